@@ -36,7 +36,13 @@ struct InvTask {
   int32_t* bad;     // set when a pivot is refused
   int32_t ncol;     // columns the sweep transforms (n; npiv when the rest columns are formed by one
                     // GEMM afterwards, see schur_split in the engine)
-  int32_t pad;
+  int32_t trail;    // 1: only the trailing block is formed (S; LU form, panel.cuh), 0: the full sweep
+  // Scratch of the panel kernels of panel.cuh: the scaled pivot rows of a panel (kb x kb) and its row
+  // permutation; FP64 matrices: the update's operands and their exponents (ozaki.cuh).
+  void* prows;
+  int32_t* perm;
+  unsigned char *oa, *ob;
+  int32_t *ea, *eb;
 };
 
 constexpr int GJ_KB = 32;
@@ -455,7 +461,8 @@ __global__ void __launch_bounds__(TCU_THREADS, 2) tc_update_kernel(const InvTask
 }
 // Undo the row interchanges as column interchanges (last first), as cycles of the resulting column
 // permutation: every thread moves its own rows, no barrier per interchange. Shared memory: cperm,
-// the cycle list and a visited mark (3 x npiv ints). Reports refused pivots.
+// the cycle list and a visited mark (3 x npiv ints). Reports refused pivots. grid (matrices, row
+// chunks): every CTA finds the cycles for itself.
 __host__ __device__ inline int64_t finish_bytes(int npiv) { return 3 * (int64_t)npiv * 4 + 16; }
 
 template <typename T>
@@ -465,12 +472,13 @@ __global__ void __launch_bounds__(256) inv_finish_kernel(const InvTask* __restri
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const InvTask t = tasks[blockIdx.x];
   if (*t.bad) {
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && blockIdx.y == 0) {
       if (t.front < 0) status[t.job] = ST_SINGULAR;
       else jobs[t.job].fail[t.front] = 1;
     }
     return;
   }
+  if ((int)(blockIdx.y * blockDim.x) >= t.n) return;
   const int np = t.npiv;
   int* cperm = reinterpret_cast<int*>(smem_raw);
   int* cyc = cperm + np;
@@ -500,7 +508,7 @@ __global__ void __launch_bounds__(256) inv_finish_kernel(const InvTask* __restri
   __syncthreads();
   V* A = static_cast<V*>(t.a);
   const int len = ncyc;
-  for (int i = threadIdx.x; i < t.n; i += blockDim.x) {
+  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < t.n; i += gridDim.y * blockDim.x) {
     int q = 0;
     while (q < len) {
       // Cycle c_0 .. c_L-1 with cperm[c_a] = c_a+1: column c_a takes column c_a+1, the last c_0.

@@ -29,6 +29,7 @@
 #include "sweep.cuh"
 #include "disorder.cuh"
 #include "leadsig.cuh"
+#include "panel.cuh"
 #include "tcgemm.cuh"
 
 using namespace caroli;
@@ -78,7 +79,14 @@ struct DevPlan {
   Entry* entries = nullptr;
   int32_t* vidx = nullptr;
   SweepRow* srows = nullptr;
+  size_t oz_bytes = 0;  // FP64 update operands: of its largest level, or of the root
   void upload(cudaStream_t s) {
+    std::vector<size_t> per(std::max(1, host.levels), 0);
+    for (size_t k = 0; k + 1 < host.fronts.size(); ++k) {
+      const FrontDesc& f = host.fronts[k];
+      if (f.n > SMALL_MAX_F64 && f.ne > 0) per[f.level] += oz::bytes(f.n);
+    }
+    oz_bytes = std::max(*std::max_element(per.begin(), per.end()), oz::bytes(host.fronts[host.root].n));
     fronts = dalloc<FrontDesc>(host.fronts.size());
     vidx = dalloc<int32_t>(std::max<size_t>(1, host.vidx.size()));
     if (!host.vidx.empty())
@@ -315,12 +323,14 @@ struct TaskCache {
   std::vector<Task> tasks;
   std::vector<TaskLevel> levels;
   std::vector<InvTask> inv;
-  std::vector<size_t> inv_piv_off, inv_y_off, inv_bt_off;
-  size_t inv_piv = 0, inv_y = 0, inv_bt = 0, root0 = 0, rinv0 = 0;
+  // Scratch offsets of every large front and root. The levels run one after the other, so each level's
+  // (and the roots') start again at 0; the sizes are those of the largest level.
+  std::vector<size_t> inv_piv_off, inv_y_off, inv_bt_off, inv_oz_off, inv_pp_off;
+  size_t inv_piv = 0, inv_y = 0, inv_bt = 0, inv_oz = 0, inv_pp = 0, root0 = 0, rinv0 = 0;
   int max_root = 0;
   double root_flops = 0.0, trace_flops = 0.0;
   const void *piv = nullptr, *y = nullptr, *bt = nullptr, *scale = nullptr, *bad = nullptr, *dinv = nullptr,
-             *dtasks = nullptr;
+             *dtasks = nullptr, *oz = nullptr, *pp = nullptr;
 };
 
 // The autotuner's choice for a plan set: the largest f32 front factored by one CTA in shared
@@ -369,7 +379,8 @@ struct caroli_ctx {
   std::vector<std::unique_ptr<System>> systems;
   Buf arena, root_arena, jobs, tasks, fail, status, tout, part, pert;
   RefineBufs rb[2];  // forward and adjoint refinement state
-  Buf inv, ipiv, iy, ibt, iscale, ibad;
+  Buf inv, ipiv, iy, ibt, iscale, ibad, ioz, ipp;
+  int max_cluster = 8;  // CTAs per cluster a panel sweep may use (16 where the GPU schedules them)
   TaskCache tcache;
   Buf grhs, gptr, gdv, gdp;
   Buf states_w;  // lead factors W_L, W_R of a scattering-states call
@@ -451,6 +462,38 @@ size_t panel_smem(int pmax, size_t vbytes) {
   const int64_t staged = panel_staged_bytes(pmax, (int)vbytes), work = panel_work_bytes(pmax, (int)vbytes);
   if (staged <= SMEM_LIMIT) return (size_t)staged;
   return work <= SMEM_LIMIT ? (size_t)work : 0;
+}
+
+// Scratch of one matrix's panel sweeps: the scaled pivot rows of a panel, its row permutation.
+constexpr size_t PANEL_PROWS = (size_t)GJ_KB * GJ_KB * sizeof(double2);
+constexpr size_t PANEL_SCRATCH = (PANEL_PROWS + PS_PERM * 4 + 255) / 256 * 256;
+constexpr int SM_COUNT = 152;
+
+// One panel of `count` matrices with at most m candidate rows, over clusters: as many CTAs per matrix
+// as leave the GPU about one CTA per SM (a panel is bound by the FP64 pipe of the SMs it runs on), at
+// least 16 candidate rows each, and enough for their rows to fit in shared memory.
+template <typename T>
+void launch_panel_sweep(caroli_ctx* ctx, const InvTask* tasks, size_t count, int k0, int m, double tol, int perturb,
+                        const JobDesc* jobs) {
+  using V = typename Cx<T>::V;
+  int c = 1;
+  while (c < ctx->max_cluster && count * (size_t)(2 * c) <= (size_t)SM_COUNT && 16 * c < m) c *= 2;
+  while (c < ctx->max_cluster && panel_sweep_bytes(panel_rows(m, c), c, sizeof(V)) > (size_t)SMEM_LIMIT) c *= 2;
+  const int r = panel_rows(m, c);
+  const size_t sm = panel_sweep_bytes(r, c, sizeof(V));
+  if (sm > (size_t)SMEM_LIMIT) throw CudaError{cudaErrorInvalidValue, "front too large for a panel sweep"};
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(count * c));
+  cfg.blockDim = dim3(PS_THREADS);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)c;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  CK(cudaLaunchKernelEx(&cfg, panel_sweep_kernel<T>, tasks, k0, tol, perturb, r, jobs));
 }
 
 // Launches `fn(first, count)` over a task range in pieces of at most 65535 (grid y/z limit).
@@ -1248,6 +1291,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     while (end < nj) {
       const FrontPlan& P = specs[end].plan->host;
       size_t b = (size_t)P.arena_elems * vb + (size_t)P.fronts[P.root].n * P.fronts[P.root].n * vr;
+      if (vr == sizeof(double2)) b += vb == sizeof(double2) ? specs[end].plan->oz_bytes : oz::bytes(P.fronts[P.root].n);
       if (mixed) {
         const SigmaSlot& sg = specs[end].sys->slots[specs[end].slot];
         const size_t c = states ? (size_t)(states->cl[end] + states->cr[end]) : (size_t)sg.channels[specs[end].block];
@@ -1329,6 +1373,25 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     std::vector<size_t>& inv_bt_off = tc.inv_bt_off;
     std::vector<size_t>& inv_piv_off = tc.inv_piv_off;
     std::vector<size_t>& inv_y_off = tc.inv_y_off;
+    size_t y_at = 0, bt_at = 0, oz_at = 0, pp_at = 0;  // the level's scratch so far
+    auto scratch_of = [&](int n, size_t v) {  // a matrix of n rows of v-byte elements
+      inv_y_off.push_back(v == sizeof(double2) ? SIZE_MAX : y_at);
+      inv_bt_off.push_back(v == sizeof(float2) ? bt_at : SIZE_MAX);
+      tc.inv_oz_off.push_back(v == sizeof(double2) ? oz_at : SIZE_MAX);
+      tc.inv_pp_off.push_back(v == sizeof(double2) ? pp_at : SIZE_MAX);
+      if (v == sizeof(float2)) {
+        y_at += (size_t)GJ_KB * n * v;
+        bt_at += tc_operand_bytes(n);
+      } else {
+        oz_at += (oz::bytes(n) + 1023) / 1024 * 1024;
+        pp_at += PANEL_SCRATCH;
+      }
+      tc.inv_y = std::max(tc.inv_y, y_at);
+      tc.inv_bt = std::max(tc.inv_bt, bt_at);
+      tc.inv_oz = std::max(tc.inv_oz, oz_at);
+      tc.inv_pp = std::max(tc.inv_pp, pp_at);
+    };
+    auto scratch_reset = [&]() { y_at = bt_at = oz_at = pp_at = 0; };
     size_t& root0 = tc.root0;
     size_t& rinv0 = tc.rinv0;
     int& max_root = tc.max_root;
@@ -1341,13 +1404,16 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     tasks.clear();
     levels.assign(max_levels, Level{});
     inv.clear();
-    inv_piv = inv_y = inv_bt = 0;
+    inv_piv = inv_y = inv_bt = tc.inv_oz = tc.inv_pp = 0;
     inv_bt_off.clear();
     inv_piv_off.clear();
     inv_y_off.clear();
+    tc.inv_oz_off.clear();
+    tc.inv_pp_off.clear();
     for (int L = 0; L < max_levels; ++L) {
       Level& lv = levels[L];
       lv = Level{};
+      scratch_reset();
       lv.tiny0 = tasks.size();
       for (size_t j = 0; j < cj; ++j) {
         const auto& fr = specs[begin + j].plan->host.fronts;
@@ -1415,9 +1481,12 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
             const double ncol = split ? ne : (double)fr[k].n;  // columns the sweep transforms
             for (int k0 = 0; k0 < fr[k].ne; k0 += GJ_KB) {
               const double kb = std::min(GJ_KB, fr[k].ne - k0), nn = fr[k].n;
-              lv.upd_flops += 8.0 * nn * (ncol - kb) * kb;  // complex n x kb times kb x (ncol - kb)
-              lv.upd_bytes += 2.0 * nn * (ncol - kb) * vb;  // the rest columns read and written
-              lv.pan_flops += 8.0 * nn * kb * kb;
+              // complex rows x kb times kb x columns, the updated block read and written: every row and the
+              // rest columns, or (FP64 fronts, trail form) the rows and columns after the panel.
+              const double ur = vb == sizeof(double2) ? nn - k0 - kb : nn, uc = vb == sizeof(double2) ? ur : ncol - kb;
+              lv.upd_flops += 8.0 * ur * uc * kb;
+              lv.upd_bytes += 2.0 * ur * uc * vb;
+              lv.pan_flops += 8.0 * (vb == sizeof(double2) ? nn - k0 : nn) * kb * kb;
             }
             if (split) {
               lv.upd_flops += 8.0 * fr[k].n * ne * nb;                           // [X; S] = [F11^-1; W] F12
@@ -1455,12 +1524,10 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
                 lv.sg_max_cols = std::max(lv.sg_max_cols, fnb);
                 lv.sg_flops += 8.0 * fr[k].n * (double)fne * fnb;
               }
+              it.trail = vb == sizeof(double2) ? 1 : 0;
               inv_piv_off.push_back(inv_piv);
-              inv_y_off.push_back(inv_y);
-              inv_bt_off.push_back(vb == sizeof(float2) ? inv_bt : SIZE_MAX);
               inv_piv += fr[k].ne;
-              inv_y += (size_t)GJ_KB * fr[k].n * vb;
-              if (vb == sizeof(float2)) inv_bt += tc_operand_bytes(fr[k].n);
+              scratch_of(fr[k].n, vb);
               inv.push_back(it);
             }
           }
@@ -1490,11 +1557,9 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       it.job = (int32_t)j;
       it.front = -1;
       inv_piv_off.push_back(inv_piv);
-      inv_y_off.push_back(inv_y);
-      inv_bt_off.push_back(vr == sizeof(float2) ? inv_bt : SIZE_MAX);
       inv_piv += m;
-      inv_y += (size_t)GJ_KB * m * vr;
-      if (vr == sizeof(float2)) inv_bt += tc_operand_bytes(m);
+      if (j == 0) scratch_reset();
+      scratch_of(m, vr);
       inv.push_back(it);
     }
     }  // !hit
@@ -1502,6 +1567,8 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     int32_t* dpiv = static_cast<int32_t*>(ctx->ipiv.get(std::max<size_t>(inv_piv, 1) * sizeof(int32_t)));
     unsigned char* dy = static_cast<unsigned char*>(ctx->iy.get(std::max<size_t>(inv_y, 16)));
     unsigned char* dbt = static_cast<unsigned char*>(ctx->ibt.get(std::max<size_t>(inv_bt, 16)));
+    unsigned char* doz = static_cast<unsigned char*>(ctx->ioz.fit(std::max<size_t>(tc.inv_oz, 16)));
+    unsigned char* dpp = static_cast<unsigned char*>(ctx->ipp.get(std::max<size_t>(tc.inv_pp, 16)));
     double* dscale = static_cast<double*>(ctx->iscale.get(std::max<size_t>(inv.size(), 1) * sizeof(double)));
     int32_t* dbad = static_cast<int32_t*>(ctx->ibad.get(std::max<size_t>(inv.size(), 1) * sizeof(int32_t)));
     InvTask* dinv = static_cast<InvTask*>(ctx->inv.get(std::max<size_t>(inv.size(), 1) * sizeof(InvTask)));
@@ -1511,14 +1578,23 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     TGTask* dsgt = static_cast<TGTask*>(ctx->sgt_list.get(std::max<size_t>(tc.sgt.size(), 1) * sizeof(TGTask)));
     const bool same_scratch = hit && tc.piv == dpiv && tc.y == dy && tc.bt == dbt && tc.scale == dscale &&
                               tc.bad == dbad && tc.dinv == dinv && tc.dtasks == dtasks && tc.f12_stage == f12_stage &&
-                              tc.f12_dev == df12 && tc.sgt_dev == dsgt && tc.status_dev == status;
+                              tc.f12_dev == df12 && tc.sgt_dev == dsgt && tc.status_dev == status && tc.oz == doz &&
+                              tc.pp == dpp;
     if (!same_scratch) {
       for (size_t q = 0; q < inv.size(); ++q) {
         inv[q].piv = dpiv + inv_piv_off[q];
-        inv[q].y = dy + inv_y_off[q];
+        inv[q].y = inv_y_off[q] == SIZE_MAX ? nullptr : dy + inv_y_off[q];
         inv[q].bt = inv_bt_off[q] == SIZE_MAX ? nullptr : dbt + inv_bt_off[q];
         inv[q].scale2 = dscale + q;
         inv[q].bad = dbad + q;
+        if (tc.inv_oz_off[q] != SIZE_MAX) {
+          inv[q].prows = dpp + tc.inv_pp_off[q];
+          inv[q].perm = reinterpret_cast<int32_t*>(dpp + tc.inv_pp_off[q] + PANEL_PROWS);
+          inv[q].oa = doz + tc.inv_oz_off[q];
+          inv[q].ob = inv[q].oa + oz::a_bytes(inv[q].n);
+          inv[q].ea = reinterpret_cast<int32_t*>(inv[q].ob + oz::b_bytes(inv[q].n));
+          inv[q].eb = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(inv[q].ea) + oz::e_bytes(inv[q].n));
+        }
       }
       if (!inv.empty())
         CK(cudaMemcpyAsync(dinv, inv.data(), inv.size() * sizeof(InvTask), cudaMemcpyHostToDevice, s));
@@ -1536,6 +1612,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       if (!tc.sgt.empty())
         CK(cudaMemcpyAsync(dsgt, tc.sgt.data(), tc.sgt.size() * sizeof(TGTask), cudaMemcpyHostToDevice, s));
       tc.piv = dpiv; tc.y = dy; tc.bt = dbt; tc.scale = dscale; tc.bad = dbad; tc.dinv = dinv; tc.dtasks = dtasks;
+      tc.oz = doz; tc.pp = dpp;
       tc.f12_stage = f12_stage; tc.f12_dev = df12; tc.sgt_dev = dsgt; tc.status_dev = status;
     }
     tc.plans = key_plans;
@@ -1549,7 +1626,41 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     tc.split = split;
     tc.valid = true;
 
-    // Batched blocked inverse of `count` matrices starting at dinv + first, largest n.
+    // FP64 sweeps: panels over clusters, updates from exact digit products on the tensor cores
+    // (panel.cuh, ozaki.cuh).
+    auto sweep_f64 = [&](size_t first, size_t count, int nmax, int pmax, double tol, bool trail, KClass cls, double flops,
+                         KClass ucls, double uflops, double ubytes) {
+      const size_t smf = (size_t)finish_bytes(pmax);
+      if (smf > (size_t)SMEM_LIMIT) throw CudaError{cudaErrorInvalidValue, "front too large for a panel sweep"};
+      const int panels = (pmax + GJ_KB - 1) / GJ_KB;
+      CK(cudaMemsetAsync(dscale + first, 0, count * sizeof(double), s));
+      CK(cudaMemsetAsync(dbad + first, 0, count * sizeof(int32_t), s));
+      if (tol > 0.0) {
+        // A few column chunks per matrix while the matrices alone do not fill the GPU.
+        const unsigned ch = (unsigned)std::max<size_t>(1, std::min<size_t>((pmax + 7) / 8, 608 / count));
+        launch(cls, 0.0, 0.0, [&] { panel_scale_kernel<double><<<dim3((unsigned)count, ch), 256, 0, s>>>(dinv + first); });
+      }
+      for (int k0 = 0; k0 < pmax; k0 += GJ_KB) {
+        launch(cls, flops / panels, 0.0, [&] { launch_panel_sweep<double>(ctx, dinv + first, count, k0, pmax - k0, tol, 0, djobs); });
+        const int rows = trail ? nmax - k0 : nmax;  // rows and columns of the update, at most
+        const unsigned rp = (unsigned)((rows + PR_ROWS - 1) / PR_ROWS), cp = (unsigned)((rows + PR_COLS - 1) / PR_COLS);
+        launch(cls, 0.0, 0.0, [&] {
+          panel_rest_kernel<double><<<dim3((unsigned)count, rp + cp), PR_THREADS, 0, s>>>(dinv + first, k0, (int)rp);
+        });
+        const size_t rt = (size_t)(rows + oz::ROWS - 1) / oz::ROWS, ct = (size_t)(rows + oz::COLS - 1) / oz::COLS;
+        // Column tiles per CTA: A' is copied once per CTA, so as many as still leave two CTAs per SM.
+        const size_t group = std::max<size_t>(1, std::min(ct, rt * ct * count / (2 * SM_COUNT)));
+        in_pieces(count, [&](size_t f0, size_t c) {
+          launch(ucls, uflops / panels * c / count, ubytes / panels * c / count, [&] {
+            oz::update_kernel<<<dim3((unsigned)rt, (unsigned)c, (unsigned)((ct + group - 1) / group)), oz::THREADS, oz::SMEM,
+                                s>>>(dinv + first + f0, k0, (int)group, status);
+          });
+        });
+      }
+      if (trail) return;  // refused pivots are reported by the sweeps
+      const unsigned ch = (unsigned)std::max<size_t>(1, std::min<size_t>((nmax + 255) / 256, 2 * SM_COUNT / count));
+      launch(cls, 0.0, 0.0, [&] { inv_finish_kernel<double><<<dim3((unsigned)count, ch), 256, smf, s>>>(dinv + first, djobs, status); });
+    };
     // Batched blocked sweep of `count` fronts starting at dinv + first: largest size nmax, largest
     // pivot count pmax.
     // Work attribution (kernel-class accounting): the panel sweeps to `cls` with `flops`, the
@@ -1559,6 +1670,10 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       using TT = decltype(tag);
       using VV = typename Cx<TT>::V;
       if (!count || nmax <= 0 || pmax <= 0) return;
+      if constexpr (std::is_same<TT, double>::value) {
+        sweep_f64(first, count, nmax, pmax, tol, cls == K_PANEL, cls, flops, ucls, uflops, ubytes);
+        return;
+      }
       const size_t sm = panel_smem(pmax, sizeof(VV));
       const size_t smf = (size_t)finish_bytes(pmax);
       if (!sm || smf > (size_t)SMEM_LIMIT) throw CudaError{cudaErrorInvalidValue, "front too large for a panel sweep"};
@@ -2184,7 +2299,8 @@ int caroli_ctx_create(int device_ordinal, caroli_ctx** out) {
     ctx->mem_budget = free_b / 2;
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_ordinal));
-    for (auto* k : {(const void*)tc_update_kernel, (const void*)tc_sweep_gemm_kernel,
+    for (auto* k : {(const void*)tc_update_kernel, (const void*)tc_sweep_gemm_kernel, (const void*)oz::update_kernel,
+                    (const void*)panel_sweep_kernel<double>,
                     (const void*)small_front_kernel<double, false>, (const void*)small_front_kernel<float, false>,
                     (const void*)small_front_kernel<double, true>, (const void*)small_front_kernel<float, true>,
                     (const void*)small_front_wide_kernel<double, false>, (const void*)small_front_wide_kernel<float, false>,
@@ -2204,6 +2320,24 @@ int caroli_ctx_create(int device_ordinal, caroli_ctx** out) {
       CK(cudaFuncGetAttributes(&fa, k));
       const int room = std::min<int>(SMEM_LIMIT, optin - (int)fa.sharedSizeBytes);
       CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+    }
+    CK(cudaFuncSetAttribute((const void*)panel_sweep_kernel<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    {
+      // Clusters of 16 need 16 SMs of one GPU processing cluster free at once: used where a full-size one fits.
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(16);
+      cfg.blockDim = dim3(PS_THREADS);
+      cfg.dynamicSmemBytes = SMEM_LIMIT;
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = 16;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, panel_sweep_kernel<double>, &cfg) == cudaSuccess && clusters > 0)
+        ctx->max_cluster = 16;
+      (void)cudaGetLastError();
     }
     // The allocation-free entry point's static scratch: its device address on this device, once,
     // so that caroli_solve_batch_noalloc itself only launches kernels and copies.

@@ -1,0 +1,334 @@
+// FP64 rank-32 updates on the tcgen05 tensor cores: the products of inv_update_kernel<double> from
+// exact integer products of operand digits (the Ozaki scheme, K. Ozaki, T. Ogita, S. Oishi, S. M. Rump,
+// "Error-free transformations of matrix multiplication by using fast routines of matrix
+// multiplication and its applications", Numer. Algorithms 59, 2012; with f16 inputs and f32
+// accumulation as D. Mukunoki, K. Ozaki, T. Ogita, T. Imamura, ISC High Performance 2020).
+//
+// GB300's FP64 pipe does about two multiply-adds per clock and SM; the f16 tensor cores do 4 096. A
+// row of the left factor (32 complex entries, K = 64 real) is scaled by the power of two above its
+// largest component and written as seven signed base-512 digits (62 bits, so an entry keeps 53 bits
+// down to 2^-9 of the row's largest); a column of the right factor likewise. Digits are at most 256 in
+// modulus, exact in f16; a product of digits is at most 2^16 and a sum of 64 of them 2^22, so the
+// f32 accumulators hold exact integers while fewer than five digit pairs share one (levels i + j <= 3)
+// and, past that, unless nearly every digit has its largest value: then a rounding of 2^-24 of a level
+// that itself weighs 2^-36 or less. Levels i + j <= 6 are kept (28 pairs); what is left out weighs
+// 2^-63 of (row's largest) x (column's largest) per term. The levels are put together in 64-bit
+// integers and rounded once to FP64 (integer arithmetic: the FP64 pipe only does the final add).
+//
+// A 128 x 32 complex tile takes 28 x 4 MMAs (29 Mflop on the f16 cores) in place of 1.05 Mflop on the FP64
+// pipe (159 us on one SM). Measured: the updates of two 48 x 24 x 24 cubic wires' fronts 121 -> 12.8 ms
+// (a factor 1.4 of it from the trailing form), of 16 BHZ 200 x 64 solves 58.8 -> 6.9 ms; T
+// against 64 bits equal to the FP64 pipe's within its scatter (1e-15 to 5e-12 on these devices).
+//
+// The complex product is a real GEMM D = A' B'^T with the row's 32 complex entries as K = 64 and
+// two columns of D per complex column:
+//     A'[i][2c] = Re P[i, c], A'[i][2c+1] = Im P[i, c]
+//     B'[2j][2c] = Re Y[c, j], B'[2j][2c+1] = -Im Y[c, j], B'[2j+1][2c] = Im Y, B'[2j+1][2c+1] = Re Y
+// so a lane of tensor memory is a complex row and 32 lanes read and write 512 consecutive bytes of a
+// column of the matrix.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "dense.cuh"
+
+namespace caroli {
+namespace oz {
+
+constexpr int S = 7;                             // digits per operand
+constexpr int ROWS = 128;                        // complex rows per tile (the MMA's M)
+constexpr int COLS = 32;                         // complex columns per tile (N = 64)
+constexpr int A_SLICE = ROWS * 2 * GJ_KB * 2;    // bytes of one digit of A': 128 x 64 f16
+constexpr int B_SLICE = 2 * COLS * 2 * GJ_KB * 2;
+constexpr int A_TILE = S * A_SLICE, B_TILE = S * B_SLICE;
+constexpr int SMEM = A_TILE + B_TILE + 1024;
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 32 * (2 + EPI_WARPS);
+constexpr int NOT_FINITE = 1 << 20;              // exponent of a row or column holding Inf or NaN
+
+// Operand bytes of a matrix of n rows and columns: A' and B' tiles, row and column exponents.
+__host__ __device__ inline size_t a_bytes(int n) { return (size_t)((n + ROWS - 1) / ROWS) * A_TILE; }
+__host__ __device__ inline size_t b_bytes(int n) { return (size_t)((n + COLS - 1) / COLS) * B_TILE; }
+__host__ __device__ inline size_t e_bytes(int n) { return ((size_t)n * 4 + 255) / 256 * 256; }
+__host__ __device__ inline size_t bytes(int n) { return a_bytes(n) + b_bytes(n) + 2 * e_bytes(n); }
+
+// Byte offset of element (row, k) of an f16 operand: K-slices of 16 elements (one kind::f16 MMA) in the
+// core-matrix layout of tc.cuh (8 rows x 16 bytes; leading offset 128, stride offset 256).
+__device__ __forceinline__ uint32_t offset(int row, int k, int rows) {
+  return (uint32_t)((k >> 4) * rows * 32 + (row >> 3) * 256 + ((k >> 3) & 1) * 128 + (row & 7) * 16 + (k & 7) * 2);
+}
+
+__device__ __forceinline__ int biased_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// x as a 62-bit fixed-point number: x 2^(1084 - e), e the biased exponent of the largest entry.
+__device__ __forceinline__ long long fixed(double x, int e) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+  int ex = (int)(bits >> 52) & 0x7ff;
+  unsigned long long m = bits & 0xfffffffffffffull;
+  if (ex) m |= 1ull << 52;
+  else ex = 1;
+  const int sh = 9 + ex - e;  // at most 9
+  long long v = sh >= 0 ? (long long)(m << sh) : (sh > -64 ? (long long)(m >> -sh) : 0ll);
+  return (long long)bits < 0 ? -v : v;
+}
+// The signed base-512 digits of v (most significant first), each in [-256, 256].
+__device__ __forceinline__ void digits(long long v, int (&d)[S]) {
+#pragma unroll
+  for (int s = S - 1; s > 0; --s) {
+    const int low = ((int)v & 511 ^ 256) - 256;
+    d[s] = low;
+    v = (v - low) >> 9;
+  }
+  d[0] = (int)v;
+}
+// Two digits as a pair of f16: 1536 + d is 0x6600 + d in f16's binade [1024, 2048).
+__device__ __forceinline__ uint32_t pack(int lo, int hi) {
+  const uint32_t b = (uint32_t)(0x6600 + lo) | ((uint32_t)(0x6600 + hi) << 16);
+  const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&b), __half2half2(__ushort_as_half(0x6600)));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// Row q of A' from eight of its entries per lane (lane h of four: entries 8h .. 8h + 7, i.e. K-slice h).
+__device__ __forceinline__ void write_a(unsigned char* oa, int32_t* ea, int q, int h, bool act, const double2 (&a)[8]) {
+  int e = 1;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) e = max(e, max(biased_exponent(a[c].x), biased_exponent(a[c].y)));
+  e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
+  e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
+  if (!act) return;
+  if (h == 0) ea[q] = e == 0x7ff ? NOT_FINITE : e;
+  unsigned char* tile = oa + (size_t)(q / ROWS) * A_TILE;
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {  // eight f16 (four complex entries): one 16-byte core-matrix row
+    uint32_t w[S][4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      int re[S], im[S];
+      digits(fixed(a[4 * g + c].x, e), re);
+      digits(fixed(a[4 * g + c].y, e), im);
+#pragma unroll
+      for (int s = 0; s < S; ++s) w[s][c] = pack(re[s], im[s]);
+    }
+    const uint32_t off = offset(q % ROWS, 16 * h + 8 * g, ROWS);
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+      *reinterpret_cast<uint4*>(tile + s * A_SLICE + off) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+  }
+}
+
+// Column r of B' (rows 2r and 2r + 1), lane c holding entry c of the column.
+__device__ __forceinline__ void write_b(unsigned char* ob, int32_t* eb, int r, int lane, double2 y) {
+  const int e = __reduce_max_sync(0xffffffffu, max(1, max(biased_exponent(y.x), biased_exponent(y.y))));
+  if (lane == 0) eb[r] = e == 0x7ff ? NOT_FINITE : e;
+  int re[S], im[S];
+  digits(fixed(y.x, e), re);
+  digits(fixed(y.y, e), im);
+  unsigned char* tile = ob + (size_t)(r / COLS) * B_TILE;
+  const int row = 2 * (r % COLS);
+  const uint32_t o0 = offset(row, 2 * lane, 2 * COLS), o1 = offset(row + 1, 2 * lane, 2 * COLS);
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    *reinterpret_cast<uint32_t*>(tile + s * B_SLICE + o0) = pack(re[s], -im[s]);
+    *reinterpret_cast<uint32_t*>(tile + s * B_SLICE + o1) = pack(im[s], re[s]);
+  }
+}
+
+// The seven level sums of one output as FP64: 2^(e - 2114) Σ_l a_l 512^(6 - l), rounded once. e: sum of
+// the row's and the column's biased exponents.
+__device__ __forceinline__ double combine(const float (&a)[S], int e) {
+  int v[S];
+#pragma unroll
+  for (int l = 0; l < S; ++l) v[l] = __float2int_rn(a[l]);
+  const long long hi = ((long long)v[0] << 18) + ((long long)v[1] << 9) + v[2];
+  const long long lo = ((long long)v[3] << 27) + ((long long)v[4] << 18) + ((long long)v[5] << 9) + v[6];
+  const long long w = (hi << 22) + (lo >> 14);  // unit 2^(e - 2100)
+  if (e >= NOT_FINITE) return __longlong_as_double(0x7ff8000000000000ll);
+  if (w == 0) return 0.0;
+  const unsigned long long u = w < 0 ? (unsigned long long)(-w) : (unsigned long long)w;
+  const int lz = __clzll((long long)u);
+  const unsigned long long norm = u << lz;
+  // 53 bits rounded to nearest (ties up); the carry of the rounding moves the exponent.
+  const unsigned long long mant = (norm >> 11) + ((norm >> 10) & 1ull);
+  const int ex = 1023 + 63 - lz + e - 2100;
+  unsigned long long bits;
+  if (ex <= 0) bits = 0ull;
+  else if (ex >= 2046) bits = 0x7ff0000000000000ull;
+  else bits = ((unsigned long long)(ex - 1) << 52) + mant;
+  return __longlong_as_double((long long)(bits | (w < 0 ? 1ull << 63 : 0ull)));
+}
+
+__host__ __device__ constexpr uint32_t idesc_f16(int m, int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);  // D: f32; A, B: f16, K-major
+}
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate) {
+  const uint32_t acc = accumulate ? 1u : 0u;
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The update of one panel (operands written by panel_rest_kernel). A CTA takes 128 rows of a matrix and
+// `group` tiles of 32 columns: warp 0 (one thread) bulk-copies A' once and each B' tile, warp 1 (one
+// thread) issues 28 x 4 MMAs of 128 x 64 x 16 per tile into seven 64-column accumulators, warps 2-9 add
+// the tile to the old values (zero on the pivot rows of the full form). Waits are bounded as in
+// tc_update_kernel. grid (row tiles, matrices, column groups).
+__global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __restrict__ tasks, int k0, int group,
+                                                            int32_t* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint32_t tslot;
+  __shared__ __align__(8) uint64_t afull, bfull, bempty, tfull, tempty;
+  __shared__ int abort_flag;
+  const InvTask t = tasks[blockIdx.y];
+  const int n = t.n;
+  if (k0 >= t.npiv || *t.bad) return;
+  const int kb = min(GJ_KB, t.npiv - k0);
+  const bool trail = t.trail != 0;
+  const int base = trail ? k0 + kb : 0;
+  const int rows = n - base, rest = trail ? rows : n - kb;
+  const int i0 = blockIdx.x * ROWS;
+  const int tile0 = blockIdx.z * group;
+  const int tiles = min((rest + COLS - 1) / COLS - tile0, group);
+  if (i0 >= rows || tiles <= 0) return;
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  unsigned char* sa = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sb = sa + A_TILE;
+  if (w == 0) tc::tmem_alloc(&tslot, 512);
+  if (tid == 0) {
+    tc::mbar_init(&afull, 1);
+    tc::mbar_init(&bfull, 1);
+    tc::mbar_init(&bempty, 1);
+    tc::mbar_init(&tfull, 1);
+    tc::mbar_init(&tempty, EPI_WARPS);
+    abort_flag = 0;
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tbase = tslot;
+  volatile int* abort_v = &abort_flag;
+  auto fail = [&]() {
+    *abort_v = 1;
+    status[t.job] = ST_TIMEOUT;
+  };
+  int copies = 0, mma_tiles = 0;
+  if (w == 0) {
+    if (lane == 0) {
+      tc::mbar_arrive_expect_tx(&afull, A_TILE);
+      for (int s = 0; s < S; ++s)
+        tc::bulk_copy_g2s(sa + s * A_SLICE, t.oa + (size_t)blockIdx.x * A_TILE + s * A_SLICE, A_SLICE, &afull);
+      for (int ct = 0; ct < tiles && !*abort_v; ++ct) {
+        if (ct >= 1 && !tc::mbar_wait(&bempty, (uint32_t)((ct - 1) & 1), TCU_WAIT)) { fail(); break; }
+        tc::mbar_arrive_expect_tx(&bfull, B_TILE);
+        tc::bulk_copy_g2s(sb, t.ob + (size_t)(tile0 + ct) * B_TILE, B_TILE, &bfull);
+        ++copies;
+      }
+    }
+  } else if (w == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = idesc_f16(ROWS, 2 * COLS);
+      if (!tc::mbar_wait(&afull, 0, TCU_WAIT)) fail();
+      for (int ct = 0; ct < tiles && !*abort_v; ++ct) {
+        if (!tc::mbar_wait(&bfull, (uint32_t)(ct & 1), TCU_WAIT)) { fail(); break; }
+        if (ct >= 1 && !tc::mbar_wait(&tempty, (uint32_t)((ct - 1) & 1), TCU_WAIT)) { fail(); break; }
+        tc::fence_after_sync();
+        for (int l = 0; l < S; ++l)
+          for (int i = 0; i <= l; ++i) {
+            const uint32_t pa = tc::smem_addr(sa + i * A_SLICE), pb = tc::smem_addr(sb + (l - i) * B_SLICE);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+              mma_f16(tbase + (uint32_t)(l * 2 * COLS), tc::smem_desc(pa + ks * ROWS * 32, 128, 256),
+                      tc::smem_desc(pb + ks * 2 * COLS * 32, 128, 256), idesc, i > 0 || ks > 0);
+          }
+        tc::mma_commit(&bempty);
+        tc::mma_commit(&tfull);
+        ++mma_tiles;
+      }
+    }
+  } else {
+    // Warp's lane quarter of tensor memory (rows) and half of the tile's columns; four complex
+    // columns at a time, their old values requested one step ahead.
+    const int q = w & 3, half = (w - 2) >> 2;
+    const int r = i0 + 32 * q + lane, gi = base + r;
+    const bool row_in = r < rows;
+    const bool keep_old = row_in && (trail || gi < k0 || gi >= k0 + kb);
+    const int er = row_in ? t.ea[r] : 1;
+    double2* Ai = static_cast<double2*>(t.a) + gi;
+    const int64_t ld = t.ld;
+    constexpr int CW = COLS / 2;  // complex columns per warp and tile
+    auto col_of = [&](int c) { return trail ? base + c : (c < k0 ? c : c + kb); };
+    for (int ct = 0; ct < tiles; ++ct) {
+      const int c0 = (tile0 + ct) * COLS + half * CW;
+      double2 old[4];
+      auto fetch = [&](int c) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          old[j] = (keep_old && c + j < rest) ? Ai[(int64_t)col_of(c + j) * ld] : make_double2(0.0, 0.0);
+      };
+      fetch(c0);
+      bool ok = !*abort_v && tc::mbar_wait(&tfull, (uint32_t)(ct & 1), TCU_WAIT);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (lane == 0) fail();
+        break;
+      }
+      tc::fence_after_sync();
+#pragma unroll
+      for (int g = 0; g < CW / 4; ++g) {
+        float v[S][8];
+#pragma unroll
+        for (int l = 0; l < S; ++l)
+          tmem_ld8(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(l * 2 * COLS + half * 2 * CW + 8 * g), v[l]);
+        tc::tmem_ld_wait();
+        if (g == CW / 4 - 1) {
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&tempty);
+        }
+        double2 now[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) now[j] = old[j];
+        if (g + 1 < CW / 4) fetch(c0 + 4 * (g + 1));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int c = c0 + 4 * g + j;
+          if (c >= rest) continue;
+          const int e = er + t.eb[c];
+          float x[S], y[S];
+#pragma unroll
+          for (int l = 0; l < S; ++l) {
+            x[l] = v[l][2 * j];
+            y[l] = v[l][2 * j + 1];
+          }
+          // trail: old - L Y; full: old + (swept panel) Y.
+          const double re = combine(x, e), im = combine(y, e);
+          const double2 out = trail ? make_double2(now[j].x - re, now[j].y - im) : make_double2(now[j].x + re, now[j].y + im);
+          if (row_in) Ai[(int64_t)col_of(c) * ld] = out;
+        }
+      }
+    }
+  }
+  // Drain what this thread issued before tensor memory and shared memory go away.
+  if (*abort_v) {
+    if (w == 0 && lane == 0) {
+      tc::mbar_wait(&afull, 0, TCU_WAIT);
+      if (copies > 0) tc::mbar_wait(&bfull, (uint32_t)((copies - 1) & 1), TCU_WAIT);
+    }
+    if (w == 1 && lane == 0 && mma_tiles > 0) tc::mbar_wait(&bempty, (uint32_t)((mma_tiles - 1) & 1), TCU_WAIT);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (w == 0) tc::tmem_dealloc(tbase, 512);
+}
+
+}  // namespace oz
+}  // namespace caroli

@@ -470,14 +470,14 @@ constexpr size_t PANEL_SCRATCH = (PANEL_PROWS + PS_PERM * 4 + 255) / 256 * 256;
 constexpr int SM_COUNT = 152;
 
 // One panel of `count` matrices with at most m candidate rows, over clusters: as many CTAs per matrix
-// as leave the GPU about one CTA per SM (a panel is bound by the FP64 pipe of the SMs it runs on), at
-// least 16 candidate rows each, and enough for their rows to fit in shared memory.
+// as leave the GPU at most two CTAs per SM (a panel is bound by the FP64 pipe of the SMs it runs on), at
+// least eight candidate rows each, and enough for their rows to fit in shared memory.
 template <typename T>
 void launch_panel_sweep(caroli_ctx* ctx, const InvTask* tasks, size_t count, int k0, int m, double tol, int perturb,
-                        const JobDesc* jobs) {
+                        const JobDesc* jobs, int32_t* status) {
   using V = typename Cx<T>::V;
   int c = 1;
-  while (c < ctx->max_cluster && count * (size_t)(2 * c) <= (size_t)SM_COUNT && 16 * c < m) c *= 2;
+  while (c < ctx->max_cluster && count * (size_t)(2 * c) <= (size_t)(2 * SM_COUNT) && 8 * c < m) c *= 2;
   while (c < ctx->max_cluster && panel_sweep_bytes(panel_rows(m, c), c, sizeof(V)) > (size_t)SMEM_LIMIT) c *= 2;
   const int r = panel_rows(m, c);
   const size_t sm = panel_sweep_bytes(r, c, sizeof(V));
@@ -493,7 +493,7 @@ void launch_panel_sweep(caroli_ctx* ctx, const InvTask* tasks, size_t count, int
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  CK(cudaLaunchKernelEx(&cfg, panel_sweep_kernel<T>, tasks, k0, tol, perturb, r, jobs));
+  CK(cudaLaunchKernelEx(&cfg, panel_sweep_kernel<T>, tasks, k0, tol, perturb, r, jobs, status));
 }
 
 // Launches `fn(first, count)` over a task range in pieces of at most 65535 (grid y/z limit).
@@ -1641,15 +1641,25 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
         launch(cls, 0.0, 0.0, [&] { panel_scale_kernel<double><<<dim3((unsigned)count, ch), 256, 0, s>>>(dinv + first); });
       }
       for (int k0 = 0; k0 < pmax; k0 += GJ_KB) {
-        launch(cls, flops / panels, 0.0, [&] { launch_panel_sweep<double>(ctx, dinv + first, count, k0, pmax - k0, tol, 0, djobs); });
+        launch(cls, flops / panels, 0.0, [&] { launch_panel_sweep<double>(ctx, dinv + first, count, k0, pmax - k0, tol, 0, djobs, status); });
         const int rows = trail ? nmax - k0 : nmax;  // rows and columns of the update, at most
-        const unsigned rp = (unsigned)((rows + PR_ROWS - 1) / PR_ROWS), cp = (unsigned)((rows + PR_COLS - 1) / PR_COLS);
+        // Pieces of 16 rows and columns, or of 4 while those are fewer than two per scheduler.
+        const bool fine = (size_t)((rows + 15) / 16) * 2 * count < (size_t)(4 * SM_COUNT);
+        const unsigned rp = (unsigned)((rows + (fine ? 3 : 15)) / (fine ? 4 : 16));
         launch(cls, 0.0, 0.0, [&] {
-          panel_rest_kernel<double><<<dim3((unsigned)count, rp + cp), PR_THREADS, 0, s>>>(dinv + first, k0, (int)rp);
+          if (fine) panel_rest_kernel<double, 16><<<dim3((unsigned)count, 2 * rp), PR_THREADS, 0, s>>>(dinv + first, k0, (int)rp);
+          else panel_rest_kernel<double, 4><<<dim3((unsigned)count, 2 * rp), PR_THREADS, 0, s>>>(dinv + first, k0, (int)rp);
         });
+        // Column tiles per CTA, one CTA per SM: the fewest tile times over all waves (a CTA's start, mostly
+        // the copy of A', counted as 1.5 tiles).
         const size_t rt = (size_t)(rows + oz::ROWS - 1) / oz::ROWS, ct = (size_t)(rows + oz::COLS - 1) / oz::COLS;
-        // Column tiles per CTA: A' is copied once per CTA, so as many as still leave two CTAs per SM.
-        const size_t group = std::max<size_t>(1, std::min(ct, rt * ct * count / (2 * SM_COUNT)));
+        size_t group = ct;
+        double least = 1e300;
+        for (size_t parts = 1; parts <= std::min<size_t>(ct, 16); ++parts) {
+          const size_t g = (ct + parts - 1) / parts, ctas = rt * count * ((ct + g - 1) / g);
+          const double cost = (double)((ctas + SM_COUNT - 1) / SM_COUNT) * (g + 1.5);
+          if (cost < least) { least = cost; group = g; }
+        }
         in_pieces(count, [&](size_t f0, size_t c) {
           launch(ucls, uflops / panels * c / count, ubytes / panels * c / count, [&] {
             oz::update_kernel<<<dim3((unsigned)rt, (unsigned)c, (unsigned)((ct + group - 1) / group)), oz::THREADS, oz::SMEM,

@@ -110,6 +110,26 @@ template <typename V> __device__ __forceinline__ V cinv(V a) {
   }
   return r;
 }
+// FP64: an FP64 instruction holds a scheduler's pipe for 64 clocks here whatever its active lanes, and
+// Smith's form takes three divisions (about 2 000 clocks, on the critical path of every pivot step).
+// conj(a) / |a|^2 with one reciprocal takes a third of that and has as small an error while |a|^2 can
+// neither overflow nor lose bits to underflow.
+template <> __device__ __forceinline__ double2 cinv<double2>(double2 a) {
+  const int e = max((__double2hiint(a.x) >> 20) & 0x7ff, (__double2hiint(a.y) >> 20) & 0x7ff);
+  if (e > 1023 - 400 && e < 1023 + 400) {
+    const double r = 1.0 / fma(a.x, a.x, a.y * a.y);
+    return make_double2(a.x * r, -(a.y * r));
+  }
+  double2 r;
+  if (fabs(a.x) >= fabs(a.y)) {
+    const double q = a.y / a.x, d = a.x + a.y * q;
+    r.x = 1.0 / d; r.y = -q / d;
+  } else {
+    const double q = a.x / a.y, d = a.x * q + a.y;
+    r.x = q / d; r.y = -1.0 / d;
+  }
+  return r;
+}
 template <typename V> __device__ __forceinline__ double cabs2(V a) {
   return (double)a.x * (double)a.x + (double)a.y * (double)a.y;
 }

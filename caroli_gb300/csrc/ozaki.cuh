@@ -15,9 +15,9 @@
 // 2^-63 of (row's largest) x (column's largest) per term. The levels are put together in 64-bit
 // integers and rounded once to FP64 (integer arithmetic: the FP64 pipe only does the final add).
 //
-// A 128 x 32 complex tile takes 28 x 4 MMAs (29 Mflop on the f16 cores) in place of 1.05 Mflop on the FP64
-// pipe (159 us on one SM). Measured: the updates of two 48 x 24 x 24 cubic wires' fronts 121 -> 12.8 ms
-// (a factor 1.4 of it from the trailing form), of 16 BHZ 200 x 64 solves 58.8 -> 6.9 ms; T
+// A 128 x 16 complex tile takes 15 Mflop on the f16 cores in place of 0.52 Mflop on the FP64 pipe (80 us
+// on one SM). Measured: the updates of two 48 x 24 x 24 cubic wires' fronts 121 -> 6.9 ms
+// (a factor 1.4 of it from the trailing form), of 16 BHZ 200 x 64 solves 58.8 -> 3.9 ms; T
 // against 64 bits equal to the FP64 pipe's within its scatter (1e-15 to 5e-12 on these devices).
 //
 // The complex product is a real GEMM D = A' B'^T with the row's 32 complex entries as K = 64 and
@@ -36,12 +36,17 @@ namespace oz {
 
 constexpr int S = 7;                             // digits per operand
 constexpr int ROWS = 128;                        // complex rows per tile (the MMA's M)
-constexpr int COLS = 32;                         // complex columns per tile (N = 64)
+constexpr int COLS = 16;                         // complex columns per tile (N = 32)
 constexpr int A_SLICE = ROWS * 2 * GJ_KB * 2;    // bytes of one digit of A': 128 x 64 f16
-constexpr int B_SLICE = 2 * COLS * 2 * GJ_KB * 2;
-constexpr int A_TILE = S * A_SLICE, B_TILE = S * B_SLICE;
-constexpr int SMEM = A_TILE + B_TILE + 1024;
-constexpr int EPI_WARPS = 8;
+constexpr int A_TILE = S * A_SLICE;
+// B' of a tile stacks its digits along N (row 32 s + j: digit s of B' row j), so that one MMA multiplies
+// a digit i of A' with the digits 0 .. 6 - i of B' into the accumulators of the levels i .. 6.
+constexpr int B_ROWS = S * 2 * COLS;
+constexpr int B_TILE = B_ROWS * 2 * GJ_KB * 2;
+constexpr int STAGES = 3;                        // B' tiles in shared memory
+constexpr int SMEM = A_TILE + STAGES * B_TILE + 1024;
+constexpr int ACC = 256;                         // tensor-memory columns of one of two accumulator sets (S x 32 used)
+constexpr int EPI_WARPS = 16;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
 constexpr int NOT_FINITE = 1 << 20;              // exponent of a row or column holding Inf or NaN
 
@@ -87,48 +92,56 @@ __device__ __forceinline__ uint32_t pack(int lo, int hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// Row q of A' from eight of its entries per lane (lane h of four: entries 8h .. 8h + 7, i.e. K-slice h).
-__device__ __forceinline__ void write_a(unsigned char* oa, int32_t* ea, int q, int h, bool act, const double2 (&a)[8]) {
+// The largest exponent of the entries LPR lanes hold (at least 1).
+template <int LPR> __device__ __forceinline__ int row_exponent(const double2 (&a)[GJ_KB / LPR]) {
   int e = 1;
 #pragma unroll
-  for (int c = 0; c < 8; ++c) e = max(e, max(biased_exponent(a[c].x), biased_exponent(a[c].y)));
-  e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
-  e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
+  for (int i = 0; i < GJ_KB / LPR; ++i) e = max(e, max(biased_exponent(a[i].x), biased_exponent(a[i].y)));
+#pragma unroll
+  for (int o = 1; o < LPR; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+  return e;
+}
+
+// Row q of A' from LPR lanes, lane h holding the entries LPR i + h: four lanes' 4-byte pairs (re, im) fill
+// a 16-byte core-matrix row.
+template <int LPR>
+__device__ __forceinline__ void write_a(unsigned char* oa, int32_t* ea, int q, int h, bool act,
+                                        const double2 (&a)[GJ_KB / LPR]) {
+  const int e = row_exponent<LPR>(a);
   if (!act) return;
   if (h == 0) ea[q] = e == 0x7ff ? NOT_FINITE : e;
   unsigned char* tile = oa + (size_t)(q / ROWS) * A_TILE;
 #pragma unroll
-  for (int g = 0; g < 2; ++g) {  // eight f16 (four complex entries): one 16-byte core-matrix row
-    uint32_t w[S][4];
+  for (int i = 0; i < GJ_KB / LPR; ++i) {
+    int re[S], im[S];
+    digits(fixed(a[i].x, e), re);
+    digits(fixed(a[i].y, e), im);
+    const uint32_t off = offset(q % ROWS, 2 * (LPR * i + h), ROWS);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      int re[S], im[S];
-      digits(fixed(a[4 * g + c].x, e), re);
-      digits(fixed(a[4 * g + c].y, e), im);
-#pragma unroll
-      for (int s = 0; s < S; ++s) w[s][c] = pack(re[s], im[s]);
-    }
-    const uint32_t off = offset(q % ROWS, 16 * h + 8 * g, ROWS);
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-      *reinterpret_cast<uint4*>(tile + s * A_SLICE + off) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+    for (int s = 0; s < S; ++s) *reinterpret_cast<uint32_t*>(tile + s * A_SLICE + off) = pack(re[s], im[s]);
   }
 }
 
-// Column r of B' (rows 2r and 2r + 1), lane c holding entry c of the column.
-__device__ __forceinline__ void write_b(unsigned char* ob, int32_t* eb, int r, int lane, double2 y) {
-  const int e = __reduce_max_sync(0xffffffffu, max(1, max(biased_exponent(y.x), biased_exponent(y.y))));
-  if (lane == 0) eb[r] = e == 0x7ff ? NOT_FINITE : e;
-  int re[S], im[S];
-  digits(fixed(y.x, e), re);
-  digits(fixed(y.y, e), im);
+// Column r of B' (rows 2r and 2r + 1) from LPR lanes, laid out over the lanes as in write_a.
+template <int LPR>
+__device__ __forceinline__ void write_b(unsigned char* ob, int32_t* eb, int r, int h, bool act,
+                                        const double2 (&y)[GJ_KB / LPR]) {
+  const int e = row_exponent<LPR>(y);
+  if (!act) return;
+  if (h == 0) eb[r] = e == 0x7ff ? NOT_FINITE : e;
   unsigned char* tile = ob + (size_t)(r / COLS) * B_TILE;
   const int row = 2 * (r % COLS);
-  const uint32_t o0 = offset(row, 2 * lane, 2 * COLS), o1 = offset(row + 1, 2 * lane, 2 * COLS);
 #pragma unroll
-  for (int s = 0; s < S; ++s) {
-    *reinterpret_cast<uint32_t*>(tile + s * B_SLICE + o0) = pack(re[s], -im[s]);
-    *reinterpret_cast<uint32_t*>(tile + s * B_SLICE + o1) = pack(im[s], re[s]);
+  for (int i = 0; i < GJ_KB / LPR; ++i) {
+    int re[S], im[S];
+    digits(fixed(y[i].x, e), re);
+    digits(fixed(y[i].y, e), im);
+    const int k = 2 * (LPR * i + h);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      *reinterpret_cast<uint32_t*>(tile + offset(2 * COLS * s + row, k, B_ROWS)) = pack(re[s], -im[s]);
+      *reinterpret_cast<uint32_t*>(tile + offset(2 * COLS * s + row + 1, k, B_ROWS)) = pack(im[s], re[s]);
+    }
   }
 }
 
@@ -178,15 +191,18 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 }
 
 // The update of one panel (operands written by panel_rest_kernel). A CTA takes 128 rows of a matrix and
-// `group` tiles of 32 columns: warp 0 (one thread) bulk-copies A' once and each B' tile, warp 1 (one
-// thread) issues 28 x 4 MMAs of 128 x 64 x 16 per tile into seven 64-column accumulators, warps 2-9 add
-// the tile to the old values (zero on the pivot rows of the full form). Waits are bounded as in
-// tc_update_kernel. grid (row tiles, matrices, column groups).
+// `group` tiles of 16 columns: warp 0 (one thread) bulk-copies A' once and the B' tiles into a ring of
+// three, warp 1 (one thread) issues 7 x 4 MMAs per tile (N = 224, 192, ... 32: 1 792 clocks at the full f16
+// rate; a 128 x 32 x 16 MMA per digit pair took 53 clocks, 6 000 per tile) into one of two sets of seven
+// 32-column accumulators, warps 2-17 (four per lane quarter, four complex columns each) add the other set's
+// tile to the old values (zero on the pivot rows of the full form): their FP64 adds, the only FP64 work
+// left, keep that pipe 62 % busy, the bound. Two sets of 32-column tiles would not
+// fit in tensor memory. Waits are bounded as in tc_update_kernel. grid (row tiles, matrices, column groups).
 __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __restrict__ tasks, int k0, int group,
                                                             int32_t* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t tslot;
-  __shared__ __align__(8) uint64_t afull, bfull, bempty, tfull, tempty;
+  __shared__ __align__(8) uint64_t afull, bfull[STAGES], bempty[STAGES], tfull[2], tempty[2];
   __shared__ int abort_flag;
   const InvTask t = tasks[blockIdx.y];
   const int n = t.n;
@@ -202,13 +218,17 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   unsigned char* sa = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sb = sa + A_TILE;
-  if (w == 0) tc::tmem_alloc(&tslot, 512);
+  if (w == 0) tc::tmem_alloc(&tslot, 2 * ACC);
   if (tid == 0) {
     tc::mbar_init(&afull, 1);
-    tc::mbar_init(&bfull, 1);
-    tc::mbar_init(&bempty, 1);
-    tc::mbar_init(&tfull, 1);
-    tc::mbar_init(&tempty, EPI_WARPS);
+    for (int i = 0; i < STAGES; ++i) {
+      tc::mbar_init(&bfull[i], 1);
+      tc::mbar_init(&bempty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&tfull[i], 1);
+      tc::mbar_init(&tempty[i], EPI_WARPS);
+    }
     abort_flag = 0;
   }
   tc::fence_before_sync();
@@ -227,93 +247,85 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
       for (int s = 0; s < S; ++s)
         tc::bulk_copy_g2s(sa + s * A_SLICE, t.oa + (size_t)blockIdx.x * A_TILE + s * A_SLICE, A_SLICE, &afull);
       for (int ct = 0; ct < tiles && !*abort_v; ++ct) {
-        if (ct >= 1 && !tc::mbar_wait(&bempty, (uint32_t)((ct - 1) & 1), TCU_WAIT)) { fail(); break; }
-        tc::mbar_arrive_expect_tx(&bfull, B_TILE);
-        tc::bulk_copy_g2s(sb, t.ob + (size_t)(tile0 + ct) * B_TILE, B_TILE, &bfull);
+        const int st = ct % STAGES;
+        if (ct >= STAGES && !tc::mbar_wait(&bempty[st], (uint32_t)((ct / STAGES - 1) & 1), TCU_WAIT)) { fail(); break; }
+        tc::mbar_arrive_expect_tx(&bfull[st], B_TILE);
+        tc::bulk_copy_g2s(sb + st * B_TILE, t.ob + (size_t)(tile0 + ct) * B_TILE, B_TILE, &bfull[st]);
         ++copies;
       }
     }
   } else if (w == 1) {
     if (lane == 0) {
-      constexpr uint32_t idesc = idesc_f16(ROWS, 2 * COLS);
       if (!tc::mbar_wait(&afull, 0, TCU_WAIT)) fail();
       for (int ct = 0; ct < tiles && !*abort_v; ++ct) {
-        if (!tc::mbar_wait(&bfull, (uint32_t)(ct & 1), TCU_WAIT)) { fail(); break; }
-        if (ct >= 1 && !tc::mbar_wait(&tempty, (uint32_t)((ct - 1) & 1), TCU_WAIT)) { fail(); break; }
+        const int st = ct % STAGES, a = ct & 1;
+        if (!tc::mbar_wait(&bfull[st], (uint32_t)((ct / STAGES) & 1), TCU_WAIT)) { fail(); break; }
+        if (ct >= 2 && !tc::mbar_wait(&tempty[a], (uint32_t)(((ct >> 1) - 1) & 1), TCU_WAIT)) { fail(); break; }
         tc::fence_after_sync();
-        for (int l = 0; l < S; ++l)
-          for (int i = 0; i <= l; ++i) {
-            const uint32_t pa = tc::smem_addr(sa + i * A_SLICE), pb = tc::smem_addr(sb + (l - i) * B_SLICE);
+        // One MMA per digit i of A' and K-slice: N = 32 (7 - i).
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-              mma_f16(tbase + (uint32_t)(l * 2 * COLS), tc::smem_desc(pa + ks * ROWS * 32, 128, 256),
-                      tc::smem_desc(pb + ks * 2 * COLS * 32, 128, 256), idesc, i > 0 || ks > 0);
-          }
-        tc::mma_commit(&bempty);
-        tc::mma_commit(&tfull);
+        for (int i = 0; i < S; ++i) {
+          const uint32_t pa = tc::smem_addr(sa + i * A_SLICE), pb = tc::smem_addr(sb + st * B_TILE);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            mma_f16(tbase + (uint32_t)(a * ACC + i * 2 * COLS), tc::smem_desc(pa + ks * ROWS * 32, 128, 256),
+                    tc::smem_desc(pb + ks * B_ROWS * 32, 128, 256), idesc_f16(ROWS, 2 * COLS * (S - i)), i > 0 || ks > 0);
+        }
+        tc::mma_commit(&bempty[st]);
+        tc::mma_commit(&tfull[a]);
         ++mma_tiles;
       }
     }
   } else {
-    // Warp's lane quarter of tensor memory (rows) and half of the tile's columns; four complex
-    // columns at a time, their old values requested one step ahead.
-    const int q = w & 3, half = (w - 2) >> 2;
+    // The warp's lane quarter of tensor memory (rows) and four of the tile's complex columns; their old
+    // values are requested while the tile is multiplied.
+    const int q = w & 3, part = (w - 2) >> 2;
     const int r = i0 + 32 * q + lane, gi = base + r;
     const bool row_in = r < rows;
     const bool keep_old = row_in && (trail || gi < k0 || gi >= k0 + kb);
     const int er = row_in ? t.ea[r] : 1;
     double2* Ai = static_cast<double2*>(t.a) + gi;
     const int64_t ld = t.ld;
-    constexpr int CW = COLS / 2;  // complex columns per warp and tile
+    constexpr int CW = 4 * COLS / EPI_WARPS;  // complex columns per warp and tile
+    static_assert(CW == 4, "eight accumulator columns per load");
     auto col_of = [&](int c) { return trail ? base + c : (c < k0 ? c : c + kb); };
     for (int ct = 0; ct < tiles; ++ct) {
-      const int c0 = (tile0 + ct) * COLS + half * CW;
-      double2 old[4];
-      auto fetch = [&](int c) {
+      const int c0 = (tile0 + ct) * COLS + part * CW, a = ct & 1;
+      double2 old[CW];
+      int ec[CW];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          old[j] = (keep_old && c + j < rest) ? Ai[(int64_t)col_of(c + j) * ld] : make_double2(0.0, 0.0);
-      };
-      fetch(c0);
-      bool ok = !*abort_v && tc::mbar_wait(&tfull, (uint32_t)(ct & 1), TCU_WAIT);
+      for (int j = 0; j < CW; ++j) {
+        const bool in = c0 + j < rest;
+        old[j] = (keep_old && in) ? Ai[(int64_t)col_of(c0 + j) * ld] : make_double2(0.0, 0.0);
+        ec[j] = in ? er + t.eb[c0 + j] : 2;
+      }
+      bool ok = !*abort_v && tc::mbar_wait(&tfull[a], (uint32_t)((ct >> 1) & 1), TCU_WAIT);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
         if (lane == 0) fail();
         break;
       }
       tc::fence_after_sync();
+      float v[S][2 * CW];
 #pragma unroll
-      for (int g = 0; g < CW / 4; ++g) {
-        float v[S][8];
+      for (int l = 0; l < S; ++l)
+        tmem_ld8(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * ACC + l * 2 * COLS + part * 2 * CW), v[l]);
+      tc::tmem_ld_wait();
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&tempty[a]);
 #pragma unroll
-        for (int l = 0; l < S; ++l)
-          tmem_ld8(tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(l * 2 * COLS + half * 2 * CW + 8 * g), v[l]);
-        tc::tmem_ld_wait();
-        if (g == CW / 4 - 1) {
-          tc::fence_before_sync();
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(&tempty);
+      for (int j = 0; j < CW; ++j) {
+        float x[S], y[S];
+#pragma unroll
+        for (int l = 0; l < S; ++l) {
+          x[l] = v[l][2 * j];
+          y[l] = v[l][2 * j + 1];
         }
-        double2 now[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) now[j] = old[j];
-        if (g + 1 < CW / 4) fetch(c0 + 4 * (g + 1));
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int c = c0 + 4 * g + j;
-          if (c >= rest) continue;
-          const int e = er + t.eb[c];
-          float x[S], y[S];
-#pragma unroll
-          for (int l = 0; l < S; ++l) {
-            x[l] = v[l][2 * j];
-            y[l] = v[l][2 * j + 1];
-          }
-          // trail: old - L Y; full: old + (swept panel) Y.
-          const double re = combine(x, e), im = combine(y, e);
-          const double2 out = trail ? make_double2(now[j].x - re, now[j].y - im) : make_double2(now[j].x + re, now[j].y + im);
-          if (row_in) Ai[(int64_t)col_of(c) * ld] = out;
-        }
+        // trail: old - L Y; full: old + (swept panel) Y.
+        const double re = combine(x, ec[j]), im = combine(y, ec[j]);
+        const double2 out = trail ? make_double2(old[j].x - re, old[j].y - im) : make_double2(old[j].x + re, old[j].y + im);
+        if (row_in && c0 + j < rest) Ai[(int64_t)col_of(c0 + j) * ld] = out;
       }
     }
   }
@@ -321,13 +333,15 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
   if (*abort_v) {
     if (w == 0 && lane == 0) {
       tc::mbar_wait(&afull, 0, TCU_WAIT);
-      if (copies > 0) tc::mbar_wait(&bfull, (uint32_t)((copies - 1) & 1), TCU_WAIT);
+      for (int ct = max(0, copies - STAGES); ct < copies; ++ct)
+        tc::mbar_wait(&bfull[ct % STAGES], (uint32_t)((ct / STAGES) & 1), TCU_WAIT);
     }
-    if (w == 1 && lane == 0 && mma_tiles > 0) tc::mbar_wait(&bempty, (uint32_t)((mma_tiles - 1) & 1), TCU_WAIT);
+    if (w == 1 && lane == 0 && mma_tiles > 0)
+      tc::mbar_wait(&bempty[(mma_tiles - 1) % STAGES], (uint32_t)(((mma_tiles - 1) / STAGES) & 1), TCU_WAIT);
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (w == 0) tc::tmem_dealloc(tbase, 512);
+  if (w == 0) tc::tmem_dealloc(tbase, 2 * ACC);
 }
 
 }  // namespace oz

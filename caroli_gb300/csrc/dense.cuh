@@ -84,7 +84,36 @@ __host__ __device__ inline int64_t panel_staged_bytes(int m, int vbytes) {
   return (int64_t)m * GJ_KB * vbytes + panel_work_bytes(m, vbytes);
 }
 
-// Sweeps panel [k0, k0 + kb) of every matrix, one CTA per matrix:
+// The row permutation of a panel's interchanges piv[0 .. kb) (positions past the panel's first row), by one
+// warp: perm[c] the original row of the one now at position c < kb; then the positions at or past kb that
+// hold another row now (each is some piv[k], listed once) from perm[GJ_KB] on, their original rows from
+// perm[2 GJ_KB] on, and their number at perm[3 GJ_KB].
+__device__ __forceinline__ void panel_permutation(const int* piv, int kb, int* perm) {
+  const int lane = threadIdx.x & 31;
+  auto origin = [&](int x) {  // the interchanges undone, last first
+    for (int k = kb - 1; k >= 0; --k) {
+      const int p = piv[k];
+      x = x == k ? p : (x == p ? k : x);
+    }
+    return x;
+  };
+  if (lane < kb) perm[lane] = origin(lane);
+  const int p = lane < kb ? piv[lane] : -1;
+  const int from = lane < kb && p >= kb ? origin(p) : p;
+  const bool moved = lane < kb && p >= kb && from != p;
+  const unsigned same = __match_any_sync(0xffffffffu, moved ? p : -1 - lane);
+  const bool leader = moved && (__ffs(same) - 1 == lane);
+  const unsigned bal = __ballot_sync(0xffffffffu, leader);
+  if (leader) {
+    const int at = __popc(bal & ((1u << lane) - 1u));
+    perm[GJ_KB + at] = p;
+    perm[2 * GJ_KB + at] = from;
+  }
+  if (lane == 0) perm[3 * GJ_KB] = __popc(bal);
+}
+
+// Sweeps panel [k0, k0 + kb) of every matrix, one CTA per matrix (with InvTask::prows set only step 1; the
+// others are panel_rest_kernel's, which spreads them over many CTAs):
 //  1. Gauss-Jordan sweep of the m = npiv - k0 candidate rows of the panel columns (in shared
 //     memory when they fit), pivots from those rows: the pivot block P becomes P^-1 and the other
 //     candidate rows -a P^-1;
@@ -144,6 +173,19 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) inv_panel_kernel(
   if (staged)
     for (int c = w; c < kb; c += nw)
       for (int i = lane; i < m; i += 32) A[(k0 + i) + (int64_t)(k0 + c) * ld] = C[i + c * ldc];
+  if (t.prows) {
+    // The rest of the matrix is panel_rest_kernel's: the steps' pivot rows and the permutation for it.
+    V* pg = static_cast<V*>(t.prows);
+    for (int e = threadIdx.x; e < kb * GJ_KB; e += blockDim.x) {
+      const int k = e / GJ_KB, c = e & (GJ_KB - 1);
+      if (c < kb) pg[e] = prows[k * kb + c];
+    }
+    if (w == 0) {
+      if (lane < kb) t.piv[k0 + lane] = k0 + piv[lane];
+      panel_permutation(piv, kb, t.perm);
+    }
+    return;
+  }
   if (threadIdx.x == 0)
     for (int k = 0; k < kb; ++k) {
       t.piv[k0 + k] = k0 + piv[k];

@@ -255,6 +255,7 @@ struct SectorRequest {
 struct RefineBufs {
   Buf rdesc, rx, rr, rd, rtb, rhb, rt, rerr, rdone, rgx, stasks;
   Buf gV, gZ, gH, gg, gcs, gsn, gy, gbeta, gcol, gflags;
+  Buf csum;                                // partial sums of the convergence check
   Buf segs, ctasks, ccount, cjobs, ojobs;  // task and job lists compacted to the solves still iterating
   Buf tg_fr, tg_tasks, tg_stage;    // tensor-core sweeps of many-column solves (tcgemm.cuh)
   // The vectors (one column per channel; the bulk of a mixed batch's memory besides the fronts).
@@ -553,6 +554,7 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
   double* rt_out = static_cast<double*>(rb.rt.get(cj * sizeof(double)));
   double* rerr = static_cast<double*>(rb.rerr.get(cj * sizeof(double)));
   int32_t* rdone = static_cast<int32_t*>(rb.rdone.get(cj * sizeof(int32_t)));
+  double* csum = static_cast<double*>(rb.csum.get(cj * CHECK_PARTS * 3 * sizeof(double)));
   CK(cudaMemsetAsync(rt_out, 0, cj * sizeof(double), s));
   CK(cudaMemsetAsync(rerr, 0, cj * sizeof(double), s));
   const size_t M = GM_M;
@@ -918,7 +920,7 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
     } else {
       in_pieces((size_t)nj, [&](size_t f0, size_t c) {
         launch(K_REF_ROOT, 0.0, 0.0, [&] {
-          sweep_root_kernel<CB><<<dim3(cchunks, (unsigned)c), 256, (size_t)max_root * CB * sizeof(float2), s>>>(
+          sweep_root_kernel<CB><<<dim3(cchunks, (unsigned)((max_root + SW_ROWS - 1) / SW_ROWS), (unsigned)c), 256, (size_t)max_root * CB * sizeof(float2), s>>>(
               drd, jobs + f0, src, dst);
         });
       });
@@ -1015,8 +1017,9 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
     });
     for (int side = 0; side < nsides; ++side) slice_products(set_res + side, K_REF_RES, ojobs, no);
     slice_products(set_gam, K_REF_CHECK, ojobs, no);
+    launch(K_REF_CHECK, 0.0, 0.0, [&] { refine_sums_kernel<<<dim3((unsigned)cj, CHECK_PARTS), 256, 0, s>>>(drd, csum); });
     launch(K_REF_CHECK, 0.0, 0.0, [&] {
-      refine_check_kernel<<<(unsigned)cj, 256, 0, s>>>(drd, ctx->refine_tol, ctx->max_iters, rt_out, rerr, rdone);
+      refine_check_kernel<<<(unsigned)cj, 32, 0, s>>>(drd, csum, ctx->refine_tol, ctx->max_iters, rt_out, rerr, rdone);
     });
     compact(0);
     CK(cudaMemcpyAsync(dh.data(), rdone, cj * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -1212,7 +1215,8 @@ void gradient(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, s
   }
   double2* rhs = static_cast<double2*>(ctx->grhs.get(std::max<size_t>(ro, 1) * sizeof(double2)));
   double* dv = static_cast<double*>(ctx->gdv.get(std::max<size_t>(dvo, 1) * sizeof(double)));
-  double* dp = static_cast<double*>(ctx->gdp.get(std::max<size_t>(cj * std::max(grad.nparams, 1), 1) * sizeof(double)));
+  const size_t ndp = std::max<size_t>(cj * std::max(grad.nparams, 1), 1);
+  double* dp = static_cast<double*>(ctx->gdp.get(ndp * (1 + GRAD_PARTS) * sizeof(double)));  // sums, then their parts
   // Pointer tables: rhs per job, dv per job, dH per job.
   std::vector<const void*> ptrs(3 * cj);
   std::vector<const double2*> rhs_ptr(cj);
@@ -1240,14 +1244,15 @@ void gradient(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, s
                                                             reinterpret_cast<double* const*>(dptrs + cj) + f0);
     });
   });
-  if (grad.nparams > 0 && grad.dvals)
-    in_pieces(cj, [&](size_t f0, size_t c) {
-      launch(K_REF_RES, 0.0, 0.0, [&] {
-        grad_p_kernel<<<dim3((unsigned)c, (unsigned)grad.nparams), 256, 0, s>>>(
-            fwd + f0, adj + f0, reinterpret_cast<const double2* const*>(dptrs + 2 * cj) + f0, grad.nnz,
-            dp + f0 * grad.nparams, grad.nparams);
-      });
+  if (grad.nparams > 0 && grad.dvals) {
+    double* part = dp + ndp;
+    launch(K_REF_RES, 0.0, 0.0, [&] {
+      grad_p_kernel<<<dim3((unsigned)cj, (unsigned)grad.nparams, GRAD_PARTS), 256, 0, s>>>(
+          fwd, adj, reinterpret_cast<const double2* const*>(dptrs + 2 * cj), grad.nnz, part, grad.nparams);
     });
+    const int count = (int)(cj * grad.nparams);
+    launch(K_REF_RES, 0.0, 0.0, [&] { grad_p_finish_kernel<<<(count + 127) / 128, 128, 0, s>>>(part, dp, count); });
+  }
   std::vector<double> dvh(dvo), dph(cj * std::max(grad.nparams, 1));
   CK(cudaMemcpyAsync(dvh.data(), dv, dvo * sizeof(double), cudaMemcpyDeviceToHost, s));
   if (grad.nparams > 0 && grad.dvals)
@@ -1378,13 +1383,13 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       inv_y_off.push_back(v == sizeof(double2) ? SIZE_MAX : y_at);
       inv_bt_off.push_back(v == sizeof(float2) ? bt_at : SIZE_MAX);
       tc.inv_oz_off.push_back(v == sizeof(double2) ? oz_at : SIZE_MAX);
-      tc.inv_pp_off.push_back(v == sizeof(double2) ? pp_at : SIZE_MAX);
+      tc.inv_pp_off.push_back(pp_at);
+      pp_at += PANEL_SCRATCH;
       if (v == sizeof(float2)) {
         y_at += (size_t)GJ_KB * n * v;
         bt_at += tc_operand_bytes(n);
       } else {
         oz_at += (oz::bytes(n) + 1023) / 1024 * 1024;
-        pp_at += PANEL_SCRATCH;
       }
       tc.inv_y = std::max(tc.inv_y, y_at);
       tc.inv_bt = std::max(tc.inv_bt, bt_at);
@@ -1587,9 +1592,9 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
         inv[q].bt = inv_bt_off[q] == SIZE_MAX ? nullptr : dbt + inv_bt_off[q];
         inv[q].scale2 = dscale + q;
         inv[q].bad = dbad + q;
+        inv[q].prows = dpp + tc.inv_pp_off[q];
+        inv[q].perm = reinterpret_cast<int32_t*>(dpp + tc.inv_pp_off[q] + PANEL_PROWS);
         if (tc.inv_oz_off[q] != SIZE_MAX) {
-          inv[q].prows = dpp + tc.inv_pp_off[q];
-          inv[q].perm = reinterpret_cast<int32_t*>(dpp + tc.inv_pp_off[q] + PANEL_PROWS);
           inv[q].oa = doz + tc.inv_oz_off[q];
           inv[q].ob = inv[q].oa + oz::a_bytes(inv[q].n);
           inv[q].ea = reinterpret_cast<int32_t*>(inv[q].ob + oz::b_bytes(inv[q].n));
@@ -1626,6 +1631,21 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     tc.split = split;
     tc.valid = true;
 
+    // max|F11| of every matrix and cleared flags: a few column chunks per matrix while the matrices alone
+    // do not fill the GPU.
+    auto scale_of = [&](auto tag, size_t first, size_t count, int pmax, KClass cls) {
+      CK(cudaMemsetAsync(dscale + first, 0, count * sizeof(double), s));
+      CK(cudaMemsetAsync(dbad + first, 0, count * sizeof(int32_t), s));
+      if (!pmax) return;
+      const unsigned ch = (unsigned)std::max<size_t>(1, std::min<size_t>((pmax + 7) / 8, 4 * SM_COUNT / count));
+      launch(cls, 0.0, 0.0, [&] { panel_scale_kernel<decltype(tag)><<<dim3((unsigned)count, ch), 256, 0, s>>>(dinv + first); });
+    };
+    auto finish_of = [&](auto tag, size_t first, size_t count, int nmax, size_t smf, KClass cls) {
+      const unsigned ch = (unsigned)std::max<size_t>(1, std::min<size_t>((nmax + 255) / 256, 2 * SM_COUNT / count));
+      launch(cls, 0.0, 0.0, [&] {
+        inv_finish_kernel<decltype(tag)><<<dim3((unsigned)count, ch), 256, smf, s>>>(dinv + first, djobs, status);
+      });
+    };
     // FP64 sweeps: panels over clusters, updates from exact digit products on the tensor cores
     // (panel.cuh, ozaki.cuh).
     auto sweep_f64 = [&](size_t first, size_t count, int nmax, int pmax, double tol, bool trail, KClass cls, double flops,
@@ -1633,13 +1653,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       const size_t smf = (size_t)finish_bytes(pmax);
       if (smf > (size_t)SMEM_LIMIT) throw CudaError{cudaErrorInvalidValue, "front too large for a panel sweep"};
       const int panels = (pmax + GJ_KB - 1) / GJ_KB;
-      CK(cudaMemsetAsync(dscale + first, 0, count * sizeof(double), s));
-      CK(cudaMemsetAsync(dbad + first, 0, count * sizeof(int32_t), s));
-      if (tol > 0.0) {
-        // A few column chunks per matrix while the matrices alone do not fill the GPU.
-        const unsigned ch = (unsigned)std::max<size_t>(1, std::min<size_t>((pmax + 7) / 8, 608 / count));
-        launch(cls, 0.0, 0.0, [&] { panel_scale_kernel<double><<<dim3((unsigned)count, ch), 256, 0, s>>>(dinv + first); });
-      }
+      scale_of(0.0, first, count, tol > 0.0 ? pmax : 0, cls);  // a root refuses zero pivots only
       for (int k0 = 0; k0 < pmax; k0 += GJ_KB) {
         launch(cls, flops / panels, 0.0, [&] { launch_panel_sweep<double>(ctx, dinv + first, count, k0, pmax - k0, tol, 0, djobs, status); });
         const int rows = trail ? nmax - k0 : nmax;  // rows and columns of the update, at most
@@ -1647,8 +1661,8 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
         const bool fine = (size_t)((rows + 15) / 16) * 2 * count < (size_t)(4 * SM_COUNT);
         const unsigned rp = (unsigned)((rows + (fine ? 3 : 15)) / (fine ? 4 : 16));
         launch(cls, 0.0, 0.0, [&] {
-          if (fine) panel_rest_kernel<double, 16><<<dim3((unsigned)count, 2 * rp), PR_THREADS, 0, s>>>(dinv + first, k0, (int)rp);
-          else panel_rest_kernel<double, 4><<<dim3((unsigned)count, 2 * rp), PR_THREADS, 0, s>>>(dinv + first, k0, (int)rp);
+          if (fine) panel_rest_kernel<double, 16, 64><<<dim3((unsigned)count, 2 * rp), 64, 0, s>>>(dinv + first, k0, (int)rp);
+          else panel_rest_kernel<double, 4, 64><<<dim3((unsigned)count, 2 * rp), 64, 0, s>>>(dinv + first, k0, (int)rp);
         });
         // Column tiles per CTA, one CTA per SM: the fewest tile times over all waves (a CTA's start, mostly
         // the copy of A', counted as 1.5 tiles).
@@ -1668,8 +1682,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
         });
       }
       if (trail) return;  // refused pivots are reported by the sweeps
-      const unsigned ch = (unsigned)std::max<size_t>(1, std::min<size_t>((nmax + 255) / 256, 2 * SM_COUNT / count));
-      launch(cls, 0.0, 0.0, [&] { inv_finish_kernel<double><<<dim3((unsigned)count, ch), 256, smf, s>>>(dinv + first, djobs, status); });
+      finish_of(0.0, first, count, nmax, smf, cls);
     };
     // Batched blocked sweep of `count` fronts starting at dinv + first: largest size nmax, largest
     // pivot count pmax.
@@ -1690,10 +1703,17 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       const int panels = (pmax + GJ_KB - 1) / GJ_KB;
       const double per = flops / panels;
       const double uper = uflops / panels, ubper = ubytes / panels;
-      launch(cls, 0.0, 0.0, [&] { inv_scale_kernel<TT><<<(unsigned)count, 256, 0, s>>>(dinv + first); });
+      scale_of(TT{}, first, count, pmax, cls);
       for (int k0 = 0; k0 < pmax; k0 += GJ_KB) {
         launch(cls, per, 0.0, [&] {
           inv_panel_kernel<TT><<<(unsigned)count, 256, sm, s>>>(dinv + first, k0, tol, perturb, (int)sm);
+        });
+        // Pieces of 64 rows and columns, or of 16 while those leave SMs without work.
+        const bool fine = (size_t)((nmax + 63) / 64) * 2 * count < (size_t)(4 * SM_COUNT);
+        const unsigned rp = (unsigned)((nmax + (fine ? 15 : 63)) / (fine ? 16 : 64));
+        launch(cls, 0.0, 0.0, [&] {
+          if (fine) panel_rest_kernel<TT, 4, 64><<<dim3((unsigned)count, 2 * rp), 64, 0, s>>>(dinv + first, k0, (int)rp);
+          else panel_rest_kernel<TT, 4, 256><<<dim3((unsigned)count, 2 * rp), 256, 0, s>>>(dinv + first, k0, (int)rp);
         });
         const unsigned rt = (unsigned)((nmax + 63) / 64);
         in_pieces(count, [&](size_t f0, size_t c) {
@@ -1708,7 +1728,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
           });
         });
       }
-      launch(cls, 0.0, 0.0, [&] { inv_finish_kernel<TT><<<(unsigned)count, 256, smf, s>>>(dinv + first, djobs, status); });
+      finish_of(TT{}, first, count, nmax, smf, cls);
     };
 
     const int perturb = mixed ? 1 : 0;

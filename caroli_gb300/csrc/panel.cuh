@@ -361,36 +361,10 @@ __global__ void __launch_bounds__(PS_THREADS) panel_sweep_kernel(const InvTask* 
   for (int j = w; j < kb; j += PS_THREADS / 32)
     for (int i = lane; i < rows; i += 32) A[(r0 + i) + (int64_t)j * t.ld] = F[i + (size_t)j * R];
   if (rank == 0 && w == 0) {
-    // Where the row now at position x came from: the interchanges undone last first.
-    auto origin = [&](int x) {
-      for (int k = kb - 1; k >= 0; --k) {
-        const int p = s_piv[k];
-        x = x == k ? p : (x == p ? k : x);
-      }
-      return x;
-    };
-    int* perm = t.perm;
-    if (lane < kb) {
-      t.piv[k0 + lane] = k0 + s_piv[lane];
-      perm[lane] = origin(lane);
-    }
-    // Positions at or past kb that hold another row now: each is some piv[k], listed once.
-    const int p = lane < kb ? s_piv[lane] : -1;
-    const int from = lane < kb && p >= kb ? origin(p) : p;
-    const bool moved = lane < kb && p >= kb && from != p;
-    const unsigned same = __match_any_sync(0xffffffffu, moved ? p : -1 - lane);
-    const bool leader = moved && (__ffs(same) - 1 == lane);
-    const unsigned bal = __ballot_sync(0xffffffffu, leader);
-    if (leader) {
-      const int at = __popc(bal & ((1u << lane) - 1u));
-      perm[GJ_KB + at] = p;
-      perm[2 * GJ_KB + at] = from;
-    }
-    if (lane == 0) perm[3 * GJ_KB] = __popc(bal);
+    if (lane < kb) t.piv[k0 + lane] = k0 + s_piv[lane];
+    panel_permutation(s_piv, kb, t.perm);
   }
 }
-
-constexpr int PR_THREADS = 64;
 
 // The recorded steps replayed on a row of the panel held by LPR lanes, lane h the entries LPR i + h:
 // step k subtracts entry k times row k of `pk` (stride GJ_KB) from the entries past k (`tri`), or from
@@ -425,19 +399,19 @@ __device__ __forceinline__ void replay_row(V (&b)[GJ_KB / LPR], const V* pk, int
   }
 }
 
-// After panel_sweep_kernel: grid (matrices, row pieces then column pieces), PR_THREADS threads, LPR lanes
-// per row or column (a piece has PR_THREADS / LPR of them).
+// After a panel's sweep: grid (matrices, row pieces then column pieces), NT threads, LPR lanes per row or
+// column (a piece has NT / LPR of them).
 // Row piece: rows outside the candidates replay the recorded steps. With oa set (FP64), every row the
 // update reads also becomes an operand row.
 // Column piece: the pivot rows of the columns outside the panel into Y (or B', or the FP64 operand), the
 // displaced rows into place. In the trail form a column is first solved with L11, by the same replay.
 // LPR: 16 while the pieces of 4 do not fill the GPU (a piece is then a chain of 256 FP64
 // instructions per warp instead of 1 024), 4 past that (fewer shuffles per entry).
-template <typename T, int LPR>
-__global__ void __launch_bounds__(PR_THREADS) panel_rest_kernel(const InvTask* __restrict__ tasks, int k0,
+template <typename T, int LPR, int NT>
+__global__ void __launch_bounds__(NT) panel_rest_kernel(const InvTask* __restrict__ tasks, int k0,
                                                                 int row_pieces) {
   using V = typename Cx<T>::V;
-  constexpr int Q = GJ_KB / LPR, PIECE = PR_THREADS / LPR;
+  constexpr int Q = GJ_KB / LPR, PIECE = NT / LPR;
   __shared__ V sm[GJ_KB * GJ_KB];
   const InvTask t = tasks[blockIdx.x];
   const int n = t.n, np = t.npiv;
@@ -459,7 +433,7 @@ __global__ void __launch_bounds__(PR_THREADS) panel_rest_kernel(const InvTask* _
     const bool any = __syncthreads_or(out);
     if (any) {
       const V* pg = static_cast<const V*>(t.prows);
-      for (int e = threadIdx.x; e < kb * GJ_KB; e += PR_THREADS) sm[e] = (e & (GJ_KB - 1)) < kb ? pg[e] : cx<V>(0.0, 0.0);
+      for (int e = threadIdx.x; e < kb * GJ_KB; e += NT) sm[e] = (e & (GJ_KB - 1)) < kb ? pg[e] : cx<V>(0.0, 0.0);
     } else if (sizeof(T) == 4) {
       return;
     }
@@ -494,7 +468,7 @@ __global__ void __launch_bounds__(PR_THREADS) panel_rest_kernel(const InvTask* _
   if (trail) {
     // L11^T with each column of L11 scaled by its pivot's reciprocal (the steps then use the raw pivot-row
     // entries), the reciprocals on the diagonal.
-    for (int e = threadIdx.x; e < kb * GJ_KB; e += PR_THREADS) {
+    for (int e = threadIdx.x; e < kb * GJ_KB; e += NT) {
       const int c = e & (GJ_KB - 1), k = e / GJ_KB;
       V v = cx<V>(0.0, 0.0);
       if (c < kb && c >= k) {

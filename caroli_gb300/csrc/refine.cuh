@@ -136,46 +136,65 @@ __global__ void __launch_bounds__(256) refine_residual_kernel(RefineDesc* __rest
 // residual rho, the remaining relative error of x_L is about corr * rho: converged when that is
 // below `tol`; stalled when not finite, growing, or out of outer steps. Error estimate
 // |T| * 2 * corr * rho.
-__global__ void __launch_bounds__(256) refine_check_kernel(RefineDesc* __restrict__ rd, double tol, int max_iters,
-                                                           double* __restrict__ t_out, double* __restrict__ err_out,
-                                                           int32_t* __restrict__ done_out) {
-  __shared__ double red[3][32];
-  RefineDesc& R = rd[blockIdx.x];
-  if (R.done) {
-    if (threadIdx.x == 0) done_out[blockIdx.x] = R.stalled ? 2 : 1;
-    return;
-  }
-  double tl = 0.0, dn = 0.0, xn = 0.0;
-  if (R.whole)  // every orbital's value matters (dT/dV_a, ψ): the correction of the whole vector
-    for (int64_t q = threadIdx.x; q < (int64_t)R.nblk * R.c; q += blockDim.x) {
+// The sums of the check of every job: part[(job * CHECK_PARTS + y) * 3 + (T, |d|^2, |x|^2)] over the elements
+// of part y. grid (jobs, CHECK_PARTS): with convergence on the whole vector there are nblk x c elements, and
+// one CTA per job took 1.1 ms for 16 jobs of 16 384 x 21 (the FP64 pipe of 16 SMs).
+constexpr int CHECK_PARTS = 32;
+__global__ void __launch_bounds__(256) refine_sums_kernel(const RefineDesc* __restrict__ rd, double* __restrict__ part) {
+  __shared__ double red[3][8];
+  const RefineDesc& R = rd[blockIdx.x];
+  if (R.done) return;
+  double vals[3] = {0.0, 0.0, 0.0};
+  const int64_t stride = (int64_t)gridDim.y * blockDim.x, first = blockIdx.y * (int64_t)blockDim.x + threadIdx.x;
+  if (R.whole) {  // every orbital's value matters (dT/dV_a, ψ): the correction of the whole vector
+    for (int64_t q = first; q < (int64_t)R.nblk * R.c; q += stride) {
       const float2 dv = R.d[q];
       const double2 xv = R.x[q];
-      dn += (double)dv.x * dv.x + (double)dv.y * dv.y;
-      xn += xv.x * xv.x + xv.y * xv.y;
+      vals[1] += (double)dv.x * dv.x + (double)dv.y * dv.y;
+      vals[2] += xv.x * xv.x + xv.y * xv.y;
     }
-  for (int idx = threadIdx.x; idx < (R.whole ? 0 : R.nl * R.c); idx += blockDim.x) {
-    const int a = idx % R.nl, j = idx / R.nl;
-    const double2* xj = R.x + (int64_t)j * R.nblk;
-    const int row = R.left_local[a];
-    const double2 g = R.gx[a + (int64_t)j * R.nl];  // (Γ_L x_L)[a], from slice_gemm_kernel
-    const double2 xa = xj[row];
-    tl += xa.x * g.x + xa.y * g.y;
-    const float2 dv = R.d[row + (int64_t)j * R.nblk];
-    dn += (double)dv.x * dv.x + (double)dv.y * dv.y;
-    xn += xa.x * xa.x + xa.y * xa.y;
+  } else {
+    for (int64_t idx = first; idx < (int64_t)R.nl * R.c; idx += stride) {
+      const int a = (int)(idx % R.nl), j = (int)(idx / R.nl);
+      const int64_t q = R.left_local[a] + (int64_t)j * R.nblk;
+      const double2 g = R.gx[a + (int64_t)j * R.nl], xa = R.x[q];  // (Γ_L x_L)[a] from slice products
+      const float2 dv = R.d[q];
+      vals[0] += xa.x * g.x + xa.y * g.y;
+      vals[1] += (double)dv.x * dv.x + (double)dv.y * dv.y;
+      vals[2] += xa.x * xa.x + xa.y * xa.y;
+    }
   }
-  double vals[3] = {tl, dn, xn};
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
   for (int k = 0; k < 3; ++k) {
     double v = vals[k];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (l == 0) red[k][w] = v;
   }
   __syncthreads();
+  if (threadIdx.x < 3) {
+    double v = 0.0;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) v += red[threadIdx.x][q];
+    part[((int64_t)blockIdx.x * CHECK_PARTS + blockIdx.y) * 3 + threadIdx.x] = v;
+  }
+}
+
+// The decision from those sums: a warp per job.
+__global__ void __launch_bounds__(32) refine_check_kernel(RefineDesc* __restrict__ rd, const double* __restrict__ part,
+                                                          double tol, int max_iters, double* __restrict__ t_out,
+                                                          double* __restrict__ err_out, int32_t* __restrict__ done_out) {
+  RefineDesc& R = rd[blockIdx.x];
+  if (R.done) {
+    if (threadIdx.x == 0) done_out[blockIdx.x] = R.stalled ? 2 : 1;
+    return;
+  }
+  double sum[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    sum[k] = part[((int64_t)blockIdx.x * CHECK_PARTS + threadIdx.x) * 3 + k];
+    for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+  }
   if (threadIdx.x == 0) {
-    double sum[3] = {0.0, 0.0, 0.0};
-    for (int k = 0; k < 3; ++k)
-      for (int q = 0; q < (int)(blockDim.x >> 5); ++q) sum[k] += red[k][q];
     const double corr = sum[2] > 0.0 ? sqrt(sum[1] / sum[2]) : (sum[1] > 0.0 ? INFINITY : 0.0);
     const double prev = R.corr;
     R.iters += 1;
@@ -439,19 +458,21 @@ __global__ void __launch_bounds__(256) gm_update_kernel(RefineDesc* __restrict__
   if (R.done) return;
   const int q = blockIdx.y * 256 + threadIdx.x;
   if (q >= R.nblk) return;
-  const int steps = R.inner;  // Arnoldi vectors of this outer step (coefficients past them are 0)
+  const int steps = R.inner;  // Arnoldi vectors of this outer step (mostly two to four)
   for (int j = 0; j < R.c; ++j) {
-    // The coefficients first, then every preconditioned vector's element at once.
-    double2 yv[GM_M];
-    float2 zv[GM_M];
-#pragma unroll
-    for (int t = 0; t < GM_M; ++t) yv[t] = t < steps ? R.y[(int64_t)j * GM_M + t] : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int t = 0; t < GM_M; ++t)
-      zv[t] = t < steps ? R.Z[(int64_t)t * R.nblk * R.c + (int64_t)j * R.nblk + q] : make_float2(0.f, 0.f);
+    // Four vectors at a time, their elements requested together; none past the steps taken (all GM_M, with
+    // zero coefficients, were 1.0 ms of FP64 multiply-adds in place of 0.3 on 256 solves of 25 600 rows).
     double2 acc = make_double2(0.0, 0.0);
+    for (int t0 = 0; t0 < steps; t0 += 4) {
+      float2 zv[4];
 #pragma unroll
-    for (int t = 0; t < GM_M; ++t) acc = cfma(acc, yv[t], make_double2((double)zv[t].x, (double)zv[t].y));
+      for (int u = 0; u < 4; ++u)
+        zv[u] = t0 + u < steps ? R.Z[(int64_t)(t0 + u) * R.nblk * R.c + (int64_t)j * R.nblk + q] : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (t0 + u < steps)
+          acc = cfma(acc, R.y[(int64_t)j * GM_M + t0 + u], make_double2((double)zv[u].x, (double)zv[u].y));
+    }
     const int64_t o = q + (int64_t)j * R.nblk;
     R.x[o].x += acc.x;
     R.x[o].y += acc.y;
@@ -751,10 +772,12 @@ __global__ void __launch_bounds__(256) grad_v_kernel(const RefineDesc* __restric
   out[blockIdx.x][i] = 2.0 * s;  // block-local order
 }
 
-// dT/dp = 2 Re Σ_j z_j^† (dH/dp) x_j for each parameter (dH given as values on the CSR pattern).
-// grid (jobs, parameters); partial sums per CTA in `part`.
+// dT/dp = 2 Re Σ_j z_j^† (dH/dp) x_j for each parameter (dH given as values on the CSR pattern), in
+// GRAD_PARTS partial sums per (job, parameter). grid (jobs, parameters, GRAD_PARTS). Entries that are zero
+// (a parameter touches few sites) cost their load only.
+constexpr int GRAD_PARTS = 32;
 __global__ void __launch_bounds__(256) grad_p_kernel(const RefineDesc* __restrict__ fwd, const RefineDesc* __restrict__ adj,
-                                                     const double2* const* dh, int64_t nnz, double* __restrict__ out,
+                                                     const double2* const* dh, int64_t nnz, double* __restrict__ part,
                                                      int nparams) {
   __shared__ double red[32];
   const RefineDesc& X = fwd[blockIdx.x];
@@ -762,16 +785,26 @@ __global__ void __launch_bounds__(256) grad_p_kernel(const RefineDesc* __restric
   const int k = blockIdx.y;
   const double2* d = dh[blockIdx.x] + (int64_t)k * nnz;
   double s = 0.0;
-  for (int i = threadIdx.x; i < X.nblk; i += blockDim.x)
-    for (int j = 0; j < X.c; ++j) {
-      double2 hx = make_double2(0.0, 0.0);
-      const double2* xj = X.x + (int64_t)j * X.nblk;
-      for (int q = X.csr_ptr[i]; q < X.csr_ptr[i + 1]; ++q) hx = cfma(hx, d[X.csr_q[q]], xj[X.csr_col[q]]);
-      const double2 z = Z.x[i + (int64_t)j * X.nblk];
-      s += z.x * hx.x + z.y * hx.y;  // Re(conj(z) hx)
+  for (int i = blockIdx.z * blockDim.x + threadIdx.x; i < X.nblk; i += gridDim.z * blockDim.x)
+    for (int q = X.csr_ptr[i]; q < X.csr_ptr[i + 1]; ++q) {
+      const double2 v = d[X.csr_q[q]];
+      if (!((__double_as_longlong(v.x) | __double_as_longlong(v.y)) << 1)) continue;  // +-0
+      const int col = X.csr_col[q];
+      for (int j = 0; j < X.c; ++j) {
+        const double2 hx = cmul(v, X.x[col + (int64_t)j * X.nblk]);
+        const double2 z = Z.x[i + (int64_t)j * X.nblk];
+        s += z.x * hx.x + z.y * hx.y;  // Re(conj(z) hx)
+      }
     }
   s = block_sum(s, red);
-  if (threadIdx.x == 0) out[(int64_t)blockIdx.x * nparams + k] = 2.0 * s;
+  if (threadIdx.x == 0) part[((int64_t)blockIdx.x * nparams + k) * GRAD_PARTS + blockIdx.z] = s;
+}
+__global__ void grad_p_finish_kernel(const double* __restrict__ part, double* __restrict__ out, int count) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= count) return;
+  double s = 0.0;
+  for (int z = 0; z < GRAD_PARTS; ++z) s += part[(int64_t)q * GRAD_PARTS + z];
+  out[q] = 2.0 * s;
 }
 
 }  // namespace caroli

@@ -320,18 +320,22 @@ __global__ void __launch_bounds__(256) sweep_rows_bwd_kernel(const RefineDesc* _
 }
 
 // ---- root: x = F_root^-1 z (the conjugate transpose for the adjoint) ---------------------------
-// grid (column chunks, jobs); dynamic shared memory z (m x CB).
+// grid (column chunks, row tiles of 64, jobs); dynamic shared memory z (m x CB). The inner dimension is
+// split four ways as in sweep_rows_*; the adjoint reads rows of the stored inverse's transpose, a warp per
+// row. (One CTA per job and column chunk took 270 us for 16 roots of 512 and 21 columns.)
 template <int CB>
 __global__ void __launch_bounds__(256) sweep_root_kernel(const RefineDesc* __restrict__ rd, const int32_t* __restrict__ jobs,
                                                          int src, int dst) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const RefineDesc& R = rd[jobs ? jobs[blockIdx.y] : blockIdx.y];
+  __shared__ float2 part[SW_SLICES - 1][SW_ROWS][CB];
+  const RefineDesc& R = rd[jobs ? jobs[blockIdx.z] : blockIdx.z];
   const int j0 = blockIdx.x * CB;
   if (sweep_idle(R, src) || j0 >= R.c) return;
+  const FrontDesc& f = R.fronts[R.root_front];
+  const int m = f.n, r0 = blockIdx.y * SW_ROWS;
+  if (r0 >= m) return;
   const double2* rin = sweep_src(R, src);
   float2* dout = sweep_dst(R, dst);
-  const FrontDesc& f = R.fronts[R.root_front];
-  const int m = f.n;
   float2* z = reinterpret_cast<float2*>(smem_raw);
   for (int p = threadIdx.x; p < m; p += blockDim.x) {
     float2 zz[CB];
@@ -340,32 +344,59 @@ __global__ void __launch_bounds__(256) sweep_root_kernel(const RefineDesc* __res
     for (int j = 0; j < CB; ++j) z[p * CB + j] = zz[j];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    float2 acc[CB];
+  if (R.adjoint) {
+    const int lane = threadIdx.x & 31;
+    for (int i = r0 + (threadIdx.x >> 5); i < min(m, r0 + SW_ROWS); i += 8) {
+      float2 acc[CB];
 #pragma unroll
-    for (int j = 0; j < CB; ++j) acc[j] = make_float2(0.f, 0.f);
-    if (R.adjoint) {
-      for (int k = 0; k < m; ++k) {
+      for (int j = 0; j < CB; ++j) acc[j] = make_float2(0.f, 0.f);
+#pragma unroll 4
+      for (int k = lane; k < m; k += 32) {
         float2 a = R.root[k + (int64_t)i * m];
         a.y = -a.y;
 #pragma unroll
         for (int j = 0; j < CB; ++j) acc[j] = cfma(acc[j], a, z[k * CB + j]);
       }
-    } else {
+#pragma unroll
+      for (int j = 0; j < CB; ++j)
+        for (int o = 16; o > 0; o >>= 1) {
+          acc[j].x += __shfl_xor_sync(0xffffffffu, acc[j].x, o);
+          acc[j].y += __shfl_xor_sync(0xffffffffu, acc[j].y, o);
+        }
+      const int v = R.srows[f.var_off + i].var;
+#pragma unroll
+      for (int j = 0; j < CB; ++j)
+        if (lane == j && j0 + j < R.c) dout[v + (int64_t)(j0 + j) * R.nblk] = acc[j];
+    }
+    return;
+  }
+  const int lr = threadIdx.x % SW_ROWS, sl = threadIdx.x / SW_ROWS;
+  const int r = r0 + lr;
+  float2 acc[CB];
+#pragma unroll
+  for (int j = 0; j < CB; ++j) acc[j] = make_float2(0.f, 0.f);
+  if (r < m) {
+    const int kper = (m + SW_SLICES - 1) / SW_SLICES;
+    const int k1 = min(m, (sl + 1) * kper);
+    const float2* F = R.root + r;
 #pragma unroll 8
-      for (int k = 0; k < m; ++k) {
-        const float2 a = R.root[i + (int64_t)k * m];
+    for (int k = sl * kper; k < k1; ++k) {
+      const float2 a = F[(int64_t)k * m];
 #pragma unroll
-        for (int j = 0; j < CB; ++j) acc[j] = cfma(acc[j], a, z[k * CB + j]);
-      }
+      for (int j = 0; j < CB; ++j) acc[j] = cfma(acc[j], a, z[k * CB + j]);
     }
-    const int v = R.srows[f.var_off + i].var;
+  }
+  if (sl > 0)
 #pragma unroll
-    for (int j = 0; j < CB; ++j) {
-      const int col = j0 + j;
-      if (col >= R.c) break;
-      dout[v + (int64_t)col * R.nblk] = acc[j];
-    }
+    for (int j = 0; j < CB; ++j) part[sl - 1][lr][j] = acc[j];
+  __syncthreads();
+  if (sl != 0 || r >= m) return;
+  const int v = R.srows[f.var_off + r].var;
+#pragma unroll
+  for (int j = 0; j < CB; ++j) {
+#pragma unroll
+    for (int q = 0; q < SW_SLICES - 1; ++q) { acc[j].x += part[q][lr][j].x; acc[j].y += part[q][lr][j].y; }
+    if (j0 + j < R.c) dout[v + (int64_t)(j0 + j) * R.nblk] = acc[j];
   }
 }
 

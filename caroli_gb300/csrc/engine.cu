@@ -29,6 +29,7 @@
 #include "sweep.cuh"
 #include "disorder.cuh"
 #include "leadsig.cuh"
+#include "ozgemm.cuh"
 #include "panel.cuh"
 #include "tcgemm.cuh"
 
@@ -242,25 +243,24 @@ struct JobSpec {
 };
 
 // Sector transmissions of multi-terminal jobs: trace labels in place of the leads. Label k of a
-// block sits at the positions of its lead (lptr/lpos per block, device and host copies); its Γ per
-// (instance, block) in a device table of P pointers.
+// block sits at the positions hptr[k] .. hptr[k + 1] of the block's device list lpos, in its lead's order.
 struct SectorRequest {
   int P = 0, nblocks = 0;
   std::vector<std::vector<int32_t>> hptr;
-  std::vector<const int32_t*> lptr, lpos;       // per block
-  std::vector<const double2* const*> gam;       // per (instance, block)
+  std::vector<const int32_t*> lpos;             // per block
+  std::vector<const double2*> gam;              // per (instance, block, label)
 };
 
 // Device state of one refinement (forward, or the adjoint of the gradient).
 struct RefineBufs {
-  Buf rdesc, rx, rr, rd, rtb, rhb, rt, rerr, rdone, rgx, stasks;
+  Buf rdesc, rx, rr, rd, rtb, rhb, rt, rerr, rdone, rgx, spack, sdig, svec, sgemm;  // s*: slice products (tasks, digits of Σ and Γ, of the vectors)
   Buf gV, gZ, gH, gg, gcs, gsn, gy, gbeta, gcol, gflags;
   Buf csum;                                // partial sums of the convergence check
   Buf segs, ctasks, ccount, cjobs, ojobs;  // task and job lists compacted to the solves still iterating
   Buf tg_fr, tg_tasks, tg_stage;    // tensor-core sweeps of many-column solves (tcgemm.cuh)
   // The vectors (one column per channel; the bulk of a mixed batch's memory besides the fronts).
   void release_vectors() {
-    for (Buf* b : {&rx, &rr, &rd, &rtb, &rhb, &rgx, &gV, &gZ, &tg_stage}) b->release();
+    for (Buf* b : {&rx, &rr, &rd, &rtb, &rhb, &rgx, &gV, &gZ, &tg_stage, &sdig, &svec}) b->release();
   }
 };
 
@@ -392,10 +392,10 @@ struct caroli_ctx {
   // (instance, block) job, copied out after the root inverse.
   std::vector<std::vector<double2>>* green_out = nullptr;
   int green_blocks = 0;
-  Buf sec_pos, sec_ptr, sec_gam, sec_tab;
-  Buf mjobs, mscratch, mout;  // multi-terminal traces
+  Buf sec_pos, sec_gam;
+  Buf tr_tasks, tr_dig, tr_c, tr_part;  // traces: task lists, digits, products, partial sums
   Buf dent, dspin, dscal, dcoef, dflag, dtab, dclean;  // on-device disorder
-  Buf lead_d, lead_cols, lead_w;                       // self-energies from lead modes
+  Buf lead_d, lead_cols, lead_w, lead_status;                       // self-energies from lead modes
   double inner_tol = 1e-10;
   bool tensor_cores = true;  // f32 rank-kb updates on tcgen05 (3xTF32); else on the CUDA cores
   int max_iters = 6;
@@ -624,43 +624,97 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
   }
   RefineDesc* drd = static_cast<RefineDesc*>(rb.rdesc.get(cj * sizeof(RefineDesc)));
   CK(cudaMemcpyAsync(drd, rdh.data(), cj * sizeof(RefineDesc), cudaMemcpyHostToDevice, s));
-  // Dense slice products (Σ_L, Σ_R of A and Γ_L of the trace): one task per job and product,
-  // built once. Matvec of step k: V_{k+1} -= Σ Z_k; residual: r += Σ x; check: gx = Γ_L x_L.
-  // Left and right slices run as separate launches (they may share rows).
-  const int nsides = 2;
-  const size_t per_set = cj;  // tasks of one (product, side) set
-  const size_t set_mv = 0, set_res = (size_t)GM_M * nsides, set_gam = set_res + nsides;
-  const size_t nsets = set_gam + 1;
-  std::vector<SliceTask> sth(nsets * per_set);
+  // Dense slice products on the tensor cores (ozgemm.cuh): V_{k+1} -= Σ Z_k, r += Σ x, gx = Γ_L x_L. The
+  // digits of each distinct Σ_L, Σ_R (Γ_L) are written once here; a product writes its vectors' digits, then
+  // multiplies. Two tasks (left, right) per job for the Σ products, one for Γ_L. The sides add into
+  // different rows unless the slices are the same (a device of one slice): they then take a launch each.
+  constexpr int SLICE_SIDES = 2;
+  const size_t nst = cj * SLICE_SIDES;
+  std::vector<oz::PackTask> packs;               // Σ and Γ of the distinct slots, then per job and side the vectors
+  std::vector<oz::GemmTask> gemms(2 * nst + cj); // matvec, residual (per job and side), Γ_L (per job)
+  std::vector<oz::PackTask> vec(2 * nst + cj);
+  std::map<const double2*, size_t> packed;       // first element -> its pack task
+  std::vector<size_t> dig_off, vec_off(nst), vec_eoff(nst), exp_off;
+  size_t digs = 0, vecs = 0;
   int slice_m = 1;
+  bool same_rows = false;
+  double fl_sigma = 0.0, fl_gamma = 0.0;
+  int max_pack = 1;
   for (size_t j = 0; j < cj; ++j) {
     const RefineDesc& R = rdh[j];
-    const RefineDesc* dR = drd + j;
-    for (int side = 0; side < nsides; ++side) {
+    const FrontPlan& P = specs[begin + j].plan->host;
+    if (R.c == 0) continue;
+    same_rows |= P.nr > 0 && P.rpos == 0 && P.nl > 0;
+    auto matrix = [&](const double2* p, int m) -> size_t {
+      auto it = packed.find(p);
+      if (it != packed.end()) return it->second;
+      oz::PackTask t{};
+      t.p = p; t.ld = m; t.rows = t.k = m;
+      t.trans = t.conj = R.adjoint;
+      dig_off.push_back(digs);
+      digs += oz::pack_a_bytes(m, m);
+      exp_off.push_back(digs);
+      digs += oz::pack_e_bytes(m, m);
+      packs.push_back(t);
+      max_pack = std::max(max_pack, m * oz::chunks_of(m));
+      packed.emplace(p, packs.size() - 1);
+      return packs.size() - 1;
+    };
+    for (int side = 0; side < SLICE_SIDES; ++side) {
       const double2* sg = side == 0 ? R.sigma_l : R.sigma_r;
       const int m = side == 0 ? R.nl : R.nr;
       const int32_t* rows = side == 0 ? R.left_local : R.right_local;
+      if (!sg || m <= 0) continue;
       slice_m = std::max(slice_m, m);
-      SliceTask base{};
-      base.rd = dR; base.s = sg; base.irow = rows; base.orow = rows; base.ldi = base.ldo = R.nblk;
-      base.m = (sg && m > 0) ? m : 0; base.c = R.c; base.adj = R.adjoint; base.accumulate = 1;
-      for (int k = 0; k < GM_M; ++k) {
-        SliceTask t = base;
-        t.in = R.Z + (size_t)k * R.nblk * R.c; t.in_f32 = 1; t.out = R.V + (size_t)(k + 1) * R.nblk * R.c;
-        t.mode = 0; t.sign = -1.0;
-        sth[(set_mv + (size_t)k * nsides + side) * per_set + j] = t;
+      const size_t q = j * SLICE_SIDES + side, mat = matrix(sg, m);
+      vec_off[q] = vecs;
+      vecs += oz::pack_b_bytes(R.c, m);
+      vec_eoff[q] = vecs;
+      vecs += oz::pack_e_bytes(R.c, m);
+      oz::PackTask v{};
+      v.ld = R.nblk; v.kmap = rows; v.rows = R.c; v.k = m; v.trans = 1; v.b = 1; v.rd = drd + j;
+      oz::GemmTask g{};
+      g.crow = rows; g.rd = drd + j; g.m = m; g.n = R.c; g.chunks = oz::chunks_of(m);
+      g.ea = reinterpret_cast<const int32_t*>(mat);  // the pack task, until the buffers are known
+      v.src = 1; g.dst = 1; g.sign = -1.0;
+      vec[q] = v; gemms[q] = g;
+      v.src = 2; g.dst = 2; g.sign = 1.0;
+      vec[nst + q] = v; gemms[nst + q] = g;
+      fl_sigma += 8.0 * m * (double)m * R.c;
+      if (side == 0 && R.gamma_l && !R.whole) {
+        g.dst = 3; g.crow = nullptr;  // takes the digits of x_L that the residual wrote
+        g.ea = reinterpret_cast<const int32_t*>(matrix(R.gamma_l, m));
+        vec[2 * nst + j] = v; gemms[2 * nst + j] = g;
+        fl_gamma += 8.0 * m * (double)m * R.c;
       }
-      SliceTask t = base;
-      t.in = R.x; t.in_f32 = 0; t.out = R.r; t.mode = 1; t.sign = 1.0;
-      sth[(set_res + side) * per_set + j] = t;
     }
-    SliceTask t{};
-    t.rd = dR; t.s = R.gamma_l; t.irow = R.left_local; t.orow = nullptr; t.in = R.x; t.out = R.gx;
-    t.ldi = R.nblk; t.ldo = R.nl; t.m = (R.gamma_l && !R.whole) ? R.nl : 0; t.c = R.c; t.mode = 1; t.sign = 1.0;
-    sth[set_gam * per_set + j] = t;
   }
-  SliceTask* dst_tasks = static_cast<SliceTask*>(rb.stasks.get(sth.size() * sizeof(SliceTask)));
-  CK(cudaMemcpyAsync(dst_tasks, sth.data(), sth.size() * sizeof(SliceTask), cudaMemcpyHostToDevice, s));
+  unsigned char* ddig = static_cast<unsigned char*>(rb.sdig.get(std::max<size_t>(digs, 16)));
+  unsigned char* dvec = static_cast<unsigned char*>(rb.svec.get(std::max<size_t>(vecs, 16)));
+  for (size_t k = 0; k < packs.size(); ++k) {
+    packs[k].dig = ddig + dig_off[k];
+    packs[k].exp = reinterpret_cast<int32_t*>(ddig + exp_off[k]);
+  }
+  for (size_t e = 0; e < gemms.size(); ++e) {
+    if (!gemms[e].m) continue;
+    const size_t mat = reinterpret_cast<size_t>(gemms[e].ea), q = e < 2 * nst ? e % nst : (e - 2 * nst) * SLICE_SIDES;
+    gemms[e].a = packs[mat].dig;
+    gemms[e].ea = packs[mat].exp;
+    gemms[e].b = vec[e].dig = dvec + vec_off[q];
+    vec[e].exp = reinterpret_cast<int32_t*>(dvec + vec_eoff[q]);
+    gemms[e].eb = vec[e].exp;
+  }
+  const size_t npacks = packs.size();
+  packs.insert(packs.end(), vec.begin(), vec.end());
+  oz::PackTask* dpacks = static_cast<oz::PackTask*>(rb.spack.get(packs.size() * sizeof(oz::PackTask)));
+  oz::GemmTask* dgemms = static_cast<oz::GemmTask*>(rb.sgemm.get(gemms.size() * sizeof(oz::GemmTask)));
+  CK(cudaMemcpyAsync(dpacks, packs.data(), packs.size() * sizeof(oz::PackTask), cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(dgemms, gemms.data(), gemms.size() * sizeof(oz::GemmTask), cudaMemcpyHostToDevice, s));
+  in_pieces(npacks, [&](size_t f0, size_t c) {
+    launch(K_REF_RES, 0.0, 0.0, [&] {
+      oz::pack_kernel<<<dim3((unsigned)((max_pack + 63) / 64), (unsigned)c), 256, 0, s>>>(dpacks + f0, nullptr, 1, 0);
+    });
+  });
   // Solves with many columns (TG_MIN_COLS or more channels) sweep their large fronts and the root
   // as tensor-core GEMMs (tcgemm.cuh): per level, the fronts' right-hand sides are gathered into a
   // staging block, then one GEMM task per output block. The lists hold every large front of every
@@ -799,23 +853,24 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
       });
     });
   };
-  // Launches the slice products of one set for the `nl` jobs listed in `jl`; flops for the
-  // accounting (the set's flops over all jobs, in proportion to the jobs listed).
-  auto slice_products = [&](size_t set, KClass cls, const int32_t* jl, size_t nl) {
-    double fl = 0.0;
-    for (size_t j = 0; j < cj; ++j) fl += 8.0 * sth[set * per_set + j].m * (double)sth[set * per_set + j].m * sth[set * per_set + j].c;
+  // One kind of slice products (0: matvec of step k, 1: residual, 2: Γ_L) for the `nl` jobs listed in `jl`.
+  auto slice_products = [&](int kind, int k, KClass cls, const int32_t* jl, size_t nl) {
+    const double fl = kind == 2 ? fl_gamma : fl_sigma;
     if (fl == 0.0 || nl == 0) return;
-    const dim3 grid((unsigned)((slice_m + SG_ROWS - 1) / SG_ROWS), (unsigned)((std::max(1, cmax) + SG_COLS - 1) / SG_COLS));
-    const unsigned rchunks = (unsigned)((slice_m + 127) / 128);
-    in_pieces(nl, [&](size_t f0, size_t c) {
-      launch(cls, fl * c / cj, 0.0, [&] {
-        const SliceTask* tk = dst_tasks + set * per_set;
-        if (cmax <= 1) slice_rows_kernel<1><<<dim3(rchunks, (unsigned)c), 128, 0, s>>>(tk, jl + f0);
-        else if (cmax <= 2) slice_rows_kernel<2><<<dim3(rchunks, (unsigned)c), 128, 0, s>>>(tk, jl + f0);
-        else if (cmax <= 4) slice_rows_kernel<4><<<dim3(rchunks, (unsigned)c), 128, 0, s>>>(tk, jl + f0);
-        else if (cmax <= 8) slice_rows_kernel<8><<<dim3(rchunks, (unsigned)c), 128, 0, s>>>(tk, jl + f0);
-        else slice_gemm_kernel<<<dim3(grid.x, grid.y, (unsigned)c), 256, 0, s>>>(tk, jl + f0);
-      });
+    const int per = kind == 2 ? 1 : SLICE_SIDES, sides = same_rows ? per : 1;  // launches, tasks per job and launch
+    const unsigned px = (unsigned)(((size_t)std::max(1, cmax) * oz::chunks_of(slice_m) + 63) / 64);
+    const dim3 grid((unsigned)((slice_m + oz::ROWS - 1) / oz::ROWS), (unsigned)((std::max(1, cmax) + oz::COLS - 1) / oz::COLS));
+    const size_t t0 = kind * nst;
+    in_pieces_of(nl, 65535 / per, [&](size_t f0, size_t c) {
+      if (kind < 2)
+        launch(cls, 0.0, 0.0, [&] {
+          oz::pack_kernel<<<dim3(px, (unsigned)(c * per)), 256, 0, s>>>(dpacks + npacks + t0, jl + f0, per, k);
+        });
+      for (int sd = 0; sd < sides; ++sd)
+        launch(cls, fl * c / cj / sides, 0.0, [&] {
+          oz::gemm_kernel<<<dim3(grid.x, grid.y, (unsigned)(c * (sides > 1 ? 1 : per))), oz::THREADS, oz::GEMM_SMEM, s>>>(
+              dgemms + t0, jl + f0, per, k, sides > 1 ? sd : -1);
+        });
     });
   };
   // Right-hand-side columns per CTA: the batch's largest channel count, rounded up to 1, 2, 4, 8.
@@ -972,7 +1027,7 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
         launch(K_REF_RES, resid_flops * c / cj, 0.0,
                [&] { gm_matvec_kernel<<<dim3((unsigned)c, rows), 256, 0, s>>>(drd, jl + f0, k); });
       });
-      for (int side = 0; side < nsides; ++side) slice_products(set_mv + (size_t)k * nsides + side, K_REF_RES, jl, nl);
+      slice_products(0, k, K_REF_RES, jl, nl);
       // Classical Gram-Schmidt, one pass (gm_dot_kernel pass 0): right-preconditioned by the f32
       // factors, A M^-1 is close to the identity and its few Krylov vectors stay orthogonal to
       // working accuracy; the outer step checks the true FP64 residual either way.
@@ -1015,8 +1070,8 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
       launch(K_REF_RES, resid_flops * c / cj, 0.0,
              [&] { refine_residual_kernel<<<dim3((unsigned)c, rows), 256, 0, s>>>(drd, ojobs + f0); });
     });
-    for (int side = 0; side < nsides; ++side) slice_products(set_res + side, K_REF_RES, ojobs, no);
-    slice_products(set_gam, K_REF_CHECK, ojobs, no);
+    slice_products(1, 0, K_REF_RES, ojobs, no);
+    slice_products(2, 0, K_REF_CHECK, ojobs, no);
     launch(K_REF_CHECK, 0.0, 0.0, [&] { refine_sums_kernel<<<dim3((unsigned)cj, CHECK_PARTS), 256, 0, s>>>(drd, csum); });
     launch(K_REF_CHECK, 0.0, 0.0, [&] {
       refine_check_kernel<<<(unsigned)cj, 32, 0, s>>>(drd, csum, ctx->refine_tol, ctx->max_iters, rt_out, rerr, rdone);
@@ -1270,6 +1325,119 @@ void gradient(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, s
   (void)eh;
 }
 
+// One trace Tr[Γ_p G Γ_q G^†]: G the np x nq block of a root inverse at rows r0 + rmap, columns c0 + cmap.
+struct TracePair {
+  const void* g;
+  int64_t ld;
+  const double2 *gp, *gq;
+  const int32_t *rmap, *cmap;
+  double* part;   // oz::DOT_PARTS partial sums
+  size_t part_at;
+  int32_t* status;
+  int r0, c0, np, nq;
+};
+
+// Σ_ij Re[(Γ_p G)_ij conj((G Γ_q)_ij)] of every pair (caroli-green/src/lib.rs:106-113): both products as FP64
+// GEMMs on the tensor cores (ozgemm.cuh), in batches of about a gigabyte of digits; each Γ of a batch is
+// written as digits once. Against a thread per element on the FP64 pipe: two solves with slices of 576
+// orbitals 6.4 -> 0.3 ms, all pairs of four leads of 128 orbitals at eight energies 4.9 -> 0.4 ms.
+template <typename LaunchT>
+void trace_pairs(caroli_ctx* ctx, const std::vector<TracePair>& pairs, double flops, LaunchT& launch) {
+  cudaStream_t s = ctx->stream;
+  constexpr size_t BATCH = size_t(1) << 30;
+  for (size_t first = 0; first < pairs.size();) {
+    std::vector<oz::PackTask> packs;
+    std::vector<oz::GemmTask> gemms;
+    std::vector<oz::DotTask> dots;
+    std::vector<size_t> dig, exps, mats;  // digit and exponent offsets per pack; per GEMM its two packs
+    std::map<std::pair<const double2*, int>, size_t> gammas;
+    size_t at = 0, cat = 0;
+    int max_pack = 1, max_m = 1, max_n = 1;
+    auto add = [&](oz::PackTask t) {
+      dig.push_back(at);
+      at += t.b ? oz::pack_b_bytes(t.rows, t.k) : oz::pack_a_bytes(t.rows, t.k);
+      exps.push_back(at);
+      at += oz::pack_e_bytes(t.rows, t.k);
+      max_pack = std::max(max_pack, t.rows * oz::chunks_of(t.k));
+      packs.push_back(t);
+      return packs.size() - 1;
+    };
+    auto gamma = [&](const double2* p, int m, int b) {
+      auto it = gammas.find({p, b});
+      if (it != gammas.end()) return it->second;
+      oz::PackTask t{};
+      t.p = p; t.ld = m; t.rows = t.k = m; t.trans = t.b = b;
+      return gammas[{p, b}] = add(t);
+    };
+    size_t next = first;
+    for (; next < pairs.size() && (next == first || at < BATCH); ++next) {
+      const TracePair& q = pairs[next];
+      oz::PackTask g{};
+      g.p = q.g; g.ld = q.ld;
+      g.r0 = q.r0; g.rmap = q.rmap; g.rows = q.np;
+      g.k0 = q.c0; g.kmap = q.cmap; g.k = q.nq;
+      const size_t ga = add(g);  // G as the left factor
+      std::swap(g.r0, g.k0);
+      std::swap(g.rmap, g.kmap);
+      std::swap(g.rows, g.k);
+      g.trans = g.b = 1;
+      const size_t gb = add(g);  // and as the right one
+      oz::GemmTask t{};
+      t.m = q.np; t.n = q.nq; t.ldc = q.np; t.sign = 1.0; t.status = q.status;
+      max_m = std::max(max_m, q.np);
+      max_n = std::max(max_n, q.nq);
+      oz::DotTask d{};
+      d.count = (int64_t)q.np * q.nq;
+      d.part = q.part;
+      for (int side = 0; side < 2; ++side) {
+        mats.push_back(side == 0 ? gamma(q.gp, q.np, 0) : ga);
+        mats.push_back(side == 0 ? gb : gamma(q.gq, q.nq, 1));
+        t.chunks = oz::chunks_of(side == 0 ? q.np : q.nq);
+        gemms.push_back(t);
+      }
+      dots.push_back(d);
+      cat += 2 * (size_t)d.count;
+    }
+    unsigned char* ddig = static_cast<unsigned char*>(ctx->tr_dig.get(at));
+    double2* dc = static_cast<double2*>(ctx->tr_c.get(std::max<size_t>(cat, 1) * sizeof(double2)));
+    for (size_t k = 0; k < packs.size(); ++k) {
+      packs[k].dig = ddig + dig[k];
+      packs[k].exp = reinterpret_cast<int32_t*>(ddig + exps[k]);
+    }
+    size_t co = 0;
+    for (size_t k = 0; k < gemms.size(); ++k) {
+      const oz::PackTask &a = packs[mats[2 * k]], &b = packs[mats[2 * k + 1]];
+      gemms[k].a = a.dig; gemms[k].ea = a.exp;
+      gemms[k].b = b.dig; gemms[k].eb = b.exp;
+      gemms[k].c = dc + co;
+      (k % 2 ? dots[k / 2].y : dots[k / 2].x) = dc + co;
+      co += (size_t)gemms[k].m * gemms[k].n;
+    }
+    const size_t pb = packs.size() * sizeof(oz::PackTask), gb = gemms.size() * sizeof(oz::GemmTask),
+                 db = dots.size() * sizeof(oz::DotTask);
+    unsigned char* dt = static_cast<unsigned char*>(ctx->tr_tasks.get(pb + gb + db));
+    CK(cudaMemcpyAsync(dt, packs.data(), pb, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(dt + pb, gemms.data(), gb, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(dt + pb + gb, dots.data(), db, cudaMemcpyHostToDevice, s));
+    const oz::PackTask* dp = reinterpret_cast<const oz::PackTask*>(dt);
+    const oz::GemmTask* dg = reinterpret_cast<const oz::GemmTask*>(dt + pb);
+    const oz::DotTask* dd = reinterpret_cast<const oz::DotTask*>(dt + pb + gb);
+    in_pieces(packs.size(), [&](size_t f0, size_t c) {
+      launch(K_TRACE, 0.0, 0.0, [&] {
+        oz::pack_kernel<<<dim3((unsigned)((max_pack + 63) / 64), (unsigned)c), 256, 0, s>>>(dp + f0, nullptr, 1, 0);
+      });
+    });
+    const dim3 grid((unsigned)((max_m + oz::ROWS - 1) / oz::ROWS), (unsigned)((max_n + oz::COLS - 1) / oz::COLS));
+    in_pieces(gemms.size(), [&](size_t f0, size_t c) {
+      launch(K_TRACE, flops * c / (2.0 * pairs.size()), 0.0, [&] {
+        oz::gemm_kernel<<<dim3(grid.x, grid.y, (unsigned)c), oz::THREADS, oz::GEMM_SMEM, s>>>(dg + f0, nullptr, 1, 0, -1);
+      });
+    });
+    launch(K_TRACE, 0.0, 0.0, [&] { oz::dot_kernel<<<dim3((unsigned)dots.size(), oz::DOT_PARTS), 256, 0, s>>>(dd); });
+    first = next;
+  }
+}
+
 // Runs `specs` in `mode`: complex f64 fronts (DOUBLE), complex f32 fronts under an f64 root
 // (SINGLE), or complex f32 factors refined in FP64 (MIXED). T: front precision, TR: root precision.
 template <typename T, typename TR>
@@ -1303,7 +1471,10 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
         const size_t nblk = (size_t)specs[end].sys->blocks[specs[end].block].nblk;
         const size_t per = c * (nblk * (16 * (GM_M + 1) + 8 * GM_M + 16 + 16 + 8) +
                                 (size_t)(P.sum_ne + P.sum_nb) * 8 + (size_t)P.nl * 16);
-        b += per * (grad ? 2 : 1);
+        // Digits of the slice products: Σ_L, Σ_R, Γ_L and the vectors on the slices.
+        const size_t dig = 2 * oz::pack_a_bytes(P.nl, P.nl) + oz::pack_a_bytes(P.nr, P.nr) +
+                           oz::pack_b_bytes((int)c, P.nl) + oz::pack_b_bytes((int)c, P.nr);
+        b += (per + dig) * (grad ? 2 : 1);
       }
       if (end > begin && bytes + b > ctx->mem_budget) break;
       bytes += b;
@@ -1314,7 +1485,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     std::vector<size_t> arena_off(cj), root_off(cj), fail_off(cj);
     size_t aoff = 0, roff = 0, foff = 0;
     int max_levels = 0;
-    size_t parts_per_job = 1;
+    const size_t parts_per_job = oz::DOT_PARTS;
     for (size_t j = 0; j < cj; ++j) {
       const FrontPlan& P = specs[begin + j].plan->host;
       arena_off[j] = aoff;
@@ -1324,7 +1495,6 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       fail_off[j] = foff;
       foff += P.fronts.size();
       max_levels = std::max(max_levels, P.levels);
-      parts_per_job = std::max(parts_per_job, (size_t)(P.nr + 7) / 8);
     }
     V* arena = static_cast<V*>(ctx->arena.fit(std::max<size_t>(aoff, 1) * vb));
     VR* rarena = static_cast<VR*>(ctx->root_arena.fit(std::max<size_t>(roff, 1) * vr));
@@ -1894,12 +2064,58 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     std::vector<double> th(cj), eh(cj, 0.0);
     std::vector<int32_t> sh(cj, ST_OK), ih(cj, 0);
     if (!mixed) {
-      in_pieces(cj, [&](size_t f0, size_t c) {
-        launch(K_TRACE, trace_flops * c / cj, 0.0, [&] {
-          trace_kernel<TR><<<dim3((unsigned)parts_per_job, (unsigned)c), 256, 0, s>>>(djobs + f0, part + f0 * parts_per_job,
-                                                                                    (int)parts_per_job);
-        });
-      });
+      // Traces Tr[Γ_p G_pq Γ_q G_pq^†] from the root inverses: one pair of slices per two-terminal block, every
+      // pair of leads (or sector labels) of a multi-terminal one.
+      std::vector<TracePair> pairs;
+      std::vector<size_t> midx, mfirst;  // multi-terminal jobs and their first pair's parts
+      size_t mparts = 0;
+      CK(cudaMemsetAsync(part, 0, cj * parts_per_job * sizeof(double), s));
+      if constexpr (std::is_same<TR, double>::value) {
+        const SectorRequest* sec = ctx->sector;
+        for (size_t j = 0; j < cj; ++j) {
+          const JobSpec& sp = specs[begin + j];
+          const FrontPlan& P = sp.plan->host;
+          const SigmaSlot& sg = sp.sys->slots[sp.slot];
+          TracePair t{};
+          t.g = rarena + root_off[j];
+          t.ld = P.fronts[P.root].n;
+          t.status = status + j;
+          t.r0 = P.nd;
+          if (sp.sys->nleads <= 0) {
+            t.gp = sg.gl[sp.block]; t.gq = sg.gr[sp.block];
+            t.np = P.nl; t.nq = P.nr;
+            t.c0 = P.nd + P.rpos;
+            t.part = part + j * parts_per_job;
+            if (t.np && t.nq) pairs.push_back(t);
+            continue;
+          }
+          const bool labels = sec && sp.inst >= 0;
+          const int np = labels ? sec->P : sp.sys->nleads;
+          const std::vector<int32_t>& lp = labels ? sec->hptr[sp.block] : sp.sys->mptr[sp.block];
+          const int32_t* pos = labels ? sec->lpos[sp.block] : sp.sys->dmpos[sp.block];
+          midx.push_back(j);
+          mfirst.push_back(mparts);
+          for (int a = 0; a < np; ++a)
+            for (int b = 0; b < np; ++b) {
+              auto gamma = [&](int q) {
+                return labels ? sec->gam[((size_t)sp.inst * sec->nblocks + sp.block) * sec->P + q]
+                              : (const double2*)sg.mgam[(size_t)sp.block * np + q];
+              };
+              t.gp = gamma(a); t.gq = gamma(b);
+              t.np = lp[a + 1] - lp[a]; t.nq = lp[b + 1] - lp[b];
+              t.rmap = pos + lp[a]; t.cmap = pos + lp[b];
+              t.c0 = P.nd;
+              t.part_at = mparts;
+              mparts += parts_per_job;
+              if (t.np && t.nq) pairs.push_back(t);
+            }
+        }
+        double* mpart = static_cast<double*>(ctx->tr_part.get(std::max<size_t>(mparts, 1) * sizeof(double)));
+        if (mparts) CK(cudaMemsetAsync(mpart, 0, mparts * sizeof(double), s));
+        for (TracePair& t : pairs)
+          if (!t.part) t.part = mpart + t.part_at;
+        trace_pairs(ctx, pairs, trace_flops, launch);
+      }
       launch(K_TRACE, 0.0, 0.0, [&] {
         trace_finish_kernel<<<(unsigned)((cj + 127) / 128), 128, 0, s>>>(part, (int)parts_per_job, (int)cj, tdev, status);
       });
@@ -1918,71 +2134,18 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
                                    cudaMemcpyDeviceToHost, s));
           }
       }
-      // Multi-terminal blocks: every T_pq from the root inverse.
-      std::vector<MultiJob> mj;
-      std::vector<size_t> midx;
-      int64_t smax = 1;
-      int pmax = 0;
-      const SectorRequest* sec = ctx->sector;
-      for (size_t j = 0; j < cj; ++j) {
-        const JobSpec& sp = specs[begin + j];
-        if (sp.sys->nleads <= 0) continue;
-        const bool labels = sec && sp.inst >= 0;
-        const int P = labels ? sec->P : sp.sys->nleads;
-        const std::vector<int32_t>& lp = labels ? sec->hptr[sp.block] : sp.sys->mptr[sp.block];
-        for (int a = 0; a < P; ++a)
-          for (int b = 0; b < P; ++b)
-            smax = std::max<int64_t>(smax, (int64_t)(lp[a + 1] - lp[a]) * (lp[b + 1] - lp[b]));
-        pmax = std::max(pmax, P);
-        MultiJob m{};
-        m.g = rarena + root_off[j];
-        if (labels) {
-          m.lpos = sec->lpos[sp.block];
-          m.lptr = sec->lptr[sp.block];
-          m.gamma = sec->gam[(size_t)sp.inst * sec->nblocks + sp.block];
-        } else {
-          m.lpos = sp.sys->dmpos[sp.block];
-          m.lptr = sp.sys->dmptr[sp.block];
-          m.gamma = sp.sys->slots[sp.slot].mtab[sp.block];
-        }
-        m.m = sp.plan->host.fronts[sp.plan->host.root].n;
-        m.nd = sp.plan->host.nd;
-        m.P = P;
-        mj.push_back(m);
-        midx.push_back(j);
-      }
-      std::vector<double> mh;
-      if (!mj.empty()) {
-        const size_t pairs = (size_t)pmax * pmax;
-        double2* scratch = static_cast<double2*>(ctx->mscratch.get(mj.size() * pairs * smax * sizeof(double2)));
-        double* mout = static_cast<double*>(ctx->mout.get(mj.size() * pairs * sizeof(double)));
-        for (size_t k = 0; k < mj.size(); ++k) {
-          mj[k].scratch = scratch + k * pairs * smax;
-          mj[k].out = mout + k * pairs;
-        }
-        MultiJob* dmj = static_cast<MultiJob*>(ctx->mjobs.get(mj.size() * sizeof(MultiJob)));
-        CK(cudaMemcpyAsync(dmj, mj.data(), mj.size() * sizeof(MultiJob), cudaMemcpyHostToDevice, s));
-        in_pieces(mj.size(), [&](size_t f0, size_t c) {
-          launch(K_TRACE, 0.0, 0.0, [&] {
-            multi_trace_kernel<TR><<<dim3((unsigned)pairs, (unsigned)c), 256, 0, s>>>(dmj + f0, smax);
-          });
-        });
-        mh.resize(mj.size() * pairs);
-        CK(cudaMemcpyAsync(mh.data(), mout, mh.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-        for (size_t k = 0; k < mj.size(); ++k) {
-          JobOut& o = out[begin + midx[k]];
-          o.tm.clear();
-          o.tm.resize((size_t)mj[k].P * mj[k].P);  // filled after the synchronisation below
-        }
-      }
+      std::vector<double> mh(mparts);
+      if (mparts) CK(cudaMemcpyAsync(mh.data(), ctx->tr_part.p, mparts * sizeof(double), cudaMemcpyDeviceToHost, s));
       CK(cudaEventRecord(ctx->ev1, s));
       CK(cudaMemcpyAsync(th.data(), tdev, cj * sizeof(double), cudaMemcpyDeviceToHost, s));
-      if (!mj.empty()) {
+      if (mparts) {
         CK(cudaStreamSynchronize(s));
-        const size_t pairs = (size_t)pmax * pmax;
-        for (size_t k = 0; k < mj.size(); ++k) {
-          JobOut& o = out[begin + midx[k]];
-          for (size_t q = 0; q < o.tm.size(); ++q) o.tm[q] = mh[k * pairs + q];
+        for (size_t k = 0; k < midx.size(); ++k) {  // T[p * P + q]: the pair's partial sums in order
+          const size_t last = k + 1 < midx.size() ? mfirst[k + 1] : mparts, count = (last - mfirst[k]) / parts_per_job;
+          std::vector<double>& tm = out[begin + midx[k]].tm;
+          tm.assign(count, 0.0);
+          for (size_t q = 0; q < count; ++q)
+            for (size_t e = 0; e < parts_per_job; ++e) tm[q] += mh[mfirst[k] + q * parts_per_job + e];
         }
       }
     } else {
@@ -2329,7 +2492,7 @@ int caroli_ctx_create(int device_ordinal, caroli_ctx** out) {
     ctx->mem_budget = free_b / 2;
     int optin = 0;
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_ordinal));
-    for (auto* k : {(const void*)tc_update_kernel, (const void*)tc_sweep_gemm_kernel, (const void*)oz::update_kernel,
+    for (auto* k : {(const void*)tc_update_kernel, (const void*)tc_sweep_gemm_kernel, (const void*)oz::update_kernel, (const void*)oz::gemm_kernel,
                     (const void*)panel_sweep_kernel<double>,
                     (const void*)small_front_kernel<double, false>, (const void*)small_front_kernel<float, false>,
                     (const void*)small_front_kernel<double, true>, (const void*)small_front_kernel<float, true>,
@@ -3170,6 +3333,37 @@ namespace {
 // The device buffers of energy slot `slot` (sized by the blocks' lead slices, W_R for up to nr
 // channels), allocated on first use: uploading the next energy into a slot only copies. The slot
 // is marked unset until its caller has filled it.
+// S = sc Y diag(d) Y^† (n x n, column-major; d on the device): the left factor's digits are written from
+// Y diag(d), the right one's from Y^†. 576 orbitals: 1.8 ms on the FP64 pipe, 0.1 ms here. A wait that runs
+// out sets *status.
+void lead_sigma(caroli_ctx* ctx, const double2* y, int n, const double2* d, double sc, double2* out, int32_t* status) {
+  cudaStream_t s = ctx->stream;
+  const size_t a = oz::pack_a_bytes(n, n), b = oz::pack_b_bytes(n, n), e = oz::pack_e_bytes(n, n);
+  unsigned char* dig = static_cast<unsigned char*>(ctx->tr_dig.get(a + b + 2 * e));
+  oz::PackTask pk[2] = {};
+  for (oz::PackTask& t : pk) {
+    t.p = y; t.ld = n; t.rows = t.k = n;
+  }
+  pk[0].kscale = d;
+  pk[0].dig = dig;
+  pk[0].exp = reinterpret_cast<int32_t*>(dig + a + b);
+  pk[1].conj = pk[1].b = 1;
+  pk[1].dig = dig + a;
+  pk[1].exp = reinterpret_cast<int32_t*>(dig + a + b + e);
+  oz::GemmTask g{};
+  g.a = pk[0].dig; g.ea = pk[0].exp; g.b = pk[1].dig; g.eb = pk[1].exp;
+  g.c = out; g.ldc = g.m = g.n = n; g.chunks = oz::chunks_of(n); g.sign = sc; g.status = status;
+  unsigned char* dt = static_cast<unsigned char*>(ctx->tr_tasks.get(sizeof(pk) + sizeof(g)));
+  CK(cudaMemcpyAsync(dt, pk, sizeof(pk), cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(dt + sizeof(pk), &g, sizeof(g), cudaMemcpyHostToDevice, s));
+  oz::pack_kernel<<<dim3((unsigned)(((size_t)n * oz::chunks_of(n) + 63) / 64), 2), 256, 0, s>>>(
+      reinterpret_cast<const oz::PackTask*>(dt), nullptr, 1, 0);
+  CK(cudaGetLastError());
+  oz::gemm_kernel<<<dim3((unsigned)((n + oz::ROWS - 1) / oz::ROWS), (unsigned)((n + oz::COLS - 1) / oz::COLS), 1), oz::THREADS,
+                    oz::GEMM_SMEM, s>>>(reinterpret_cast<const oz::GemmTask*>(dt + sizeof(pk)), nullptr, 1, 0, -1);
+  CK(cudaGetLastError());
+}
+
 SigmaSlot& slot_buffers(System* sys, int slot) {
   if ((int)sys->slots.size() <= slot) sys->slots.resize(slot + 1);
   SigmaSlot& sg = sys->slots[slot];
@@ -3380,8 +3574,8 @@ int caroli_multi_sector_transmissions(caroli_ctx* ctx, int plan_id, int count, c
     rq.P = P;
     rq.nblocks = nb;
     // Label positions per block: those of the label's lead.
-    std::vector<int32_t> hpos, hptr;
-    std::vector<size_t> pos_off(nb), ptr_off(nb);
+    std::vector<int32_t> hpos;
+    std::vector<size_t> pos_off(nb);
     for (int b = 0; b < nb; ++b) {
       std::vector<int32_t> lp(1, 0);
       pos_off[b] = hpos.size();
@@ -3390,19 +3584,12 @@ int caroli_multi_sector_transmissions(caroli_ctx* ctx, int plan_id, int count, c
         for (int32_t q = sys->mptr[b][p]; q < sys->mptr[b][p + 1]; ++q) hpos.push_back(sys->mpos[b][q]);
         lp.push_back((int32_t)(hpos.size() - pos_off[b]));
       }
-      ptr_off[b] = hptr.size();
-      hptr.insert(hptr.end(), lp.begin(), lp.end());
       rq.hptr.push_back(lp);
     }
     int32_t* dpos = static_cast<int32_t*>(ctx->sec_pos.get(std::max<size_t>(hpos.size(), 1) * sizeof(int32_t)));
-    int32_t* dptr = static_cast<int32_t*>(ctx->sec_ptr.get(std::max<size_t>(hptr.size(), 1) * sizeof(int32_t)));
     if (!hpos.empty()) CK(cudaMemcpyAsync(dpos, hpos.data(), hpos.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(dptr, hptr.data(), hptr.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    for (int b = 0; b < nb; ++b) {
-      rq.lpos.push_back(dpos + pos_off[b]);
-      rq.lptr.push_back(dptr + ptr_off[b]);
-    }
-    // Γ of every (instance, block, label), and per (instance, block) a table of P pointers.
+    for (int b = 0; b < nb; ++b) rq.lpos.push_back(dpos + pos_off[b]);
+    // Γ of every (instance, block, label).
     size_t gel = 0;
     std::vector<size_t> goff((size_t)count * nb * P);
     for (int i = 0; i < count; ++i)
@@ -3413,21 +3600,15 @@ int caroli_multi_sector_transmissions(caroli_ctx* ctx, int plan_id, int count, c
           gel += np * np;
         }
     double2* dg = static_cast<double2*>(ctx->sec_gam.get(std::max<size_t>(gel, 1) * sizeof(double2)));
-    const double2** dtab =
-        static_cast<const double2**>(ctx->sec_tab.get(std::max<size_t>((size_t)count * nb * P, 1) * sizeof(double2*)));
-    std::vector<const double2*> htab((size_t)count * nb * P);
+    rq.gam.resize((size_t)count * nb * P);
     for (int i = 0; i < count; ++i)
       for (int b = 0; b < nb; ++b)
         for (int k = 0; k < P; ++k) {
           const size_t q = ((size_t)i * nb + b) * P + k;
           const size_t np = (size_t)(rq.hptr[b][k + 1] - rq.hptr[b][k]);
-          htab[q] = dg + goff[q];
+          rq.gam[q] = dg + goff[q];
           if (np) CK(cudaMemcpyAsync(dg + goff[q], gammas[q], np * np * sizeof(double2), cudaMemcpyHostToDevice, s));
         }
-    if (!htab.empty())
-      CK(cudaMemcpyAsync(dtab, htab.data(), htab.size() * sizeof(double2*), cudaMemcpyHostToDevice, s));
-    for (int i = 0; i < count; ++i)
-      for (int b = 0; b < nb; ++b) rq.gam.push_back(dtab + ((size_t)i * nb + b) * P);
     CK(cudaStreamSynchronize(s));
     std::vector<JobSpec> specs;
     for (int i = 0; i < count; ++i)
@@ -3664,6 +3845,9 @@ int caroli_sigma_from_modes(caroli_ctx* ctx, int plan_id, int slot, double energ
     double2* dd = static_cast<double2*>(ctx->lead_d.get(2 * (size_t)nmax * sizeof(double2)));
     int32_t* dcols = static_cast<int32_t*>(ctx->lead_cols.get((size_t)nmax * sizeof(int32_t)));
     double* dw = static_cast<double*>(ctx->lead_w.get((size_t)nmax * sizeof(double)));
+    int32_t* dstat = static_cast<int32_t*>(ctx->lead_status.get(sizeof(int32_t)));
+    int32_t hstat = 0;
+    CK(cudaMemsetAsync(dstat, 0, sizeof(int32_t), s));
     for (int b = 0; b < nb; ++b) {
       const FrontPlan& P = sys->plans[b]->host;
       for (int side = 0; side < 2; ++side) {
@@ -3673,9 +3857,7 @@ int caroli_sigma_from_modes(caroli_ctx* ctx, int plan_id, int slot, double energ
         CK(cudaMemcpyAsync(d, side == 0 ? d_left[b] : d_right[b], (size_t)n * sizeof(double2), cudaMemcpyHostToDevice, s));
         double2* S = side == 0 ? sg.sl[b] : sg.sr[b];
         double2* G = side == 0 ? sg.gl[b] : sg.gr[b];
-        const unsigned t = (unsigned)((n + LS_TILE - 1) / LS_TILE);
-        lead_sigma_kernel<<<dim3(t, t), 256, 0, s>>>(sys->lead_y[side][b], n, d, sys->lead_sc[side][b], S);
-        CK(cudaGetLastError());
+        lead_sigma(ctx, sys->lead_y[side][b], n, d, sys->lead_sc[side][b], S, dstat);
         lead_gamma_kernel<<<(unsigned)(((int64_t)n * n + 255) / 256), 256, 0, s>>>(S, n, G);
         CK(cudaGetLastError());
       }
@@ -3689,7 +3871,9 @@ int caroli_sigma_from_modes(caroli_ctx* ctx, int plan_id, int slot, double energ
       }
       sg.channels[b] = nc;
       // The host vectors of this block must outlive the copies: synchronise per block.
+      CK(cudaMemcpyAsync(&hstat, dstat, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
+      if (hstat) return fail_with(ctx, CAROLI_ECUDA, "caroli_sigma_from_modes: a device wait ran out");
     }
     sg.energy = energy;
     sg.set = true;

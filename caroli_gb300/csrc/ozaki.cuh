@@ -106,11 +106,11 @@ template <int LPR> __device__ __forceinline__ int row_exponent(const double2 (&a
 // a 16-byte core-matrix row.
 template <int LPR>
 __device__ __forceinline__ void write_a(unsigned char* oa, int32_t* ea, int q, int h, bool act,
-                                        const double2 (&a)[GJ_KB / LPR]) {
+                                        const double2 (&a)[GJ_KB / LPR], size_t tile_stride = A_TILE) {
   const int e = row_exponent<LPR>(a);
   if (!act) return;
   if (h == 0) ea[q] = e == 0x7ff ? NOT_FINITE : e;
-  unsigned char* tile = oa + (size_t)(q / ROWS) * A_TILE;
+  unsigned char* tile = oa + (size_t)(q / ROWS) * tile_stride;
 #pragma unroll
   for (int i = 0; i < GJ_KB / LPR; ++i) {
     int re[S], im[S];
@@ -125,11 +125,11 @@ __device__ __forceinline__ void write_a(unsigned char* oa, int32_t* ea, int q, i
 // Column r of B' (rows 2r and 2r + 1) from LPR lanes, laid out over the lanes as in write_a.
 template <int LPR>
 __device__ __forceinline__ void write_b(unsigned char* ob, int32_t* eb, int r, int h, bool act,
-                                        const double2 (&y)[GJ_KB / LPR]) {
+                                        const double2 (&y)[GJ_KB / LPR], size_t tile_stride = B_TILE) {
   const int e = row_exponent<LPR>(y);
   if (!act) return;
   if (h == 0) eb[r] = e == 0x7ff ? NOT_FINITE : e;
-  unsigned char* tile = ob + (size_t)(r / COLS) * B_TILE;
+  unsigned char* tile = ob + (size_t)(r / COLS) * tile_stride;
   const int row = 2 * (r % COLS);
 #pragma unroll
   for (int i = 0; i < GJ_KB / LPR; ++i) {
@@ -188,6 +188,19 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
                : "memory");
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The products of a tile's digits (one thread): one MMA per digit i of A' and K-slice, N = 32 (7 - i).
+__device__ __forceinline__ void mma_tile(uint32_t acc, const unsigned char* sa, const unsigned char* sb) {
+  const uint32_t pb = tc::smem_addr(sb);
+#pragma unroll
+  for (int i = 0; i < S; ++i) {
+    const uint32_t pa = tc::smem_addr(sa + i * A_SLICE);
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+      mma_f16(acc + (uint32_t)(i * 2 * COLS), tc::smem_desc(pa + ks * ROWS * 32, 128, 256),
+              tc::smem_desc(pb + ks * B_ROWS * 32, 128, 256), idesc_f16(ROWS, 2 * COLS * (S - i)), i > 0 || ks > 0);
+  }
 }
 
 // The update of one panel (operands written by panel_rest_kernel). A CTA takes 128 rows of a matrix and
@@ -262,15 +275,7 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
         if (!tc::mbar_wait(&bfull[st], (uint32_t)((ct / STAGES) & 1), TCU_WAIT)) { fail(); break; }
         if (ct >= 2 && !tc::mbar_wait(&tempty[a], (uint32_t)(((ct >> 1) - 1) & 1), TCU_WAIT)) { fail(); break; }
         tc::fence_after_sync();
-        // One MMA per digit i of A' and K-slice: N = 32 (7 - i).
-#pragma unroll
-        for (int i = 0; i < S; ++i) {
-          const uint32_t pa = tc::smem_addr(sa + i * A_SLICE), pb = tc::smem_addr(sb + st * B_TILE);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            mma_f16(tbase + (uint32_t)(a * ACC + i * 2 * COLS), tc::smem_desc(pa + ks * ROWS * 32, 128, 256),
-                    tc::smem_desc(pb + ks * B_ROWS * 32, 128, 256), idesc_f16(ROWS, 2 * COLS * (S - i)), i > 0 || ks > 0);
-        }
+        mma_tile(tbase + (uint32_t)(a * ACC), sa, sb + st * B_TILE);
         tc::mma_commit(&bempty[st]);
         tc::mma_commit(&tfull[a]);
         ++mma_tiles;

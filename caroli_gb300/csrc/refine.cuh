@@ -70,7 +70,7 @@ struct RefineDesc {
   // left slice, the others by W_R on the right slice; cl = 0 for a transmission.
   const double2* w_l;
   int32_t cl, pad2;
-  // Γ_L x_L of the current x (nl x c, column-major), formed by slice_gemm_kernel for the check.
+  // Γ_L x_L of the current x (nl x c, column-major), formed by a slice product (ozgemm.cuh) for the check.
   double2* gx;
 };
 
@@ -101,7 +101,7 @@ __device__ __forceinline__ float2* sweep_dst(const RefineDesc& R, int dst) {
 }
 
 // x += d, then the FP64 residual r = B - A x of every row: grid (jobs, row chunks of 256). The
-// residual kernel applies B - (z - H) x; the slices' Σ x follow as slice_gemm_kernel launches.
+// residual kernel applies B - (z - H) x; the slices' Σ x follow as slice products (ozgemm.cuh).
 __global__ void __launch_bounds__(256) refine_update_kernel(RefineDesc* __restrict__ rd) {
   RefineDesc& R = rd[blockIdx.x];
   if (R.done) return;
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(256) refine_residual_kernel(RefineDesc* __rest
     acc.x -= R.energy * xj[i].x;
     acc.y -= R.energy * xj[i].y;
     for (int q = R.csr_ptr[i]; q < R.csr_ptr[i + 1]; ++q) acc = cfma(acc, R.vals[R.csr_q[q]], xj[R.csr_col[q]]);
-    R.r[i + (int64_t)j * R.nblk] = acc;  // + Σ_L x + Σ_R x on the slices: slice_gemm_kernel
+    R.r[i + (int64_t)j * R.nblk] = acc;  // + Σ_L x + Σ_R x on the slices: slice products
   }
 }
 
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(256) gm_start_kernel(RefineDesc* __restrict__ 
 }
 
 // w = A z_k into V_{k+1}, A = z - H - Σ_L - Σ_R in FP64: z - H here, grid (jobs, row chunks of
-// 256); the dense Σ blocks of the slices follow as slice_gemm_kernel launches.
+// 256); the dense Σ blocks of the slices follow as slice products (ozgemm.cuh).
 __global__ void __launch_bounds__(256) gm_matvec_kernel(RefineDesc* __restrict__ rd, const int32_t* __restrict__ jl,
                                                         int k) {
   const RefineDesc& R = rd[jl[blockIdx.x]];
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(256) gm_matvec_kernel(RefineDesc* __restrict__
     acc.x *= R.energy;
     acc.y *= R.energy;
     for (int q = R.csr_ptr[i]; q < R.csr_ptr[i + 1]; ++q) acc = cfms(acc, R.vals[R.csr_q[q]], zd(R.csr_col[q]));
-    W[i + (int64_t)j * R.nblk] = acc;  // - Σ_L z - Σ_R z on the slices: slice_gemm_kernel
+    W[i + (int64_t)j * R.nblk] = acc;  // - Σ_L z - Σ_R z on the slices: slice products
   }
 }
 
@@ -500,180 +500,6 @@ __global__ void gm_residual_kernel(RefineDesc* __restrict__ rd, int njobs) {
 }  // namespace caroli
 
 namespace caroli {
-
-// ---- Dense slice products --------------------------------------------------------------------
-// The lead blocks of A (Σ_L, Σ_R: m x m, dense, on the slices' orbitals) and Γ_L of the trace,
-// applied to the c right-hand-side columns of a job at once: for i < m, j < c,
-//     out[orow[i] + j ldo] = (accumulate ? out : 0) + sign Σ_a S(i, a) in[irow[a] + j ldi],
-// S(i, a) = S[i + a m], or conj(S[a + i m]) for the adjoint solve. A batched complex FP64 GEMM:
-// 64 x 32 output tiles, K in steps of 16 staged in shared memory, a 4 x 2 complex tile per thread;
-// with hundreds of channels (a 32 x 32-site lead) these products carry most of the refinement's
-// FP64 work.
-struct SliceTask {
-  const RefineDesc* rd;  // skipped once the job is done (mode 0: or its inner solve is done)
-  const double2* s;
-  const int32_t* irow;   // rows of the input (block-local), m entries
-  const int32_t* orow;   // rows of the output, m entries; null: row i
-  const void* in;        // double2, or float2 with in_f32
-  double2* out;
-  int64_t ldi, ldo;
-  int32_t m, c, adj, in_f32, mode, accumulate;
-  double sign;
-};
-
-constexpr int SG_ROWS = 64, SG_COLS = 32, SG_K = 16;
-
-// Both slice kernels take the tasks of the jobs in `jl` (a job's task is tasks[job]).
-__global__ void __launch_bounds__(256) slice_gemm_kernel(const SliceTask* __restrict__ tasks,
-                                                         const int32_t* __restrict__ jl) {
-  __shared__ double2 As[SG_K][SG_ROWS];
-  __shared__ double2 Bs[SG_K][SG_COLS];
-  const SliceTask t = tasks[jl[blockIdx.z]];
-  const RefineDesc& R = *t.rd;
-  if (R.done || (t.mode == 0 && R.inner_done)) return;
-  const int i0 = blockIdx.x * SG_ROWS, j0 = blockIdx.y * SG_COLS;
-  if (i0 >= t.m || j0 >= t.c) return;
-  const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4;
-  // Three real products per complex one (the 3M form): p1 = Σ ar br, p2 = Σ ai bi,
-  // p3 = Σ (ar + ai)(br + bi); the product is (p1 - p2, p3 - p1 - p2). A quarter fewer FP64
-  // multiply-adds than the four-product form on a part bound by the FP64 pipe.
-  double p1[4][2], p2[4][2], p3[4][2];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int q = 0; q < 2; ++q) p1[r][q] = p2[r][q] = p3[r][q] = 0.0;
-  for (int k0 = 0; k0 < t.m; k0 += SG_K) {
-    // S tile: rows i0.., columns k0.. (coalesced along the stored dimension).
-    for (int e = tid; e < SG_ROWS * SG_K; e += 256) {
-      int ii, kk;
-      if (t.adj) { kk = e % SG_K; ii = e / SG_K; }
-      else { ii = e % SG_ROWS; kk = e / SG_ROWS; }
-      const int i = i0 + ii, k = k0 + kk;
-      double2 v = make_double2(0.0, 0.0);
-      if (i < t.m && k < t.m) {
-        if (t.adj) { v = t.s[k + (int64_t)i * t.m]; v.y = -v.y; }
-        else v = t.s[i + (int64_t)k * t.m];
-      }
-      As[kk][ii] = v;
-    }
-    // Input tile: rows irow[k0..], columns j0.. (coalesced along the rows).
-    for (int e = tid; e < SG_K * SG_COLS; e += 256) {
-      const int kk = e % SG_K, jj = e / SG_K;
-      const int k = k0 + kk, j = j0 + jj;
-      double2 v = make_double2(0.0, 0.0);
-      if (k < t.m && j < t.c) {
-        const int64_t q = t.irow[k] + (int64_t)j * t.ldi;
-        if (t.in_f32) {
-          const float2 f = static_cast<const float2*>(t.in)[q];
-          v = make_double2((double)f.x, (double)f.y);
-        } else {
-          v = static_cast<const double2*>(t.in)[q];
-        }
-      }
-      Bs[kk][jj] = v;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int kk = 0; kk < SG_K; ++kk) {
-      double2 a[4], b[2];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = As[kk][ti + 16 * r];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) b[q] = Bs[kk][tj + 16 * q];
-      double as[4], bs[2];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) as[r] = a[r].x + a[r].y;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) bs[q] = b[q].x + b[q].y;
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          p1[r][q] = fma(a[r].x, b[q].x, p1[r][q]);
-          p2[r][q] = fma(a[r].y, b[q].y, p2[r][q]);
-          p3[r][q] = fma(as[r], bs[q], p3[r][q]);
-        }
-    }
-    __syncthreads();
-  }
-  double2 acc[4][2];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int q = 0; q < 2; ++q) acc[r][q] = make_double2(p1[r][q] - p2[r][q], p3[r][q] - p1[r][q] - p2[r][q]);
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + ti + 16 * r;
-    if (i >= t.m) continue;
-    const int64_t orow = t.orow ? t.orow[i] : i;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int j = j0 + tj + 16 * q;
-      if (j >= t.c) continue;
-      double2& o = t.out[orow + (int64_t)j * t.ldo];
-      const double2 v = make_double2(t.sign * acc[r][q].x, t.sign * acc[r][q].y);
-      if (t.accumulate) { o.x += v.x; o.y += v.y; }
-      else o = v;
-    }
-  }
-}
-
-// The same products for jobs with few columns (at most CB, the ribbons' few channels): a thread per
-// output row holding its CB sums, the input rows of a K step staged in shared memory. A 64 x 32
-// tile would leave most of its columns empty there. grid (row chunks of 128, tasks), 128 threads.
-template <int CB>
-__global__ void __launch_bounds__(128) slice_rows_kernel(const SliceTask* __restrict__ tasks,
-                                                         const int32_t* __restrict__ jl) {
-  constexpr int KS = 64;
-  __shared__ double2 Xs[KS][CB];
-  const SliceTask t = tasks[jl[blockIdx.y]];
-  const RefineDesc& R = *t.rd;
-  if (R.done || (t.mode == 0 && R.inner_done)) return;
-  const int i0 = blockIdx.x * 128;
-  if (i0 >= t.m) return;
-  const int i = i0 + threadIdx.x;
-  double2 acc[CB];
-#pragma unroll
-  for (int j = 0; j < CB; ++j) acc[j] = make_double2(0.0, 0.0);
-  for (int k0 = 0; k0 < t.m; k0 += KS) {
-    for (int e = threadIdx.x; e < KS * CB; e += 128) {
-      const int kk = e % KS, j = e / KS, k = k0 + kk;
-      double2 v = make_double2(0.0, 0.0);
-      if (k < t.m && j < t.c) {
-        const int64_t q = t.irow[k] + (int64_t)j * t.ldi;
-        if (t.in_f32) {
-          const float2 f = static_cast<const float2*>(t.in)[q];
-          v = make_double2((double)f.x, (double)f.y);
-        } else {
-          v = static_cast<const double2*>(t.in)[q];
-        }
-      }
-      Xs[kk][j] = v;
-    }
-    __syncthreads();
-    if (i < t.m) {
-      const int k1 = min(KS, t.m - k0);
-      for (int kk = 0; kk < k1; ++kk) {
-        double2 a;
-        if (t.adj) { a = t.s[(k0 + kk) + (int64_t)i * t.m]; a.y = -a.y; }
-        else a = t.s[i + (int64_t)(k0 + kk) * t.m];
-#pragma unroll
-        for (int j = 0; j < CB; ++j) acc[j] = cfma(acc[j], a, Xs[kk][j]);
-      }
-    }
-    __syncthreads();
-  }
-  if (i >= t.m) return;
-  const int64_t orow = t.orow ? t.orow[i] : i;
-#pragma unroll
-  for (int j = 0; j < CB; ++j) {
-    if (j >= t.c) break;
-    double2& o = t.out[orow + (int64_t)j * t.ldo];
-    const double2 v = make_double2(t.sign * acc[j].x, t.sign * acc[j].y);
-    if (t.accumulate) { o.x += v.x; o.y += v.y; }
-    else o = v;
-  }
-}
 
 // Transmission matrix t = W_L^† x_L of each job after its refinement (x = G W_R): t is
 // cl x c column-major, W_L nl x cl. grid (jobs), threads over the entries of t.

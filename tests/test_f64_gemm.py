@@ -1,0 +1,50 @@
+"""The FP64 GEMMs on the tensor cores (traces, slice products, lead self-energies) at the edges of their
+tiles (16 columns, 32 inner entries, 128 rows), against a dense solve in numpy.
+
+A two-slice square device of width W has slices of W orbitals and no tree: its trace multiplies W x W
+blocks, the refined solve multiplies Σ with as many columns as the right lead has open channels, and the
+self-energies formed on the device are W x W x W products."""
+import numpy as np
+import pytest
+
+from caroli_gb300 import NestedTwoTerminal, Precision, Region, square
+from caroli_gb300.disorder import ScalarPotential
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+
+
+def _dense_transmission(s, sigma):
+    y = s.system
+    h = np.zeros((y.n, y.n), complex)
+    h[np.repeat(np.arange(y.n), np.diff(y.row_ptr)), y.cols.astype(int)] = y.values[0]
+    a = sigma.energy * np.eye(y.n) - h
+    blk, (sl, sr) = y.blocks[0], sigma.blocks[0]
+    a[np.ix_(blk.left, blk.left)] -= sl
+    a[np.ix_(blk.right, blk.right)] -= sr
+    g = np.linalg.inv(a)[np.ix_(blk.left, blk.right)]
+    gl, gr = 1j * (sl - sl.conj().T), 1j * (sr - sr.conj().T)
+    return np.trace(gl @ g @ gr @ g.conj().T).real, np.linalg.cond(a)
+
+
+# Widths around one and two tiles of every kind; lengths 1 (one slice that is both) and 2.
+@pytest.mark.parametrize("length,width", [(2, 1), (2, 15), (2, 16), (2, 17), (2, 31), (2, 32), (2, 33), (2, 64), (1, 33),
+                                          (2, 96), (2, 127), (2, 128), (2, 129), (2, 161)])
+def test_transmission_against_dense(length, width):
+    clean = square()
+    region = Region.cuboid(clean.lattice, [length, width, 0])
+    pot = np.random.RandomState(width).uniform(-0.7, 0.7, length * width)
+    s = NestedTwoTerminal.from_model(clean.with_onsite_term(ScalarPotential(pot, width, 1, 1)), clean, region, 0)
+    sigma = s.self_energies(0.37)
+    ref, cond = _dense_transmission(s, sigma)
+    # n eps cond(A) for G, twice for |G|^2, against at most one per channel.
+    bound = 4 * length * width * EPS * cond * width
+    assert abs(s.transmission_with(sigma) - ref) <= bound
+    on_device = s.self_energies_on_device(0.37)
+    assert abs(s.transmission_with(on_device) - ref) <= bound
+    s.plan().ctx.set_mixed_max_channels(1000)
+    try:
+        assert abs(s.transmission_with_precision(sigma, Precision.MIXED) - ref) <= 1e-8 + bound
+        assert abs(s.transmission_with_precision(on_device, Precision.MIXED) - ref) <= 1e-8 + bound
+    finally:
+        s.plan().ctx.set_mixed_max_channels()

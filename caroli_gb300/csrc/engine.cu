@@ -81,7 +81,19 @@ struct DevPlan {
   int32_t* vidx = nullptr;
   SweepRow* srows = nullptr;
   size_t oz_bytes = 0;  // FP64 update operands: of its largest level, or of the root
+  // Tree fronts level by level, largest first (ties by index): those of level L from level_at[L] on.
+  std::vector<int32_t> by_size;
+  std::vector<size_t> level_at;
   void upload(cudaStream_t s) {
+    by_size.resize(host.fronts.size() - 1);
+    std::iota(by_size.begin(), by_size.end(), 0);
+    std::stable_sort(by_size.begin(), by_size.end(), [&](int32_t a, int32_t b) {
+      const FrontDesc &x = host.fronts[a], &y = host.fronts[b];
+      return x.level != y.level ? x.level < y.level : x.n > y.n;
+    });
+    level_at.assign((size_t)host.levels + 1, by_size.size());
+    for (size_t q = by_size.size(); q-- > 0;)
+      for (int L = host.fronts[by_size[q]].level; L >= 0 && level_at[L] > q; --L) level_at[L] = q;
     std::vector<size_t> per(std::max(1, host.levels), 0);
     for (size_t k = 0; k + 1 < host.fronts.size(); ++k) {
       const FrontDesc& f = host.fronts[k];
@@ -116,6 +128,7 @@ struct DevPlan {
 struct SigmaSlot {
   double energy = 0.0;
   bool set = false;
+  double2* base = nullptr;                   // one allocation for the matrices below
   std::vector<double2*> sl, sr, gl, gr, wr;  // per block, device
   std::vector<int> channels;                // columns of W_R per block
   // Multi-terminal systems: Γ_p of every (block, lead), and per block a device table of the P
@@ -179,7 +192,8 @@ struct System {
     cudaFree(vals);
     cudaFree(dvals);
     for (auto& s : slots) {
-      for (auto* v : {&s.sl, &s.sr, &s.gl, &s.gr, &s.wr, &s.mgam, &s.mw})
+      cudaFree(s.base);
+      for (auto* v : {&s.mgam, &s.mw})
         for (auto* p : *v) cudaFree(p);
       for (auto* p : s.mtab) cudaFree(p);
     }
@@ -259,6 +273,11 @@ struct RefineBufs {
   Buf segs, ctasks, ccount, cjobs, ojobs;  // task and job lists compacted to the solves still iterating
   Buf tg_fr, tg_tasks, tg_stage;    // tensor-core sweeps of many-column solves (tcgemm.cuh)
   // The vectors (one column per channel; the bulk of a mixed batch's memory besides the fronts).
+  size_t vector_bytes() const {
+    size_t sum = 0;
+    for (const Buf* b : {&rx, &rr, &rd, &rtb, &rhb, &rgx, &gV, &gZ, &tg_stage, &sdig, &svec}) sum += b->bytes;
+    return sum;
+  }
   void release_vectors() {
     for (Buf* b : {&rx, &rr, &rd, &rtb, &rhb, &rgx, &gV, &gZ, &tg_stage, &sdig, &svec}) b->release();
   }
@@ -378,11 +397,14 @@ struct caroli_ctx {
   double factor_ms = 0.0, root_ms = 0.0, tail_ms = 0.0;
   std::string err;
   std::vector<std::unique_ptr<System>> systems;
-  Buf arena, root_arena, jobs, tasks, fail, status, tout, part, pert;
+  Buf arena, root_arena, jobs, fail, status, tout, part, pert;
   RefineBufs rb[2];  // forward and adjoint refinement state
-  Buf inv, ipiv, iy, ibt, iscale, ibad, ioz, ipp;
+  Buf ipiv, iy, ibt, iscale, ibad, ioz, ipp;
   int max_cluster = 8;  // CTAs per cluster a panel sweep may use (16 where the GPU schedules them)
-  TaskCache tcache;
+  // Task lists and their device copies, f32 and f64 fronts apart: a mixed batch whose last solves are
+  // recomputed in FP64 finds its own lists again on the next call.
+  TaskCache tcache[2];
+  Buf tasks[2], inv[2];
   Buf grhs, gptr, gdv, gdp;
   Buf states_w;  // lead factors W_L, W_R of a scattering-states call
   Buf states_rhs;  // multi-terminal sources
@@ -728,7 +750,7 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
   size_t root_fr0 = 0, root_nfr = 0, root_t0 = 0;
   int root_m = 1;
   if (wide) {
-    const std::vector<Task>& htasks = ctx->tcache.tasks;
+    const std::vector<Task>& htasks = ctx->tcache[0].tasks;
     std::vector<TGFront> frs;
     std::vector<TGTask> tgs;
     std::vector<size_t> stage_off_f, stage_off_b;  // per entry of frs (forward and backward stages)
@@ -1451,10 +1473,6 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
   const bool mixed = mode == MODE_MIXED;
   out.assign(nj, JobOut{});
   Launcher launch{ctx, s};
-  // The memory budget of a batch covers its fronts and, in mixed precision, its refinement vectors;
-  // a batch without refinement gives the idle vectors of an earlier mixed batch back first.
-  if (!mixed)
-    for (RefineBufs& b : ctx->rb) b.release_vectors();
   size_t begin = 0;
   while (begin < nj) {
     // Chunk of jobs within the memory budget: the fronts and, in mixed precision, the refinement's
@@ -1496,8 +1514,29 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       foff += P.fronts.size();
       max_levels = std::max(max_levels, P.levels);
     }
-    V* arena = static_cast<V*>(ctx->arena.fit(std::max<size_t>(aoff, 1) * vb));
-    VR* rarena = static_cast<VR*>(ctx->root_arena.fit(std::max<size_t>(roff, 1) * vr));
+    // The memory budget of a batch covers its fronts and, in mixed precision, its refinement vectors. What an
+    // earlier batch left (larger fronts, vectors a batch without refinement does not need) is kept while it
+    // fits the same budget, and given back otherwise or when an allocation fails: a mixed batch with a few
+    // solves recomputed in FP64 paid 120 ms a call for freeing and allocating 25 GB (256 block solves).
+    const size_t need_a = std::max<size_t>(aoff, 1) * vb, need_r = std::max<size_t>(roff, 1) * vr;
+    size_t vectors = ctx->rb[0].vector_bytes() + ctx->rb[1].vector_bytes();
+    if (mixed && bytes > need_a + need_r) vectors = std::max(vectors, bytes - need_a - need_r);
+    const bool keep = std::max(ctx->arena.bytes, need_a) + std::max(ctx->root_arena.bytes, need_r) + ctx->ioz.bytes +
+                          vectors <= ctx->mem_budget;
+    if (!mixed && !keep)
+      for (RefineBufs& b : ctx->rb) b.release_vectors();
+    auto room = [&](Buf& b, size_t need) -> void* {
+      if (!keep) return b.fit(need);
+      try {
+        return b.get(need);
+      } catch (const CudaError&) {
+        if (mixed) throw;
+        for (RefineBufs& v : ctx->rb) v.release_vectors();
+        return b.get(need);
+      }
+    };
+    V* arena = static_cast<V*>(room(ctx->arena, need_a));
+    VR* rarena = static_cast<VR*>(room(ctx->root_arena, need_r));
     uint8_t* fail = static_cast<uint8_t*>(ctx->fail.get(std::max<size_t>(foff, 1)));
     int32_t* status = static_cast<int32_t*>(ctx->status.get(cj * sizeof(int32_t)));
     int* pert = static_cast<int*>(ctx->pert.get(cj * sizeof(int)));
@@ -1529,7 +1568,8 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     // Built once per distinct batch (the plans of the chunk, precisions and arena addresses) and
     // kept with its device copies: a repeated batch reuses them without host work.
     using Level = TaskLevel;
-    TaskCache& tc = ctx->tcache;
+    constexpr int prec = sizeof(T) == 8 ? 1 : 0;
+    TaskCache& tc = ctx->tcache[prec];
     const int small_max = sizeof(T) == 8 ? SMALL_MAX_F64 : ctx->small_max_f32;
     // Split Schur update: the panel sweeps transform only the pivot columns, then one tensor-core
     // GEMM per front forms [X; S] = [F11^-1; W] F12 + [0; F22] (f32 fronts below the root).
@@ -1589,51 +1629,52 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       Level& lv = levels[L];
       lv = Level{};
       scratch_reset();
-      lv.tiny0 = tasks.size();
-      for (size_t j = 0; j < cj; ++j) {
-        const auto& fr = specs[begin + j].plan->host.fronts;
-        const FrontDesc* dfr = specs[begin + j].plan->fronts;
-        for (size_t k = 0; k + 1 < fr.size(); ++k)
-          if (fr[k].level == L && fr[k].n <= TINY_MAX) {
-            tasks.push_back({(int32_t)j, (int32_t)k, dfr + k});
-            const double ne = fr[k].ne, nb = fr[k].n - fr[k].ne;
-            lv.tiny_flops += 8.0 / 3 * ne * ne * ne + 8 * ne * ne * nb + 8 * nb * nb * ne;
-            lv.max_tiny_n = std::max(lv.max_tiny_n, fr[k].n);
-            lv.tiny_bytes += ((double)fr[k].n * fr[k].n + (mixed ? (double)fr[k].n * fr[k].n : nb * nb)) * vb;
+      // The level's fronts with lo < n <= hi of every job, largest first: the eight warps of a tiny-front CTA get
+      // fronts of about one size (a CTA lasts as long as its largest front), and the longest CTAs start first.
+      auto collect = [&](int lo, int hi, auto fn) {
+        std::vector<size_t> at(cj), end(cj);
+        for (size_t j = 0; j < cj; ++j) {
+          const DevPlan& P = *specs[begin + j].plan;
+          const auto& fr = P.host.fronts;
+          const size_t l0 = L < P.host.levels ? P.level_at[L] : P.by_size.size();
+          end[j] = L < P.host.levels ? P.level_at[L + 1] : l0;
+          at[j] = (size_t)(std::partition_point(P.by_size.begin() + l0, P.by_size.begin() + end[j],
+                                                [&](int32_t k) { return fr[k].n > hi; }) - P.by_size.begin());
+        }
+        for (int n = hi; n > lo; --n)
+          for (size_t j = 0; j < cj; ++j) {
+            const DevPlan& P = *specs[begin + j].plan;
+            for (; at[j] < end[j] && P.host.fronts[P.by_size[at[j]]].n == n; ++at[j]) {
+              const int32_t k = P.by_size[at[j]];
+              tasks.push_back({(int32_t)j, k, P.fronts + k});
+              fn(P.host.fronts[k]);
+            }
           }
-      }
-      lv.tiny_n = tasks.size() - lv.tiny0;
-      // Largest fronts first: the eight warps of a tiny-front CTA get fronts of about one size (a
-      // CTA lasts as long as its largest front), and the longest CTAs start first.
-      auto by_size = [&](size_t a0, size_t a1) {
-        std::stable_sort(tasks.begin() + a0, tasks.begin() + a1, [&](const Task& x, const Task& y) {
-          return specs[begin + x.job].plan->host.fronts[x.front].n > specs[begin + y.job].plan->host.fronts[y.front].n;
-        });
       };
-      by_size(lv.tiny0, tasks.size());
+      lv.tiny0 = tasks.size();
+      collect(-1, TINY_MAX, [&](const FrontDesc& f) {
+        const double ne = f.ne, nb = f.n - f.ne;
+        lv.tiny_flops += 8.0 / 3 * ne * ne * ne + 8 * ne * ne * nb + 8 * nb * nb * ne;
+        lv.max_tiny_n = std::max(lv.max_tiny_n, f.n);
+        lv.tiny_bytes += ((double)f.n * f.n + (mixed ? (double)f.n * f.n : nb * nb)) * vb;
+      });
+      lv.tiny_n = tasks.size() - lv.tiny0;
       lv.small0 = tasks.size();
       const int bucket_hi[3] = {48, 64, small_max};
       for (int b = 0; b < 3; ++b) {
         const int lo = b == 0 ? TINY_MAX : bucket_hi[b - 1], hi = bucket_hi[b];
         lv.sb0[b] = tasks.size();
-        for (size_t j = 0; j < cj; ++j) {
-          const auto& fr = specs[begin + j].plan->host.fronts;
-          const FrontDesc* dfr = specs[begin + j].plan->fronts;
-          for (size_t k = 0; k + 1 < fr.size(); ++k)
-            if (fr[k].level == L && fr[k].n > lo && fr[k].n <= hi) {
-              tasks.push_back({(int32_t)j, (int32_t)k, dfr + k});
-              const double ne = fr[k].ne, nb = fr[k].n - fr[k].ne;
-              lv.max_small_n = std::max(lv.max_small_n, fr[k].n);
-              lv.max_small_ne = std::max(lv.max_small_ne, fr[k].ne);
-              lv.sb_n[b] = std::max(lv.sb_n[b], fr[k].n);
-              lv.sb_ne[b] = std::max(lv.sb_ne[b], fr[k].ne);
-              lv.small_flops += 8.0 / 3 * ne * ne * ne + 8 * ne * ne * nb + 8 * nb * nb * ne;
-              // The front written (mixed keeps all of it, else S) and the children's blocks read.
-              lv.small_bytes += ((double)fr[k].n * fr[k].n + (mixed ? (double)fr[k].n * fr[k].n : nb * nb)) * vb;
-            }
-        }
+        collect(lo, hi, [&](const FrontDesc& f) {
+          const double ne = f.ne, nb = f.n - f.ne;
+          lv.max_small_n = std::max(lv.max_small_n, f.n);
+          lv.max_small_ne = std::max(lv.max_small_ne, f.ne);
+          lv.sb_n[b] = std::max(lv.sb_n[b], f.n);
+          lv.sb_ne[b] = std::max(lv.sb_ne[b], f.ne);
+          lv.small_flops += 8.0 / 3 * ne * ne * ne + 8 * ne * ne * nb + 8 * nb * nb * ne;
+          // The front written (mixed keeps all of it, else S) and the children's blocks read.
+          lv.small_bytes += ((double)f.n * f.n + (mixed ? (double)f.n * f.n : nb * nb)) * vb;
+        });
         lv.sbn[b] = tasks.size() - lv.sb0[b];
-        by_size(lv.sb0[b], tasks.size());
         if (hi >= small_max) break;
       }
       lv.small_n = tasks.size() - lv.small0;
@@ -1642,70 +1683,72 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       lv.f12_0 = tc.f12.size();
       lv.sg0 = tc.sgt.size();
       for (size_t j = 0; j < cj; ++j) {
-        const auto& fr = specs[begin + j].plan->host.fronts;
-        const FrontDesc* dfr = specs[begin + j].plan->fronts;
-        for (size_t k = 0; k + 1 < fr.size(); ++k)
-          if (fr[k].level == L && fr[k].n > small_max) {
-            tasks.push_back({(int32_t)j, (int32_t)k, dfr + k});
-            const double ne = fr[k].ne, nb = fr[k].n - fr[k].ne;
-            lv.max_large_n = std::max(lv.max_large_n, fr[k].n);
-            lv.max_large_ne = std::max(lv.max_large_ne, fr[k].ne);
-            lv.inv_flops += 8.0 / 3 * ne * ne * ne;
-            lv.gemm0_flops += 8 * ne * ne * nb;
-            lv.gemm1_flops += 8 * nb * nb * ne;
-            const double ncol = split ? ne : (double)fr[k].n;  // columns the sweep transforms
-            for (int k0 = 0; k0 < fr[k].ne; k0 += GJ_KB) {
-              const double kb = std::min(GJ_KB, fr[k].ne - k0), nn = fr[k].n;
-              // complex rows x kb times kb x columns, the updated block read and written: every row and the
-              // rest columns, or (FP64 fronts, trail form) the rows and columns after the panel.
-              const double ur = vb == sizeof(double2) ? nn - k0 - kb : nn, uc = vb == sizeof(double2) ? ur : ncol - kb;
-              lv.upd_flops += 8.0 * ur * uc * kb;
-              lv.upd_bytes += 2.0 * ur * uc * vb;
-              lv.pan_flops += 8.0 * (vb == sizeof(double2) ? nn - k0 : nn) * kb * kb;
-            }
-            if (split) {
-              lv.upd_flops += 8.0 * fr[k].n * ne * nb;                           // [X; S] = [F11^-1; W] F12
-              lv.upd_bytes += ((double)fr[k].n * ne + 3.0 * ne * nb + 2.0 * nb * nb) * vb;  // A, F12 twice, X, F22
-            }
-            lv.asm_bytes += (double)fr[k].n * fr[k].n * vb;
-            if (fr[k].ne > 0) {
-              InvTask it{};
-              it.a = arena + arena_off[j] + fr[k].arena_off;
-              it.ld = fr[k].n;
-              it.n = fr[k].n;
-              it.npiv = fr[k].ne;
-              it.ncol = split ? fr[k].ne : fr[k].n;
-              it.job = (int32_t)j;
-              it.front = (int32_t)k;
-              if (split && fr[k].n > fr[k].ne) {
-                const int fne = fr[k].ne, fnb = fr[k].n - fr[k].ne;
-                float2* fa = reinterpret_cast<float2*>(arena + arena_off[j] + fr[k].arena_off);
-                const size_t ci = tc.f12.size();
-                tc.f12.push_back({fa, nullptr, fr[k].n, fne, nullptr});
-                tc.f12_off.push_back(tc.f12_elems);
-                tc.f12_inv.push_back(inv.size());
-                tc.f12_elems += (size_t)fne * fnb;
-                TGTask tx{};
-                tx.a = fa; tx.lda = fr[k].n; tx.ldb = fne; tx.c = fa + (size_t)fne * fr[k].n; tx.ldc = fr[k].n;
-                tx.m = fne; tx.n = fnb; tx.k = fne; tx.sign = 1.f; tx.job = (int32_t)j;
-                TGTask ts = tx;
-                ts.a = fa + fne; ts.add = fa + fne + (size_t)fne * fr[k].n; ts.ldadd = fr[k].n;
-                ts.c = fa + fne + (size_t)fne * fr[k].n; ts.m = fnb;
-                tc.sgt.push_back(tx);
-                tc.sgt_stage.push_back({ci, 0});
-                tc.sgt.push_back(ts);
-                tc.sgt_stage.push_back({ci, 1});
-                lv.sg_max_m = std::max(lv.sg_max_m, std::max(fne, fnb));
-                lv.sg_max_cols = std::max(lv.sg_max_cols, fnb);
-                lv.sg_flops += 8.0 * fr[k].n * (double)fne * fnb;
-              }
-              it.trail = vb == sizeof(double2) ? 1 : 0;
-              inv_piv_off.push_back(inv_piv);
-              inv_piv += fr[k].ne;
-              scratch_of(fr[k].n, vb);
-              inv.push_back(it);
-            }
+        const DevPlan& DP = *specs[begin + j].plan;
+        const auto& fr = DP.host.fronts;
+        const FrontDesc* dfr = DP.fronts;
+        for (size_t q = L < DP.host.levels ? DP.level_at[L] : DP.by_size.size(); q < DP.by_size.size(); ++q) {
+          const size_t k = DP.by_size[q];
+          if (fr[k].level != L || fr[k].n <= small_max) break;  // the level's larger fronts come first
+          tasks.push_back({(int32_t)j, (int32_t)k, dfr + k});
+          const double ne = fr[k].ne, nb = fr[k].n - fr[k].ne;
+          lv.max_large_n = std::max(lv.max_large_n, fr[k].n);
+          lv.max_large_ne = std::max(lv.max_large_ne, fr[k].ne);
+          lv.inv_flops += 8.0 / 3 * ne * ne * ne;
+          lv.gemm0_flops += 8 * ne * ne * nb;
+          lv.gemm1_flops += 8 * nb * nb * ne;
+          const double ncol = split ? ne : (double)fr[k].n;  // columns the sweep transforms
+          for (int k0 = 0; k0 < fr[k].ne; k0 += GJ_KB) {
+            const double kb = std::min(GJ_KB, fr[k].ne - k0), nn = fr[k].n;
+            // complex rows x kb times kb x columns, the updated block read and written: every row and the
+            // rest columns, or (FP64 fronts, trail form) the rows and columns after the panel.
+            const double ur = vb == sizeof(double2) ? nn - k0 - kb : nn, uc = vb == sizeof(double2) ? ur : ncol - kb;
+            lv.upd_flops += 8.0 * ur * uc * kb;
+            lv.upd_bytes += 2.0 * ur * uc * vb;
+            lv.pan_flops += 8.0 * (vb == sizeof(double2) ? nn - k0 : nn) * kb * kb;
           }
+          if (split) {
+            lv.upd_flops += 8.0 * fr[k].n * ne * nb;                           // [X; S] = [F11^-1; W] F12
+            lv.upd_bytes += ((double)fr[k].n * ne + 3.0 * ne * nb + 2.0 * nb * nb) * vb;  // A, F12 twice, X, F22
+          }
+          lv.asm_bytes += (double)fr[k].n * fr[k].n * vb;
+          if (fr[k].ne > 0) {
+            InvTask it{};
+            it.a = arena + arena_off[j] + fr[k].arena_off;
+            it.ld = fr[k].n;
+            it.n = fr[k].n;
+            it.npiv = fr[k].ne;
+            it.ncol = split ? fr[k].ne : fr[k].n;
+            it.job = (int32_t)j;
+            it.front = (int32_t)k;
+            if (split && fr[k].n > fr[k].ne) {
+              const int fne = fr[k].ne, fnb = fr[k].n - fr[k].ne;
+              float2* fa = reinterpret_cast<float2*>(arena + arena_off[j] + fr[k].arena_off);
+              const size_t ci = tc.f12.size();
+              tc.f12.push_back({fa, nullptr, fr[k].n, fne, nullptr});
+              tc.f12_off.push_back(tc.f12_elems);
+              tc.f12_inv.push_back(inv.size());
+              tc.f12_elems += (size_t)fne * fnb;
+              TGTask tx{};
+              tx.a = fa; tx.lda = fr[k].n; tx.ldb = fne; tx.c = fa + (size_t)fne * fr[k].n; tx.ldc = fr[k].n;
+              tx.m = fne; tx.n = fnb; tx.k = fne; tx.sign = 1.f; tx.job = (int32_t)j;
+              TGTask ts = tx;
+              ts.a = fa + fne; ts.add = fa + fne + (size_t)fne * fr[k].n; ts.ldadd = fr[k].n;
+              ts.c = fa + fne + (size_t)fne * fr[k].n; ts.m = fnb;
+              tc.sgt.push_back(tx);
+              tc.sgt_stage.push_back({ci, 0});
+              tc.sgt.push_back(ts);
+              tc.sgt_stage.push_back({ci, 1});
+              lv.sg_max_m = std::max(lv.sg_max_m, std::max(fne, fnb));
+              lv.sg_max_cols = std::max(lv.sg_max_cols, fnb);
+              lv.sg_flops += 8.0 * fr[k].n * (double)fne * fnb;
+            }
+            it.trail = vb == sizeof(double2) ? 1 : 0;
+            inv_piv_off.push_back(inv_piv);
+            inv_piv += fr[k].ne;
+            scratch_of(fr[k].n, vb);
+            inv.push_back(it);
+          }
+        }
       }
       lv.large_n = tasks.size() - lv.large0;
       lv.f12_n = tc.f12.size() - lv.f12_0;
@@ -1742,12 +1785,12 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     int32_t* dpiv = static_cast<int32_t*>(ctx->ipiv.get(std::max<size_t>(inv_piv, 1) * sizeof(int32_t)));
     unsigned char* dy = static_cast<unsigned char*>(ctx->iy.get(std::max<size_t>(inv_y, 16)));
     unsigned char* dbt = static_cast<unsigned char*>(ctx->ibt.get(std::max<size_t>(inv_bt, 16)));
-    unsigned char* doz = static_cast<unsigned char*>(ctx->ioz.fit(std::max<size_t>(tc.inv_oz, 16)));
+    unsigned char* doz = static_cast<unsigned char*>(room(ctx->ioz, std::max<size_t>(tc.inv_oz, 16)));
     unsigned char* dpp = static_cast<unsigned char*>(ctx->ipp.get(std::max<size_t>(tc.inv_pp, 16)));
     double* dscale = static_cast<double*>(ctx->iscale.get(std::max<size_t>(inv.size(), 1) * sizeof(double)));
     int32_t* dbad = static_cast<int32_t*>(ctx->ibad.get(std::max<size_t>(inv.size(), 1) * sizeof(int32_t)));
-    InvTask* dinv = static_cast<InvTask*>(ctx->inv.get(std::max<size_t>(inv.size(), 1) * sizeof(InvTask)));
-    Task* dtasks = static_cast<Task*>(ctx->tasks.get(tasks.size() * sizeof(Task)));
+    InvTask* dinv = static_cast<InvTask*>(ctx->inv[prec].get(std::max<size_t>(inv.size(), 1) * sizeof(InvTask)));
+    Task* dtasks = static_cast<Task*>(ctx->tasks[prec].get(tasks.size() * sizeof(Task)));
     float2* f12_stage = static_cast<float2*>(ctx->f12_stage.get(std::max<size_t>(tc.f12_elems, 1) * sizeof(float2)));
     F12Copy* df12 = static_cast<F12Copy*>(ctx->f12_list.get(std::max<size_t>(tc.f12.size(), 1) * sizeof(F12Copy)));
     TGTask* dsgt = static_cast<TGTask*>(ctx->sgt_list.get(std::max<size_t>(tc.sgt.size(), 1) * sizeof(TGTask)));
@@ -3369,17 +3412,22 @@ SigmaSlot& slot_buffers(System* sys, int slot) {
   SigmaSlot& sg = sys->slots[slot];
   const size_t nblocks = sys->plans.size();
   if (sg.sl.size() != nblocks) {
-    for (auto* v : {&sg.sl, &sg.sr, &sg.gl, &sg.gr, &sg.wr}) {
-      for (auto* p : *v) cudaFree(p);
-      v->clear();
-    }
+    for (auto* v : {&sg.sl, &sg.sr, &sg.gl, &sg.gr, &sg.wr}) v->clear();
+    cudaFree(sg.base);
+    sg.base = nullptr;
+    size_t total = 0;
+    std::vector<size_t> at;
     for (size_t b = 0; b < nblocks; ++b) {
       const size_t nl = sys->plans[b]->host.nl, nr = sys->plans[b]->host.nr;
-      sg.sl.push_back(dalloc<double2>(std::max<size_t>(nl * nl, 1)));
-      sg.sr.push_back(dalloc<double2>(std::max<size_t>(nr * nr, 1)));
-      sg.gl.push_back(dalloc<double2>(std::max<size_t>(nl * nl, 1)));
-      sg.gr.push_back(dalloc<double2>(std::max<size_t>(nr * nr, 1)));
-      sg.wr.push_back(dalloc<double2>(std::max<size_t>(nr * nr, 1)));
+      for (size_t m : {nl, nr, nl, nr, nr}) {
+        at.push_back(total);
+        total += (std::max<size_t>(m * m, 1) + 15) / 16 * 16;  // 256-byte steps
+      }
+    }
+    sg.base = dalloc<double2>(total);
+    for (size_t b = 0; b < nblocks; ++b) {
+      size_t q = 5 * b;
+      for (auto* v : {&sg.sl, &sg.sr, &sg.gl, &sg.gr, &sg.wr}) v->push_back(sg.base + at[q++]);
     }
   }
   sg.channels.assign(nblocks, 0);

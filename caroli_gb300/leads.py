@@ -171,23 +171,19 @@ class LeadSolver:
     def _definite_roots(self, e):
         s, c, theta, y = self.cell
         mu = -(theta - e) / (s * c)
-        lam_r = np.empty(len(mu), np.complex128)
-        lam_l = np.empty(len(mu), np.complex128)
-        for k, m in enumerate(mu):
-            if abs(m) < 2.0:
-                root = complex(m / 2.0, np.sqrt(4.0 - m * m) / 2.0)
-                if 2.0 * root.imag < DEGENERATE_TOL:
-                    raise GreenError("Singular", f"subband edge near E = {e}")
-                # Current J = -2 s c Im λ: the root with s Im λ < 0 goes right.
-                r, l = (root, root.conjugate()) if s < 0 else (root.conjugate(), root)
-                if abs(2.0 * r.imag / c) < VELOCITY_TOL * self.scale:
-                    raise GreenError("Singular", f"subband edge near E = {e}")
-                lam_r[k], lam_l[k] = r, l
-            else:
-                big = (m + np.sign(m) * np.sqrt(m * m - 4.0)) / 2.0
-                if abs(big) <= 1.0 + UNIT_TOL:
-                    raise GreenError("Singular", f"subband edge near E = {e}")
-                lam_r[k], lam_l[k] = 1.0 / big, big
+        # Propagating modes (|mu| < 2): the two roots on the unit circle; the current is J = -2 s c Im λ, so the
+        # root with s Im λ < 0 goes right. Evanescent ones: λ and 1/λ, the decaying one to the right.
+        prop = np.abs(mu) < 2.0
+        im = np.sqrt(np.where(prop, 4.0 - mu * mu, 4.0)) / 2.0
+        if np.any(prop & ((2.0 * im < DEGENERATE_TOL) | (np.abs(2.0 * im / c) < VELOCITY_TOL * self.scale))):
+            raise GreenError("Singular", f"subband edge near E = {e}")
+        big = (mu + np.sign(mu) * np.sqrt(np.where(prop, 4.0, mu * mu) - 4.0)) / 2.0
+        if np.any(~prop & (np.abs(big) <= 1.0 + UNIT_TOL)):
+            raise GreenError("Singular", f"subband edge near E = {e}")
+        root = mu / 2.0 + 1j * (im if s < 0 else -im)
+        big = np.where(prop, 1.0, big)
+        lam_r = np.where(prop, root, 1.0 / big)
+        lam_l = np.where(prop, root.conj(), big)
         return lam_l, lam_r
 
     # -- general coupling: the 2n pencil ---------------------------------------------------------

@@ -310,6 +310,8 @@ struct StatesRequest {
 struct TaskLevel {
   size_t tiny0 = 0, tiny_n = 0;
   size_t small0 = 0, small_n = 0, large0 = 0, large_n = 0;
+  size_t big_n = 0;  // the first of the large fronts, above SWEEP_WIDE_MAX variables
+  int max_wide_n = 0, max_wide_ne = 0;  // of the others
   int max_small_n = 0, max_small_ne = 0, max_large_n = 0, max_large_ne = 0, max_n = 0;
   // Small fronts in size buckets (one launch each, shared memory sized to the bucket).
   size_t sb0[3] = {0, 0, 0}, sbn[3] = {0, 0, 0};
@@ -491,6 +493,7 @@ size_t panel_smem(int pmax, size_t vbytes) {
 constexpr size_t PANEL_PROWS = (size_t)GJ_KB * GJ_KB * sizeof(double2);
 constexpr size_t PANEL_SCRATCH = (PANEL_PROWS + PS_PERM * 4 + 255) / 256 * 256;
 constexpr int SM_COUNT = 152;
+constexpr int SWEEP_FEW = 8 * SM_COUNT;  // fronts (times column chunks) below which a sweep takes row tiles
 
 // One panel of `count` matrices with at most m candidate rows, over clusters: as many CTAs per matrix
 // as leave the GPU at most two CTAs per SM (a panel is bound by the FP64 pipe of the SMs it runs on), at
@@ -530,7 +533,9 @@ template <typename F> void in_pieces_of(size_t count, size_t piece, F fn) {
 struct LevelRange {
   size_t tiny0, tiny_n;  // fronts of at most TINY_MAX variables (one warp each)
   size_t mid0, mid_n;    // fronts of at most 96 variables (one warp each, three rows per lane)
-  size_t first, count;   // the others
+  size_t first, count;   // the others, largest first
+  size_t big;            // those above SWEEP_WIDE_MAX variables (row tiles; the rest a warp each where there are many)
+  int mid_n_max, mid_ne_max, wide_n_max, wide_ne_max;
   int max_n;
   int max_ne;            // bound on the eliminated variables of the others
 };
@@ -906,13 +911,14 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
   const unsigned rows = (unsigned)((max_blk + 255) / 256);
   const unsigned cols = (unsigned)std::max(1, cmax);
   // Task segments (per level: tiny fronts, then the others) and their compacted copies.
-  const int nseg = 3 * nlev;
+  const int nseg = 4 * nlev;
   std::vector<TaskSeg> segs(nseg);
   int64_t seg_max = 0;
   for (int L = 0; L < nlev; ++L) {
-    segs[3 * L] = {(int64_t)lr[L].tiny0, (int64_t)lr[L].tiny_n};
-    segs[3 * L + 1] = {(int64_t)lr[L].mid0, (int64_t)lr[L].mid_n};
-    segs[3 * L + 2] = {(int64_t)lr[L].first, (int64_t)lr[L].count};
+    segs[4 * L] = {(int64_t)lr[L].tiny0, (int64_t)lr[L].tiny_n};
+    segs[4 * L + 1] = {(int64_t)lr[L].mid0, (int64_t)lr[L].mid_n};
+    segs[4 * L + 2] = {(int64_t)lr[L].first, (int64_t)lr[L].big};
+    segs[4 * L + 3] = {(int64_t)(lr[L].first + lr[L].big), (int64_t)(lr[L].count - lr[L].big)};
     seg_max = std::max<int64_t>(seg_max, std::max(std::max(lr[L].tiny_n, lr[L].mid_n), lr[L].count));
   }
   size_t ntask_all = 0;
@@ -951,28 +957,62 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
   auto sweep_cb = [&](auto cbt, int src, int dst) {
     constexpr int CB = decltype(cbt)::value;
     // Warp-per-front launches over a segment, at most 65535 blocks of TINY_WARPS (grid y).
-    auto warp_fwd = [&](auto rplt, size_t seg0, int cnt) {
+    auto warp_fwd = [&](auto rplt, size_t seg0, int cnt, int zmax) {
       constexpr int RPL = decltype(rplt)::value;
       in_pieces_of((size_t)cnt, (size_t)65535 * TINY_WARPS, [&](size_t f0, size_t c) {
         launch(K_REF_FWD, 0.0, 0.0, [&] {
-          sweep_warp_fwd_kernel<CB, RPL><<<dim3(cchunks, (unsigned)((c + TINY_WARPS - 1) / TINY_WARPS)), 256, 0, s>>>(
-              drd, ctasks + seg0 + f0, (int)c, src);
+          sweep_warp_fwd_kernel<CB, RPL><<<dim3(cchunks, (unsigned)((c + TINY_WARPS - 1) / TINY_WARPS)), 256,
+                                           (size_t)TINY_WARPS * std::max(1, zmax) * CB * sizeof(float2), s>>>(drd, ctasks + seg0 + f0, (int)c,
+                                                                                                 src, zmax);
         });
       });
     };
-    auto warp_bwd = [&](auto rplt, size_t seg0, int cnt) {
+    auto warp_bwd = [&](auto rplt, size_t seg0, int cnt, int zmax) {
       constexpr int RPL = decltype(rplt)::value;
       in_pieces_of((size_t)cnt, (size_t)65535 * TINY_WARPS, [&](size_t f0, size_t c) {
         launch(K_REF_BWD, 0.0, 0.0, [&] {
-          sweep_warp_bwd_kernel<CB, RPL><<<dim3(cchunks, (unsigned)((c + TINY_WARPS - 1) / TINY_WARPS)), 256, 0, s>>>(
-              drd, ctasks + seg0 + f0, (int)c, src, dst);
+          sweep_warp_bwd_kernel<CB, RPL><<<dim3(cchunks, (unsigned)((c + TINY_WARPS - 1) / TINY_WARPS)), 256,
+                                           (size_t)TINY_WARPS * std::max(1, zmax) * CB * sizeof(float2), s>>>(drd, ctasks + seg0 + f0, (int)c,
+                                                                                                 src, dst, zmax);
         });
       });
     };
+    // Row tiles of at most max_n variables, max_ne of them eliminated.
+    auto rows_fwd = [&](size_t seg0, int cnt, int max_n, int max_ne) {
+      const size_t sm = (size_t)std::max(1, max_ne) * CB * sizeof(float2);
+      const unsigned tiles = (unsigned)((max_n + SW_ROWS - 1) / SW_ROWS);
+      in_pieces((size_t)cnt, [&](size_t f0, size_t c) {
+        launch(K_REF_FWD, 0.0, sweep_bytes * 0.5 / nlev, [&] {
+          sweep_rows_fwd_kernel<CB><<<dim3(cchunks, tiles, (unsigned)c), 256, sm, s>>>(drd, ctasks + seg0 + f0, src);
+        });
+      });
+    };
+    auto rows_bwd = [&](size_t seg0, int cnt, int max_n, int max_ne) {
+      const size_t sm = (size_t)std::max(1, max_n) * CB * sizeof(float2);
+      const unsigned tiles = (unsigned)((std::max(1, max_ne) + SW_ROWS - 1) / SW_ROWS);
+      in_pieces((size_t)cnt, [&](size_t f0, size_t c) {
+        launch(K_REF_BWD, 0.0, sweep_bytes * 0.5 / nlev, [&] {
+          sweep_rows_bwd_kernel<CB><<<dim3(cchunks, tiles, (unsigned)c), 256, sm, s>>>(drd, ctasks + seg0 + f0, src, dst);
+        });
+      });
+    };
+    // A warp per front where the fronts fill the GPU, else row tiles; up to 192 variables only while a warp's
+    // sums stay in registers (CB <= 4).
+    auto as_warps = [&](int cnt) { return (size_t)cnt * cchunks >= (size_t)SWEEP_FEW; };
+    auto rpl = [](int rows, auto fn) {  // rows per lane of a warp: 1, 2, 3, 4 or 6
+      if (rows <= 32) fn(std::integral_constant<int, 1>{});
+      else if (rows <= 64) fn(std::integral_constant<int, 2>{});
+      else if (CB == 8 || rows <= 96) fn(std::integral_constant<int, 3>{});
+      else if constexpr (CB <= 4) {
+        if (rows <= 128) fn(std::integral_constant<int, 4>{});
+        else fn(std::integral_constant<int, 6>{});
+      }
+    };
     for (int L = 0; L < nlev; ++L) {
-      const int nt = hcount[3 * L], nm = hcount[3 * L + 1], nr = hcount[3 * L + 2];
-      if (nt) warp_fwd(std::integral_constant<int, 1>{}, lr[L].tiny0, nt);
-      if (nm) warp_fwd(std::integral_constant<int, 3>{}, lr[L].mid0, nm);
+      const int nt = hcount[4 * L], nm = hcount[4 * L + 1], nr = hcount[4 * L + 2], nw = hcount[4 * L + 3];
+      if (nt) rpl(TINY_MAX, [&](auto q) { warp_fwd(q, lr[L].tiny0, nt, TINY_MAX); });
+      if (nm && as_warps(nm)) rpl(lr[L].mid_n_max, [&](auto q) { warp_fwd(q, lr[L].mid0, nm, lr[L].mid_ne_max); });
+      else if (nm) rows_fwd(lr[L].mid0, nm, lr[L].mid_n_max, lr[L].mid_ne_max);
       if (wide) {
         if (wl[L].nfr) {
           tg_gather(true, wl[L].fr0, wl[L].nfr, src, dst, K_REF_FWD);
@@ -980,15 +1020,14 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
         }
         continue;
       }
-      if (!nr) continue;
-      const size_t sm = (size_t)std::max(1, lr[L].max_ne) * CB * sizeof(float2);
-      const unsigned tiles = (unsigned)((lr[L].max_n + SW_ROWS - 1) / SW_ROWS);
-      in_pieces((size_t)nr, [&](size_t f0, size_t c) {
-        launch(K_REF_FWD, 0.0, sweep_bytes * 0.5 / nlev, [&] {
-          sweep_rows_fwd_kernel<CB><<<dim3(cchunks, tiles, (unsigned)c), 256, sm, s>>>(drd, ctasks + lr[L].first + f0,
-                                                                                     src);
-        });
-      });
+      if (nr) rows_fwd(lr[L].first, nr, lr[L].max_n, lr[L].max_ne);
+      const size_t w0 = lr[L].first + lr[L].big;
+      if constexpr (CB <= 4)
+        if (nw && as_warps(nw)) {
+          rpl(lr[L].wide_n_max, [&](auto q) { warp_fwd(q, w0, nw, lr[L].wide_ne_max); });
+          continue;
+        }
+      if (nw) rows_fwd(w0, nw, lr[L].wide_n_max, lr[L].wide_ne_max);
     }
     const int nj = hcount[nseg];
     if (wide) {
@@ -1003,9 +1042,10 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
       });
     }
     for (int L = nlev - 1; L >= 0; --L) {
-      const int nt = hcount[3 * L], nm = hcount[3 * L + 1], nr = hcount[3 * L + 2];
-      if (nt) warp_bwd(std::integral_constant<int, 1>{}, lr[L].tiny0, nt);
-      if (nm) warp_bwd(std::integral_constant<int, 3>{}, lr[L].mid0, nm);
+      const int nt = hcount[4 * L], nm = hcount[4 * L + 1], nr = hcount[4 * L + 2], nw = hcount[4 * L + 3];
+      if (nt) rpl(TINY_MAX, [&](auto q) { warp_bwd(q, lr[L].tiny0, nt, TINY_MAX); });
+      if (nm && as_warps(nm)) rpl(lr[L].mid_ne_max, [&](auto q) { warp_bwd(q, lr[L].mid0, nm, lr[L].mid_n_max); });
+      else if (nm) rows_bwd(lr[L].mid0, nm, lr[L].mid_n_max, lr[L].mid_ne_max);
       if (wide) {
         if (wl[L].nfr) {
           tg_gather(false, wl[L].fr0, wl[L].nfr, src, dst, K_REF_BWD);
@@ -1013,15 +1053,14 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
         }
         continue;
       }
-      if (!nr) continue;
-      const size_t sm = (size_t)std::max(1, lr[L].max_n) * CB * sizeof(float2);
-      const unsigned tiles = (unsigned)((std::max(1, lr[L].max_ne) + SW_ROWS - 1) / SW_ROWS);
-      in_pieces((size_t)nr, [&](size_t f0, size_t c) {
-        launch(K_REF_BWD, 0.0, sweep_bytes * 0.5 / nlev, [&] {
-          sweep_rows_bwd_kernel<CB><<<dim3(cchunks, tiles, (unsigned)c), 256, sm, s>>>(drd, ctasks + lr[L].first + f0,
-                                                                                     src, dst);
-        });
-      });
+      if (nr) rows_bwd(lr[L].first, nr, lr[L].max_n, lr[L].max_ne);
+      const size_t w0 = lr[L].first + lr[L].big;
+      if constexpr (CB <= 4)
+        if (nw && as_warps(nw)) {
+          rpl(lr[L].wide_ne_max, [&](auto q) { warp_bwd(q, w0, nw, lr[L].wide_n_max); });
+          continue;
+        }
+      if (nw) rows_bwd(w0, nw, lr[L].wide_n_max, lr[L].wide_ne_max);
     }
   };
   auto sweep = [&](int src, int dst) {
@@ -1647,12 +1686,12 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
             for (; at[j] < end[j] && P.host.fronts[P.by_size[at[j]]].n == n; ++at[j]) {
               const int32_t k = P.by_size[at[j]];
               tasks.push_back({(int32_t)j, k, P.fronts + k});
-              fn(P.host.fronts[k]);
+              fn(j, k, P.host.fronts[k]);
             }
           }
       };
       lv.tiny0 = tasks.size();
-      collect(-1, TINY_MAX, [&](const FrontDesc& f) {
+      collect(-1, TINY_MAX, [&](size_t, int32_t, const FrontDesc& f) {
         const double ne = f.ne, nb = f.n - f.ne;
         lv.tiny_flops += 8.0 / 3 * ne * ne * ne + 8 * ne * ne * nb + 8 * nb * nb * ne;
         lv.max_tiny_n = std::max(lv.max_tiny_n, f.n);
@@ -1664,7 +1703,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       for (int b = 0; b < 3; ++b) {
         const int lo = b == 0 ? TINY_MAX : bucket_hi[b - 1], hi = bucket_hi[b];
         lv.sb0[b] = tasks.size();
-        collect(lo, hi, [&](const FrontDesc& f) {
+        collect(lo, hi, [&](size_t, int32_t, const FrontDesc& f) {
           const double ne = f.ne, nb = f.n - f.ne;
           lv.max_small_n = std::max(lv.max_small_n, f.n);
           lv.max_small_ne = std::max(lv.max_small_ne, f.ne);
@@ -1682,74 +1721,78 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       lv.inv0 = inv.size();
       lv.f12_0 = tc.f12.size();
       lv.sg0 = tc.sgt.size();
+      int level_max = 0;
       for (size_t j = 0; j < cj; ++j) {
-        const DevPlan& DP = *specs[begin + j].plan;
-        const auto& fr = DP.host.fronts;
-        const FrontDesc* dfr = DP.fronts;
-        for (size_t q = L < DP.host.levels ? DP.level_at[L] : DP.by_size.size(); q < DP.by_size.size(); ++q) {
-          const size_t k = DP.by_size[q];
-          if (fr[k].level != L || fr[k].n <= small_max) break;  // the level's larger fronts come first
-          tasks.push_back({(int32_t)j, (int32_t)k, dfr + k});
-          const double ne = fr[k].ne, nb = fr[k].n - fr[k].ne;
-          lv.max_large_n = std::max(lv.max_large_n, fr[k].n);
-          lv.max_large_ne = std::max(lv.max_large_ne, fr[k].ne);
-          lv.inv_flops += 8.0 / 3 * ne * ne * ne;
-          lv.gemm0_flops += 8 * ne * ne * nb;
-          lv.gemm1_flops += 8 * nb * nb * ne;
-          const double ncol = split ? ne : (double)fr[k].n;  // columns the sweep transforms
-          for (int k0 = 0; k0 < fr[k].ne; k0 += GJ_KB) {
-            const double kb = std::min(GJ_KB, fr[k].ne - k0), nn = fr[k].n;
-            // complex rows x kb times kb x columns, the updated block read and written: every row and the
-            // rest columns, or (FP64 fronts, trail form) the rows and columns after the panel.
-            const double ur = vb == sizeof(double2) ? nn - k0 - kb : nn, uc = vb == sizeof(double2) ? ur : ncol - kb;
-            lv.upd_flops += 8.0 * ur * uc * kb;
-            lv.upd_bytes += 2.0 * ur * uc * vb;
-            lv.pan_flops += 8.0 * (vb == sizeof(double2) ? nn - k0 : nn) * kb * kb;
-          }
-          if (split) {
-            lv.upd_flops += 8.0 * fr[k].n * ne * nb;                           // [X; S] = [F11^-1; W] F12
-            lv.upd_bytes += ((double)fr[k].n * ne + 3.0 * ne * nb + 2.0 * nb * nb) * vb;  // A, F12 twice, X, F22
-          }
-          lv.asm_bytes += (double)fr[k].n * fr[k].n * vb;
-          if (fr[k].ne > 0) {
-            InvTask it{};
-            it.a = arena + arena_off[j] + fr[k].arena_off;
-            it.ld = fr[k].n;
-            it.n = fr[k].n;
-            it.npiv = fr[k].ne;
-            it.ncol = split ? fr[k].ne : fr[k].n;
-            it.job = (int32_t)j;
-            it.front = (int32_t)k;
-            if (split && fr[k].n > fr[k].ne) {
-              const int fne = fr[k].ne, fnb = fr[k].n - fr[k].ne;
-              float2* fa = reinterpret_cast<float2*>(arena + arena_off[j] + fr[k].arena_off);
-              const size_t ci = tc.f12.size();
-              tc.f12.push_back({fa, nullptr, fr[k].n, fne, nullptr});
-              tc.f12_off.push_back(tc.f12_elems);
-              tc.f12_inv.push_back(inv.size());
-              tc.f12_elems += (size_t)fne * fnb;
-              TGTask tx{};
-              tx.a = fa; tx.lda = fr[k].n; tx.ldb = fne; tx.c = fa + (size_t)fne * fr[k].n; tx.ldc = fr[k].n;
-              tx.m = fne; tx.n = fnb; tx.k = fne; tx.sign = 1.f; tx.job = (int32_t)j;
-              TGTask ts = tx;
-              ts.a = fa + fne; ts.add = fa + fne + (size_t)fne * fr[k].n; ts.ldadd = fr[k].n;
-              ts.c = fa + fne + (size_t)fne * fr[k].n; ts.m = fnb;
-              tc.sgt.push_back(tx);
-              tc.sgt_stage.push_back({ci, 0});
-              tc.sgt.push_back(ts);
-              tc.sgt_stage.push_back({ci, 1});
-              lv.sg_max_m = std::max(lv.sg_max_m, std::max(fne, fnb));
-              lv.sg_max_cols = std::max(lv.sg_max_cols, fnb);
-              lv.sg_flops += 8.0 * fr[k].n * (double)fne * fnb;
-            }
-            it.trail = vb == sizeof(double2) ? 1 : 0;
-            inv_piv_off.push_back(inv_piv);
-            inv_piv += fr[k].ne;
-            scratch_of(fr[k].n, vb);
-            inv.push_back(it);
-          }
-        }
+        const DevPlan& P = *specs[begin + j].plan;
+        if (L < P.host.levels && P.level_at[L] < P.level_at[L + 1])
+          level_max = std::max(level_max, P.host.fronts[P.by_size[P.level_at[L]]].n);
       }
+      collect(small_max, level_max, [&](size_t j, int32_t k, const FrontDesc& f) {
+        if (f.n > SWEEP_WIDE_MAX) {
+          ++lv.big_n;
+        } else {
+          lv.max_wide_n = std::max(lv.max_wide_n, f.n);
+          lv.max_wide_ne = std::max(lv.max_wide_ne, f.ne);
+        }
+        const double ne = f.ne, nb = f.n - f.ne;
+        lv.max_large_n = std::max(lv.max_large_n, f.n);
+        lv.max_large_ne = std::max(lv.max_large_ne, f.ne);
+        lv.inv_flops += 8.0 / 3 * ne * ne * ne;
+        lv.gemm0_flops += 8 * ne * ne * nb;
+        lv.gemm1_flops += 8 * nb * nb * ne;
+        const double ncol = split ? ne : (double)f.n;  // columns the sweep transforms
+        for (int k0 = 0; k0 < f.ne; k0 += GJ_KB) {
+          const double kb = std::min(GJ_KB, f.ne - k0), nn = f.n;
+          // complex rows x kb times kb x columns, the updated block read and written: every row and the
+          // rest columns, or (FP64 fronts, trail form) the rows and columns after the panel.
+          const double ur = vb == sizeof(double2) ? nn - k0 - kb : nn, uc = vb == sizeof(double2) ? ur : ncol - kb;
+          lv.upd_flops += 8.0 * ur * uc * kb;
+          lv.upd_bytes += 2.0 * ur * uc * vb;
+          lv.pan_flops += 8.0 * (vb == sizeof(double2) ? nn - k0 : nn) * kb * kb;
+        }
+        if (split) {
+          lv.upd_flops += 8.0 * f.n * ne * nb;                           // [X; S] = [F11^-1; W] F12
+          lv.upd_bytes += ((double)f.n * ne + 3.0 * ne * nb + 2.0 * nb * nb) * vb;  // A, F12 twice, X, F22
+        }
+        lv.asm_bytes += (double)f.n * f.n * vb;
+        if (f.ne > 0) {
+          InvTask it{};
+          it.a = arena + arena_off[j] + f.arena_off;
+          it.ld = f.n;
+          it.n = f.n;
+          it.npiv = f.ne;
+          it.ncol = split ? f.ne : f.n;
+          it.job = (int32_t)j;
+          it.front = (int32_t)k;
+          if (split && f.n > f.ne) {
+            const int fne = f.ne, fnb = f.n - f.ne;
+            float2* fa = reinterpret_cast<float2*>(arena + arena_off[j] + f.arena_off);
+            const size_t ci = tc.f12.size();
+            tc.f12.push_back({fa, nullptr, f.n, fne, nullptr});
+            tc.f12_off.push_back(tc.f12_elems);
+            tc.f12_inv.push_back(inv.size());
+            tc.f12_elems += (size_t)fne * fnb;
+            TGTask tx{};
+            tx.a = fa; tx.lda = f.n; tx.ldb = fne; tx.c = fa + (size_t)fne * f.n; tx.ldc = f.n;
+            tx.m = fne; tx.n = fnb; tx.k = fne; tx.sign = 1.f; tx.job = (int32_t)j;
+            TGTask ts = tx;
+            ts.a = fa + fne; ts.add = fa + fne + (size_t)fne * f.n; ts.ldadd = f.n;
+            ts.c = fa + fne + (size_t)fne * f.n; ts.m = fnb;
+            tc.sgt.push_back(tx);
+            tc.sgt_stage.push_back({ci, 0});
+            tc.sgt.push_back(ts);
+            tc.sgt_stage.push_back({ci, 1});
+            lv.sg_max_m = std::max(lv.sg_max_m, std::max(fne, fnb));
+            lv.sg_max_cols = std::max(lv.sg_max_cols, fnb);
+            lv.sg_flops += 8.0 * f.n * (double)fne * fnb;
+          }
+          it.trail = vb == sizeof(double2) ? 1 : 0;
+          inv_piv_off.push_back(inv_piv);
+          inv_piv += f.ne;
+          scratch_of(f.n, vb);
+          inv.push_back(it);
+        }
+      });
       lv.large_n = tasks.size() - lv.large0;
       lv.f12_n = tc.f12.size() - lv.f12_0;
       lv.sg_n = tc.sgt.size() - lv.sg0;
@@ -2195,9 +2238,8 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       if constexpr (std::is_same<T, float>::value && std::is_same<TR, float>::value) {
         std::vector<LevelRange> lr;
         for (const Level& lv : levels) {
-          // Every small bucket (at most 96 variables) sweeps a warp per front; the large fronts follow.
-          const size_t mid = lv.small_n;
-          lr.push_back({lv.tiny0, lv.tiny_n, lv.small0, mid, lv.small0 + mid, lv.small_n - mid + lv.large_n, lv.max_n,
+          lr.push_back({lv.tiny0, lv.tiny_n, lv.small0, lv.small_n, lv.large0, lv.large_n, lv.big_n, lv.max_small_n,
+                        lv.max_small_ne, lv.max_wide_n, lv.max_wide_ne, lv.max_n,
                         std::max(lv.max_large_ne, lv.max_small_n)});
         }
         // Transmissions only: a stalled solve is recomputed in FP64 there (not so for gradients and
@@ -2545,6 +2587,24 @@ int caroli_ctx_create(int device_ordinal, caroli_ctx** out) {
                     (const void*)inv_panel_kernel<double>, (const void*)inv_panel_kernel<float>,
                     (const void*)tiny_front_kernel<double, false>, (const void*)tiny_front_kernel<double, true>,
                     (const void*)tiny_front_kernel<float, false>, (const void*)tiny_front_kernel<float, true>,
+                    (const void*)sweep_warp_fwd_kernel<1, 1>, (const void*)sweep_warp_bwd_kernel<1, 1>,
+                    (const void*)sweep_warp_fwd_kernel<1, 2>, (const void*)sweep_warp_bwd_kernel<1, 2>,
+                    (const void*)sweep_warp_fwd_kernel<1, 3>, (const void*)sweep_warp_bwd_kernel<1, 3>,
+                    (const void*)sweep_warp_fwd_kernel<1, 4>, (const void*)sweep_warp_bwd_kernel<1, 4>,
+                    (const void*)sweep_warp_fwd_kernel<1, 6>, (const void*)sweep_warp_bwd_kernel<1, 6>,
+                    (const void*)sweep_warp_fwd_kernel<2, 1>, (const void*)sweep_warp_bwd_kernel<2, 1>,
+                    (const void*)sweep_warp_fwd_kernel<2, 2>, (const void*)sweep_warp_bwd_kernel<2, 2>,
+                    (const void*)sweep_warp_fwd_kernel<2, 3>, (const void*)sweep_warp_bwd_kernel<2, 3>,
+                    (const void*)sweep_warp_fwd_kernel<2, 4>, (const void*)sweep_warp_bwd_kernel<2, 4>,
+                    (const void*)sweep_warp_fwd_kernel<2, 6>, (const void*)sweep_warp_bwd_kernel<2, 6>,
+                    (const void*)sweep_warp_fwd_kernel<4, 1>, (const void*)sweep_warp_bwd_kernel<4, 1>,
+                    (const void*)sweep_warp_fwd_kernel<4, 2>, (const void*)sweep_warp_bwd_kernel<4, 2>,
+                    (const void*)sweep_warp_fwd_kernel<4, 3>, (const void*)sweep_warp_bwd_kernel<4, 3>,
+                    (const void*)sweep_warp_fwd_kernel<4, 4>, (const void*)sweep_warp_bwd_kernel<4, 4>,
+                    (const void*)sweep_warp_fwd_kernel<4, 6>, (const void*)sweep_warp_bwd_kernel<4, 6>,
+                    (const void*)sweep_warp_fwd_kernel<8, 1>, (const void*)sweep_warp_bwd_kernel<8, 1>,
+                    (const void*)sweep_warp_fwd_kernel<8, 2>, (const void*)sweep_warp_bwd_kernel<8, 2>,
+                    (const void*)sweep_warp_fwd_kernel<8, 3>, (const void*)sweep_warp_bwd_kernel<8, 3>,
                     (const void*)sweep_rows_fwd_kernel<1>, (const void*)sweep_rows_fwd_kernel<2>,
                     (const void*)sweep_rows_fwd_kernel<4>, (const void*)sweep_rows_fwd_kernel<8>,
                     (const void*)sweep_rows_bwd_kernel<1>, (const void*)sweep_rows_bwd_kernel<2>,

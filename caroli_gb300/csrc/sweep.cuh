@@ -7,9 +7,8 @@
 // The sweeps stream each front's factor columns once ([F11^-1; W] forward, X backward) against
 // CB right-hand-side columns (the channels of W_R, mostly one or two), so they are bound by HBM
 // bandwidth and by the latency of the gathers in front of the streams. Each front row finds its
-// sources in one 16-byte SweepRow (built with the plan); fronts of at most 64 variables run one per
-// warp with the right-hand side in registers (broadcast by shuffles), larger ones as row tiles of
-// 64 with the inner dimension split four ways.
+// sources in one 16-byte SweepRow (built with the plan); the smaller fronts run one per warp, larger or
+// few ones as row tiles of 64 with the inner dimension split four ways.
 //
 // Tasks come from lists compacted to the solves still iterating (compact_kernel), so a batch in
 // which a few solves need more GMRES steps does not sweep the others' tasks again.
@@ -43,21 +42,24 @@ __device__ __forceinline__ bool sweep_idle(const RefineDesc& R, int src) {
 }
 
 // ---- fronts of at most 32 RPL variables: a warp each --------------------------------------------
-// Lane l owns rows l, l + 32, ... (RPL rows); the right-hand side of row k comes from lane k % 32 of
-// register k / 32 by a shuffle, so a warp needs no shared memory and no barrier. RPL = 1 serves
-// the tiny fronts (n <= 32), RPL = 2 the fronts up to 64 variables.
-template <int RPL, int CB>
-__device__ __forceinline__ float2 lane_value(const float2 (&v)[RPL][CB], int k, int j) {
-  float2 src = v[0][j];
-#pragma unroll
-  for (int u = 1; u < RPL; ++u)
-    if ((k >> 5) == u) src = v[u][j];
-  return make_float2(__shfl_sync(0xffffffffu, src.x, k & 31), __shfl_sync(0xffffffffu, src.y, k & 31));
-}
+// Lane l owns rows l, l + 32, ... (RPL rows); the entries a column multiplies are broadcast from the warp's
+// part of shared memory (zmax x CB). The factors stream in batches of U columns, the first requested before
+// the right-hand side is gathered: the gather is a chain of dependent loads (task, descriptors, sources,
+// values), and a front lasts as long as that chain plus its stream. Up to 192 variables when there are enough
+// such fronts to fill the GPU (SWEEP_FEW; fewer are faster as row tiles, several CTAs each). RPL covers the
+// level's largest front (forward: its rows; backward: its eliminated rows): registers decide how many
+// warps an SM holds.
+// Against shuffled registers and four columns at a time, and row tiles from 97 variables on: 256 solves of
+// BHZ 200 x 64, forward + backward 15.6 -> 11.7 ms per pass.
+constexpr int SWEEP_WIDE_MAX = 192;
+// Columns in flight: fewer where more would take the registers of another CTA per SM.
+template <int CB, int RPL> constexpr int SWEEP_BATCH = RPL == 1 ? 4 : (RPL >= 4 ? 2 : (RPL * CB > 12 ? 4 : 8));
 
 template <int CB, int RPL>
-__global__ void __launch_bounds__(256) sweep_warp_fwd_kernel(const RefineDesc* __restrict__ rd,
-                                                             const Task* __restrict__ tasks, int ntasks, int src) {
+__global__ void __launch_bounds__(256, RPL == 1 && CB <= 2 ? 6 : 2) sweep_warp_fwd_kernel(const RefineDesc* __restrict__ rd,
+                                                             const Task* __restrict__ tasks, int ntasks, int src, int zmax) {
+  constexpr int U = SWEEP_BATCH<CB, RPL>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ti = blockIdx.y * TINY_WARPS + w;
   if (ti >= ntasks) return;
@@ -67,29 +69,46 @@ __global__ void __launch_bounds__(256) sweep_warp_fwd_kernel(const RefineDesc* _
   if (sweep_idle(R, src) || j0 >= R.c) return;
   const FrontDesc& f = *tk.fd;
   const int n = f.n, ne = f.ne;
+  const float2* F = R.arena + f.arena_off + lane;  // rows lane + 32 u of [F11^-1; W]
+  float2 a[U][RPL];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int x = 0; x < U; ++x)
+#pragma unroll
+      for (int u = 0; u < RPL; ++u)
+        a[x][u] = (k0 + x < ne && lane + 32 * u < n) ? F[32 * u + (int64_t)(k0 + x) * n] : make_float2(0.f, 0.f);
+  };
+  load(0);
   const double2* rin = sweep_src(R, src);
-  float2 z[RPL][CB], acc[RPL][CB];
+  float2* z = reinterpret_cast<float2*>(smem_raw) + (size_t)w * zmax * CB;
+  float2 acc[RPL][CB];
 #pragma unroll
   for (int u = 0; u < RPL; ++u) {
     const int r = lane + 32 * u;
-    if (r < n) load_z<CB>(R, rin, R.srows[f.var_off + r], j0, z[u]);
-    else
 #pragma unroll
-      for (int j = 0; j < CB; ++j) z[u][j] = make_float2(0.f, 0.f);
+    for (int j = 0; j < CB; ++j) acc[u][j] = make_float2(0.f, 0.f);
+    if (r < n) {
+      float2 v[CB];
+      load_z<CB>(R, rin, R.srows[f.var_off + r], j0, v);
 #pragma unroll
-    for (int j = 0; j < CB; ++j) acc[u][j] = r < ne ? make_float2(0.f, 0.f) : z[u][j];
+      for (int j = 0; j < CB; ++j) {
+        if (r < ne) z[r * CB + j] = v[j];
+        else acc[u][j] = v[j];
+      }
+    }
   }
-  const float2* F = R.arena + f.arena_off + lane;  // rows lane + 32 u of [F11^-1; W]
-#pragma unroll 4
-  for (int k = 0; k < ne; ++k) {
-    float2 a[RPL];
+  __syncwarp();
+  for (int k0 = 0; k0 < ne; k0 += U) {
+    if (k0) load(k0);
 #pragma unroll
-    for (int u = 0; u < RPL; ++u) a[u] = lane + 32 * u < n ? F[32 * u + (int64_t)k * n] : make_float2(0.f, 0.f);
+    for (int x = 0; x < U; ++x) {
+      const int k = min(k0 + x, ne - 1);  // past the last column a is zero
 #pragma unroll
-    for (int j = 0; j < CB; ++j) {
-      const float2 zk = lane_value<RPL, CB>(z, k, j);
+      for (int j = 0; j < CB; ++j) {
+        const float2 zk = z[k * CB + j];
 #pragma unroll
-      for (int u = 0; u < RPL; ++u) acc[u][j] = cfma(acc[u][j], a[u], zk);
+        for (int u = 0; u < RPL; ++u) acc[u][j] = cfma(acc[u][j], a[x][u], zk);
+      }
     }
   }
 #pragma unroll
@@ -106,10 +125,15 @@ __global__ void __launch_bounds__(256) sweep_warp_fwd_kernel(const RefineDesc* _
   }
 }
 
+// Backward, RPL rows per lane covering ne. Few eliminated rows (ne <= 16): lane = r + ne2 s (ne2 = ne rounded up to a power of two, s < 32 / ne2) sums
+// X[r, p] x_b[p] over p = s (mod 32 / ne2); the slices meet by shuffles at the end. More: lane r, one column
+// at a time per load.
 template <int CB, int RPL>
-__global__ void __launch_bounds__(256) sweep_warp_bwd_kernel(const RefineDesc* __restrict__ rd,
+__global__ void __launch_bounds__(256, RPL == 1 && CB <= 2 ? 6 : 2) sweep_warp_bwd_kernel(const RefineDesc* __restrict__ rd,
                                                              const Task* __restrict__ tasks, int ntasks, int src,
-                                                             int dst) {
+                                                             int dst, int zmax) {
+  constexpr int U = SWEEP_BATCH<CB, RPL>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ti = blockIdx.y * TINY_WARPS + w;
   if (ti >= ntasks) return;
@@ -121,69 +145,57 @@ __global__ void __launch_bounds__(256) sweep_warp_bwd_kernel(const RefineDesc* _
   const int n = f.n, ne = f.ne, nb = n - ne;
   if (ne == 0) return;
   float2* dout = sweep_dst(R, dst);
-  float2 xb[RPL][CB], acc[RPL][CB];
+  float2* xb = reinterpret_cast<float2*>(smem_raw) + (size_t)w * zmax * CB;
+  const bool few = ne <= 16;
+  const int ne2 = ne <= 1 ? 1 : ne <= 2 ? 2 : ne <= 4 ? 4 : ne <= 8 ? 8 : 16;
+  const int S = few ? 32 / ne2 : 1, r0 = few ? lane & (ne2 - 1) : lane, sl = few ? lane / ne2 : 0;
+  const float2* X = R.arena + f.arena_off + r0 + (int64_t)ne * n;  // row r0 of X
+  float2 a[U][RPL];
+  auto load = [&](int p0) {
+#pragma unroll
+    for (int x = 0; x < U; ++x) {
+      const int p = p0 + x * S + sl;
+#pragma unroll
+      for (int u = 0; u < RPL; ++u)
+        a[x][u] = (p < nb && r0 + 32 * u < ne) ? X[32 * u + (int64_t)p * n] : make_float2(0.f, 0.f);
+    }
+  };
+  load(0);
+  float2 acc[RPL][CB];  // t - (this slice's part of X x_b); t in slice 0
 #pragma unroll
   for (int u = 0; u < RPL; ++u) {
-    const int p = lane + 32 * u, r = lane + 32 * u;
-    const int vb = p < nb ? R.srows[f.var_off + ne + p].var : 0;
+    const int r = lane + 32 * u;
 #pragma unroll
-    for (int j = 0; j < CB; ++j) {
-      const int col = j0 + j;
-      xb[u][j] = (p < nb && col < R.c) ? dout[vb + (int64_t)col * R.nblk] : make_float2(0.f, 0.f);
-      acc[u][j] = (r < ne && col < R.c) ? R.tb[(f.toff + r) + (int64_t)col * R.sum_ne] : make_float2(0.f, 0.f);
-    }
+    for (int j = 0; j < CB; ++j)
+      acc[u][j] = (r < ne && j0 + j < R.c) ? R.tb[(f.toff + r) + (int64_t)(j0 + j) * R.sum_ne] : make_float2(0.f, 0.f);
   }
-  if (ne <= 16) {
-    // Few eliminated rows: lane = r + ne2 s (ne2 = ne rounded up to a power of two, s < 32 / ne2)
-    // sums X[r, p] x_b[p] over p = s (mod 32 / ne2); the slices meet by shuffles at the end.
-    const int ne2 = ne <= 1 ? 1 : ne <= 2 ? 2 : ne <= 4 ? 4 : ne <= 8 ? 8 : 16;
-    const int S = 32 / ne2, r = lane & (ne2 - 1), sl = lane / ne2;
-    const float2* X = R.arena + f.arena_off + r + (int64_t)ne * n;  // row r of X
-    float2 part[CB];
+  for (int r = lane; r < nb; r += 32) {
+    const int vb = R.srows[f.var_off + ne + r].var;
 #pragma unroll
-    for (int j = 0; j < CB; ++j) part[j] = make_float2(0.f, 0.f);
-    for (int p0 = 0; p0 < nb; p0 += S) {
-      const int p = p0 + sl;
-      const float2 a = (r < ne && p < nb) ? X[(int64_t)p * n] : make_float2(0.f, 0.f);
-      const int u = p0 >> 5;  // the same for the whole warp: S divides 32
+    for (int j = 0; j < CB; ++j)
+      xb[r * CB + j] = j0 + j < R.c ? dout[vb + (int64_t)(j0 + j) * R.nblk] : make_float2(0.f, 0.f);
+  }
+  __syncwarp();
+  for (int p0 = 0; p0 < nb; p0 += U * S) {
+    if (p0) load(p0);
 #pragma unroll
-      for (int j = 0; j < CB; ++j) {
-        float2 src = xb[0][j];
-#pragma unroll
-        for (int q = 1; q < RPL; ++q)
-          if (u == q) src = xb[q][j];
-        const float2 xp = make_float2(__shfl_sync(0xffffffffu, src.x, p & 31), __shfl_sync(0xffffffffu, src.y, p & 31));
-        part[j] = cfma(part[j], a, xp);
-      }
-    }
-    for (int o = ne2; o < 32; o <<= 1)
+    for (int x = 0; x < U; ++x) {
+      const int p = min(p0 + x * S + sl, nb - 1);  // past the last column a is zero
 #pragma unroll
       for (int j = 0; j < CB; ++j) {
-        part[j].x += __shfl_xor_sync(0xffffffffu, part[j].x, o);
-        part[j].y += __shfl_xor_sync(0xffffffffu, part[j].y, o);
-      }
-    // Lane r (slice 0) holds row r's sum: bring it to the lane that owns row r's output.
+        const float2 xp = xb[p * CB + j];
 #pragma unroll
-    for (int j = 0; j < CB; ++j) {
-      const float2 sum = make_float2(__shfl_sync(0xffffffffu, part[j].x, lane & (ne2 - 1)),
-                                     __shfl_sync(0xffffffffu, part[j].y, lane & (ne2 - 1)));
-      if (lane < ne) { acc[0][j].x -= sum.x; acc[0][j].y -= sum.y; }
-    }
-  } else {
-    const float2* F = R.arena + f.arena_off + lane + (int64_t)ne * n;  // rows lane + 32 u of X
-#pragma unroll 4
-    for (int p = 0; p < nb; ++p) {
-      float2 a[RPL];
-#pragma unroll
-      for (int u = 0; u < RPL; ++u) a[u] = lane + 32 * u < ne ? F[32 * u + (int64_t)p * n] : make_float2(0.f, 0.f);
-#pragma unroll
-      for (int j = 0; j < CB; ++j) {
-        const float2 xp = lane_value<RPL, CB>(xb, p, j);
-#pragma unroll
-        for (int u = 0; u < RPL; ++u) acc[u][j] = cfms(acc[u][j], a[u], xp);
+        for (int u = 0; u < RPL; ++u) acc[u][j] = cfms(acc[u][j], a[x][u], xp);
       }
     }
   }
+  if (few)
+#pragma unroll
+    for (int j = 0; j < CB; ++j)
+      for (int o = ne2; o < 32; o <<= 1) {  // lane r then holds row r's sum
+        acc[0][j].x += __shfl_xor_sync(0xffffffffu, acc[0][j].x, o);
+        acc[0][j].y += __shfl_xor_sync(0xffffffffu, acc[0][j].y, o);
+      }
 #pragma unroll
   for (int u = 0; u < RPL; ++u) {
     const int r = lane + 32 * u;

@@ -2029,7 +2029,10 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
             else if (wide_cta)
               small_front_wide_kernel<T, false><<<nblk, 512, sm, s>>>(djobs, st, Prec<T>::tol, perturb, pert);
             else
-              small_front_kernel<T, false><<<nblk, 256, sm, s>>>(djobs, st, Prec<T>::tol, perturb, pert);
+              // FP64: four warps, one per scheduler, once the fronts fill the SMs (16 BHZ 200 x 64 solves: 8.88
+              // -> 8.71 ms); with few fronts the eight warps' overlap counts (one 32 x 32 square: 0.48 -> 0.46).
+              small_front_kernel<T, false><<<nblk, sizeof(T) == 8 && nblk >= 4 * SM_COUNT ? 128 : 256, sm, s>>>(
+                  djobs, st, Prec<T>::tol, perturb, pert);
           });
         }
         if (lv.large_n) {

@@ -371,8 +371,9 @@ __device__ __forceinline__ void column_order(const int* piv, int npiv, int* cper
 // two divergent loops: a column j != k becomes F[i, j] - c_i pr_j (pr_j = F[p, j] / pivot), the
 // pivot column -c_i / pivot, which is the same update from a zero column (`zeros`, rows zeros in
 // shared memory) with pr = 1 / pivot. Rows k and p, which the interchange treats apart, are
-// rewritten after the loop.
-template <typename T>
+// rewritten after the loop. TRAIL: only the pivots and prows are wanted, so the rows up to k are left alone
+// (half of the multiply-adds).
+template <typename T, bool TRAIL>
 __device__ bool gj_sweep_cols(typename Cx<T>::V* F, int ld, int rows, int cols, double scale2, double tol,
                               typename Cx<T>::V* cb, int* piv, bool perturb, int* perturbed,
                               typename Cx<T>::V* prows, const typename Cx<T>::V* zeros) {
@@ -429,7 +430,7 @@ __device__ bool gj_sweep_cols(typename Cx<T>::V* F, int ld, int rows, int cols, 
       prows[k * cols + j] = pr;
       const bool fill = j == k + 1;
 #pragma unroll 4
-      for (int i = 0; i < rows; ++i) {
+      for (int i = TRAIL ? k + 1 : 0; i < rows; ++i) {
         const V nv = cfms(src[i], ck[i], pr);
         Fj[i] = nv;
         if (fill) cn[i] = nv;
@@ -439,8 +440,10 @@ __device__ bool gj_sweep_cols(typename Cx<T>::V* F, int ld, int rows, int cols, 
         Fj[p] = nv;
         if (fill) cn[p] = nv;
       }
-      Fj[k] = pr;
-      if (fill) cn[k] = pr;
+      if (!TRAIL) {
+        Fj[k] = pr;
+        if (fill) cn[k] = pr;
+      }
     }
     asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
   }
@@ -496,6 +499,45 @@ __device__ __forceinline__ void replay_boundary(typename Cx<T>::V* F, int ld, in
         const int col = lane + 32 * q;
         if (i0 + u < n && col < n) F[i0 + u + col * ld] = r[u][q];
       }
+  }
+}
+
+// Boundary rows of an FP64 front of at most 64 variables whose factors are not kept, straight to the Schur
+// complement in `out`: eight lanes per row, lane h the entries h + 8 i, four rows per warp. Step k updates
+// the entries past k only. An FP64 instruction costs the same with one active lane as with 32, and these fronts
+// are bound by that pipe: against whole rows per warp (replay_boundary), 64 lanes' worth for 33 columns and
+// every column at every step, the small and tiny fronts of 16 BHZ 200 x 64 solves took 9.13 ms, now 8.71 (with
+// four warps per front), those of graphene over 64 energies 0.95, now 0.87.
+__device__ __forceinline__ void replay_schur(const double2* F, int ld, int n, int ne, const double2* prows, double2* out) {
+  constexpr int Q = 8;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, h = lane & 7;
+  const int nq = (n + 7) >> 3;
+  for (int i0 = ne + 4 * w; i0 < n; i0 += 4 * nw) {
+    const int row = i0 + (lane >> 3);
+    double2 r[Q];
+#pragma unroll
+    for (int i = 0; i < Q; ++i)
+      r[i] = (row < n && 8 * i + h < n) ? F[row + (8 * i + h) * ld] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int kq = 0; kq < Q; ++kq) {
+      if (8 * kq >= ne) break;
+      for (int kk = 0; kk < 8; ++kk) {
+        const int k = 8 * kq + kk;
+        if (k >= ne) break;
+        const int src = (lane & ~7) | kk;
+        const double2 a = make_double2(__shfl_sync(0xffffffffu, r[kq].x, src), __shfl_sync(0xffffffffu, r[kq].y, src));
+        const double2* pk = prows + k * n + h;
+        if (h > kk) r[kq] = cfms(r[kq], a, pk[8 * kq]);
+#pragma unroll
+        for (int i = kq + 1; i < Q; ++i)
+          if (i < nq) r[i] = cfms(r[i], a, pk[8 * i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      const int col = 8 * i + h;
+      if (row < n && col >= ne && col < n) out[row + (int64_t)col * n] = r[i];
+    }
   }
 }
 
@@ -611,7 +653,7 @@ __device__ __forceinline__ void small_front_body(const JobDesc* __restrict__ job
   // other warps wait at the block barrier.
   __shared__ int ok_flag;
   if (w < (n + 31) / 32) {
-    const bool okc = gj_sweep_cols<T>(F, ld, ne, n, scale2, tol, cb, piv, perturb != 0,
+    const bool okc = gj_sweep_cols<T, !KEEP && sizeof(T) == 8>(F, ld, ne, n, scale2, tol, cb, piv, perturb != 0,
                                       perturbed ? perturbed + t.job : nullptr, prows, zeros);
     if (threadIdx.x == 0) ok_flag = okc ? 1 : 0;
   }
@@ -619,6 +661,10 @@ __device__ __forceinline__ void small_front_body(const JobDesc* __restrict__ job
   const bool ok = ok_flag != 0;
   if (!ok) {
     if (threadIdx.x == 0) J.fail[t.front] = 1;
+    return;
+  }
+  if constexpr (!KEEP && sizeof(T) == 8) {
+    replay_schur(F, ld, n, ne, prows, out);
     return;
   }
   // Boundary rows: the recorded steps replayed.

@@ -53,6 +53,21 @@ def test_root_green_against_dense_inverse(length, width, spread):
     assert np.linalg.norm(greens[0][0] - ref) <= bound * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("length,width", [(40, 6), (40, 9), (33, 12), (50, 15), (37, 16), (64, 17), (45, 21), (70, 8)])
+def test_small_fronts_against_dense_inverse(length, width):
+    """Narrow devices: fronts of up to 64 variables, eight lanes per boundary row of any remainder."""
+    s = _device(length, width, 1, 7 * length + width)
+    sigma = s.self_energies(0.21)
+    a = _dense(s, sigma)
+    blk = s.system.blocks[0]
+    kept = np.concatenate([blk.left, blk.right])
+    ref = np.linalg.inv(a)[np.ix_(kept, kept)]
+    greens, st = s.plan().root_green([s._slot(sigma)], [0], [len(kept)])
+    assert st[0] == 0
+    bound = len(a) * EPS * np.linalg.cond(a)  # as above
+    assert np.linalg.norm(greens[0][0] - ref) <= bound * np.linalg.norm(ref)
+
+
 def test_batches_fill_clusters_differently():
     """One solve takes clusters of 16 CTAs per matrix, forty take one CTA each: the sums run in the same
     order either way, so every T is the same to the last bit."""

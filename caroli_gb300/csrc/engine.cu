@@ -31,6 +31,7 @@
 #include "leadsig.cuh"
 #include "ozgemm.cuh"
 #include "panel.cuh"
+#include "trail.cuh"
 #include "tcgemm.cuh"
 
 using namespace caroli;
@@ -1913,10 +1914,20 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       for (int k0 = 0; k0 < pmax; k0 += GJ_KB) {
         launch(cls, flops / panels, 0.0, [&] { launch_panel_sweep<double>(ctx, dinv + first, count, k0, pmax - k0, tol, 0, djobs, status); });
         const int rows = trail ? nmax - k0 : nmax;  // rows and columns of the update, at most
-        // Pieces of 16 rows and columns, or of 4 while those are fewer than two per scheduler.
-        const bool fine = (size_t)((rows + 15) / 16) * 2 * count < (size_t)(4 * SM_COUNT);
-        const unsigned rp = (unsigned)((rows + (fine ? 3 : 15)) / (fine ? 4 : 16));
         launch(cls, 0.0, 0.0, [&] {
+          if (trail) {
+            // Waves of tiles (one CTA of 128 rows and columns per SM, 62 us full) or of pieces (two CTAs per SM, 28 us).
+            const size_t tiles = (size_t)((rows + 127) / 128), pieces = (size_t)((rows + 31) / 32);
+            if (62 * ((count * tiles + SM_COUNT - 1) / SM_COUNT) < 28 * ((2 * count * pieces + 2 * SM_COUNT - 1) / (2 * SM_COUNT)))
+              trail::rest_kernel<1><<<dim3((unsigned)count, (unsigned)tiles), 256, trail::COARSE_SMEM, s>>>(dinv + first, k0, status);
+            else
+              trail::rest_kernel<4><<<dim3((unsigned)count, (unsigned)pieces, 2), 128, trail::FINE_SMEM, s>>>(
+                  dinv + first, k0, status);
+            return;
+          }
+          // Pieces of 16 rows and columns, or of 4 while those are fewer than two per scheduler.
+          const bool fine = (size_t)((rows + 15) / 16) * 2 * count < (size_t)(4 * SM_COUNT);
+          const unsigned rp = (unsigned)((rows + (fine ? 3 : 15)) / (fine ? 4 : 16));
           if (fine) panel_rest_kernel<double, 16, 64><<<dim3((unsigned)count, 2 * rp), 64, 0, s>>>(dinv + first, k0, (int)rp);
           else panel_rest_kernel<double, 4, 64><<<dim3((unsigned)count, 2 * rp), 64, 0, s>>>(dinv + first, k0, (int)rp);
         });
@@ -2601,6 +2612,7 @@ int caroli_ctx_create(int device_ordinal, caroli_ctx** out) {
                     (const void*)sweep_warp_fwd_kernel<2, 4>, (const void*)sweep_warp_bwd_kernel<2, 4>,
                     (const void*)sweep_warp_fwd_kernel<2, 6>, (const void*)sweep_warp_bwd_kernel<2, 6>,
                     (const void*)sweep_warp_fwd_kernel<4, 1>, (const void*)sweep_warp_bwd_kernel<4, 1>,
+                    (const void*)trail::rest_kernel<1>, (const void*)trail::rest_kernel<4>,
                     (const void*)sweep_warp_fwd_kernel<4, 2>, (const void*)sweep_warp_bwd_kernel<4, 2>,
                     (const void*)sweep_warp_fwd_kernel<4, 3>, (const void*)sweep_warp_bwd_kernel<4, 3>,
                     (const void*)sweep_warp_fwd_kernel<4, 4>, (const void*)sweep_warp_bwd_kernel<4, 4>,

@@ -64,32 +64,29 @@ __device__ __forceinline__ uint32_t offset(int row, int k, int rows) {
 
 __device__ __forceinline__ int biased_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 
-// x as a 62-bit fixed-point number: x 2^(1084 - e), e the biased exponent of the largest entry.
-__device__ __forceinline__ long long fixed(double x, int e) {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
-  int ex = (int)(bits >> 52) & 0x7ff;
-  unsigned long long m = bits & 0xfffffffffffffull;
-  if (ex) m |= 1ull << 52;
-  else ex = 1;
-  const int sh = 9 + ex - e;  // at most 9
-  long long v = sh >= 0 ? (long long)(m << sh) : (sh > -64 ? (long long)(m >> -sh) : 0ll);
-  return (long long)bits < 0 ? -v : v;
+// x as a 62-bit fixed-point number, x 2^(1084 - e) rounded toward zero (e the biased exponent of the largest
+// entry, at least 1), plus 256 in the place of each base-512 digit: the digits of the sum, less 256, are the signed digits of x.
+__device__ __forceinline__ unsigned long long biased_digits(double x, int e) {
+  const int hi = __double2hiint(x);
+  const int ex = (hi >> 20) & 0x7ff;
+  const unsigned mh = (unsigned)(hi & 0xfffff) | (ex ? 0x100000u : 0u), ml = (unsigned)__double2loint(x);
+  const unsigned long long m = ((unsigned long long)mh << 32 | ml) << 9;
+  const unsigned long long v = m >> min(e - max(ex, 1), 63);
+  constexpr unsigned long long BIAS = 0x4020100804020100ull;  // 256 x (1 + 512 + ... + 512^6)
+  return hi < 0 ? BIAS - v : BIAS + v;
 }
-// The signed base-512 digits of v (most significant first), each in [-256, 256].
-__device__ __forceinline__ void digits(long long v, int (&d)[S]) {
+// The seven signed digits of a complex entry, most significant first, each in [-256, 256], as pairs (re, im) of
+// f16: 0x6400 + u is 1024 + u in f16's binade [1024, 2048), from which 1280 is taken.
+__device__ __forceinline__ void digit_pairs(double2 x, int e, uint32_t (&d)[S]) {
+  const unsigned long long re = biased_digits(x.x, e), im = biased_digits(x.y, e);
 #pragma unroll
-  for (int s = S - 1; s > 0; --s) {
-    const int low = ((int)v & 511 ^ 256) - 256;
-    d[s] = low;
-    v = (v - low) >> 9;
+  for (int s = 0; s < S; ++s) {
+    const int at = 9 * (S - 1 - s);
+    const unsigned mask = s ? 511u : 1023u;
+    const uint32_t b = ((uint32_t)(re >> at) & mask) | ((((uint32_t)(im >> at) & mask) | 0x6400u) << 16) | 0x6400u;
+    const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&b), __half2half2(__ushort_as_half(0x6500)));
+    d[s] = *reinterpret_cast<const uint32_t*>(&v);
   }
-  d[0] = (int)v;
-}
-// Two digits as a pair of f16: 1536 + d is 0x6600 + d in f16's binade [1024, 2048).
-__device__ __forceinline__ uint32_t pack(int lo, int hi) {
-  const uint32_t b = (uint32_t)(0x6600 + lo) | ((uint32_t)(0x6600 + hi) << 16);
-  const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&b), __half2half2(__ushort_as_half(0x6600)));
-  return *reinterpret_cast<const uint32_t*>(&v);
 }
 
 // The largest exponent of the entries LPR lanes hold (at least 1).
@@ -113,12 +110,11 @@ __device__ __forceinline__ void write_a(unsigned char* oa, int32_t* ea, int q, i
   unsigned char* tile = oa + (size_t)(q / ROWS) * tile_stride;
 #pragma unroll
   for (int i = 0; i < GJ_KB / LPR; ++i) {
-    int re[S], im[S];
-    digits(fixed(a[i].x, e), re);
-    digits(fixed(a[i].y, e), im);
+    uint32_t d[S];
+    digit_pairs(a[i], e, d);
     const uint32_t off = offset(q % ROWS, 2 * (LPR * i + h), ROWS);
 #pragma unroll
-    for (int s = 0; s < S; ++s) *reinterpret_cast<uint32_t*>(tile + s * A_SLICE + off) = pack(re[s], im[s]);
+    for (int s = 0; s < S; ++s) *reinterpret_cast<uint32_t*>(tile + s * A_SLICE + off) = d[s];
   }
 }
 
@@ -133,14 +129,13 @@ __device__ __forceinline__ void write_b(unsigned char* ob, int32_t* eb, int r, i
   const int row = 2 * (r % COLS);
 #pragma unroll
   for (int i = 0; i < GJ_KB / LPR; ++i) {
-    int re[S], im[S];
-    digits(fixed(y[i].x, e), re);
-    digits(fixed(y[i].y, e), im);
+    uint32_t d[S];
+    digit_pairs(y[i], e, d);
     const int k = 2 * (LPR * i + h);
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-      *reinterpret_cast<uint32_t*>(tile + offset(2 * COLS * s + row, k, B_ROWS)) = pack(re[s], -im[s]);
-      *reinterpret_cast<uint32_t*>(tile + offset(2 * COLS * s + row + 1, k, B_ROWS)) = pack(im[s], re[s]);
+      *reinterpret_cast<uint32_t*>(tile + offset(2 * COLS * s + row, k, B_ROWS)) = d[s] ^ 0x80000000u;
+      *reinterpret_cast<uint32_t*>(tile + offset(2 * COLS * s + row + 1, k, B_ROWS)) = __funnelshift_l(d[s], d[s], 16);
     }
   }
 }

@@ -10,7 +10,8 @@
 //                       exchange and no CTA computes a reciprocal or a pivot search twice;
 //   panel_rest_kernel   what is independent per row (the rows outside the candidates replay the
 //                       steps) and per column (the pivot rows of the other columns), over as many
-//                       CTAs as there are pieces of 4 to 16 rows and columns.
+//                       CTAs as there are pieces of 4 to 16 rows and columns; trail::rest_kernel
+//                       (trail.cuh) in its place in the trailing form.
 //
 // Two forms (InvTask::trail):
 //   full   Gauss-Jordan, as inv_panel_kernel: the swept panel holds [P^-1; -a P^-1] and every other
@@ -367,44 +368,29 @@ __global__ void __launch_bounds__(PS_THREADS) panel_sweep_kernel(const InvTask* 
 }
 
 // The recorded steps replayed on a row of the panel held by LPR lanes, lane h the entries LPR i + h:
-// step k subtracts entry k times row k of `pk` (stride GJ_KB) from the entries past k (`tri`), or from
-// all others with entry k becoming -a pk[k]. Interleaved so that the lanes stay equally busy as the
-// triangle shrinks: an FP64 instruction costs the same with one active lane as with 32.
+// step k subtracts entry k times row k of `pk` (stride GJ_KB) from all others, entry k becoming -a pk[k].
 template <int LPR, typename V>
-__device__ __forceinline__ void replay_row(V (&b)[GJ_KB / LPR], const V* pk, int kb, int h, bool tri) {
+__device__ __forceinline__ void replay_row(V (&b)[GJ_KB / LPR], const V* pk, int kb, int h) {
   constexpr int Q = GJ_KB / LPR;
   const int lane = threadIdx.x & 31;
-  if (tri) {
 #pragma unroll
-    for (int k = 0; k < GJ_KB; ++k) {
-      if (k >= kb) break;
-      const V own = b[k / LPR];
-      const int src = (lane & ~(LPR - 1)) | (k % LPR);
-      const V ak = cx<V>(__shfl_sync(0xffffffffu, own.x, src), __shfl_sync(0xffffffffu, own.y, src));
-      if (h > k % LPR) b[k / LPR] = cfms_pk(b[k / LPR], ak, pk[k * GJ_KB + k / LPR * LPR + h]);
+  for (int k = 0; k < GJ_KB; ++k) {
+    if (k >= kb) break;
+    const V own = b[k / LPR];
+    const int src = (lane & ~(LPR - 1)) | (k % LPR);
+    const V ak = cx<V>(__shfl_sync(0xffffffffu, own.x, src), __shfl_sync(0xffffffffu, own.y, src));
+    if (h == k % LPR) b[k / LPR] = cx<V>(0.0, 0.0);  // entry k: 0 - a pk[k]
 #pragma unroll
-      for (int i = k / LPR + 1; i < Q; ++i) b[i] = cfms_pk(b[i], ak, pk[k * GJ_KB + LPR * i + h]);
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < GJ_KB; ++k) {
-      if (k >= kb) break;
-      const V own = b[k / LPR];
-      const int src = (lane & ~(LPR - 1)) | (k % LPR);
-      const V ak = cx<V>(__shfl_sync(0xffffffffu, own.x, src), __shfl_sync(0xffffffffu, own.y, src));
-      if (h == k % LPR) b[k / LPR] = cx<V>(0.0, 0.0);  // entry k: 0 - a pk[k]
-#pragma unroll
-      for (int i = 0; i < Q; ++i) b[i] = cfms_pk(b[i], ak, pk[k * GJ_KB + LPR * i + h]);
-    }
+    for (int i = 0; i < Q; ++i) b[i] = cfms_pk(b[i], ak, pk[k * GJ_KB + LPR * i + h]);
   }
 }
 
-// After a panel's sweep: grid (matrices, row pieces then column pieces), NT threads, LPR lanes per row or
-// column (a piece has NT / LPR of them).
+// After a panel's sweep in the full form (the trailing form: trail.cuh): grid (matrices, row pieces then
+// column pieces), NT threads, LPR lanes per row or column (a piece has NT / LPR of them).
 // Row piece: rows outside the candidates replay the recorded steps. With oa set (FP64), every row the
 // update reads also becomes an operand row.
 // Column piece: the pivot rows of the columns outside the panel into Y (or B', or the FP64 operand), the
-// displaced rows into place. In the trail form a column is first solved with L11, by the same replay.
+// displaced rows into place.
 // LPR: 16 while the pieces of 4 do not fill the GPU (a piece is then a chain of 256 FP64
 // instructions per warp instead of 1 024), 4 past that (fewer shuffles per entry).
 template <typename T, int LPR, int NT>
@@ -417,18 +403,14 @@ __global__ void __launch_bounds__(NT) panel_rest_kernel(const InvTask* __restric
   const int n = t.n, np = t.npiv;
   if (k0 >= np || *t.bad) return;
   const int kb = min(GJ_KB, np - k0);
-  const bool trail = t.trail != 0;
   const int h = threadIdx.x % LPR;
   V* A = static_cast<V*>(t.a);
   const int64_t ld = t.ld;
-  const int base = trail ? k0 + kb : 0;  // first row (and, for trail, column) of the update
   if ((int)blockIdx.y < row_pieces) {
-    const int total = n - base;
-    const int q0 = blockIdx.y * PIECE;
-    if (q0 >= total) return;
-    const int q = q0 + threadIdx.x / LPR;
-    const int row = base + q;
-    const bool act = q < total;
+    const int row0 = blockIdx.y * PIECE;
+    if (row0 >= n) return;
+    const int row = row0 + threadIdx.x / LPR;
+    const bool act = row < n;
     const bool out = act && (row < k0 || row >= np);
     const bool any = __syncthreads_or(out);
     if (any) {
@@ -446,7 +428,7 @@ __global__ void __launch_bounds__(NT) panel_rest_kernel(const InvTask* __restric
       V b[Q];
 #pragma unroll
       for (int i = 0; i < Q; ++i) b[i] = a[i];
-      replay_row<LPR>(b, sm, kb, h, trail);
+      replay_row<LPR>(b, sm, kb, h);
       if (out)
 #pragma unroll
         for (int i = 0; i < Q; ++i)
@@ -456,32 +438,18 @@ __global__ void __launch_bounds__(NT) panel_rest_kernel(const InvTask* __restric
           }
     }
     if constexpr (sizeof(T) == 8) {
-      if (t.oa) oz::write_a<LPR>(t.oa, t.ea, q, h, act, a);
+      if (t.oa) oz::write_a<LPR>(t.oa, t.ea, row, h, act, a);
     }
     return;
   }
-  const int total = (trail ? n : t.ncol) - (trail ? base : kb);
+  const int total = t.ncol - kb;
   const int c0 = ((int)blockIdx.y - row_pieces) * PIECE;
   if (c0 >= total) return;
   const int* perm = t.perm;
   const int nd = perm[3 * GJ_KB];
-  if (trail) {
-    // L11^T with each column of L11 scaled by its pivot's reciprocal (the steps then use the raw pivot-row
-    // entries), the reciprocals on the diagonal.
-    for (int e = threadIdx.x; e < kb * GJ_KB; e += NT) {
-      const int c = e & (GJ_KB - 1), k = e / GJ_KB;
-      V v = cx<V>(0.0, 0.0);
-      if (c < kb && c >= k) {
-        v = A[(k0 + c) + (int64_t)(k0 + k) * ld];
-        if (c > k) v = cmul(v, A[(k0 + k) + (int64_t)(k0 + k) * ld]);
-      }
-      sm[e] = v;
-    }
-    __syncthreads();
-  }
   const int r = c0 + threadIdx.x / LPR;
   const bool act = r < total;
-  const int j = trail ? base + r : (r < k0 ? r : r + kb);
+  const int j = r < k0 ? r : r + kb;
   V* Aj = A + (int64_t)j * ld;
   V y[Q], dv[Q];
 #pragma unroll
@@ -495,14 +463,6 @@ __global__ void __launch_bounds__(NT) panel_rest_kernel(const InvTask* __restric
   for (int i = 0; i < Q; ++i) {
     const int c = LPR * i + h;
     if (act && c < nd) Aj[k0 + perm[GJ_KB + c]] = dv[i];
-  }
-  if (trail) {
-    replay_row<LPR>(y, sm, kb, h, true);
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-      const int c = LPR * i + h;
-      if (c < kb) y[i] = cmul(y[i], sm[c + c * GJ_KB]);
-    }
   }
   if constexpr (sizeof(T) == 8) {
     if (t.ob) {

@@ -76,3 +76,22 @@ def test_batches_fill_clusters_differently():
     together = s.transmissions_with(sigmas)
     alone = [s.transmission_with(x) for x in sigmas]
     assert together == alone
+
+
+@pytest.mark.parametrize("length,width", [(30, 40), (40, 48), (26, 56), (44, 41), (33, 57), (70, 72), (36, 90)])
+def test_trailing_panels_of_many_solves(length, width):
+    """Panels of every remainder (1, 8, 9, 16, 24, 25, ... columns) with the vectors of a matrix over several
+    tiles: 330 solves take a CTA per 128 rows and columns, one takes a CTA per 32 of either. Bit for bit the same,
+    and the one against a dense inverse."""
+    s = _device(length, width, 1, length + 3 * width)
+    sigmas = [s.self_energies(e) for e in np.linspace(-0.8, 0.7, 11)]
+    alone = [s.transmission_with(x) for x in sigmas]
+    assert s.transmissions_with(sigmas * 30) == alone * 30
+    a = _dense(s, sigmas[4])
+    blk = s.system.blocks[0]
+    kept = np.concatenate([blk.left, blk.right])
+    ref = np.linalg.inv(a)[np.ix_(kept, kept)]
+    greens, st = s.plan().root_green([s._slot(sigmas[4])], [0], [len(kept)])
+    assert st[0] == 0
+    bound = len(a) * EPS * np.linalg.cond(a)  # as above
+    assert np.linalg.norm(greens[0][0] - ref) <= bound * np.linalg.norm(ref)

@@ -153,38 +153,6 @@ __device__ __forceinline__ double block_max(double v, double* red) {
   return r;
 }
 
-// Largest value, ties to the smaller index (the reference keeps the first maximum). NaN values
-// never win, so a column of NaN reports -1 and fails the pivot test.
-__device__ __forceinline__ void argmax_pair(double& v, int& i, double v2, int i2) {
-  if (v2 > v || (v2 == v && i2 < i)) { v = v2; i = i2; }
-}
-__device__ __forceinline__ int block_argmax(double v, int i, double* redv, int* redi, double* out_v) {
-  for (int o = 16; o > 0; o >>= 1) {
-    double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-    int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-    argmax_pair(v, i, v2, i2);
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
-  __syncthreads();
-  if (l == 0) { redv[w] = v; redi[w] = i; }
-  __syncthreads();
-  if (w == 0) {
-    v = l < nw ? redv[l] : -1.0;
-    i = l < nw ? redi[l] : 0x7fffffff;
-    for (int o = 16; o > 0; o >>= 1) {
-      double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-      int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-      argmax_pair(v, i, v2, i2);
-    }
-    if (l == 0) { redv[0] = v; redi[0] = i; }
-  }
-  __syncthreads();
-  int r = redi[0];
-  *out_v = redv[0];
-  __syncthreads();
-  return r;
-}
-
 // ---- assembly -----------------------------------------------------------------------------------
 // Assembly: element (i, j) of a front before its H entries is the children's handed blocks through
 // their index maps, plus z on the diagonal of the own separator, minus Σ on the root.
@@ -225,8 +193,8 @@ struct ChildBlocks {
     for (int c = 0; c < 2; ++c)
       if (a[c] >= 0 && b[c] >= 0) {
         const auto w = base[c][a[c] + (int64_t)b[c] * ld[c]];
-        v.x += (T)w.x;
-        v.y += (T)w.y;
+        v.x = c == 0 ? (T)w.x : v.x + (T)w.x;
+        v.y = c == 0 ? (T)w.y : v.y + (T)w.y;
       }
     return v;
   }
@@ -247,24 +215,51 @@ __device__ __forceinline__ void apply_entries(const JobDesc& J, const FrontDesc&
 }
 
 // ---- Gauss-Jordan sweep -------------------------------------------------------------------------
-// Largest value of a warp, ties to the smaller index (the reference keeps the first maximum); NaN
-// never wins, so a column of NaN reports -1 and fails the pivot test.
-// v is a lane's largest |c|^2 (never NaN) or -1 for no candidate. In f32 two warp reductions do
-// it: the maximum of v's bits (non-negative floats order as unsigned integers; +1 so that 0 means
-// no candidate), then the minimum index among the lanes holding it.
-template <typename T> __device__ __forceinline__ void warp_argmax(T& v, int& i) {
-  if constexpr (sizeof(T) == 4) {
-    const unsigned key = v >= 0 ? __float_as_uint((float)v) + 1u : 0u;
-    const unsigned top = __reduce_max_sync(0xffffffffu, key);
-    i = __reduce_min_sync(0xffffffffu, key == top ? i : 0x7fffffff);
-    v = top ? (T)__uint_as_float(top - 1u) : (T)-1;
-  } else {
-    for (int o = 16; o > 0; o >>= 1) {
-      const T v2 = __shfl_xor_sync(0xffffffffu, v, o);
-      const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-      if (v2 > v || (v2 == v && i2 < i)) { v = v2; i = i2; }
-    }
-  }
+// Pivot search on integers: a squared modulus as its bits + 1 (non-negative floating-point numbers order as
+// unsigned integers), 0 for no candidate and NaN. An FP64 compare or conversion holds a scheduler's FP64 pipe
+// for 64 clocks: the f32 tiny fronts, which only compared with an FP64 threshold and converted energies in
+// their loops, kept that pipe 66 % busy.
+__device__ __forceinline__ unsigned long long norm_key(double m) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(m);
+  return b <= 0x7ff0000000000000ull ? b + 1ull : 0ull;
+}
+__device__ __forceinline__ unsigned norm_key(float m) {
+  const unsigned b = __float_as_uint(m);
+  return b <= 0x7f800000u ? b + 1u : 0u;
+}
+template <typename T> using NormKey = decltype(norm_key(T()));
+// The largest key of a refused pivot: |d|^2 > thresh is key > refuse_key(thresh) (a NaN threshold refuses all).
+template <typename T> __device__ __forceinline__ NormKey<T> refuse_key(double thresh) {
+  NormKey<T> k;
+  if constexpr (sizeof(T) == 8) k = norm_key(thresh);
+  else k = norm_key(__double2float_rd(thresh));
+  return k ? k : ~(NormKey<T>)0;
+}
+template <typename T> __device__ __forceinline__ double key_norm(unsigned long long key) {
+  if constexpr (sizeof(T) == 8) return __longlong_as_double((long long)(key - 1ull));
+  else return (double)__uint_as_float((unsigned)(key - 1ull));
+}
+// The warp's largest key; `i`: its index, ties to the smaller one (the reference keeps the first maximum).
+__device__ __forceinline__ unsigned warp_top(unsigned key, int& i) {
+  const unsigned top = __reduce_max_sync(0xffffffffu, key);
+  i = __reduce_min_sync(0xffffffffu, key == top ? i : 0x7fffffff);
+  return top;
+}
+__device__ __forceinline__ unsigned long long warp_top(unsigned long long key, int& i) {
+  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+  const unsigned th = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned tl = __reduce_max_sync(0xffffffffu, hi == th ? lo : 0u);
+  i = __reduce_min_sync(0xffffffffu, hi == th && lo == tl ? i : 0x7fffffff);
+  return (unsigned long long)th << 32 | tl;
+}
+// The block's largest key (`red`: 32 words of shared memory; synchronises the block).
+template <typename K> __device__ __forceinline__ K block_top(K key, unsigned long long* red) {
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+  int i = 0;
+  key = warp_top(key, i);
+  if (l == 0) red[w] = key;
+  __syncthreads();
+  return warp_top(l < nw ? (K)red[l] : (K)0, i);
 }
 
 // In-place Gauss-Jordan sweep of the leading `npiv` columns of a rows x cols matrix F (column-major,
@@ -290,24 +285,23 @@ __device__ bool gj_sweep(typename Cx<T>::V* F, int ld, int rows, int cols, int n
                          typename Cx<T>::V* prows = nullptr) {
   using V = typename Cx<T>::V;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const double thresh = tol * tol * scale2;
+  const NormKey<T> refuse = refuse_key<T>(tol * tol * scale2);
   for (int k = 0; k < npiv; ++k) {
     const V* ck = cb + (k & 1) * rows;
     V* cn = cb + ((k + 1) & 1) * rows;
-    T best = -1;
+    NormKey<T> best = 0;
     int p = 0x7fffffff;
     for (int i = k + lane; i < cand; i += 32) {
-      const T m = cnorm(ck[i]);
-      if (m > best) { best = m; p = i; }
+      const NormKey<T> q = norm_key(cnorm(ck[i]));
+      if (q > best) { best = q; p = i; }
     }
-    warp_argmax(best, p);
-    const double big = (double)best;
+    best = warp_top(best, p);
     V d;
-    if (!(big > thresh) || p >= cand) {
+    if (!(best > refuse)) {
       // NaN or an empty column: nothing sensible to perturb.
-      if (!perturb || !(big >= 0.0) || !(scale2 > 0.0) || p >= cand) return false;
+      if (!perturb || !best || !(scale2 > 0.0)) return false;
       d = ck[p];
-      const double mag = sqrt(big), target = tol * sqrt(scale2);
+      const double mag = sqrt(key_norm<T>(best)), target = tol * sqrt(scale2);
       if (mag > 0.0) { d.x = (T)(d.x / mag * target); d.y = (T)(d.y / mag * target); }
       else { d.x = (T)target; d.y = (T)0; }
       if (threadIdx.x == 0 && perturbed) atomicAdd(perturbed, 1);
@@ -381,38 +375,31 @@ __device__ bool gj_sweep_cols(typename Cx<T>::V* F, int ld, int rows, int cols, 
   const int lane = threadIdx.x & 31;
   const int j = threadIdx.x;  // this lane's column
   const int nthreads = ((cols + 31) / 32) * 32;
-  const double thresh = tol * tol * scale2;
+  const NormKey<T> refuse = refuse_key<T>(tol * tol * scale2);
   V* Fj = F + (int64_t)j * ld;
   for (int k = 0; k < rows; ++k) {
     const V* ck = cb + (k & 1) * rows;
     V* cn = cb + ((k + 1) & 1) * rows;
-    T best = -1;
+    NormKey<T> best = 0;
     int p = 0x7fffffff;
     if (sizeof(T) == 4 && rows - k <= 32) {
-      // One candidate per lane: the largest |c|^2 by a warp max of its bits (non-negative floats
-      // order as unsigned integers; +1 so that 0 means no candidate or NaN), the smallest row
-      // among equal maxima by a ballot. Same result as the shuffle reduction below.
+      // One candidate per lane: the smallest row among equal maxima by a ballot.
       const int i = k + lane;
-      const float m = i < rows ? (float)cnorm(ck[i]) : -1.f;
-      const unsigned key = (i < rows && m == m) ? __float_as_uint(m) + 1u : 0u;
-      const unsigned top = __reduce_max_sync(0xffffffffu, key);
-      if (top != 0u) {
-        p = k + __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
-        best = (T)__uint_as_float(top - 1u);
-      }
+      const unsigned key = i < rows ? (unsigned)norm_key(cnorm(ck[i])) : 0u;
+      best = __reduce_max_sync(0xffffffffu, key);
+      p = k + __ffs(__ballot_sync(0xffffffffu, key == (unsigned)best)) - 1;
     } else {
       for (int i = k + lane; i < rows; i += 32) {
-        const T m = cnorm(ck[i]);
-        if (m > best) { best = m; p = i; }
+        const NormKey<T> q = norm_key(cnorm(ck[i]));
+        if (q > best) { best = q; p = i; }
       }
-      warp_argmax(best, p);
+      best = warp_top(best, p);
     }
-    const double big = (double)best;
     V d;
-    if (!(big > thresh) || p >= rows) {
-      if (!perturb || !(big >= 0.0) || !(scale2 > 0.0) || p >= rows) return false;
+    if (!(best > refuse)) {
+      if (!perturb || !best || !(scale2 > 0.0)) return false;
       d = ck[p];
-      const double mag = sqrt(big), target = tol * sqrt(scale2);
+      const double mag = sqrt(key_norm<T>(best)), target = tol * sqrt(scale2);
       if (mag > 0.0) { d.x = (T)(d.x / mag * target); d.y = (T)(d.y / mag * target); }
       else { d.x = (T)target; d.y = (T)0; }
       if (threadIdx.x == 0 && perturbed) atomicAdd(perturbed, 1);
@@ -569,7 +556,7 @@ __device__ __forceinline__ void small_front_body(const JobDesc* __restrict__ job
   V* prows = F + (int64_t)ld * n;
   V* cb = prows + (int64_t)ne * n;
   V* zeros = cb + 2 * n;
-  double* red = reinterpret_cast<double*>(zeros + n);
+  unsigned long long* red = reinterpret_cast<unsigned long long*>(zeros + n);
   int* piv = reinterpret_cast<int*>(red + 32);
   int* cperm = piv + n;
   int* cmap = cperm + n;  // 2 x n: child c's position of variable i, -1 where it has none
@@ -594,12 +581,10 @@ __device__ __forceinline__ void small_front_body(const JobDesc* __restrict__ job
       cmap[n + i] = a[1];
     }
     int ar[3][2];
-    bool own[3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const int i = lane + 32 * q;
-      own[q] = i < n && J.own[f.own_off + i];
-    }
+    // The energy goes to the diagonal of the warp's columns w + nw l at once, lane l (n <= 32 nw).
+    const int dj = w + nw * lane;
+    const bool own = dj < n && J.own[f.own_off + dj];
+    const T energy = (T)J.energy;
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -615,11 +600,11 @@ __device__ __forceinline__ void small_front_body(const JobDesc* __restrict__ job
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const int i = lane + 32 * q;
-        if (i >= n) continue;
-        if (i == j && own[q]) v[q].x += (T)J.energy;
-        F[i + j * ld] = v[q];
+        if (i < n) F[i + j * ld] = v[q];
       }
     }
+    __syncwarp();
+    if (own) F[dj + dj * ld].x += energy;
   }
   __syncthreads();
   if (has0) {
@@ -641,14 +626,15 @@ __device__ __forceinline__ void small_front_body(const JobDesc* __restrict__ job
       for (int i = lane; i < n; i += 32) out[i + (int64_t)j * n] = F[i + j * ld];
     return;
   }
-  T local = 0;
+  NormKey<T> local = 0;
   for (int j = w; j < ne; j += nw)
-    for (int i = lane; i < ne; i += 32) local = fmax(local, cnorm(F[i + j * ld]));
+    for (int i = lane; i < ne; i += 32) local = max(local, norm_key(cnorm(F[i + j * ld])));
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     if (i < ne) cb[i] = F[i];
     zeros[i] = cx<V>(0.0, 0.0);
   }
-  const double scale2 = block_max((double)local, red);  // also publishes cb
+  local = block_top(local, red);  // also publishes cb
+  const double scale2 = local ? key_norm<T>(local) : 0.0;
   // Pivot rows: a lane per column in the first ceil(n / 32) warps (named barrier per pivot); the
   // other warps wait at the block barrier.
   __shared__ int ok_flag;

@@ -46,13 +46,6 @@ __host__ __device__ inline size_t panel_sweep_bytes(int r, int c, size_t vbytes)
   return ((size_t)r * GJ_KB + 2 * (size_t)r + 2 * (size_t)c * GJ_KB + 2 * GJ_KB) * vbytes + 2 * (size_t)c * 16 + 16;
 }
 
-// Orders squared moduli as unsigned integers; 0: no candidate (also NaN).
-__device__ __forceinline__ unsigned long long norm_key(double m) {
-  return m >= 0.0 ? (unsigned long long)__double_as_longlong(m) + 1ull : 0ull;
-}
-__device__ __forceinline__ unsigned long long norm_key(float m) {
-  return m >= 0.f ? (unsigned long long)__float_as_uint(m) + 1ull : 0ull;
-}
 // The lane holding the largest key of the warp, ties to the smallest index; -1 when every key is 0. The
 // upper words mostly decide it: one warp reduction and a vote.
 __device__ __forceinline__ int key_argmax(unsigned long long key, int idx) {
@@ -67,16 +60,6 @@ __device__ __forceinline__ int key_argmax(unsigned long long key, int idx) {
   }
   return __ffs(in) - 1;
 }
-// The largest key a refused pivot can have: |d|^2 > thresh is key > refuse_key(thresh).
-template <typename T> __device__ __forceinline__ unsigned long long refuse_key(double thresh) {
-  if constexpr (sizeof(T) == 8) return norm_key(thresh);
-  else return norm_key(__double2float_rd(thresh));
-}
-template <typename T> __device__ __forceinline__ double key_norm(unsigned long long key) {
-  if constexpr (sizeof(T) == 8) return __longlong_as_double((long long)(key - 1ull));
-  else return (double)__uint_as_float((unsigned)(key - 1ull));
-}
-
 // Shared-memory address of the same location in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
   uint32_t r;
@@ -124,11 +107,13 @@ __global__ void __launch_bounds__(256) panel_scale_kernel(const InvTask* __restr
   const InvTask t = tasks[blockIdx.x];
   const V* A = static_cast<const V*>(t.a);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  T mt = 0;
+  NormKey<T> mt = 0;
   for (int j = blockIdx.y * 8 + w; j < t.npiv; j += gridDim.y * 8)
-    for (int i = lane; i < t.npiv; i += 32) mt = fmax(mt, cnorm(A[i + (int64_t)j * t.ld]));
-  const unsigned long long key = (unsigned long long)__double_as_longlong((double)mt);
-  if (key_argmax(key, lane) == lane && key) atomicMax(reinterpret_cast<unsigned long long*>(t.scale2), key);
+    for (int i = lane; i < t.npiv; i += 32) mt = max(mt, norm_key(cnorm(A[i + (int64_t)j * t.ld])));
+  int first = 0;
+  mt = warp_top(mt, first);
+  if (lane == 0 && mt)
+    atomicMax(reinterpret_cast<unsigned long long*>(t.scale2), (unsigned long long)__double_as_longlong(key_norm<T>(mt)));
 }
 
 // grid: matrices x cluster (clusters along x), PS_THREADS threads. R: rows per CTA.

@@ -54,13 +54,14 @@ __global__ void __launch_bounds__(256) tiny_front_kernel(const JobDesc* __restri
     int ai[2];
     kids.index(lane < n ? lane : 0, ai);
     const bool own = lane < n && J.own[f.own_off + lane];
+    const T energy = (T)J.energy;
 #pragma unroll 8
     for (int j = 0; j < n; ++j) {
       const int bj[2] = {__shfl_sync(0xffffffffu, ai[0], j), __shfl_sync(0xffffffffu, ai[1], j)};
-      V v = kids.template at<T>(ai, bj);
-      if (j == lane && own) v.x += (T)J.energy;
+      const V v = kids.template at<T>(ai, bj);
       if (lane < n) F[lane + j * LD] = v;
     }
+    if (own) F[lane + lane * LD].x += energy;
   }
   __syncwarp();
   if (has0) {
@@ -78,31 +79,25 @@ __global__ void __launch_bounds__(256) tiny_front_kernel(const JobDesc* __restri
   __syncwarp();
   V* out = static_cast<V*>(J.arena) + f.arena_off;
   if (ne > 0) {
-    T s2 = 0;
+    NormKey<T> s2 = 0;
     if (lane < ne)
-      for (int j = 0; j < ne; ++j) s2 = fmax(s2, cnorm(F[lane + j * LD]));
-    for (int o = 16; o > 0; o >>= 1) s2 = fmax(s2, __shfl_xor_sync(0xffffffffu, s2, o));
-    const double scale2 = (double)s2;
-    const double thresh = tol * tol * scale2;
+      for (int j = 0; j < ne; ++j) s2 = max(s2, norm_key(cnorm(F[lane + j * LD])));
+    int any = 0;
+    s2 = warp_top(s2, any);
+    const double scale2 = s2 ? key_norm<T>(s2) : 0.0;
+    const NormKey<T> refuse = refuse_key<T>(tol * tol * scale2);
     int mypiv = 0;  // lane k keeps piv[k]
     for (int k = 0; k < ne; ++k) {
-      T bt = (T)-1;
-      int bi = 0x7fffffff;
-      if (lane >= k && lane < ne) {
-        const T m = cnorm(F[lane + k * LD]);
-        if (m > bt) { bt = m; bi = lane; }  // NaN is no candidate
-      }
-      warp_argmax(bt, bi);
-      const double best = (double)bt;
-      int p = bi;
-      if (!(best > thresh) || p >= ne) {
-        if (!perturb || !(best >= 0.0) || !(scale2 > 0.0) || p >= ne) {
+      int p = lane;
+      const NormKey<T> best = warp_top(lane >= k && lane < ne ? norm_key(cnorm(F[lane + k * LD])) : (NormKey<T>)0, p);
+      if (!(best > refuse)) {
+        if (!perturb || !best || !(scale2 > 0.0)) {  // NaN: no candidate
           if (lane == 0) J.fail[t.front] = 1;
           return;
         }
         if (lane == 0) {
           V& d = F[p + k * LD];
-          const double mag = sqrt(best), target = tol * sqrt(scale2);
+          const double mag = sqrt(key_norm<T>(best)), target = tol * sqrt(scale2);
           if (mag > 0.0) { d.x = (T)(d.x / mag * target); d.y = (T)(d.y / mag * target); }
           else { d.x = (T)target; d.y = (T)0; }
           if (perturbed) atomicAdd(perturbed + t.job, 1);

@@ -11,6 +11,12 @@
 // but need seven products, with 48 outputs per vector to put together in place of 32, and their
 // eight operand columns are half of an MMA's K.
 //
+// Digits are cut relative to the largest entry of a row of L and of a column of U, and the pivot rows are scaled
+// by the pivots' reciprocals: behind a small pivot p, row k of U (of size 1 / p) would take its place in the
+// digits of every column, also for rows of L that are zero in column k. So the digits are taken of L D^-1 and
+// D U, D_kk the power of two next to |p_k|^(1/2): the same product, and neither side exceeds its other
+// entries by more than p^(-1/2). (U11 likewise; L11's columns are at most 1 against their pivots.)
+//
 // Measured against the whole replay on the FP64 pipe: 3 584 fronts of 16 BHZ 200 x 64 solves (first panel)
 // 1.47 -> 0.78 ms, all panels of these solves 9.0 -> 5.3 ms; the panels (with their sweeps) of two
 // 48 x 24 x 24 cubic wires 11.1 -> 9.9 ms. The FP64 pipe is then busy half of the time, one or two warps per
@@ -28,23 +34,30 @@ constexpr int B16_BYTES = oz::S * 32 * 32 * 2;  // digits of 16 complex columns 
 constexpr int SIDE = A_BYTES + 2 * B8_BYTES + B16_BYTES + GJ_KB * GJ_KB * 16;  // shared memory of the rows or the columns
 constexpr int COARSE_SMEM = 2 * SIDE + 128, FINE_SMEM = SIDE + 128;
 
+// Biased exponent of an entry times 2^shift.
+constexpr int LEAST = -4096;
+__device__ __forceinline__ int exponent(double2 v, int shift) {
+  const int e = max(1, max(oz::biased_exponent(v.x), oz::biased_exponent(v.y)));
+  return e == 0x7ff ? 2 * oz::NOT_FINITE : e + shift;
+}
+
 // Column r of the digits of a W x W block T[c0 .. c0 + W)[c0 + W ..) (row stride GJ_KB), W / 8 entries per
-// lane of eight; returns the column's exponent.
+// lane of eight, entry k times 2^(mul half[k]); returns the column's exponent.
 template <int W>
-__device__ __forceinline__ int put_block(unsigned char* dst, const double2* T, int c0, int r, int h) {
+__device__ __forceinline__ int put_block(unsigned char* dst, const double2* T, int c0, int r, int h, const int* half, int mul) {
   double2 y[W / 8];
-  int e = 1;
+  int e = LEAST;
 #pragma unroll
   for (int i = 0; i < W / 8; ++i) {
     y[i] = T[(c0 + 8 * i + h) * GJ_KB + c0 + W + r];
-    e = max(e, max(oz::biased_exponent(y[i].x), oz::biased_exponent(y[i].y)));
+    e = max(e, exponent(y[i], mul * half[c0 + 8 * i + h]));
   }
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
 #pragma unroll
   for (int i = 0; i < W / 8; ++i) {
     uint32_t d[oz::S];
-    oz::digit_pairs(y[i], e, d);
+    oz::digit_pairs(y[i], e - mul * half[c0 + 8 * i + h], d);
     const int k = 2 * (8 * i + h);
 #pragma unroll
     for (int s = 0; s < oz::S; ++s) {
@@ -52,12 +65,13 @@ __device__ __forceinline__ int put_block(unsigned char* dst, const double2* T, i
       *reinterpret_cast<uint32_t*>(dst + oz::offset(2 * W * s + 2 * r + 1, k, oz::S * 2 * W)) = __funnelshift_l(d[s], d[s], 16);
     }
   }
-  return e == 0x7ff ? oz::NOT_FINITE : e;
+  return e;
 }
 
-// Steps 8 b .. 8 b + 7 replayed on the columns up to 8 b + 7; returns the largest exponent of those columns.
+// Steps 8 b .. 8 b + 7 replayed on the columns up to 8 b + 7; returns the largest exponent
+// of those columns (times 2^(mul half[k])).
 template <int LPR, int b>
-__device__ __forceinline__ int replay_block(double2 (&v)[GJ_KB / LPR], const double2* T, int h, bool any) {
+__device__ __forceinline__ int replay_block(double2 (&v)[GJ_KB / LPR], const double2* T, int h, bool any, const int* half, int mul) {
   constexpr int C0 = B * b;
   const int lane = threadIdx.x & 31;
   if (any) {
@@ -73,9 +87,9 @@ __device__ __forceinline__ int replay_block(double2 (&v)[GJ_KB / LPR], const dou
       for (int i = k / LPR + 1; i < (C0 + B) / LPR; ++i) v[i] = cfms(v[i], ak, T[k * GJ_KB + LPR * i + h]);
     }
   }
-  int e = 1;
+  int e = LEAST;
 #pragma unroll
-  for (int i = C0 / LPR; i < (C0 + B) / LPR; ++i) e = max(e, max(oz::biased_exponent(v[i].x), oz::biased_exponent(v[i].y)));
+  for (int i = C0 / LPR; i < (C0 + B) / LPR; ++i) e = max(e, exponent(v[i], mul * half[LPR * i + h]));
 #pragma unroll
   for (int o = 1; o < LPR; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
   return e;
@@ -97,6 +111,7 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
   __shared__ uint32_t tslot;
   __shared__ __align__(8) uint64_t done[2];
   __shared__ int s_eb[2][GJ_KB];
+  __shared__ __align__(16) int s_half[GJ_KB];
   const InvTask t = tasks[blockIdx.x];
   const int n = t.n, np = t.npiv;
   if (k0 >= np || *t.bad) return;
@@ -142,11 +157,17 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
     tc::mbar_init(&done[0], 1);
     tc::mbar_init(&done[1], 1);
   }
+  if (threadIdx.x < GJ_KB) {  // half of the pivot's exponent
+    const double2 inv = static_cast<const double2*>(t.prows)[threadIdx.x * (GJ_KB + 1)];
+    s_half[threadIdx.x] = (int)threadIdx.x < kb ? (1023 - exponent(inv, 0)) >> 1 : 0;
+  }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tacc = tslot + (uint32_t)(slot * 256);
 
+  // Entry k of a row times 2^-half[k], row k of U11 and entry k of a column times 2^half[k]: see above.
+  const int inner = columns ? 0 : -1;
   bool late = false;
   uint32_t phase = 0, issued = 0;
   constexpr int NE = 4 / LPR;  // entries per lane of a group of four columns
@@ -179,14 +200,14 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
   };
   // Digits of the groups g0 .. g0 + ng - 1 as row `row` of an operand: digit s at dst + s slice, 16 bytes (four entries)
   // per store where a thread holds them.
-  auto put = [&](unsigned char* dst, uint32_t slice, int row, int rows, int g0, int ng, int e) {
+  auto put = [&](unsigned char* dst, uint32_t slice, int row, int rows, int g0, int ng, int e, int mul) {
 #pragma unroll UNROLL
     for (int g = 0; g < ng; ++g) {
       double2 o[NE];
       fetch(g0 + g, o);
       uint32_t d[NE][oz::S];
 #pragma unroll
-      for (int i = 0; i < NE; ++i) oz::digit_pairs(o[i], e, d[i]);
+      for (int i = 0; i < NE; ++i) oz::digit_pairs(o[i], e - mul * s_half[4 * (g0 + g) + LPR * i + h], d[i]);
       unsigned char* at = dst + oz::offset(row, 8 * g + 2 * h, rows);
 #pragma unroll
       for (int s = 0; s < oz::S; ++s) {
@@ -199,8 +220,7 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
   // A', the MMAs of a digit of A' with all digits of B' it still meets (level sums of 2 W columns), the sums put
   // together.
   auto product = [&](int c0, int W, const unsigned char* sb, const int* eb, int e) {
-    put(sa, 128 * 4 * W, m, 128, c0 / 4, W / 4, e);
-    if (e == 0x7ff) e = oz::NOT_FINITE;
+    put(sa, 128 * 4 * W, m, 128, c0 / 4, W / 4, e, inner);
     tc::fence_smem_async();
     tc::fence_before_sync();
     side_sync();
@@ -272,8 +292,8 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
     int* eb = s_eb[slot];
     {
       const int r = tid >> 3, h8 = tid & 7;
-      const int e16 = put_block<16>(sb16, T, 0, r, h8);
-      const int e8 = put_block<8>(sb8 + (tid >> 6) * B8_BYTES, T, 16 * (tid >> 6), r & 7, h8);
+      const int e16 = put_block<16>(sb16, T, 0, r, h8, s_half, -inner);
+      const int e8 = put_block<8>(sb8 + (tid >> 6) * B8_BYTES, T, 16 * (tid >> 6), r & 7, h8, s_half, -inner);
       if (h8 == 0) {
         eb[r] = e16;
         eb[16 + r] = e8;
@@ -281,7 +301,7 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
     }
     // A warp without vectors to solve only takes part in the barriers.
     const bool any = __any_sync(0xffffffffu, out);
-    int e0 = 1;  // largest exponent of the block solved last
+    int e0 = LEAST;  // largest exponent of the block solved last
 #pragma unroll 1
     for (int b = 0; b < GJ_KB / B && B * b < kb; ++b) {
       if (b > 0) {
@@ -289,10 +309,10 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
         product(b == 3 ? 16 : 0, wide ? 16 : 8, wide ? sb16 : sb8 + (b >> 1) * B8_BYTES, eb + (wide ? 0 : 16 + 8 * (b >> 1)), e0);
       }
       switch (b) {
-        case 0: e0 = replay_block<LPR, 0>(v, T, h, any); break;
-        case 1: e0 = max(e0, replay_block<LPR, 1>(v, T, h, any)); break;
-        case 2: e0 = replay_block<LPR, 2>(v, T, h, any); break;
-        default: e0 = replay_block<LPR, 3>(v, T, h, any); break;
+        case 0: e0 = replay_block<LPR, 0>(v, T, h, any, s_half, inner); break;
+        case 1: e0 = max(e0, replay_block<LPR, 1>(v, T, h, any, s_half, inner)); break;
+        case 2: e0 = replay_block<LPR, 2>(v, T, h, any, s_half, inner); break;
+        default: e0 = replay_block<LPR, 3>(v, T, h, any, s_half, inner); break;
       }
     }
     if (late && lane == 0) status[t.job] = ST_TIMEOUT;
@@ -316,14 +336,15 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
       v[i] = c < kb ? Ar[(int64_t)c * ld] : make_double2(0.0, 0.0);
     }
   }
-  int e = 1;
+  const int outer = columns ? 1 : -1;
+  int e = LEAST;
 #pragma unroll
-  for (int i = 0; i < Q; ++i) e = max(e, max(oz::biased_exponent(v[i].x), oz::biased_exponent(v[i].y)));
+  for (int i = 0; i < Q; ++i) e = max(e, exponent(v[i], outer * s_half[LPR * i + h]));
 #pragma unroll
   for (int o = 1; o < LPR; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
-  if (act && h == 0) (columns ? t.eb : t.ea)[q] = e == 0x7ff ? oz::NOT_FINITE : e;
+  if (act && h == 0) (columns ? t.eb : t.ea)[q] = e;
   if (act && !columns) {
-    put(t.oa + (size_t)(q / oz::ROWS) * oz::A_TILE, oz::A_SLICE, q % oz::ROWS, oz::ROWS, 0, GJ_KB / 4, e);
+    put(t.oa + (size_t)(q / oz::ROWS) * oz::A_TILE, oz::A_SLICE, q % oz::ROWS, oz::ROWS, 0, GJ_KB / 4, e, outer);
   } else if (act) {  // rows (re, -im) and (im, re) of every digit (oz::write_b)
     unsigned char* tile = t.ob + (size_t)(q / oz::COLS) * oz::B_TILE;
 #pragma unroll UNROLL
@@ -332,7 +353,7 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
       fetch(g, o);
       uint32_t d[NE][oz::S];
 #pragma unroll
-      for (int i = 0; i < NE; ++i) oz::digit_pairs(o[i], e, d[i]);
+      for (int i = 0; i < NE; ++i) oz::digit_pairs(o[i], e - s_half[4 * g + LPR * i + h], d[i]);
 #pragma unroll
       for (int s = 0; s < oz::S; ++s)
 #pragma unroll

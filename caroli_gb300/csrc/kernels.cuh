@@ -133,6 +133,13 @@ template <> __device__ __forceinline__ double2 cinv<double2>(double2 a) {
 template <typename V> __device__ __forceinline__ double cabs2(V a) {
   return (double)a.x * (double)a.x + (double)a.y * (double)a.y;
 }
+// f32 to FP64 on integers: GB300 converts two numbers per clock and SM, the rate of an FP64 multiply-add. The
+// same result; what is neither zero nor normal in f32 takes the instruction.
+__device__ __forceinline__ double wide(float x) {
+  const unsigned b = __float_as_uint(x), a = b & 0x7fffffffu;
+  if (a - 0x00800000u >= 0x7f000000u && a != 0u) return (double)x;
+  return __hiloint2double((int)((b & 0x80000000u) | (a ? (a >> 3) + 0x38000000u : 0u)), (int)(b << 29));
+}
 template <typename V> __device__ __forceinline__ V from64(double2 z) { return cx<V>(z.x, z.y); }
 
 // ---- block reductions -------------------------------------------------------------------------

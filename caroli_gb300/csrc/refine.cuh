@@ -78,6 +78,34 @@ constexpr int GM_M = 12;  // Arnoldi steps per outer step
 
 __device__ __forceinline__ float2 f2(double2 v) { return make_float2((float)v.x, (float)v.y); }
 
+// acc - h z with z in f32. Most entries of a Hamiltonian are real or imaginary: two FP64 multiply-adds in place
+// of four, the same sums (the others add a zero). With the operands converted on integers too, an entry costs
+// two FP64 instructions where it cost six; these products are bound by that pipe. (Residuals and matvecs of 128
+// BHZ 200 x 64 solves 4.6 -> 3.5 ms, of 30 graphene ribbons 3.6 -> 3.0; where disorder mixes both kinds in a warp,
+// BHZ 100 x 40 with random moments, 1.26 -> 1.33. One vote per warp instead of a branch per lane gave 3.5 and 1.33.)
+__device__ __forceinline__ bool is_zero(double x) { return ((unsigned)__double2hiint(x) << 1 | (unsigned)__double2loint(x)) == 0u; }
+__device__ __forceinline__ double2 cfms_axis(double2 acc, double2 h, float2 z) {
+  const bool real = is_zero(h.y);
+  if (real || is_zero(h.x)) {
+    const double g = real ? -h.x : -h.y;
+    acc.x = fma(g, wide(real ? z.x : -z.y), acc.x);
+    acc.y = fma(g, wide(real ? z.y : z.x), acc.y);
+    return acc;
+  }
+  return cfms(acc, h, make_double2(wide(z.x), wide(z.y)));
+}
+// acc + h x.
+__device__ __forceinline__ double2 cfma_axis(double2 acc, double2 h, double2 x) {
+  const bool real = is_zero(h.y);
+  if (real || is_zero(h.x)) {
+    const double g = real ? h.x : h.y;
+    acc.x = fma(g, real ? x.x : -x.y, acc.x);
+    acc.y = fma(g, real ? x.y : x.x, acc.y);
+    return acc;
+  }
+  return cfma(acc, h, x);
+}
+
 // Right-hand side B[i, j]: the explicit one, else W_L on the left slice (columns below cl) and
 // W_R on the right slice.
 __device__ __forceinline__ double2 rhs_at(const RefineDesc& R, int i, int j) {
@@ -126,7 +154,7 @@ __global__ void __launch_bounds__(256) refine_residual_kernel(RefineDesc* __rest
     double2 acc = rhs_at(R, i, j);
     acc.x -= R.energy * xj[i].x;
     acc.y -= R.energy * xj[i].y;
-    for (int q = R.csr_ptr[i]; q < R.csr_ptr[i + 1]; ++q) acc = cfma(acc, R.vals[R.csr_q[q]], xj[R.csr_col[q]]);
+    for (int q = R.csr_ptr[i]; q < R.csr_ptr[i + 1]; ++q) acc = cfma_axis(acc, R.vals[R.csr_q[q]], xj[R.csr_col[q]]);
     R.r[i + (int64_t)j * R.nblk] = acc;  // + Σ_L x + Σ_R x on the slices: slice products
   }
 }
@@ -280,7 +308,7 @@ __global__ void __launch_bounds__(256) gm_start_kernel(RefineDesc* __restrict__ 
   if (R.done || j >= R.c) return;
   const double2* r = R.r + (int64_t)j * R.nblk;
   double ss = 0.0;
-  for (int i = threadIdx.x; i < R.nblk; i += blockDim.x) ss += r[i].x * r[i].x + r[i].y * r[i].y;
+  for (int i = threadIdx.x; i < R.nblk; i += blockDim.x) ss = fma(r[i].x, r[i].x, fma(r[i].y, r[i].y, ss));
   const double beta = sqrt(block_sum(ss, red));
   const double inv = beta > 0.0 ? 1.0 / beta : 0.0;
   double2* v0 = R.V + (int64_t)j * R.nblk;
@@ -309,11 +337,9 @@ __global__ void __launch_bounds__(256) gm_matvec_kernel(RefineDesc* __restrict__
   double2* W = R.V + (int64_t)(k + 1) * R.nblk * R.c;
   for (int j = 0; j < R.c; ++j) {
     const float2* zj = Zk + (int64_t)j * R.nblk;
-    auto zd = [&](int q) { return make_double2((double)zj[q].x, (double)zj[q].y); };
-    double2 acc = zd(i);
-    acc.x *= R.energy;
-    acc.y *= R.energy;
-    for (int q = R.csr_ptr[i]; q < R.csr_ptr[i + 1]; ++q) acc = cfms(acc, R.vals[R.csr_q[q]], zd(R.csr_col[q]));
+    const float2 zi = zj[i];
+    double2 acc = make_double2(R.energy * wide(zi.x), R.energy * wide(zi.y));
+    for (int q = R.csr_ptr[i]; q < R.csr_ptr[i + 1]; ++q) acc = cfms_axis(acc, R.vals[R.csr_q[q]], zj[R.csr_col[q]]);
     W[i + (int64_t)j * R.nblk] = acc;  // - Σ_L z - Σ_R z on the slices: slice products
   }
 }
@@ -330,9 +356,9 @@ __global__ void __launch_bounds__(256) gm_dot_kernel(RefineDesc* __restrict__ rd
   const double2* w = R.V + (int64_t)(k + 1) * R.nblk * R.c + (int64_t)j * R.nblk;
   double re = 0.0, im = 0.0;
   for (int q = threadIdx.x; q < R.nblk; q += blockDim.x) {
-    const double2 p = cconj_mul(v[q], w[q]);
-    re += p.x;
-    im += p.y;
+    const double2 a = v[q], b = w[q];
+    re = fma(a.x, b.x, fma(a.y, b.y, re));
+    im = fma(a.x, b.y, fma(-a.y, b.x, im));
   }
   re = block_sum(re, red);
   im = block_sum(im, red);
@@ -371,7 +397,7 @@ __global__ void __launch_bounds__(256) gm_norm_kernel(RefineDesc* __restrict__ r
   if (R.done || R.inner_done || j >= R.c || R.col_done[j] != 0) return;
   double2* w = R.V + (int64_t)(k + 1) * R.nblk * R.c + (int64_t)j * R.nblk;
   double ss = 0.0;
-  for (int q = threadIdx.x; q < R.nblk; q += blockDim.x) ss += w[q].x * w[q].x + w[q].y * w[q].y;
+  for (int q = threadIdx.x; q < R.nblk; q += blockDim.x) ss = fma(w[q].x, w[q].x, fma(w[q].y, w[q].y, ss));
   const double nrm = sqrt(block_sum(ss, red));
   const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
   for (int q = threadIdx.x; q < R.nblk; q += blockDim.x) w[q] = make_double2(w[q].x * inv, w[q].y * inv);
@@ -471,12 +497,12 @@ __global__ void __launch_bounds__(256) gm_update_kernel(RefineDesc* __restrict__
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (t0 + u < steps)
-          acc = cfma(acc, R.y[(int64_t)j * GM_M + t0 + u], make_double2((double)zv[u].x, (double)zv[u].y));
+          acc = cfma(acc, R.y[(int64_t)j * GM_M + t0 + u], make_double2(wide(zv[u].x), wide(zv[u].y)));
     }
     const int64_t o = q + (int64_t)j * R.nblk;
     R.x[o].x += acc.x;
     R.x[o].y += acc.y;
-    R.d[o] = make_float2((float)acc.x, (float)acc.y);
+    R.d[o] = f2(acc);
   }
 }
 

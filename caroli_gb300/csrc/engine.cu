@@ -1962,40 +1962,40 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       if (!count || nmax <= 0 || pmax <= 0) return;
       if constexpr (std::is_same<TT, double>::value) {
         sweep_f64(first, count, nmax, pmax, tol, cls == K_PANEL, cls, flops, ucls, uflops, ubytes);
-        return;
-      }
-      const size_t sm = panel_smem(pmax, sizeof(VV));
-      const size_t smf = (size_t)finish_bytes(pmax);
-      if (!sm || smf > (size_t)SMEM_LIMIT) throw CudaError{cudaErrorInvalidValue, "front too large for a panel sweep"};
-      const int panels = (pmax + GJ_KB - 1) / GJ_KB;
-      const double per = flops / panels;
-      const double uper = uflops / panels, ubper = ubytes / panels;
-      scale_of(TT{}, first, count, pmax, cls);
-      for (int k0 = 0; k0 < pmax; k0 += GJ_KB) {
-        launch(cls, per, 0.0, [&] {
-          inv_panel_kernel<TT><<<(unsigned)count, 256, sm, s>>>(dinv + first, k0, tol, perturb, (int)sm);
-        });
-        // Pieces of 64 rows and columns, or of 16 while those leave SMs without work.
-        const bool fine = (size_t)((nmax + 63) / 64) * 2 * count < (size_t)(4 * SM_COUNT);
-        const unsigned rp = (unsigned)((nmax + (fine ? 15 : 63)) / (fine ? 16 : 64));
-        launch(cls, 0.0, 0.0, [&] {
-          if (fine) panel_rest_kernel<TT, 4, 64><<<dim3((unsigned)count, 2 * rp), 64, 0, s>>>(dinv + first, k0, (int)rp);
-          else panel_rest_kernel<TT, 4, 256><<<dim3((unsigned)count, 2 * rp), 256, 0, s>>>(dinv + first, k0, (int)rp);
-        });
-        const unsigned rt = (unsigned)((nmax + 63) / 64);
-        in_pieces(count, [&](size_t f0, size_t c) {
-          launch(ucls, uper * c / count, ubper * c / count, [&] {
-            if (std::is_same<TT, float>::value && ctx->tensor_cores && ctx->tc_choice)
-              tc_update_kernel<<<dim3((unsigned)((nmax + TCU_ROWS - 1) / TCU_ROWS), (unsigned)c,
-                                      (unsigned)((nmax + TCU_COLS * TCU_GROUP - 1) / (TCU_COLS * TCU_GROUP))),
-                                 TCU_THREADS, TCU_SMEM, s>>>(
-                  dinv + first + f0, k0, status, ctx->tc_wait_limit);
-            else
-              inv_update_kernel<TT><<<dim3(rt, rt, (unsigned)c), 256, 0, s>>>(dinv + first + f0, k0);
+      } else {
+        const size_t sm = panel_smem(pmax, sizeof(VV));
+        const size_t smf = (size_t)finish_bytes(pmax);
+        if (!sm || smf > (size_t)SMEM_LIMIT) throw CudaError{cudaErrorInvalidValue, "front too large for a panel sweep"};
+        const int panels = (pmax + GJ_KB - 1) / GJ_KB;
+        const double per = flops / panels;
+        const double uper = uflops / panels, ubper = ubytes / panels;
+        scale_of(TT{}, first, count, pmax, cls);
+        for (int k0 = 0; k0 < pmax; k0 += GJ_KB) {
+          launch(cls, per, 0.0, [&] {
+            inv_panel_kernel<TT><<<(unsigned)count, 256, sm, s>>>(dinv + first, k0, tol, perturb, (int)sm);
           });
-        });
+          // Pieces of 64 rows and columns, or of 16 while those leave SMs without work.
+          const bool fine = (size_t)((nmax + 63) / 64) * 2 * count < (size_t)(4 * SM_COUNT);
+          const unsigned rp = (unsigned)((nmax + (fine ? 15 : 63)) / (fine ? 16 : 64));
+          launch(cls, 0.0, 0.0, [&] {
+            if (fine) panel_rest_kernel<TT, 4, 64><<<dim3((unsigned)count, 2 * rp), 64, 0, s>>>(dinv + first, k0, (int)rp);
+            else panel_rest_kernel<TT, 4, 256><<<dim3((unsigned)count, 2 * rp), 256, 0, s>>>(dinv + first, k0, (int)rp);
+          });
+          const unsigned rt = (unsigned)((nmax + 63) / 64);
+          in_pieces(count, [&](size_t f0, size_t c) {
+            launch(ucls, uper * c / count, ubper * c / count, [&] {
+              if (std::is_same<TT, float>::value && ctx->tensor_cores && ctx->tc_choice)
+                tc_update_kernel<<<dim3((unsigned)((nmax + TCU_ROWS - 1) / TCU_ROWS), (unsigned)c,
+                                        (unsigned)((nmax + TCU_COLS * TCU_GROUP - 1) / (TCU_COLS * TCU_GROUP))),
+                                   TCU_THREADS, TCU_SMEM, s>>>(
+                    dinv + first + f0, k0, status, ctx->tc_wait_limit);
+              else
+                inv_update_kernel<TT><<<dim3(rt, rt, (unsigned)c), 256, 0, s>>>(dinv + first + f0, k0);
+            });
+          });
+        }
+        finish_of(TT{}, first, count, nmax, smf, cls);
       }
-      finish_of(TT{}, first, count, nmax, smf, cls);
     };
 
     const int perturb = mixed ? 1 : 0;

@@ -500,8 +500,9 @@ __device__ __forceinline__ void replay_boundary(typename Cx<T>::V* F, int ld, in
 // complement in `out`: eight lanes per row, lane h the entries h + 8 i, four rows per warp. Step k updates
 // the entries past k only. An FP64 instruction costs the same with one active lane as with 32, and these fronts
 // are bound by that pipe: against whole rows per warp (replay_boundary), 64 lanes' worth for 33 columns and
-// every column at every step, the small and tiny fronts of 16 BHZ 200 x 64 solves took 9.13 ms, now 8.71 (with
-// four warps per front), those of graphene over 64 energies 0.95, now 0.87.
+// every column at every step, the small and tiny fronts of 16 BHZ 200 x 64 solves took 9.13 ms, then 8.71 (with
+// four warps per front; 6.8 with what followed: integer pivot keys, tiny.cuh), those of graphene over 64 energies
+// 0.95, then 0.87 (0.69).
 __device__ __forceinline__ void replay_schur(const double2* F, int ld, int n, int ne, const double2* prows, double2* out) {
   constexpr int Q = 8;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, h = lane & 7;

@@ -22,8 +22,8 @@
 //          of the scaled pivot rows); L11 with the reciprocals of the pivots on its diagonal.
 // Measured with ozaki.cuh against the former FP64 path (one CTA per matrix and panel, rank-32 updates on
 // the FP64 pipe, every row and column updated): panels + updates of two 48 x 24 x 24 cubic wires (fronts
-// up to 1 728, root 1 152) 337 -> 25 ms, of 16 BHZ 200 x 64 solves (fronts up to 384) 88 -> 17 ms, of one
-// 32 x 32 square (fronts up to 94) 1.57 -> 0.38 ms.
+// up to 1 728, root 1 152) 337 -> 24 ms, of 16 BHZ 200 x 64 solves (fronts up to 384) 88 -> 13 ms, of one
+// 32 x 32 square (fronts up to 94) 1.57 -> 0.39 ms.
 //
 // The pivots (largest modulus among the candidate rows, ties to the smaller row) and the test
 // |pivot| > tol max|F11| are those of inv_panel_kernel.

@@ -128,21 +128,8 @@ __device__ __forceinline__ float2* sweep_dst(const RefineDesc& R, int dst) {
   return dst < 0 ? R.d : R.Z + (int64_t)dst * R.nblk * R.c;
 }
 
-// x += d, then the FP64 residual r = B - A x of every row: grid (jobs, row chunks of 256). The
-// residual kernel applies B - (z - H) x; the slices' Σ x follow as slice products (ozgemm.cuh).
-__global__ void __launch_bounds__(256) refine_update_kernel(RefineDesc* __restrict__ rd) {
-  RefineDesc& R = rd[blockIdx.x];
-  if (R.done) return;
-  const int i = blockIdx.y * 256 + threadIdx.x;
-  if (i >= R.nblk) return;
-  for (int j = 0; j < R.c; ++j) {
-    const int64_t q = i + (int64_t)j * R.nblk;
-    const float2 dv = R.d[q];
-    R.x[q].x += (double)dv.x;
-    R.x[q].y += (double)dv.y;
-  }
-}
-
+// The FP64 residual r = B - A x of every row: grid (jobs, row chunks of 256). This kernel applies B - (z - H) x;
+// the slices' Σ x follow as slice products (ozgemm.cuh).
 __global__ void __launch_bounds__(256) refine_residual_kernel(RefineDesc* __restrict__ rd,
                                                               const int32_t* __restrict__ jl) {
   const RefineDesc& R = rd[jl[blockIdx.x]];

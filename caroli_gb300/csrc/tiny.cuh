@@ -116,9 +116,9 @@ __global__ void __launch_bounds__(256) tiny_front_kernel(const JobDesc* __restri
       __syncwarp();
       if constexpr (!KEEP && sizeof(T) == 8) {
         // Only the Schur complement is wanted: the m x m entries past k, dealt out to the lanes two at a time
-        // (an FP64 instruction costs the same for one lane as for 32; a lane per row left those of the rows
+        // (an FP64 instruction costs the same for one lane as for 32). (A lane per row left those of the rows
         // up to k and past n idle: the FP64 tiny fronts of 16 BHZ 200 x 64 solves took 2.7 ms, now 2.1; the small and
-        // tiny ones of one 32 x 32 square 0.40, now 0.37).
+        // tiny ones of one 32 x 32 square 0.40, now 0.37.)
         const int m = n - k - 1;
         if (m > 0) {
           const int dc = 32 / m, dr = 32 - dc * m;

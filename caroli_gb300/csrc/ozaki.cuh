@@ -204,7 +204,7 @@ __device__ __forceinline__ void mma_tile(uint32_t acc, const unsigned char* sa, 
 // rate; a 128 x 32 x 16 MMA per digit pair took 53 clocks, 6 000 per tile) into one of two sets of seven
 // 32-column accumulators, warps 2-17 (four per lane quarter, four complex columns each) add the other set's
 // tile to the old values (zero on the pivot rows of the full form): their FP64 adds, the only FP64 work
-// left, keep that pipe 62 % busy, the bound. Two sets of 32-column tiles would not
+// left, keep that pipe 50 to 62 % busy, the bound. Two sets of 32-column tiles would not
 // fit in tensor memory. Waits are bounded as in tc_update_kernel. grid (row tiles, matrices, column groups).
 __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __restrict__ tasks, int k0, int group,
                                                             int32_t* __restrict__ status) {

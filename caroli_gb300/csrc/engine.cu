@@ -541,7 +541,16 @@ struct LevelRange {
   int max_ne;            // bound on the eliminated variables of the others
 };
 
-// FP64 iterative refinement of the jobs [begin, begin + cj) after their f32 factorization.
+// Gradients solve to this fraction of the refinement's tolerances, forward and adjoint: dT/dV_a = 2 Re Σ x conj(z)
+// adds the errors of two solves where single entries cancel. At the tolerances themselves the relative error of
+// dT/dV (2-norm) was 1.5e-11 in the median and up to 1.2e-9 over 60 BHZ devices with random moments, in directions set
+// by the rounding of the f32 factors, so that another order of their sums moved dT/dV by as much; at a hundredth of them
+// 1.4e-13 and 2.6e-11. It costs about a tenth more Arnoldi steps (16 solves of BHZ 100 x 40: 14.1 -> 15.2 ms; more
+// where a solve needs another outer step for it).
+constexpr double GRAD_TIGHTER = 1e-2;
+
+// FP64 iterative refinement of the jobs [begin, begin + cj) after their f32 factorization. `tighter`: the fraction of
+// the context's tolerances to aim at.
 template <typename LaunchT>
 RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, size_t begin, size_t cj,
                    const std::vector<LevelRange>& lr, int max_root, const Task* dtasks, const std::vector<JobDesc>& jd,
@@ -549,7 +558,7 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
                    const std::vector<size_t>& root_off, LaunchT& launch, std::vector<double>& th,
                    std::vector<double>& eh, std::vector<int32_t>& sh, std::vector<int32_t>& ih, RefineBufs& rb,
                    int adjoint, const std::vector<const double2*>& rhs, const StatesRequest* states = nullptr,
-                   bool allow_giveup = false) {
+                   bool allow_giveup = false, double tighter = 1.0) {
   cudaStream_t s = ctx->stream;
   std::vector<RefineDesc> rdh(cj);
   size_t xo = 0, to = 0, ho = 0;
@@ -1102,7 +1111,7 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
       });
       in_pieces(nl, [&](size_t f0, size_t c) {
         launch(K_REF_GMRES, 0.0, vec_pass * 3.0 * c / cj,
-               [&] { gm_norm_kernel<<<dim3((unsigned)c, cols), 256, 0, s>>>(drd, jl + f0, k, ctx->inner_tol); });
+               [&] { gm_norm_kernel<<<dim3((unsigned)c, cols), 256, 0, s>>>(drd, jl + f0, k, ctx->inner_tol * tighter); });
       });
       launch(K_REF_GMRES, 0.0, 0.0, [&] {
         gm_inner_check_kernel<<<(unsigned)((cj + 127) / 128), 128, 0, s>>>(drd, (int)cj, k, gflags);
@@ -1136,7 +1145,8 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
     slice_products(2, 0, K_REF_CHECK, ojobs, no);
     launch(K_REF_CHECK, 0.0, 0.0, [&] { refine_sums_kernel<<<dim3((unsigned)cj, CHECK_PARTS), 256, 0, s>>>(drd, csum); });
     launch(K_REF_CHECK, 0.0, 0.0, [&] {
-      refine_check_kernel<<<(unsigned)cj, 32, 0, s>>>(drd, csum, ctx->refine_tol, ctx->max_iters, rt_out, rerr, rdone);
+      refine_check_kernel<<<(unsigned)cj, 32, 0, s>>>(drd, csum, ctx->refine_tol * tighter, ctx->refine_tol, ctx->max_iters,
+                                                      rt_out, rerr, rdone);
     });
     compact(0);
     CK(cudaMemcpyAsync(dh.data(), rdone, cj * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -1354,7 +1364,7 @@ void gradient(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, s
   });
   std::vector<double> tz(cj), ez(cj);
   RefineDesc* adj = refine(ctx, sys, specs, begin, cj, lr, max_root, dtasks, jd, arena, arena_off, rarena, root_off,
-                           launch, tz, ez, sh, ih, ctx->rb[1], 1, rhs_ptr);
+                           launch, tz, ez, sh, ih, ctx->rb[1], 1, rhs_ptr, nullptr, false, GRAD_TIGHTER);
   in_pieces(cj, [&](size_t f0, size_t c) {
     launch(K_REF_RES, 0.0, 0.0, [&] {
       grad_v_kernel<<<dim3((unsigned)c, rows), 256, 0, s>>>(fwd + f0, adj + f0,
@@ -2263,7 +2273,8 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
         // Transmissions only: a stalled solve is recomputed in FP64 there (not so for gradients and
         // states, whose callers receive the stalled status).
         RefineDesc* fwd = refine(ctx, sys, specs, begin, cj, lr, max_root, dtasks, jd, arena, arena_off, rarena,
-                                 root_off, launch, th, eh, sh, ih, ctx->rb[0], 0, {}, states, !grad && !states);
+                                 root_off, launch, th, eh, sh, ih, ctx->rb[0], 0, {}, states, !grad && !states,
+                                 grad ? GRAD_TIGHTER : 1.0);
         for (size_t j = 0; j < cj && j < ctx->steps_tmp.size(); ++j) out[begin + j].steps = ctx->steps_tmp[j];
         if (grad) gradient(ctx, sys, specs, begin, cj, lr, max_root, dtasks, jd, arena, arena_off, rarena, root_off,
                            launch, th, eh, sh, ih, fwd, *grad, out);

@@ -149,8 +149,8 @@ __global__ void __launch_bounds__(256) refine_residual_kernel(RefineDesc* __rest
 // T = Σ_j x_Lj^† Γ_L x_Lj and the relative size of the last correction on the left slice (the only
 // rows T depends on); convergence decision. After a GMRES correction reaching inner relative
 // residual rho, the remaining relative error of x_L is about corr * rho: converged when that is
-// below `tol`; stalled when not finite, growing, or out of outer steps. Error estimate
-// |T| * 2 * corr * rho.
+// below `goal`; stalled when not finite, growing, or out of outer steps before it is below `tol`
+// (goal <= tol: a solve that cannot reach its goal is accepted at tol). Error estimate |T| * 2 * corr * rho.
 // The sums of the check of every job: part[(job * CHECK_PARTS + y) * 3 + (T, |d|^2, |x|^2)] over the elements
 // of part y. grid (jobs, CHECK_PARTS): with convergence on the whole vector there are nblk x c elements, and
 // one CTA per job took 1.1 ms for 16 jobs of 16 384 x 21 (the FP64 pipe of 16 SMs).
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256) refine_sums_kernel(const RefineDesc* __re
 
 // The decision from those sums: a warp per job.
 __global__ void __launch_bounds__(32) refine_check_kernel(RefineDesc* __restrict__ rd, const double* __restrict__ part,
-                                                          double tol, int max_iters, double* __restrict__ t_out,
+                                                          double goal, double tol, int max_iters, double* __restrict__ t_out,
                                                           double* __restrict__ err_out, int32_t* __restrict__ done_out) {
   RefineDesc& R = rd[blockIdx.x];
   if (R.done) {
@@ -218,13 +218,13 @@ __global__ void __launch_bounds__(32) refine_check_kernel(RefineDesc* __restrict
     const bool finite = isfinite(sum[0]) && isfinite(corr);
     // After a GMRES step the remaining error is about corr times the inner residual reached.
     const double rho = R.inner_res;
-    const bool conv = finite && (corr == 0.0 || corr * rho <= tol);
-    const bool stall = !finite || (!conv && R.iters >= max_iters) || (R.iters > 2 && corr > prev);
+    const bool reached = finite && (corr == 0.0 || corr * rho <= goal);
+    const bool stop = !finite || R.iters >= max_iters || (R.iters > 2 && corr > prev);
     R.corr = corr;
     R.err = fabs(sum[0]) * 2.0 * corr * rho;
-    if (conv || stall) {
+    if (reached || stop) {
       R.done = 1;
-      R.stalled = stall && !conv;
+      R.stalled = !(finite && (corr == 0.0 || corr * rho <= tol));
     }
     t_out[blockIdx.x] = sum[0];
     err_out[blockIdx.x] = R.err;

@@ -348,6 +348,7 @@ int caroli_last_refine_steps(const caroli_ctx* ctx, int64_t* job_steps, int64_t*
 /* Refinement controls of CAROLI_MIXED (defaults 6, 1e-10, 1e-10): at most max_iters outer steps
  * (FP64 residual, GMRES on the f32 factors), done when the estimated relative error of the left
  * slice of the solution is at most tol; each GMRES runs until its residual falls by inner_tol.
+ * caroli_transmission_with_grad aims at a hundredth of both and accepts tol where it cannot reach that.
  * No reference counterpart (precision::PrecisionOptions covers only the double recomputation). */
 int caroli_set_refine_options(caroli_ctx* ctx, int max_iters, double tol, double inner_tol);
 

@@ -102,3 +102,43 @@ def test_gradient_workload_64_sites():
         assert abs(dv[0, a] - fd) <= 1e-4 * abs(fd) + 1e-5, (a, dv[0, a], fd)
     fdj = (tt[-2] - tt[-1]) / (2 * h)
     assert abs(dp[0, 0] - fdj) <= 1e-4 * abs(fdj) + 1e-5
+
+
+def _dense_gradient(sys_, sigma, config, dh):
+    """T, dT/dV of every orbital and dT/dJ from a dense inverse, and cond(A)."""
+    s = sys_.system
+    rows, cols = np.repeat(np.arange(s.n), np.diff(s.row_ptr)), s.cols.astype(int)
+    a = np.zeros((s.n, s.n), complex)
+    a[rows, cols] = -s.values[config]
+    a[np.arange(s.n), np.arange(s.n)] += sigma.energy
+    gl, gr = (np.zeros((s.n, s.n), complex) for _ in range(2))
+    for blk, (sl, sr) in zip(s.blocks, sigma.blocks):
+        a[np.ix_(blk.left, blk.left)] -= sl
+        a[np.ix_(blk.right, blk.right)] -= sr
+        gl[np.ix_(blk.left, blk.left)] = 1j * (sl - sl.conj().T)
+        gr[np.ix_(blk.right, blk.right)] = 1j * (sr - sr.conj().T)
+    g = np.linalg.inv(a)
+    k = g @ gr @ g.conj().T @ gl @ g  # dT = 2 Re Tr[K dH]
+    full = np.zeros((s.n, s.n), complex)
+    full[rows, cols] = dh
+    return np.trace(gl @ g @ gr @ g.conj().T).real, 2.0 * np.diag(k).real, 2.0 * np.sum(k * full.T).real, np.linalg.cond(a)
+
+
+# Each of the two solves of a gradient aims at a relative error of 1e-12 in the norm of its vectors; their products
+# cancel to some extent in dT/dV: ten times that, and 16 eps cond(A) for the dense inverse itself.
+@pytest.mark.parametrize("length,width", [(16, 8), (23, 9), (31, 12), (40, 10)])
+def test_gradient_against_dense(length, width):
+    sys_, derivs = gradient_bhz(length, width, configs=3)
+    sys_.set_parameter_derivatives(derivs)
+    for energy in (-0.13, 0.02, 0.06):
+        sigma = sys_.self_energies(energy)
+        t, st, dv, dp = sys_.transmissions_with_grad([sigma] * 3, [0, 1, 2])
+        assert (st == 0).all(), st
+        for c in range(3):
+            rt, rv, rp, cond = _dense_gradient(sys_, sigma, c, derivs[c][0])
+            bound = 1e-11 + 16 * 2.0 ** -53 * cond
+            if abs(rt) < 1e-20:  # no open channel: both are what rounding leaves of zero
+                continue
+            assert abs(t[c] - rt) <= bound * abs(rt)
+            assert np.linalg.norm(dv[c] - rv) <= bound * np.linalg.norm(rv)
+            assert abs(dp[c, 0] - rp) <= bound * max(abs(rp), np.linalg.norm(rv))

@@ -2106,7 +2106,9 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     };
     // A batch seen twice in a row (same plans, schedule and scratch) is captured as a CUDA graph
     // on its second run and replayed afterwards: one launch in place of the level-by-level
-    // sequence. Probed runs (per-launch events) always launch directly.
+    // sequence. Probed runs (per-launch events) always launch directly. The key holds every address a
+    // captured node holds itself (kernel arguments, the buffers of scale_of's memsets); what is reached through the
+    // task lists is uploaded again when it moves.
     std::vector<uint64_t> gkey(key_plans);
     for (uint64_t v : {(uint64_t)sizeof(T), (uint64_t)sizeof(TR), (uint64_t)mixed, (uint64_t)small_max,
                        (uint64_t)(ctx->tensor_cores && ctx->tc_choice), (uint64_t)ctx->tc_wait_limit, (uint64_t)cj,
@@ -2114,7 +2116,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
                        (uint64_t)(uintptr_t)dtasks, (uint64_t)(uintptr_t)dinv, (uint64_t)(uintptr_t)pert,
                        (uint64_t)(uintptr_t)status, (uint64_t)(uintptr_t)arena, (uint64_t)(uintptr_t)rarena,
                        (uint64_t)split, (uint64_t)ctx->small_threads, (uint64_t)(uintptr_t)df12,
-                       (uint64_t)(uintptr_t)dsgt,
+                       (uint64_t)(uintptr_t)dsgt, (uint64_t)(uintptr_t)dscale, (uint64_t)(uintptr_t)dbad,
                        (uint64_t)(uintptr_t)f12_stage})
       gkey.push_back(v);
     FactorGraph& fg = ctx->fgraph;

@@ -46,6 +46,7 @@ SIGNATURES = {
     "caroli_set_tensor_cores": (ctypes.c_int, [P, ctypes.c_int]),
     "caroli_set_mixed_max_channels": (ctypes.c_int, [P, ctypes.c_int]),
     "caroli_set_wait_limit": (ctypes.c_int, [P, ctypes.c_int64]),
+    "caroli_set_f64_wait_limit": (ctypes.c_int, [P, ctypes.c_int64]),
     "caroli_set_autotune": (ctypes.c_int, [P, ctypes.c_int]),
     "caroli_set_graphs": (ctypes.c_int, [P, ctypes.c_int]),
     "caroli_set_schedule": (ctypes.c_int, [P, ctypes.c_int, ctypes.c_int]),
@@ -188,6 +189,10 @@ class Context:
     def set_wait_limit(self, polls=-1):
         """Polls of a tensor-core pipeline wait before it gives up (negative: the default)."""
         self.check(self.lib.caroli_set_wait_limit(self.h, int(polls)))
+
+    def set_f64_wait_limit(self, polls=-1):
+        """The same for the FP64 kernels (``caroli_set_f64_wait_limit``)."""
+        self.check(self.lib.caroli_set_f64_wait_limit(self.h, int(polls)))
 
     def solve_multi(self, plans, slots, configs, precision=DOUBLE):
         """T for instances of several plans of this context in one batch (``caroli_solve_multi``)."""

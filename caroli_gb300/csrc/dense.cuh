@@ -492,13 +492,16 @@ __global__ void __launch_bounds__(TCU_THREADS, 2) tc_update_kernel(const InvTask
       }
     }
   }
-  // Drain what this thread issued before tensor memory and shared memory go away.
-  if (*abort_v) {
-    if (w == 0 && lane == 0 && copies > 0) tc::mbar_wait(&bfull, (uint32_t)((copies - 1) & 1), TCU_WAIT);
-    if (w == 1 && lane == 0 && mma_tiles > 0) tc::mbar_wait(&bempty, (uint32_t)((mma_tiles - 1) & 1), TCU_WAIT);
-  }
+  // Where a wait ran out, drain what was issued before tensor memory and shared memory go away. The flag is read
+  // behind the barrier: a wait of another warp may run out after this one has left its loop.
   tc::fence_before_sync();
   __syncthreads();
+  if (abort_flag) {
+    if (w == 0 && lane == 0 && copies > 0) tc::mbar_wait(&bfull, (uint32_t)((copies - 1) & 1), TCU_WAIT);
+    if (w == 1 && lane == 0 && mma_tiles > 0) tc::mbar_wait(&bempty, (uint32_t)((mma_tiles - 1) & 1), TCU_WAIT);
+    tc::fence_before_sync();
+    __syncthreads();
+  }
   if (w == 0) tc::tmem_dealloc(tbase, 2 * TCU_COLS);
 }
 // Undo the row interchanges as column interchanges (last first), as cycles of the resulting column

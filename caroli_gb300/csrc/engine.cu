@@ -436,6 +436,7 @@ struct caroli_ctx {
   size_t mem_budget = 0;
   int mixed_max_channels = MIXED_MAX_CHANNELS;  // CAROLI_MIXED block solves with more channels run in FP64
   uint32_t tc_wait_limit = TCU_WAIT;            // polls of a pipeline wait in tc_update_kernel
+  uint32_t f64_wait_limit = TCU_WAIT;           // the same in the FP64 kernels
   unsigned char* noalloc_base = nullptr;        // device address of the allocation-free scratch array
   // Autotuner and graph replay (see run_jobs and tune_jobs).
   bool autotune = true;                         // pick the f32 factorization's schedule per plan set
@@ -906,7 +907,7 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
       for (int sd = 0; sd < sides; ++sd)
         launch(cls, fl * c / cj / sides, 0.0, [&] {
           oz::gemm_kernel<<<dim3(grid.x, grid.y, (unsigned)(c * (sides > 1 ? 1 : per))), oz::THREADS, oz::GEMM_SMEM, s>>>(
-              dgemms + t0, jl + f0, per, k, sides > 1 ? sd : -1);
+              dgemms + t0, jl + f0, per, k, sides > 1 ? sd : -1, ctx->f64_wait_limit);
         });
     });
   };
@@ -1502,7 +1503,8 @@ void trace_pairs(caroli_ctx* ctx, const std::vector<TracePair>& pairs, double fl
     const dim3 grid((unsigned)((max_m + oz::ROWS - 1) / oz::ROWS), (unsigned)((max_n + oz::COLS - 1) / oz::COLS));
     in_pieces(gemms.size(), [&](size_t f0, size_t c) {
       launch(K_TRACE, flops * c / (2.0 * pairs.size()), 0.0, [&] {
-        oz::gemm_kernel<<<dim3(grid.x, grid.y, (unsigned)c), oz::THREADS, oz::GEMM_SMEM, s>>>(dg + f0, nullptr, 1, 0, -1);
+        oz::gemm_kernel<<<dim3(grid.x, grid.y, (unsigned)c), oz::THREADS, oz::GEMM_SMEM, s>>>(dg + f0, nullptr, 1, 0, -1,
+                                                                                                    ctx->f64_wait_limit);
       });
     });
     launch(K_TRACE, 0.0, 0.0, [&] { oz::dot_kernel<<<dim3((unsigned)dots.size(), oz::DOT_PARTS), 256, 0, s>>>(dd); });
@@ -1954,7 +1956,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
         in_pieces(count, [&](size_t f0, size_t c) {
           launch(ucls, uflops / panels * c / count, ubytes / panels * c / count, [&] {
             oz::update_kernel<<<dim3((unsigned)rt, (unsigned)c, (unsigned)((ct + group - 1) / group)), oz::THREADS, oz::SMEM,
-                                s>>>(dinv + first + f0, k0, (int)group, status);
+                                s>>>(dinv + first + f0, k0, (int)group, status, ctx->f64_wait_limit);
           });
         });
       }
@@ -2111,7 +2113,8 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
     // task lists is uploaded again when it moves.
     std::vector<uint64_t> gkey(key_plans);
     for (uint64_t v : {(uint64_t)sizeof(T), (uint64_t)sizeof(TR), (uint64_t)mixed, (uint64_t)small_max,
-                       (uint64_t)(ctx->tensor_cores && ctx->tc_choice), (uint64_t)ctx->tc_wait_limit, (uint64_t)cj,
+                       (uint64_t)(ctx->tensor_cores && ctx->tc_choice), (uint64_t)ctx->tc_wait_limit,
+                       (uint64_t)ctx->f64_wait_limit, (uint64_t)cj,
                        (uint64_t)(uintptr_t)djobs,
                        (uint64_t)(uintptr_t)dtasks, (uint64_t)(uintptr_t)dinv, (uint64_t)(uintptr_t)pert,
                        (uint64_t)(uintptr_t)status, (uint64_t)(uintptr_t)arena, (uint64_t)(uintptr_t)rarena,
@@ -3495,7 +3498,8 @@ void lead_sigma(caroli_ctx* ctx, const double2* y, int n, const double2* d, doub
       reinterpret_cast<const oz::PackTask*>(dt), nullptr, 1, 0);
   CK(cudaGetLastError());
   oz::gemm_kernel<<<dim3((unsigned)((n + oz::ROWS - 1) / oz::ROWS), (unsigned)((n + oz::COLS - 1) / oz::COLS), 1), oz::THREADS,
-                    oz::GEMM_SMEM, s>>>(reinterpret_cast<const oz::GemmTask*>(dt + sizeof(pk)), nullptr, 1, 0, -1);
+                    oz::GEMM_SMEM, s>>>(reinterpret_cast<const oz::GemmTask*>(dt + sizeof(pk)), nullptr, 1, 0, -1,
+                                        ctx->f64_wait_limit);
   CK(cudaGetLastError());
 }
 
@@ -4313,6 +4317,13 @@ int caroli_set_wait_limit(caroli_ctx* ctx, int64_t polls) {
   CTX_LOCK(ctx);
   if (!ctx) return CAROLI_EINVAL;
   ctx->tc_wait_limit = polls < 0 ? TCU_WAIT : (uint32_t)std::min<int64_t>(polls, TCU_WAIT);
+  return CAROLI_OK;
+}
+
+int caroli_set_f64_wait_limit(caroli_ctx* ctx, int64_t polls) {
+  CTX_LOCK(ctx);
+  if (!ctx) return CAROLI_EINVAL;
+  ctx->f64_wait_limit = polls < 0 ? TCU_WAIT : (uint32_t)std::min<int64_t>(polls, TCU_WAIT);
   return CAROLI_OK;
 }
 

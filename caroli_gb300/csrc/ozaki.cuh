@@ -207,7 +207,7 @@ __device__ __forceinline__ void mma_tile(uint32_t acc, const unsigned char* sa, 
 // left, keep that pipe 50 to 62 % busy, the bound. Two sets of 32-column tiles would not
 // fit in tensor memory. Waits are bounded as in tc_update_kernel. grid (row tiles, matrices, column groups).
 __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __restrict__ tasks, int k0, int group,
-                                                            int32_t* __restrict__ status) {
+                                                            int32_t* __restrict__ status, uint32_t wait_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t tslot;
   __shared__ __align__(8) uint64_t afull, bfull[STAGES], bempty[STAGES], tfull[2], tempty[2];
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
         tc::bulk_copy_g2s(sa + s * A_SLICE, t.oa + (size_t)blockIdx.x * A_TILE + s * A_SLICE, A_SLICE, &afull);
       for (int ct = 0; ct < tiles && !*abort_v; ++ct) {
         const int st = ct % STAGES;
-        if (ct >= STAGES && !tc::mbar_wait(&bempty[st], (uint32_t)((ct / STAGES - 1) & 1), TCU_WAIT)) { fail(); break; }
+        if (ct >= STAGES && !tc::mbar_wait(&bempty[st], (uint32_t)((ct / STAGES - 1) & 1), wait_limit)) { fail(); break; }
         tc::mbar_arrive_expect_tx(&bfull[st], B_TILE);
         tc::bulk_copy_g2s(sb + st * B_TILE, t.ob + (size_t)(tile0 + ct) * B_TILE, B_TILE, &bfull[st]);
         ++copies;
@@ -264,11 +264,11 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
     }
   } else if (w == 1) {
     if (lane == 0) {
-      if (!tc::mbar_wait(&afull, 0, TCU_WAIT)) fail();
+      if (!tc::mbar_wait(&afull, 0, wait_limit)) fail();
       for (int ct = 0; ct < tiles && !*abort_v; ++ct) {
         const int st = ct % STAGES, a = ct & 1;
-        if (!tc::mbar_wait(&bfull[st], (uint32_t)((ct / STAGES) & 1), TCU_WAIT)) { fail(); break; }
-        if (ct >= 2 && !tc::mbar_wait(&tempty[a], (uint32_t)(((ct >> 1) - 1) & 1), TCU_WAIT)) { fail(); break; }
+        if (!tc::mbar_wait(&bfull[st], (uint32_t)((ct / STAGES) & 1), wait_limit)) { fail(); break; }
+        if (ct >= 2 && !tc::mbar_wait(&tempty[a], (uint32_t)(((ct >> 1) - 1) & 1), wait_limit)) { fail(); break; }
         tc::fence_after_sync();
         mma_tile(tbase + (uint32_t)(a * ACC), sa, sb + st * B_TILE);
         tc::mma_commit(&bempty[st]);
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
         old[j] = (keep_old && in) ? Ai[(int64_t)col_of(c0 + j) * ld] : make_double2(0.0, 0.0);
         ec[j] = in ? er + t.eb[c0 + j] : 2;
       }
-      bool ok = !*abort_v && tc::mbar_wait(&tfull[a], (uint32_t)((ct >> 1) & 1), TCU_WAIT);
+      bool ok = !*abort_v && tc::mbar_wait(&tfull[a], (uint32_t)((ct >> 1) & 1), wait_limit);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
         if (lane == 0) fail();
@@ -329,8 +329,10 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
       }
     }
   }
-  // Drain what this thread issued before tensor memory and shared memory go away.
-  if (*abort_v) {
+  // Where a wait ran out, drain what was issued (see tc_update_kernel).
+  tc::fence_before_sync();
+  __syncthreads();
+  if (abort_flag) {
     if (w == 0 && lane == 0) {
       tc::mbar_wait(&afull, 0, TCU_WAIT);
       for (int ct = max(0, copies - STAGES); ct < copies; ++ct)
@@ -338,9 +340,9 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
     }
     if (w == 1 && lane == 0 && mma_tiles > 0)
       tc::mbar_wait(&bempty[(mma_tiles - 1) % STAGES], (uint32_t)(((mma_tiles - 1) / STAGES) & 1), TCU_WAIT);
+    tc::fence_before_sync();
+    __syncthreads();
   }
-  tc::fence_before_sync();
-  __syncthreads();
   if (w == 0) tc::tmem_dealloc(tbase, 2 * ACC);
 }
 

@@ -104,7 +104,7 @@ constexpr int GEMM_STAGES = 2;
 constexpr int GEMM_SMEM = A_TILE + GEMM_STAGES * B_TILE + 1024;
 
 __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __restrict__ tasks, const int32_t* __restrict__ jl,
-                                                          int per, int step, int side) {
+                                                          int per, int step, int side, uint32_t wait_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t tslot;
   __shared__ __align__(8) uint64_t afull, aempty, bfull[GEMM_STAGES], bempty[GEMM_STAGES], tfull[2], tempty[2];
@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
       const unsigned char* gb = t.b + (size_t)blockIdx.y * nch * B_TILE;
       for (int ch = 0; ch < nch && !*abort_v; ++ch) {
         const int st = ch % GEMM_STAGES;
-        if (ch >= GEMM_STAGES && !tc::mbar_wait(&bempty[st], (uint32_t)((ch / GEMM_STAGES - 1) & 1), TCU_WAIT)) { fail(); break; }
-        if (ch >= 1 && !tc::mbar_wait(&aempty, (uint32_t)((ch - 1) & 1), TCU_WAIT)) { fail(); break; }
+        if (ch >= GEMM_STAGES && !tc::mbar_wait(&bempty[st], (uint32_t)((ch / GEMM_STAGES - 1) & 1), wait_limit)) { fail(); break; }
+        if (ch >= 1 && !tc::mbar_wait(&aempty, (uint32_t)((ch - 1) & 1), wait_limit)) { fail(); break; }
         tc::mbar_arrive_expect_tx(&bfull[st], B_TILE);
         tc::bulk_copy_g2s(sb + st * B_TILE, gb + (size_t)ch * B_TILE, B_TILE, &bfull[st]);
         tc::mbar_arrive_expect_tx(&afull, A_TILE);
@@ -166,9 +166,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
     if (lane == 0) {
       for (int ch = 0; ch < nch && !*abort_v; ++ch) {
         const int st = ch % GEMM_STAGES, a = ch & 1;
-        if (!tc::mbar_wait(&bfull[st], (uint32_t)((ch / GEMM_STAGES) & 1), TCU_WAIT)) { fail(); break; }
-        if (!tc::mbar_wait(&afull, (uint32_t)(ch & 1), TCU_WAIT)) { fail(); break; }
-        if (ch >= 2 && !tc::mbar_wait(&tempty[a], (uint32_t)(((ch >> 1) - 1) & 1), TCU_WAIT)) { fail(); break; }
+        if (!tc::mbar_wait(&bfull[st], (uint32_t)((ch / GEMM_STAGES) & 1), wait_limit)) { fail(); break; }
+        if (!tc::mbar_wait(&afull, (uint32_t)(ch & 1), wait_limit)) { fail(); break; }
+        if (ch >= 2 && !tc::mbar_wait(&tempty[a], (uint32_t)(((ch >> 1) - 1) & 1), wait_limit)) { fail(); break; }
         tc::fence_after_sync();
         mma_tile(tbase + (uint32_t)(a * ACC), sa, sb + st * B_TILE);
         tc::mma_commit(&aempty);
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
       int ec[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) ec[j] = c0 + j < t.n ? er + t.eb[(size_t)ch * t.n + c0 + j] : 2;
-      ok = !*abort_v && tc::mbar_wait(&tfull[a], (uint32_t)((ch >> 1) & 1), TCU_WAIT);
+      ok = !*abort_v && tc::mbar_wait(&tfull[a], (uint32_t)((ch >> 1) & 1), wait_limit);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
         if (lane == 0) fail();
@@ -236,16 +236,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
       }
     }
   }
-  if (*abort_v) {
+  tc::fence_before_sync();
+  __syncthreads();
+  if (abort_flag) {  // a wait ran out: drain (see tc_update_kernel)
     if (w == 0 && lane == 0 && copies > 0) {
       for (int ch = max(0, copies - GEMM_STAGES); ch < copies; ++ch)
         tc::mbar_wait(&bfull[ch % GEMM_STAGES], (uint32_t)((ch / GEMM_STAGES) & 1), TCU_WAIT);
       tc::mbar_wait(&afull, (uint32_t)((copies - 1) & 1), TCU_WAIT);
     }
     if (w == 1 && lane == 0 && mmas > 0) tc::mbar_wait(&aempty, (uint32_t)((mmas - 1) & 1), TCU_WAIT);
+    tc::fence_before_sync();
+    __syncthreads();
   }
-  tc::fence_before_sync();
-  __syncthreads();
   if (w == 0) tc::tmem_dealloc(tbase, 2 * ACC);
 }
 

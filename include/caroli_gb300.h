@@ -368,6 +368,11 @@ int caroli_set_mixed_max_channels(caroli_ctx* ctx, int channels);
  * testing that path. No reference counterpart. */
 int caroli_set_wait_limit(caroli_ctx* ctx, int64_t polls);
 
+/* The same limit for the waits of the FP64 kernels (fronts and roots, traces, refinement products, self-energies
+ * formed from lead modes). One that runs out marks its solve CAROLI_TIMEOUT; caroli_sigma_from_modes returns
+ * CAROLI_ECUDA. Meant for testing those paths. No reference counterpart. */
+int caroli_set_f64_wait_limit(caroli_ctx* ctx, int64_t polls);
+
 /* The autotuner (default on; no reference counterpart): the first time a set of plans is solved in
  * reduced precision, the f32 factorization of up to 256 of its block solves is timed under each
  * candidate schedule and the fastest is kept for that plan set and precision. Candidates: the

@@ -49,3 +49,31 @@ def test_wait_limit_timeout_reaches_caller_and_context_recovers():
     assert (np.asarray(jst) == 0).all(), jst
     for tm, r in zip(t, ref):
         assert abs(tm - r) <= 1e-8, (tm, r)
+
+
+def _f64_device():
+    return bench_system("bhz-anderson", 32)  # fronts above 64 variables: the FP64 updates run
+
+
+def test_f64_wait_limit_reaches_caller_and_context_recovers():
+    """The FP64 updates, traces and self-energies formed from lead modes given no polls: every wait gives up on a
+    barrier that has not completed, and the kernels drain what they issued."""
+    sys_ = _f64_device()
+    sigmas = [sys_.self_energies(e) for e in (-0.1, 0.3)]
+    ref, st, _ = sys_.solve_batch(sigmas, [0, 0], Precision.DOUBLE)
+    assert (st == _native.OK).all(), st
+    wire = bench_system("square-anderson", 32)
+    wref = wire.transmission_with(wire.self_energies_on_device(0.37))
+    ctx = sys_.plan().ctx
+    try:
+        ctx.set_f64_wait_limit(0)
+        _, st, _ = sys_.solve_batch(sigmas, [0, 0], Precision.DOUBLE)
+        assert (st == _native.TIMEOUT).all(), st
+        with pytest.raises(_native.NativeError, match="wait ran out"):
+            wire._slot(wire.self_energies_on_device(0.37))
+    finally:
+        ctx.set_f64_wait_limit(-1)
+    again, st, _ = sys_.solve_batch(sigmas, [0, 0], Precision.DOUBLE)
+    assert (st == _native.OK).all(), st
+    assert np.array_equal(again, ref)
+    assert wire.transmission_with(wire.self_energies_on_device(0.37)) == wref

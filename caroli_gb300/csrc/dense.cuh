@@ -518,8 +518,8 @@ __global__ void __launch_bounds__(256) inv_finish_kernel(const InvTask* __restri
   const InvTask t = tasks[blockIdx.x];
   if (*t.bad) {
     if (threadIdx.x == 0 && blockIdx.y == 0) {
-      if (t.front < 0) status[t.job] = ST_SINGULAR;
-      else jobs[t.job].fail[t.front] = 1;
+      if (t.front >= 0) jobs[t.job].fail[t.front] = 1;
+      else if (status[t.job] != ST_TIMEOUT) status[t.job] = ST_SINGULAR;  // a sweep that timed out says nothing of the root
     }
     return;
   }

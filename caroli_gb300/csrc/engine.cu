@@ -521,7 +521,7 @@ void launch_panel_sweep(caroli_ctx* ctx, const InvTask* tasks, size_t count, int
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  CK(cudaLaunchKernelEx(&cfg, panel_sweep_kernel<T>, tasks, k0, tol, perturb, r, jobs, status));
+  CK(cudaLaunchKernelEx(&cfg, panel_sweep_kernel<T>, tasks, k0, tol, perturb, r, jobs, status, ctx->f64_wait_limit));
 }
 
 // Launches `fn(first, count)` over a task range in pieces of at most 65535 (grid y/z limit).
@@ -1931,10 +1931,11 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
             // Waves of tiles (one CTA of 128 rows and columns per SM, 62 us full) or of pieces (two CTAs per SM, 28 us).
             const size_t tiles = (size_t)((rows + 127) / 128), pieces = (size_t)((rows + 31) / 32);
             if (62 * ((count * tiles + SM_COUNT - 1) / SM_COUNT) < 28 * ((2 * count * pieces + 2 * SM_COUNT - 1) / (2 * SM_COUNT)))
-              trail::rest_kernel<1><<<dim3((unsigned)count, (unsigned)tiles), 256, trail::COARSE_SMEM, s>>>(dinv + first, k0, status);
+              trail::rest_kernel<1><<<dim3((unsigned)count, (unsigned)tiles), 256, trail::COARSE_SMEM, s>>>(dinv + first, k0, status,
+                                                                                                               ctx->f64_wait_limit);
             else
               trail::rest_kernel<4><<<dim3((unsigned)count, (unsigned)pieces, 2), 128, trail::FINE_SMEM, s>>>(
-                  dinv + first, k0, status);
+                  dinv + first, k0, status, ctx->f64_wait_limit);
             return;
           }
           // Pieces of 16 rows and columns, or of 4 while those are fewer than two per scheduler.

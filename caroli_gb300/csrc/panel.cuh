@@ -81,8 +81,8 @@ __device__ __forceinline__ void store_remote(uint32_t addr, float2 v, uint32_t b
                : "memory");
 }
 // Waits (bounded) for a phase completed by other CTAs of the cluster.
-__device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t parity) {
-  for (uint32_t i = 0; i < TCU_WAIT; ++i) {
+__device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t parity, uint32_t limit) {
+  for (uint32_t i = 0; i < limit; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, "
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(256) panel_scale_kernel(const InvTask* __restr
 template <typename T>
 __global__ void __launch_bounds__(PS_THREADS) panel_sweep_kernel(const InvTask* __restrict__ tasks, int k0, double tol,
                                                                  int perturb, int R, const JobDesc* __restrict__ jobs,
-                                                                 int32_t* __restrict__ status) {
+                                                                 int32_t* __restrict__ status, uint32_t wait_limit) {
   using V = typename Cx<T>::V;
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -237,16 +237,21 @@ __global__ void __launch_bounds__(PS_THREADS) panel_sweep_kernel(const InvTask* 
   cluster_sync_all();  // every CTA of the cluster runs, its barriers armed, before its shared memory is written
   publish(0);
   const int quads = (kb + 3) / 4, groups = (rows + 7) / 8;
-  bool bad = false;
+  bool bad = false, late = false;
   for (int k = 0; k < kb; ++k) {
     const int par = k & 1;
-    const bool late = !__all_sync(0xffffffffu, cluster_wait(&arrived[par], (uint32_t)((k >> 1) & 1)));
+    // A wait that runs out marks the solve, then waits for the same stores once more with a bound of its own: no CTA
+    // may leave while they are in flight. They mostly arrive, and the sweep goes on; else it ends here.
+    bool here = cluster_wait(&arrived[par], (uint32_t)((k >> 1) & 1), wait_limit);
+    late |= !here;
+    if (!here) here = cluster_wait(&arrived[par], (uint32_t)((k >> 1) & 1), TCU_WAIT);
+    const bool lost = !__all_sync(0xffffffffu, here);
     const uint4 cd = lane < C ? cand[par * C + lane] : make_uint4(0u, 0u, 0x3fffffffu, 0u);
     const unsigned long long key = ((unsigned long long)cd.y << 32) | cd.x;
     const int id = (int)cd.z;
     const int win = key_argmax(key, id & ~(1 << 30));
     const int wid = __shfl_sync(0xffffffffu, id, max(win, 0));
-    // A refused pivot (the same decision in every CTA) or a wait that ran out ends the sweep at the block
+    // A refused pivot (the same decision in every CTA) or stores that never came end the sweep at the block
     // barrier below; what the step computes until then is dropped.
     const bool refused = win < 0 || (wid & (1 << 30));
     if (tid == 0 && k + 2 < kb) tc::mbar_arrive_expect_tx(&arrived[par], tx);
@@ -328,10 +333,9 @@ __global__ void __launch_bounds__(PS_THREADS) panel_sweep_kernel(const InvTask* 
         }
       }
     }
-    if (__syncthreads_or(refused || late)) {
-      if (late && lane == 0) {
+    if (__syncthreads_or(refused || lost)) {
+      if (lost && lane == 0) {
         *t.bad = 1;
-        status[t.job] = ST_TIMEOUT;
       } else if (rank == 0 && tid == 0) {
         *t.bad = 1;
         if (trail && t.front >= 0) jobs[t.job].fail[t.front] = 1;
@@ -341,6 +345,7 @@ __global__ void __launch_bounds__(PS_THREADS) panel_sweep_kernel(const InvTask* 
     }
     if (k + 1 < kb) publish(k + 1);
   }
+  if (__any_sync(0xffffffffu, late) && lane == 0) status[t.job] = ST_TIMEOUT;
   __syncwarp();
   cluster_sync_all();  // no CTA leaves while another may still store into it
   if (bad) return;

@@ -105,7 +105,7 @@ __device__ __forceinline__ int replay_block(double2 (&v)[GJ_KB / LPR], const dou
 // are put together beside the 32 entries.
 template <int LPR>
 __global__ void __launch_bounds__(LPR == 1 ? 256 : 128, LPR == 1 ? 1 : 2)
-rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ status) {
+rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ status, uint32_t wait_limit) {
   constexpr int Q = GJ_KB / LPR, VECS = 128 / LPR;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t tslot;
@@ -237,7 +237,7 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
       ++issued;
     }
     __syncwarp();
-    late = !__all_sync(0xffffffffu, !late && tc::mbar_wait(&done[slot], phase & 1u, TCU_WAIT));
+    late = !__all_sync(0xffffffffu, !late && tc::mbar_wait(&done[slot], phase & 1u, wait_limit));
     ++phase;
     tc::fence_after_sync();
     const int er = LPR == 1 ? e : __shfl_sync(0xffffffffu, e, 4 * (lane & 7));

@@ -11,7 +11,8 @@ import numpy as np
 import pytest
 
 from systems import bench_system, oracle_T
-from caroli_gb300 import Precision, _native
+from caroli_gb300 import NestedTwoTerminal, Precision, Region, _native, square
+from caroli_gb300.disorder import ScalarPotential
 
 pytestmark = pytest.mark.gpu
 
@@ -77,3 +78,26 @@ def test_f64_wait_limit_reaches_caller_and_context_recovers():
     assert (st == _native.OK).all(), st
     assert np.array_equal(again, ref)
     assert wire.transmission_with(wire.self_energies_on_device(0.37)) == wref
+
+
+@pytest.mark.parametrize("length,width", [(2, 9), (2, 60), (2, 150), (24, 40)])
+def test_panel_sweep_wait_that_runs_out_is_a_timeout(length, width):
+    """Every wait of the panel sweeps given no polls (clusters of 1 to 16 CTAs): the solve is marked TIMEOUT, not
+    SINGULAR, and the CTAs only leave when the rows in flight have arrived; the context is as before."""
+    clean = square()
+    pot = np.random.RandomState(width).uniform(-0.7, 0.7, length * width)
+    dev = clean.with_onsite_term(ScalarPotential(pot, width, 1, 1))
+    s = NestedTwoTerminal.from_model(dev, clean, Region.cuboid(clean.lattice, [length, width, 0]), 0)
+    slot, kept = s._slot(s.self_energies(0.37)), [2 * width]
+    ref, st = s.plan().root_green([slot], [0], kept)
+    assert st[0] == _native.OK
+    ctx = s.plan().ctx
+    try:
+        ctx.set_f64_wait_limit(0)
+        _, st = s.plan().root_green([slot], [0], kept)
+        assert st[0] == _native.TIMEOUT
+    finally:
+        ctx.set_f64_wait_limit(-1)
+    again, st = s.plan().root_green([slot], [0], kept)
+    assert st[0] == _native.OK
+    assert np.array_equal(again[0][0], ref[0][0])

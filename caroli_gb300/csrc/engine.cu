@@ -1254,7 +1254,8 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
       if (!adjoint) { th[j] = 0.0; eh[j] = 0.0; }
       if (rdh[j].c == 0) continue;
     }
-    if (!fin[j].done || fin[j].stalled) sh[j] = ST_REFINE_STALLED;
+    if (fin[j].late) sh[j] = ST_TIMEOUT;
+    else if ((!fin[j].done || fin[j].stalled) && sh[j] != ST_TIMEOUT) sh[j] = ST_REFINE_STALLED;
   }
   return drd;
 }

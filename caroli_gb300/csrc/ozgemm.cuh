@@ -37,7 +37,7 @@ struct GemmTask {
   int64_t ldc;
   const int32_t* crow;  // row i goes to row crow[i] of C (null: i)
   const RefineDesc* rd; // a refinement vector instead of c: see `dst`
-  int32_t* status;      // set to ST_TIMEOUT by a wait that runs out (null: the solve of rd is marked stalled)
+  int32_t* status;      // set to ST_TIMEOUT by a wait that runs out (null: the solve of rd is marked late)
   int32_t m, n, chunks;
   int32_t dst;          // 0: c; 1: V_{step + 1} (accumulated); 2: r (accumulated); 3: gx
   double sign;
@@ -137,13 +137,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
   volatile int* abort_v = &abort_flag;
   auto fail = [&]() {
     *abort_v = 1;
-    if (t.status) {
-      *t.status = ST_TIMEOUT;
-    } else if (t.rd) {
-      RefineDesc* R = const_cast<RefineDesc*>(t.rd);
-      R->stalled = 1;
-      R->done = 1;
-    }
+    if (t.status) *t.status = ST_TIMEOUT;
+    else if (t.rd) const_cast<RefineDesc*>(t.rd)->late = 1;
   };
   int copies = 0, mmas = 0;
   if (w == 0) {

@@ -46,7 +46,10 @@ struct RefineDesc {
   float2* tb;  // sum_ne x c
   float2* hb;  // sum_nb x c
   double t_prev, t_cur, corr, err;
-  int32_t done, iters, stalled, pad;
+  int32_t done, iters, stalled;
+  // A wait of a product ran out. Products set it and nothing else: CTAs of the same launch read `done` to leave early,
+  // which all of a CTA's warps have to decide alike. gm_inner_check_kernel and refine_check_kernel end the solve.
+  int32_t late;
   // GMRES (right-preconditioned by the f32 factors) for the correction of each outer step.
   double2* V;   // (m + 1) Arnoldi vectors, each nblk x c
   float2* Z;    // m preconditioned vectors M^-1 V_k, each nblk x c
@@ -219,12 +222,12 @@ __global__ void __launch_bounds__(32) refine_check_kernel(RefineDesc* __restrict
     // After a GMRES step the remaining error is about corr times the inner residual reached.
     const double rho = R.inner_res;
     const bool reached = finite && (corr == 0.0 || corr * rho <= goal);
-    const bool stop = !finite || R.iters >= max_iters || (R.iters > 2 && corr > prev);
+    const bool stop = !finite || R.late || R.iters >= max_iters || (R.iters > 2 && corr > prev);
     R.corr = corr;
     R.err = fabs(sum[0]) * 2.0 * corr * rho;
     if (reached || stop) {
       R.done = 1;
-      R.stalled = !(finite && (corr == 0.0 || corr * rho <= tol));
+      R.stalled = R.late || !(finite && (corr == 0.0 || corr * rho <= tol));
     }
     t_out[blockIdx.x] = sum[0];
     err_out[blockIdx.x] = R.err;
@@ -432,6 +435,7 @@ __global__ void gm_inner_check_kernel(RefineDesc* __restrict__ rd, int njobs, in
   const int job = blockIdx.x * blockDim.x + threadIdx.x;
   if (job >= njobs) return;
   RefineDesc& R = rd[job];
+  if (!R.done && R.late) R.done = R.stalled = 1;
   if (R.done) { flags[job] = 1; return; }
   if (R.inner_done) { flags[job] = 1; return; }
   R.inner = k + 1;

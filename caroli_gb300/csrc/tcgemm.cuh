@@ -22,8 +22,8 @@
 // threads wait on (bounded) before the next chunk reuses the buffers, while the next chunk's global
 // loads are in flight; two CTAs per SM overlap each other's staging and MMAs. The
 // epilogue reads the accumulator from tensor memory and writes C = add + sign A B, rows optionally
-// scattered through the fronts' SweepRow table. A wait that runs out marks the solve stalled (the
-// refinement then recomputes it in FP64) after the MMAs it issued have drained.
+// scattered through the fronts' SweepRow table. A wait that runs out marks the solve late (the
+// refinement ends it as timed out, a transmission is recomputed in FP64) after the MMAs it issued have drained.
 #pragma once
 #include "sweep.cuh"
 #include "tc.cuh"
@@ -177,13 +177,11 @@ __global__ void __launch_bounds__(TG_THREADS, 2) tc_sweep_gemm_kernel(const TGTa
     if (abort_flag) break;
   }
   if (abort_flag) {
-    // Let the issued MMAs drain (bounded) before tensor memory is freed, and send the solve to
-    // the FP64 recomputation.
+    // Let the issued MMAs drain (bounded) before tensor memory is freed, and mark the solve.
     if (issued > 0) tc::mbar_wait(&mma_done, (uint32_t)((issued - 1) & 1), TCU_WAIT);
     if (tid == 0) {
       if (Rp) {
-        Rp->stalled = 1;
-        Rp->done = 1;
+        Rp->late = 1;
       } else if (t.status) {
         t.status[t.job] = ST_TIMEOUT;
       }

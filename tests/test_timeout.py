@@ -10,7 +10,7 @@ and after the limit is restored the same context must give the oracle's results 
 import numpy as np
 import pytest
 
-from systems import bench_system, oracle_T
+from systems import bench_system, gradient_bhz, oracle_T
 from caroli_gb300 import NestedTwoTerminal, Precision, Region, _native, square
 from caroli_gb300.disorder import ScalarPotential
 
@@ -101,3 +101,26 @@ def test_panel_sweep_wait_that_runs_out_is_a_timeout(length, width):
     again, st = s.plan().root_green([slot], [0], kept)
     assert st[0] == _native.OK
     assert np.array_equal(again[0][0], ref[0][0])
+
+
+def test_refinement_products_that_time_out_are_reported():
+    """The refinement's products given no polls: gradients report TIMEOUT (not a stalled refinement), a mixed
+    transmission is recomputed in FP64, which times out as well here; the context is as before afterwards."""
+    sys_, derivs = gradient_bhz(24, 12, configs=1)
+    sys_.set_parameter_derivatives(derivs)
+    sigmas = [sys_.self_energies(e) for e in (-0.1, 0.05)]
+    ref = sys_.transmissions_with_grad(sigmas, [0, 0])
+    mixed, st, _ = sys_.solve_batch(sigmas, [0, 0], Precision.MIXED)
+    assert (ref[1] == _native.OK).all() and (st == _native.OK).all()
+    ctx = sys_.plan().ctx
+    try:
+        ctx.set_f64_wait_limit(0)
+        assert (sys_.transmissions_with_grad(sigmas, [0, 0])[1] == _native.TIMEOUT).all()
+        _, st, _ = sys_.solve_batch(sigmas, [0, 0], Precision.MIXED)
+        assert (st == _native.TIMEOUT).all(), st
+    finally:
+        ctx.set_f64_wait_limit(-1)
+    again = sys_.transmissions_with_grad(sigmas, [0, 0])
+    for a, b in zip(again, ref):
+        assert np.array_equal(a, b)
+    assert np.array_equal(sys_.solve_batch(sigmas, [0, 0], Precision.MIXED)[0], mixed)

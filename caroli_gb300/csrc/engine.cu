@@ -1923,7 +1923,9 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       const size_t smf = (size_t)finish_bytes(pmax);
       if (smf > (size_t)SMEM_LIMIT) throw CudaError{cudaErrorInvalidValue, "front too large for a panel sweep"};
       const int panels = (pmax + GJ_KB - 1) / GJ_KB;
-      scale_of(0.0, first, count, tol > 0.0 ? pmax : 0, cls);  // a root refuses zero pivots only
+      // Roots (tol = 0) refuse zero pivots only, and every pivot when an entry is Inf or its square overflows: the
+      // threshold is then 0 x Inf, a NaN. (Reading a root once more: 4 us of 0.8 ms on one 32 x 32 square.)
+      scale_of(0.0, first, count, pmax, cls);
       for (int k0 = 0; k0 < pmax; k0 += GJ_KB) {
         launch(cls, flops / panels, 0.0, [&] { launch_panel_sweep<double>(ctx, dinv + first, count, k0, pmax - k0, tol, 0, djobs, status); });
         const int rows = trail ? nmax - k0 : nmax;  // rows and columns of the update, at most

@@ -7,7 +7,7 @@ rows a cluster's CTAs take. Longer devices add fronts (the trailing form) of une
 import numpy as np
 import pytest
 
-from caroli_gb300 import NestedTwoTerminal, Region, square
+from caroli_gb300 import NestedTwoTerminal, Region, _native, square
 from caroli_gb300.disorder import ScalarPotential
 
 pytestmark = pytest.mark.gpu
@@ -95,3 +95,15 @@ def test_trailing_panels_of_many_solves(length, width):
     assert st[0] == 0
     bound = len(a) * EPS * np.linalg.cond(a)  # as above
     assert np.linalg.norm(greens[0][0] - ref) <= bound * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("length,width,at", [(2, 10, 3), (1, 12, 3), (12, 9, 4), (30, 40, 5)])
+def test_root_with_an_overflowing_square_is_singular(length, width, at):
+    """A slice orbital at an energy whose square overflows: refused as a root that is not finite, as by the other paths."""
+    clean = square()
+    pot = np.zeros(length * width)
+    pot[at] = 1e155
+    dev = clean.with_onsite_term(ScalarPotential(pot, width, 1, 1))
+    s = NestedTwoTerminal.from_model(dev, clean, Region.cuboid(clean.lattice, [length, width, 0]), 0)
+    _, st, _ = s.solve_batch([s.self_energies(0.37)], [0])
+    assert st[0] == _native.SINGULAR

@@ -11,9 +11,9 @@
 // modulus, exact in f16; a product of digits is at most 2^16 and a sum of 64 of them 2^22, so the
 // f32 accumulators hold exact integers while fewer than five digit pairs share one (levels i + j <= 3)
 // and, past that, unless nearly every digit has its largest value: then a rounding of 2^-24 of a level
-// that itself weighs 2^-36 or less. Levels i + j <= 6 are kept (28 pairs); what is left out weighs
-// 2^-63 of (row's largest) x (column's largest) per term. The levels are put together in 64-bit
-// integers and rounded once to FP64 (integer arithmetic: the FP64 pipe only does the final add).
+// that itself weighs 2^-36 or less. Levels i + j <= 6 are kept (28 pairs); what is left out, with what the digits
+// cut off, weighs 2^-59 of (row's largest) x (column's largest) per term at most. The levels are put together in
+// 64-bit integers and rounded to FP64 (integer arithmetic: the FP64 pipe only does the final add).
 //
 // A 128 x 16 complex tile takes 15 Mflop on the f16 cores in place of 0.52 Mflop on the FP64 pipe (80 us
 // on one SM). Measured: the updates of two 48 x 24 x 24 cubic wires' fronts 121 -> 6.9 ms
@@ -140,27 +140,28 @@ __device__ __forceinline__ void write_b(unsigned char* ob, int32_t* eb, int r, i
   }
 }
 
-// The seven level sums of one output as FP64: 2^(e - 2114) Σ_l a_l 512^(6 - l), rounded once. e: sum of
-// the row's and the column's biased exponents.
+// The seven level sums of one output as FP64: 2^(e - 2114) Σ_l a_l 512^(6 - l), an integer of at most 77 bits. e: sum of
+// the row's and the column's biased exponents. Taken as 64 bits, 5 or 14 of them left out (rounded) where it is below or
+// past 2^-10 of the product of the largest entries, then rounded to FP64: off by less than one last place. (14 left
+// out everywhere, rounded toward minus infinity, was up to 2^-54 of that product, the larger error of small outputs.)
 __device__ __forceinline__ double combine(const float (&a)[S], int e) {
   int v[S];
 #pragma unroll
   for (int l = 0; l < S; ++l) v[l] = __float2int_rn(a[l]);
   const long long hi = ((long long)v[0] << 18) + ((long long)v[1] << 9) + v[2];
   const long long lo = ((long long)v[3] << 27) + ((long long)v[4] << 18) + ((long long)v[5] << 9) + v[6];
-  const long long w = (hi << 22) + (lo >> 14);  // unit 2^(e - 2100)
+  const bool small = hi == (long long)(int)hi;
+  const long long w = small ? (hi << 31) + ((lo + 16) >> 5) : (hi << 22) + ((lo + 8192) >> 14);
   if (e >= NOT_FINITE) return __longlong_as_double(0x7ff8000000000000ll);
   if (w == 0) return 0.0;
   const unsigned long long u = w < 0 ? (unsigned long long)(-w) : (unsigned long long)w;
   const int lz = __clzll((long long)u);
   const unsigned long long norm = u << lz;
+  const int ex = 1023 + 63 - lz + e - (small ? 2109 : 2100);
   // 53 bits rounded to nearest (ties up); the carry of the rounding moves the exponent.
-  const unsigned long long mant = (norm >> 11) + ((norm >> 10) & 1ull);
-  const int ex = 1023 + 63 - lz + e - 2100;
   unsigned long long bits;
-  if (ex <= 0) bits = 0ull;
-  else if (ex >= 2046) bits = 0x7ff0000000000000ull;
-  else bits = ((unsigned long long)(ex - 1) << 52) + mant;
+  if (ex > 0) bits = ex > 2046 ? 0x7ff0000000000000ull : ((unsigned long long)(ex - 1) << 52) + (norm >> 11) + ((norm >> 10) & 1ull);
+  else bits = ex > -52 ? (norm >> (12 - ex)) + ((norm >> (11 - ex)) & 1ull) : 0ull;  // below the normal numbers
   return __longlong_as_double((long long)(bits | (w < 0 ? 1ull << 63 : 0ull)));
 }
 

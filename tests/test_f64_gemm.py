@@ -48,3 +48,31 @@ def test_transmission_against_dense(length, width):
         assert abs(s.transmission_with_precision(on_device, Precision.MIXED) - ref) <= 1e-8 + bound
     finally:
         s.plan().ctx.set_mixed_max_channels()
+
+
+# Entries are cut to 62 bits below twice the largest of their row: with 1 the largest, steps of 2^-61.
+@pytest.mark.parametrize("bits", [30, 50, 53, 56, 59, 61])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_cancelling_products(bits, sign):
+    """Σ_L = Y diag(d) Y^† with Y = [[1, 1], [0, 1]] and d = (1 - i δ, -1): its first entry cancels to -i δ, all that
+    Γ_L holds, so that T is proportional to what the product leaves of δ (three bits wide)."""
+    clean = square()
+    s = NestedTwoTerminal.from_model(clean, clean, Region.cuboid(clean.lattice, [2, 2, 0]), 0)
+    plan, delta = s.plan(), sign * 5.0 * 2.0 ** -bits
+    plan.lead_modes(0, 0, np.array([[1.0, 1.0], [0.0, 1.0]]), 1.0)
+    plan.lead_modes(0, 1, np.eye(2), 1.0)
+    d = [np.array([1.0 - 1j * delta, -1.0]), np.array([0.2 - 0.7j, 0.1 - 0.4j])]
+    plan.sigma_from_modes(0, 0.3, [(d[0], d[1], np.zeros(0, np.int32), np.zeros(0))])
+    y = s.system
+    a = 0.3 * np.eye(y.n, dtype=complex)
+    a[np.repeat(np.arange(y.n), np.diff(y.row_ptr)), y.cols.astype(int)] -= y.values[0]
+    blk = y.blocks[0]
+    sl, sr = np.array([[-1j * delta, -1.0], [-1.0, -1.0]]), np.diag(d[1])
+    a[np.ix_(blk.left, blk.left)] -= sl
+    a[np.ix_(blk.right, blk.right)] -= sr
+    g = np.linalg.inv(a)[np.ix_(blk.left, blk.right)]
+    gl, gr = 1j * (sl - sl.conj().T), 1j * (sr - sr.conj().T)
+    ref = np.trace(gl @ g @ gr @ g.conj().T).real
+    t, st, _ = plan.ctx.solve_multi([plan], [0], [0])
+    assert st[0] == 0
+    assert abs(t[0] - ref) <= 64 * EPS * np.linalg.cond(a) * abs(ref)

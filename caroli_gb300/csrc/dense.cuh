@@ -38,11 +38,13 @@ struct InvTask {
                     // GEMM afterwards, see schur_split in the engine)
   int32_t trail;    // 1: only the trailing block is formed (S; LU form, panel.cuh), 0: the full sweep
   // Scratch of the panel kernels of panel.cuh: the scaled pivot rows of a panel (kb x kb) and its row
-  // permutation; FP64 matrices: the update's operands and their exponents (ozaki.cuh).
+  // permutation; FP64 matrices: the update's operands, their exponents and nonzero entries (ozaki.cuh), the columns'
+  // entries in `y`.
   void* prows;
   int32_t* perm;
   unsigned char *oa, *ob;
   int32_t *ea, *eb;
+  uint32_t *ma, *mb;
 };
 
 constexpr int GJ_KB = 32;

@@ -1868,7 +1868,12 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
           inv[q].oa = doz + tc.inv_oz_off[q];
           inv[q].ob = inv[q].oa + oz::a_bytes(inv[q].n);
           inv[q].ea = reinterpret_cast<int32_t*>(inv[q].ob + oz::b_bytes(inv[q].n));
-          inv[q].eb = reinterpret_cast<int32_t*>(reinterpret_cast<unsigned char*>(inv[q].ea) + oz::e_bytes(inv[q].n));
+          const size_t eb = oz::e_bytes(inv[q].n);
+          unsigned char* at = reinterpret_cast<unsigned char*>(inv[q].ea);
+          inv[q].eb = reinterpret_cast<int32_t*>(at + eb);
+          inv[q].ma = reinterpret_cast<uint32_t*>(at + 2 * eb);
+          inv[q].mb = reinterpret_cast<uint32_t*>(at + 3 * eb);
+          inv[q].y = at + 4 * eb;
         }
       }
       if (!inv.empty())

@@ -50,11 +50,13 @@ constexpr int EPI_WARPS = 16;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
 constexpr int NOT_FINITE = 1 << 20;              // exponent of a row or column holding Inf or NaN
 
-// Operand bytes of a matrix of n rows and columns: A' and B' tiles, row and column exponents.
+// Operand bytes of a matrix of n rows and columns: A' and B' tiles, row and column exponents and masks, and the columns'
+// entries in FP64 (the rows' are in the panel).
 __host__ __device__ inline size_t a_bytes(int n) { return (size_t)((n + ROWS - 1) / ROWS) * A_TILE; }
 __host__ __device__ inline size_t b_bytes(int n) { return (size_t)((n + COLS - 1) / COLS) * B_TILE; }
 __host__ __device__ inline size_t e_bytes(int n) { return ((size_t)n * 4 + 255) / 256 * 256; }
-__host__ __device__ inline size_t bytes(int n) { return a_bytes(n) + b_bytes(n) + 2 * e_bytes(n); }
+__host__ __device__ inline size_t y_bytes(int n) { return (size_t)n * GJ_KB * sizeof(double2); }
+__host__ __device__ inline size_t bytes(int n) { return a_bytes(n) + b_bytes(n) + 4 * e_bytes(n) + y_bytes(n); }
 
 // Byte offset of element (row, k) of an f16 operand: K-slices of 16 elements (one kind::f16 MMA) in the
 // core-matrix layout of tc.cuh (8 rows x 16 bytes; leading offset 128, stride offset 256).
@@ -63,6 +65,25 @@ __device__ __forceinline__ uint32_t offset(int row, int k, int rows) {
 }
 
 __device__ __forceinline__ int biased_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// Digits are cut relative to the largest entries, so an output's error is relative to their product M, whatever its own
+// size: 2^-57 of it or so. Where the large entries of a row meet small ones of a column and the other way round, as in
+// the fronts of a device whose couplings decay over the pivots of a panel, the output is far below M; at 2^-62 M
+// nothing is left of it. An output whose old and new values are both below 2^-FAR M is therefore computed again on the
+// FP64 pipe. (Without, T of a 60 x 30 square with Anderson disorder 16, 2.5e-31, was off by 7e-5, and by decades at 30.)
+// Rows and columns that share no nonzero entry (masks) give an exact zero and stay out.
+// FAR = 12: with 8, two 48 x 24 x 24 cubic wires take 42.3 ms in place of 28.9, with 16 28.1 and with none computed again
+// 27.6; devices whose rows and columns are scaled over six decades either way come out 1.0e-13 (geometric mean)
+// off with 12, 1.1e-12 with 16 and 8e-14 on the FP64 pipe alone.
+constexpr int FAR = 12;
+__device__ __forceinline__ bool is_zero(double2 v) {
+  return ((unsigned)(__double2hiint(v.x) | __double2hiint(v.y)) << 1 | (unsigned)(__double2loint(v.x) | __double2loint(v.y))) == 0u;
+}
+__device__ __forceinline__ int top_exponent(double2 v) { return max(biased_exponent(v.x), biased_exponent(v.y)); }
+// ec: sum of the row's and the column's biased exponents; common: their common nonzero entries.
+__device__ __forceinline__ bool far_below(int ec, uint32_t common, double2 old, double2 out) {
+  return common && max(top_exponent(old), top_exponent(out)) < ec - 1023 - FAR;
+}
 
 // x as a 62-bit fixed-point number, x 2^(1084 - e) rounded toward zero (e the biased exponent of the largest
 // entry, at least 1), plus 256 in the place of each base-512 digit: the digits of the sum, less 256, are the signed digits of x.
@@ -97,6 +118,16 @@ template <int LPR> __device__ __forceinline__ int row_exponent(const double2 (&a
 #pragma unroll
   for (int o = 1; o < LPR; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
   return e;
+}
+
+// The nonzero entries of LPR lanes, lane h holding LPR i + h.
+template <int LPR> __device__ __forceinline__ uint32_t row_mask(const double2 (&a)[GJ_KB / LPR], int h) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < GJ_KB / LPR; ++i) m |= (is_zero(a[i]) ? 0u : 1u) << (LPR * i + h);
+#pragma unroll
+  for (int o = 1; o < LPR; o <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
+  return m;
 }
 
 // Row q of A' from LPR lanes, lane h holding the entries LPR i + h: four lanes' 4-byte pairs (re, im) fill
@@ -285,6 +316,8 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
     const bool row_in = r < rows;
     const bool keep_old = row_in && (trail || gi < k0 || gi >= k0 + kb);
     const int er = row_in ? t.ea[r] : 1;
+    const uint32_t mr = row_in ? t.ma[r] : 0u;
+    const double2* Y = static_cast<const double2*>(t.y);
     double2* Ai = static_cast<double2*>(t.a) + gi;
     const int64_t ld = t.ld;
     constexpr int CW = 4 * COLS / EPI_WARPS;  // complex columns per warp and tile
@@ -315,6 +348,7 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&tempty[a]);
+      uint32_t far = 0;
 #pragma unroll
       for (int j = 0; j < CW; ++j) {
         float x[S], y[S];
@@ -326,7 +360,39 @@ __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __res
         // trail: old - L Y; full: old + (swept panel) Y.
         const double re = combine(x, ec[j]), im = combine(y, ec[j]);
         const double2 out = trail ? make_double2(old[j].x - re, old[j].y - im) : make_double2(old[j].x + re, old[j].y + im);
-        if (row_in && c0 + j < rest) Ai[(int64_t)col_of(c0 + j) * ld] = out;
+        const bool in = row_in && c0 + j < rest;
+        if (in) Ai[(int64_t)col_of(c0 + j) * ld] = out;
+        if (in && far_below(ec[j], mr & t.mb[c0 + j], old[j], out)) far |= 1u << j;
+      }
+      if (__any_sync(0xffffffffu, far)) {
+        // Few rows of a column: the lanes share the sum of a row; many: a row per lane.
+        const double2* P = static_cast<const double2*>(t.a) + (int64_t)k0 * ld;  // the panel
+#pragma unroll
+        for (int j = 0; j < CW; ++j) {
+          uint32_t rows_far = __ballot_sync(0xffffffffu, far >> j & 1u);
+          const double2* Yj = Y + (int64_t)(c0 + j) * GJ_KB;
+          double2 sum = make_double2(0.0, 0.0);
+          if (__popc(rows_far) > 8) {
+            if (far >> j & 1u)
+#pragma unroll 4
+              for (int k = 0; k < kb; ++k) sum = cfma(sum, P[gi + k * ld], Yj[k]);
+          } else {
+            while (rows_far) {
+              const int src = __ffs(rows_far) - 1, i = __shfl_sync(0xffffffffu, gi, src);
+              rows_far &= rows_far - 1;
+              double2 p = lane < kb ? cmul(P[i + lane * ld], Yj[lane]) : make_double2(0.0, 0.0);
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) {
+                p.x += __shfl_xor_sync(0xffffffffu, p.x, o);
+                p.y += __shfl_xor_sync(0xffffffffu, p.y, o);
+              }
+              if (lane == src) sum = p;
+            }
+          }
+          if (far >> j & 1u)
+            Ai[(int64_t)col_of(c0 + j) * ld] =
+                trail ? make_double2(old[j].x - sum.x, old[j].y - sum.y) : make_double2(old[j].x + sum.x, old[j].y + sum.y);
+        }
       }
     }
   }

@@ -428,7 +428,9 @@ __global__ void __launch_bounds__(NT) panel_rest_kernel(const InvTask* __restric
           }
     }
     if constexpr (sizeof(T) == 8) {
-      if (t.oa) oz::write_a<LPR>(t.oa, t.ea, row, h, act, a);
+      const uint32_t mask = oz::row_mask<LPR>(a, h);
+      if (act && h == 0) t.ma[row] = mask;
+      oz::write_a<LPR>(t.oa, t.ea, row, h, act, a);
     }
     return;
   }
@@ -455,10 +457,14 @@ __global__ void __launch_bounds__(NT) panel_rest_kernel(const InvTask* __restric
     if (act && c < nd) Aj[k0 + perm[GJ_KB + c]] = dv[i];
   }
   if constexpr (sizeof(T) == 8) {
-    if (t.ob) {
-      oz::write_b<LPR>(t.ob, t.eb, r, h, act, y);
-      return;
+    const uint32_t mask = oz::row_mask<LPR>(y, h);
+    if (act) {
+      if (h == 0) t.mb[r] = mask;
+#pragma unroll
+      for (int i = 0; i < Q; ++i) static_cast<double2*>(t.y)[(int64_t)r * GJ_KB + LPR * i + h] = y[i];
     }
+    oz::write_b<LPR>(t.ob, t.eb, r, h, act, y);
+    return;
   }
   if (!act) return;
   V* Y = static_cast<V*>(t.y);

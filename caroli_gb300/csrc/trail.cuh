@@ -42,18 +42,24 @@ __device__ __forceinline__ int exponent(double2 v, int shift) {
 }
 
 // Column r of the digits of a W x W block T[c0 .. c0 + W)[c0 + W ..) (row stride GJ_KB), W / 8 entries per
-// lane of eight, entry k times 2^(mul half[k]); returns the column's exponent.
+// lane of eight, entry k times 2^(mul half[k]); returns the column's exponent, and in `mask` its nonzero entries.
 template <int W>
-__device__ __forceinline__ int put_block(unsigned char* dst, const double2* T, int c0, int r, int h, const int* half, int mul) {
+__device__ __forceinline__ int put_block(unsigned char* dst, const double2* T, int c0, int r, int h, const int* half, int mul,
+                                         uint32_t& mask) {
   double2 y[W / 8];
   int e = LEAST;
+  mask = 0;
 #pragma unroll
   for (int i = 0; i < W / 8; ++i) {
     y[i] = T[(c0 + 8 * i + h) * GJ_KB + c0 + W + r];
     e = max(e, exponent(y[i], mul * half[c0 + 8 * i + h]));
+    mask |= (oz::is_zero(y[i]) ? 0u : 1u) << (8 * i + h);
   }
 #pragma unroll
-  for (int o = 1; o < 8; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+  for (int o = 1; o < 8; o <<= 1) {
+    e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    mask |= __shfl_xor_sync(0xffffffffu, mask, o);
+  }
 #pragma unroll
   for (int i = 0; i < W / 8; ++i) {
     uint32_t d[oz::S];
@@ -111,6 +117,7 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
   __shared__ uint32_t tslot;
   __shared__ __align__(8) uint64_t done[2];
   __shared__ int s_eb[2][GJ_KB];
+  __shared__ uint32_t s_mb[2][GJ_KB];
   __shared__ __align__(16) int s_half[GJ_KB];
   const InvTask t = tasks[blockIdx.x];
   const int n = t.n, np = t.npiv;
@@ -201,13 +208,17 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
   // Digits of the groups g0 .. g0 + ng - 1 as row `row` of an operand: digit s at dst + s slice, 16 bytes (four entries)
   // per store where a thread holds them.
   auto put = [&](unsigned char* dst, uint32_t slice, int row, int rows, int g0, int ng, int e, int mul) {
+    uint32_t mask = 0;  // the vector's nonzero entries
 #pragma unroll UNROLL
     for (int g = 0; g < ng; ++g) {
       double2 o[NE];
       fetch(g0 + g, o);
       uint32_t d[NE][oz::S];
 #pragma unroll
-      for (int i = 0; i < NE; ++i) oz::digit_pairs(o[i], e - mul * s_half[4 * (g0 + g) + LPR * i + h], d[i]);
+      for (int i = 0; i < NE; ++i) {
+        oz::digit_pairs(o[i], e - mul * s_half[4 * (g0 + g) + LPR * i + h], d[i]);
+        mask |= (oz::is_zero(o[i]) ? 0u : 1u) << (4 * g + LPR * i + h);
+      }
       unsigned char* at = dst + oz::offset(row, 8 * g + 2 * h, rows);
 #pragma unroll
       for (int s = 0; s < oz::S; ++s) {
@@ -215,12 +226,13 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
         else *reinterpret_cast<uint32_t*>(at + s * slice) = d[0][s];
       }
     }
+    return mask;
   };
   // v[c0 + W .. c0 + 2 W) -= v[c0 .. c0 + W) x the block `sb`: digits of the own entries (largest exponent e) into
   // A', the MMAs of a digit of A' with all digits of B' it still meets (level sums of 2 W columns), the sums put
   // together.
-  auto product = [&](int c0, int W, const unsigned char* sb, const int* eb, int e) {
-    put(sa, 128 * 4 * W, m, 128, c0 / 4, W / 4, e, inner);
+  auto product = [&](int c0, int W, const unsigned char* sb, const int* eb, const uint32_t* mb, int e) {
+    uint32_t mask = put(sa, 128 * 4 * W, m, 128, c0 / 4, W / 4, e, inner);
     tc::fence_smem_async();
     tc::fence_before_sync();
     side_sync();
@@ -240,6 +252,8 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
     late = !__all_sync(0xffffffffu, !late && tc::mbar_wait(&done[slot], phase & 1u, wait_limit));
     ++phase;
     tc::fence_after_sync();
+#pragma unroll
+    for (int o = 1; o < LPR; o <<= 1) mask |= __shfl_xor_sync(0xffffffffu, mask, o);
     const int er = LPR == 1 ? e : __shfl_sync(0xffffffffu, e, 4 * (lane & 7));
 #pragma unroll LPR == 1 ? 1 : 2
     for (int g = 0; g < W / 4; ++g) {
@@ -264,6 +278,37 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
           d = make_double2(__shfl_sync(0xffffffffu, d.x, lane >> 2), __shfl_sync(0xffffffffu, d.y, lane >> 2));
           if (j == 0 || h == j) o[0] = d;
         }
+      }
+      // Entries far below the operands' largest: again from the vector and T (see oz::far_below).
+      double2 old[NE];
+      fetch((c0 + W) / 4 + g, old);
+      uint32_t far = 0;
+#pragma unroll
+      for (int i = 0; i < NE; ++i) {
+        const int j = 4 * g + LPR * i + h;
+        const double2 out = make_double2(old[i].x - o[i].x, old[i].y - o[i].y);
+        if (oz::far_below(e + eb[j], mask & mb[j], old[i], out)) far |= 1u << i;
+      }
+      if (__any_sync(0xffffffffu, far)) {
+        double2 sum[NE];
+#pragma unroll
+        for (int i = 0; i < NE; ++i) sum[i] = make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int kg = 0; kg < W / 4; ++kg) {
+          double2 a4[NE];
+          fetch(c0 / 4 + kg, a4);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            double2 ak = a4[k % NE];
+            if (LPR > 1)
+              ak = make_double2(__shfl_sync(0xffffffffu, ak.x, (lane & ~3) | k), __shfl_sync(0xffffffffu, ak.y, (lane & ~3) | k));
+#pragma unroll
+            for (int i = 0; i < NE; ++i) sum[i] = cfma(sum[i], ak, T[(c0 + 4 * kg + k) * GJ_KB + c0 + W + 4 * g + LPR * i + h]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < NE; ++i)
+          if (far >> i & 1u) o[i] = sum[i];
       }
       subtract((c0 + W) / 4 + g, o);
     }
@@ -290,13 +335,17 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
     }
     side_sync();
     int* eb = s_eb[slot];
+    uint32_t* mb = s_mb[slot];
     {
+      uint32_t m16, m8;
       const int r = tid >> 3, h8 = tid & 7;
-      const int e16 = put_block<16>(sb16, T, 0, r, h8, s_half, -inner);
-      const int e8 = put_block<8>(sb8 + (tid >> 6) * B8_BYTES, T, 16 * (tid >> 6), r & 7, h8, s_half, -inner);
+      const int e16 = put_block<16>(sb16, T, 0, r, h8, s_half, -inner, m16);
+      const int e8 = put_block<8>(sb8 + (tid >> 6) * B8_BYTES, T, 16 * (tid >> 6), r & 7, h8, s_half, -inner, m8);
       if (h8 == 0) {
         eb[r] = e16;
         eb[16 + r] = e8;
+        mb[r] = m16;
+        mb[16 + r] = m8;
       }
     }
     // A warp without vectors to solve only takes part in the barriers.
@@ -306,7 +355,8 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
     for (int b = 0; b < GJ_KB / B && B * b < kb; ++b) {
       if (b > 0) {
         const bool wide = b == 2;
-        product(b == 3 ? 16 : 0, wide ? 16 : 8, wide ? sb16 : sb8 + (b >> 1) * B8_BYTES, eb + (wide ? 0 : 16 + 8 * (b >> 1)), e0);
+        product(b == 3 ? 16 : 0, wide ? 16 : 8, wide ? sb16 : sb8 + (b >> 1) * B8_BYTES, eb + (wide ? 0 : 16 + 8 * (b >> 1)),
+                mb + (wide ? 0 : 16 + 8 * (b >> 1)), e0);
       }
       switch (b) {
         case 0: e0 = replay_block<LPR, 0>(v, T, h, any, s_half, inner); break;
@@ -343,8 +393,22 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
 #pragma unroll
   for (int o = 1; o < LPR; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
   if (act && h == 0) (columns ? t.eb : t.ea)[q] = e;
+  // The entries themselves for what oz::update_kernel computes again: solved rows in the panel, columns in t.y.
+  if (out && !columns && solve) {
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      const int c = LPR * i + h;
+      if (c < kb) Ar[(int64_t)c * ld] = v[i];
+    }
+  }
+  if (act && columns) {
+    double2* Y = static_cast<double2*>(t.y) + (int64_t)q * GJ_KB;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) Y[LPR * i + h] = v[i];
+  }
+  uint32_t mask = 0;
   if (act && !columns) {
-    put(t.oa + (size_t)(q / oz::ROWS) * oz::A_TILE, oz::A_SLICE, q % oz::ROWS, oz::ROWS, 0, GJ_KB / 4, e, outer);
+    mask = put(t.oa + (size_t)(q / oz::ROWS) * oz::A_TILE, oz::A_SLICE, q % oz::ROWS, oz::ROWS, 0, GJ_KB / 4, e, outer);
   } else if (act) {  // rows (re, -im) and (im, re) of every digit (oz::write_b)
     unsigned char* tile = t.ob + (size_t)(q / oz::COLS) * oz::B_TILE;
 #pragma unroll UNROLL
@@ -353,7 +417,10 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
       fetch(g, o);
       uint32_t d[NE][oz::S];
 #pragma unroll
-      for (int i = 0; i < NE; ++i) oz::digit_pairs(o[i], e - s_half[4 * g + LPR * i + h], d[i]);
+      for (int i = 0; i < NE; ++i) {
+        oz::digit_pairs(o[i], e - s_half[4 * g + LPR * i + h], d[i]);
+        mask |= (oz::is_zero(o[i]) ? 0u : 1u) << (4 * g + LPR * i + h);
+      }
 #pragma unroll
       for (int s = 0; s < oz::S; ++s)
 #pragma unroll
@@ -367,6 +434,9 @@ rest_kernel(const InvTask* __restrict__ tasks, int k0, int32_t* __restrict__ sta
         }
     }
   }
+#pragma unroll
+  for (int o = 1; o < LPR; o <<= 1) mask |= __shfl_xor_sync(0xffffffffu, mask, o);
+  if (act && h == 0) (columns ? t.mb : t.ma)[q] = mask;
   // An MMA whose wait ran out is waited for once more before its memory goes away.
   if (late && tid == 0 && issued) tc::mbar_wait(&done[slot], (issued - 1) & 1u, TCU_WAIT);
   tc::fence_before_sync();

@@ -7,8 +7,10 @@ rows a cluster's CTAs take. Longer devices add fronts (the trailing form) of une
 import numpy as np
 import pytest
 
+import caroli_gb300
 from caroli_gb300 import NestedTwoTerminal, Region, _native, square
-from caroli_gb300.disorder import ScalarPotential
+from caroli_gb300.disorder import ScalarPotential, disordered
+from systems import oracle_T
 
 pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -53
@@ -107,3 +109,68 @@ def test_root_with_an_overflowing_square_is_singular(length, width, at):
     s = NestedTwoTerminal.from_model(dev, clean, Region.cuboid(clean.lattice, [length, width, 0]), 0)
     _, st, _ = s.solve_batch([s.self_energies(0.37)], [0])
     assert st[0] == _native.SINGULAR
+
+
+def _scales(n, decades, rng):
+    return 2.0 ** np.round(rng.uniform(-decades, decades, n) * np.log2(10.0))
+
+
+@pytest.mark.parametrize("width", [20, 33, 64, 100, 161])
+@pytest.mark.parametrize("form", ["rows", "columns", "both"])
+def test_root_of_rows_and_columns_of_different_sizes(width, form):
+    """Any matrix as the root of a one-slice device (H = 0, E = 0, A = -Σ): rows and columns scaled by powers of two over
+    six decades either way, so that the exact inverse is that of the unscaled matrix, scaled."""
+    s = _device(1, width, 0, 1)
+    plan, n = s.plan(), width
+    plan.upload_values(np.zeros_like(s.system.values[:1]))
+    rng = np.random.RandomState(width)
+    a0 = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    left = _scales(n, 6, rng) if form != "columns" else np.ones(n)
+    right = _scales(n, 6, rng) if form != "rows" else np.ones(n)
+    a = left[:, None] * a0 * right
+    plan.upload_sigma(0, 0.0, [(np.asfortranarray(-a), np.zeros((n, n), complex))], [np.zeros((n, 1), complex)])
+    greens, st = plan.root_green([0], [0], [n])
+    assert st[0] == 0
+    ref = np.linalg.inv(a0) / right[:, None] / left
+    bound = n * EPS * np.linalg.cond(a0)  # as above, of the unscaled matrix
+    assert np.linalg.norm(greens[0][0] - ref) <= bound * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("length,width,decades", [(14, 40, 3), (9, 64, 6), (24, 24, 6), (6, 90, 6)])
+def test_fronts_of_rows_and_columns_of_different_sizes(length, width, decades):
+    """H and Σ scaled on both sides by powers of two over decades either way (E = 0, A = D (E - H - Σ) D)."""
+    s = _device(length, width, 0, 3 * length + width)
+    y, plan = s.system, s.plan()
+    sigma = s.self_energies(0.37)
+    a0 = _dense(s, sigma)
+    d = _scales(y.n, decades, np.random.RandomState(width))
+    rows, cols = np.repeat(np.arange(y.n), np.diff(y.row_ptr)), y.cols.astype(int)
+    blk, (sl, sr) = y.blocks[0], sigma.blocks[0]
+    h = y.values[0] - np.where(rows == cols, 0.37, 0.0)
+    plan.upload_values((d[rows] * h * d[cols])[None])
+    scaled = [np.asfortranarray(d[o][:, None] * m * d[o]) for o, m in ((blk.left, sl), (blk.right, sr))]
+    plan.upload_sigma(0, 0.0, [tuple(scaled)], [np.zeros((width, 1), complex)])
+    kept = np.concatenate([blk.left, blk.right])
+    greens, st = plan.root_green([0], [0], [len(kept)])
+    assert st[0] == 0
+    ref = np.linalg.inv(a0)[np.ix_(kept, kept)] / d[kept][:, None] / d[kept]
+    bound = y.n * EPS * np.linalg.cond(a0)  # as above, of the unscaled matrix
+    assert np.linalg.norm(greens[0][0] - ref) <= bound * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("model,shape,strength", [
+    ("square", (60, 30), 16.0), ("square", (60, 30), 60.0), ("square", (120, 24), 8.0), ("square", (40, 60), 30.0),
+    ("graphene", (60, 30), 8.0), ("graphene", (40, 40), 30.0), ("cubic", (24, 10, 10), 60.0)])
+def test_transmission_of_localised_devices(model, shape, strength):
+    """Strong disorder: T down to 1e-190, the product of couplings that decay over the pivots of a panel, relative to
+    the oracle's FP64 elimination. (Both are eliminations of the same matrices: 1e-9 leaves them four decades past
+    the 1e-13 by which such an elimination's T of these devices moves with the order of its sums.)"""
+    clean = getattr(caroli_gb300, model)()
+    region = Region.cuboid(clean.lattice, list(shape) + [0] * (3 - len(shape)))
+    device = disordered(clean, region, [{"kind": "anderson", "strength": strength}], 3)
+    s = NestedTwoTerminal.from_models([device], clean, region, 0)
+    sigma = s.self_energies(0.13)
+    ref = oracle_T(s, sigma)
+    t = s.transmission_with(sigma)
+    assert 0.0 < ref < 1e-10
+    assert abs(t - ref) <= 1e-9 * ref

@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <tuple>
 #include <memory>
 #include <mutex>
 #include <numeric>
@@ -1411,21 +1412,39 @@ struct TracePair {
   int r0, c0, np, nq;
 };
 
+// Digits of factors held at once, about: rows and columns past this are taken in strips. Memory for them is not part of
+// a batch's budget, so it stays small.
+constexpr size_t DIGITS = size_t(1) << 28;
+// Rows and columns per strip for `k` entries of the inner dimension (both factors' together) within `limit` bytes.
+inline int digit_strip(int k, size_t limit) {
+  const size_t per = (oz::A_TILE / oz::ROWS + oz::B_TILE / oz::COLS) * (size_t)oz::chunks_of(k);
+  return (int)std::max<size_t>(oz::ROWS, std::min<size_t>(limit / per, 1 << 30) / oz::ROWS * oz::ROWS);
+}
+
 // Σ_ij Re[(Γ_p G)_ij conj((G Γ_q)_ij)] of every pair (caroli-green/src/lib.rs:106-113): both products as FP64
-// GEMMs on the tensor cores (ozgemm.cuh), in batches of about a gigabyte of digits; each Γ of a batch is
-// written as digits once. Against a thread per element on the FP64 pipe: two solves with slices of 576
+// GEMMs on the tensor cores (ozgemm.cuh), in batches of about 256 MB of digits; each Γ of a batch is
+// written as digits once. Slices of more than about 1 200 orbitals go block by block (their digits, 168 bytes per entry
+// of G, would be the larger part of a solve's memory); where even a batch does not fit, a quarter of it is
+// tried. Against a thread per element on the FP64 pipe: two solves with slices of 576
 // orbitals 6.4 -> 0.3 ms, all pairs of four leads of 128 orbitals at eight energies 4.9 -> 0.4 ms.
 template <typename LaunchT>
 void trace_pairs(caroli_ctx* ctx, const std::vector<TracePair>& pairs, double flops, LaunchT& launch) {
   cudaStream_t s = ctx->stream;
-  constexpr size_t BATCH = size_t(1) << 30;
-  for (size_t first = 0; first < pairs.size();) {
+  size_t limit = DIGITS;
+  struct Place {  // a block of a pair: the `wave`-th of it
+    size_t pair;
+    int i, j, strip, wave;
+  };
+  auto strip_of = [&](const TracePair& q) { return digit_strip(q.np + q.nq, limit); };
+  Place here{0, 0, 0, pairs.empty() ? 1 : strip_of(pairs[0]), 0};
+  while (here.pair < pairs.size()) {
     std::vector<oz::PackTask> packs;
     std::vector<oz::GemmTask> gemms;
     std::vector<oz::DotTask> dots;
+    std::vector<int> waves;
     std::vector<size_t> dig, exps, mats;  // digit and exponent offsets per pack; per GEMM its two packs
-    std::map<std::pair<const double2*, int>, size_t> gammas;
-    size_t at = 0, cat = 0;
+    std::map<std::tuple<const double2*, int, int, int>, size_t> gammas;
+    size_t at = 0, cat = 0, count = 0;
     int max_pack = 1, max_m = 1, max_n = 1;
     auto add = [&](oz::PackTask t) {
       dig.push_back(at);
@@ -1436,44 +1455,66 @@ void trace_pairs(caroli_ctx* ctx, const std::vector<TracePair>& pairs, double fl
       packs.push_back(t);
       return packs.size() - 1;
     };
-    auto gamma = [&](const double2* p, int m, int b) {
-      auto it = gammas.find({p, b});
+    auto gamma = [&](const double2* p, int m, int b, int first, int rows) {  // rows (b: columns) `first` on of Γ
+      auto it = gammas.find({p, b, first, rows});
       if (it != gammas.end()) return it->second;
       oz::PackTask t{};
-      t.p = p; t.ld = m; t.rows = t.k = m; t.trans = t.b = b;
-      return gammas[{p, b}] = add(t);
+      t.p = p; t.ld = m; t.r0 = first; t.rows = rows; t.k = m; t.trans = t.b = b;
+      return gammas[{p, b, first, rows}] = add(t);
     };
-    size_t next = first;
-    for (; next < pairs.size() && (next == first || at < BATCH); ++next) {
-      const TracePair& q = pairs[next];
-      oz::PackTask g{};
-      g.p = q.g; g.ld = q.ld;
-      g.r0 = q.r0; g.rmap = q.rmap; g.rows = q.np;
-      g.k0 = q.c0; g.kmap = q.cmap; g.k = q.nq;
-      const size_t ga = add(g);  // G as the left factor
-      std::swap(g.r0, g.k0);
-      std::swap(g.rmap, g.kmap);
-      std::swap(g.rows, g.k);
-      g.trans = g.b = 1;
-      const size_t gb = add(g);  // and as the right one
+    Place next = here;
+    for (; next.pair < pairs.size() && (count == 0 || at < limit) && (count == 0 || next.wave == 0); ++count) {
+      const TracePair& q = pairs[next.pair];
+      const int m = std::min(next.strip, q.np - next.i), n = std::min(next.strip, q.nq - next.j);
+      oz::PackTask ga{}, gb{};
+      ga.p = gb.p = q.g; ga.ld = gb.ld = q.ld;
+      // Rows i.. of G as the left factor, its columns j.. as the right one.
+      ga.r0 = q.r0 + (q.rmap ? 0 : next.i); ga.rmap = q.rmap ? q.rmap + next.i : nullptr; ga.rows = m;
+      ga.k0 = q.c0; ga.kmap = q.cmap; ga.k = q.nq;
+      gb.r0 = q.c0 + (q.cmap ? 0 : next.j); gb.rmap = q.cmap ? q.cmap + next.j : nullptr; gb.rows = n;
+      gb.k0 = q.r0; gb.kmap = q.rmap; gb.k = q.np;
+      gb.trans = gb.b = 1;
+      const size_t pa = add(ga), pb = add(gb);
       oz::GemmTask t{};
-      t.m = q.np; t.n = q.nq; t.ldc = q.np; t.sign = 1.0; t.status = q.status;
-      max_m = std::max(max_m, q.np);
-      max_n = std::max(max_n, q.nq);
+      t.m = m; t.n = n; t.ldc = m; t.sign = 1.0; t.status = q.status;
+      max_m = std::max(max_m, m);
+      max_n = std::max(max_n, n);
       oz::DotTask d{};
-      d.count = (int64_t)q.np * q.nq;
+      d.count = (int64_t)m * n;
       d.part = q.part;
       for (int side = 0; side < 2; ++side) {
-        mats.push_back(side == 0 ? gamma(q.gp, q.np, 0) : ga);
-        mats.push_back(side == 0 ? gb : gamma(q.gq, q.nq, 1));
+        mats.push_back(side == 0 ? gamma(q.gp, q.np, 0, next.i, m) : pa);
+        mats.push_back(side == 0 ? pb : gamma(q.gq, q.nq, 1, next.j, n));
         t.chunks = oz::chunks_of(side == 0 ? q.np : q.nq);
         gemms.push_back(t);
       }
       dots.push_back(d);
+      waves.push_back(next.wave++);
       cat += 2 * (size_t)d.count;
+      next.j += n;
+      if (next.j == q.nq) {
+        next.j = 0;
+        next.i += m;
+      }
+      if (next.i == q.np) {
+        ++next.pair;
+        next = {next.pair, 0, 0, next.pair < pairs.size() ? strip_of(pairs[next.pair]) : 1, 0};
+      }
     }
-    unsigned char* ddig = static_cast<unsigned char*>(ctx->tr_dig.get(at));
-    double2* dc = static_cast<double2*>(ctx->tr_c.get(std::max<size_t>(cat, 1) * sizeof(double2)));
+    unsigned char* ddig;
+    double2* dc;
+    try {
+      ddig = static_cast<unsigned char*>(ctx->tr_dig.get(at));
+      dc = static_cast<double2*>(ctx->tr_c.get(std::max<size_t>(cat, 1) * sizeof(double2)));
+    } catch (const CudaError& e) {
+      if (e.e != cudaErrorMemoryAllocation) throw;
+      const size_t held = ctx->rb[0].vector_bytes() + ctx->rb[1].vector_bytes();
+      if (!held && limit < (size_t(1) << 22)) throw;
+      if (held) for (RefineBufs& v : ctx->rb) v.release_vectors();  // as for the fronts
+      else limit /= 4;
+      if (here.wave == 0) here.strip = strip_of(pairs[here.pair]);
+      continue;
+    }
     for (size_t k = 0; k < packs.size(); ++k) {
       packs[k].dig = ddig + dig[k];
       packs[k].exp = reinterpret_cast<int32_t*>(ddig + exps[k]);
@@ -1503,13 +1544,19 @@ void trace_pairs(caroli_ctx* ctx, const std::vector<TracePair>& pairs, double fl
     });
     const dim3 grid((unsigned)((max_m + oz::ROWS - 1) / oz::ROWS), (unsigned)((max_n + oz::COLS - 1) / oz::COLS));
     in_pieces(gemms.size(), [&](size_t f0, size_t c) {
-      launch(K_TRACE, flops * c / (2.0 * pairs.size()), 0.0, [&] {
+      launch(K_TRACE, flops * c / (2.0 * std::max(pairs.size(), count)), 0.0, [&] {
         oz::gemm_kernel<<<dim3(grid.x, grid.y, (unsigned)c), oz::THREADS, oz::GEMM_SMEM, s>>>(dg + f0, nullptr, 1, 0, -1,
                                                                                                     ctx->f64_wait_limit);
       });
     });
-    launch(K_TRACE, 0.0, 0.0, [&] { oz::dot_kernel<<<dim3((unsigned)dots.size(), oz::DOT_PARTS), 256, 0, s>>>(dd); });
-    first = next;
+    // Blocks of one pair add into the same sums: one launch after the other.
+    for (size_t f0 = 0; f0 < dots.size();) {
+      size_t f1 = f0 + 1;
+      while (f1 < dots.size() && waves[f1] == 0) ++f1;
+      launch(K_TRACE, 0.0, 0.0, [&] { oz::dot_kernel<<<dim3((unsigned)(f1 - f0), oz::DOT_PARTS), 256, 0, s>>>(dd + f0); });
+      f0 = f1;
+    }
+    here = next;
   }
 }
 
@@ -3477,41 +3524,50 @@ int caroli_multi_transmissions(caroli_ctx* ctx, int plan_id, int count, const in
 
 namespace {
 
+// S = sc Y diag(d) Y^† (n x n, column-major; d on the device): the left factor's digits are written from
+// Y diag(d), the right one's from Y^†. 576 orbitals: 1.8 ms on the FP64 pipe, 0.1 ms here. Slices of more than about
+// 1 700 orbitals go block by block (see DIGITS). A wait that runs out sets *status.
+void lead_sigma(caroli_ctx* ctx, const double2* y, int n, const double2* d, double sc, double2* out, int32_t* status) {
+  cudaStream_t s = ctx->stream;
+  const int strip = std::min(n, digit_strip(n, DIGITS));
+  const size_t a = oz::pack_a_bytes(strip, n), b = oz::pack_b_bytes(strip, n), e = oz::pack_e_bytes(strip, n);
+  unsigned char* dig = static_cast<unsigned char*>(ctx->tr_dig.get(a + b + 2 * e));
+  oz::PackTask pk[2] = {};
+  oz::GemmTask g{};
+  unsigned char* dt = static_cast<unsigned char*>(ctx->tr_tasks.get(sizeof(pk) + sizeof(g)));
+  for (int i = 0; i < n; i += strip)
+    for (int j = 0; j < n; j += strip) {
+      for (oz::PackTask& t : pk) {
+        t.p = y; t.ld = n; t.k = n;
+      }
+      pk[0].r0 = i;
+      pk[0].rows = std::min(strip, n - i);
+      pk[0].kscale = d;
+      pk[0].dig = dig;
+      pk[0].exp = reinterpret_cast<int32_t*>(dig + a + b);
+      pk[1].r0 = j;
+      pk[1].rows = std::min(strip, n - j);
+      pk[1].conj = pk[1].b = 1;
+      pk[1].dig = dig + a;
+      pk[1].exp = reinterpret_cast<int32_t*>(dig + a + b + e);
+      g.a = pk[0].dig; g.ea = pk[0].exp; g.b = pk[1].dig; g.eb = pk[1].exp;
+      g.c = out + i + (int64_t)j * n; g.ldc = n; g.m = pk[0].rows; g.n = pk[1].rows;
+      g.chunks = oz::chunks_of(n); g.sign = sc; g.status = status;
+      CK(cudaMemcpyAsync(dt, pk, sizeof(pk), cudaMemcpyHostToDevice, s));
+      CK(cudaMemcpyAsync(dt + sizeof(pk), &g, sizeof(g), cudaMemcpyHostToDevice, s));
+      oz::pack_kernel<<<dim3((unsigned)(((size_t)strip * oz::chunks_of(n) + 63) / 64), 2), 256, 0, s>>>(
+          reinterpret_cast<const oz::PackTask*>(dt), nullptr, 1, 0);
+      CK(cudaGetLastError());
+      oz::gemm_kernel<<<dim3((unsigned)((g.m + oz::ROWS - 1) / oz::ROWS), (unsigned)((g.n + oz::COLS - 1) / oz::COLS), 1),
+                        oz::THREADS, oz::GEMM_SMEM, s>>>(reinterpret_cast<const oz::GemmTask*>(dt + sizeof(pk)), nullptr, 1, 0, -1,
+                                                         ctx->f64_wait_limit);
+      CK(cudaGetLastError());
+    }
+}
+
 // The device buffers of energy slot `slot` (sized by the blocks' lead slices, W_R for up to nr
 // channels), allocated on first use: uploading the next energy into a slot only copies. The slot
 // is marked unset until its caller has filled it.
-// S = sc Y diag(d) Y^† (n x n, column-major; d on the device): the left factor's digits are written from
-// Y diag(d), the right one's from Y^†. 576 orbitals: 1.8 ms on the FP64 pipe, 0.1 ms here. A wait that runs
-// out sets *status.
-void lead_sigma(caroli_ctx* ctx, const double2* y, int n, const double2* d, double sc, double2* out, int32_t* status) {
-  cudaStream_t s = ctx->stream;
-  const size_t a = oz::pack_a_bytes(n, n), b = oz::pack_b_bytes(n, n), e = oz::pack_e_bytes(n, n);
-  unsigned char* dig = static_cast<unsigned char*>(ctx->tr_dig.get(a + b + 2 * e));
-  oz::PackTask pk[2] = {};
-  for (oz::PackTask& t : pk) {
-    t.p = y; t.ld = n; t.rows = t.k = n;
-  }
-  pk[0].kscale = d;
-  pk[0].dig = dig;
-  pk[0].exp = reinterpret_cast<int32_t*>(dig + a + b);
-  pk[1].conj = pk[1].b = 1;
-  pk[1].dig = dig + a;
-  pk[1].exp = reinterpret_cast<int32_t*>(dig + a + b + e);
-  oz::GemmTask g{};
-  g.a = pk[0].dig; g.ea = pk[0].exp; g.b = pk[1].dig; g.eb = pk[1].exp;
-  g.c = out; g.ldc = g.m = g.n = n; g.chunks = oz::chunks_of(n); g.sign = sc; g.status = status;
-  unsigned char* dt = static_cast<unsigned char*>(ctx->tr_tasks.get(sizeof(pk) + sizeof(g)));
-  CK(cudaMemcpyAsync(dt, pk, sizeof(pk), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(dt + sizeof(pk), &g, sizeof(g), cudaMemcpyHostToDevice, s));
-  oz::pack_kernel<<<dim3((unsigned)(((size_t)n * oz::chunks_of(n) + 63) / 64), 2), 256, 0, s>>>(
-      reinterpret_cast<const oz::PackTask*>(dt), nullptr, 1, 0);
-  CK(cudaGetLastError());
-  oz::gemm_kernel<<<dim3((unsigned)((n + oz::ROWS - 1) / oz::ROWS), (unsigned)((n + oz::COLS - 1) / oz::COLS), 1), oz::THREADS,
-                    oz::GEMM_SMEM, s>>>(reinterpret_cast<const oz::GemmTask*>(dt + sizeof(pk)), nullptr, 1, 0, -1,
-                                        ctx->f64_wait_limit);
-  CK(cudaGetLastError());
-}
-
 SigmaSlot& slot_buffers(System* sys, int slot) {
   if ((int)sys->slots.size() <= slot) sys->slots.resize(slot + 1);
   SigmaSlot& sg = sys->slots[slot];

@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
   if (w == 0) tc::tmem_dealloc(tbase, 2 * ACC);
 }
 
-// Σ_ij Re(X_ij conj(Y_ij)) of dense m x n blocks, in parts: part[task * DOT_PARTS + y]. grid (tasks, DOT_PARTS).
+// Σ_ij Re(X_ij conj(Y_ij)) of dense m x n blocks, added to the task's DOT_PARTS partial sums. grid (tasks, DOT_PARTS).
 struct DotTask {
   const double2 *x, *y;
   int64_t count;
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(256) dot_kernel(const DotTask* __restrict__ ta
     s += a.x * b.x + a.y * b.y;
   }
   s = block_sum(s, red);
-  if (threadIdx.x == 0) t.part[blockIdx.y] = s;
+  if (threadIdx.x == 0) t.part[blockIdx.y] += s;
 }
 
 }  // namespace oz

@@ -7,7 +7,7 @@ self-energies formed on the device are W x W x W products."""
 import numpy as np
 import pytest
 
-from caroli_gb300 import NestedTwoTerminal, Precision, Region, square
+from caroli_gb300 import NestedTwoTerminal, Precision, Region, _native, nested, square
 from caroli_gb300.disorder import ScalarPotential
 
 pytestmark = pytest.mark.gpu
@@ -76,3 +76,34 @@ def test_cancelling_products(bits, sign):
     t, st, _ = plan.ctx.solve_multi([plan], [0], [0])
     assert st[0] == 0
     assert abs(t[0] - ref) <= 64 * EPS * np.linalg.cond(a) * abs(ref)
+
+
+def test_wide_slices_go_block_by_block():
+    """Slices whose digits would take more than the scratch for them (256 MB): the trace and the self-energies formed
+    on the device in blocks, against a dense solve, and without more memory than the blocks take."""
+    import torch
+
+    width = 1900
+    clean = square()
+    pot = np.random.RandomState(5).uniform(-0.7, 0.7, width)
+    region = Region.cuboid(clean.lattice, [1, width, 0])
+    s = NestedTwoTerminal.from_model(clean.with_onsite_term(ScalarPotential(pot, width, 1, 1)), clean, region, 0)
+    sigma = s.self_energies(0.37)
+    ref, cond = _dense_transmission(s, sigma)
+    bound = 4 * width * EPS * cond * width  # as above
+    ctx = _native.Context(0)
+    s._plan = None
+    nested._CONTEXTS[0], kept = ctx, nested._CONTEXTS.get(0)
+    try:
+        slot = s._slot(sigma)
+        before = torch.cuda.mem_get_info()[0]
+        assert abs(s.transmission_with(sigma) - ref) <= bound
+        # The root, its operands (3.3 KB per row), products of the trace and the digits of a block; 32 MB of small things.
+        root = 16 * width * width
+        assert before - torch.cuda.mem_get_info()[0] <= 3 * root + 3400 * width + (256 << 20) + (32 << 20)
+        on_device = s.self_energies_on_device(0.37)
+        assert abs(s.transmission_with(on_device) - ref) <= bound
+    finally:
+        nested._CONTEXTS.pop(0)
+        if kept is not None:
+            nested._CONTEXTS[0] = kept

@@ -502,8 +502,8 @@ constexpr int SWEEP_FEW = 8 * SM_COUNT;  // fronts (times column chunks) below w
 // as leave the GPU at most two CTAs per SM (a panel is bound by the FP64 pipe of the SMs it runs on), at
 // least eight candidate rows each, and enough for their rows to fit in shared memory.
 template <typename T>
-void launch_panel_sweep(caroli_ctx* ctx, const InvTask* tasks, size_t count, int k0, int m, double tol, int perturb,
-                        const JobDesc* jobs, int32_t* status) {
+void launch_panel_sweep(caroli_ctx* ctx, const InvTask* tasks, size_t count, int k0, int m, double tol, const JobDesc* jobs,
+                        int32_t* status) {
   using V = typename Cx<T>::V;
   int c = 1;
   while (c < ctx->max_cluster && count * (size_t)(2 * c) <= (size_t)(2 * SM_COUNT) && 8 * c < m) c *= 2;
@@ -522,7 +522,7 @@ void launch_panel_sweep(caroli_ctx* ctx, const InvTask* tasks, size_t count, int
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  CK(cudaLaunchKernelEx(&cfg, panel_sweep_kernel<T>, tasks, k0, tol, perturb, r, jobs, status, ctx->f64_wait_limit));
+  CK(cudaLaunchKernelEx(&cfg, panel_sweep_kernel<T>, tasks, k0, tol, r, jobs, status, ctx->f64_wait_limit));
 }
 
 // Launches `fn(first, count)` over a task range in pieces of at most 65535 (grid y/z limit).
@@ -671,6 +671,7 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
   const size_t nst = cj * SLICE_SIDES;
   std::vector<oz::PackTask> packs;               // Σ and Γ of the distinct slots, then per job and side the vectors
   std::vector<oz::GemmTask> gemms(2 * nst + cj); // matvec, residual (per job and side), Γ_L (per job)
+  std::vector<size_t> left_of(2 * nst + cj);     // their left factors' pack tasks
   std::vector<oz::PackTask> vec(2 * nst + cj);
   std::map<const double2*, size_t> packed;       // first element -> its pack task
   std::vector<size_t> dig_off, vec_off(nst), vec_eoff(nst), exp_off;
@@ -714,15 +715,14 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
       v.ld = R.nblk; v.kmap = rows; v.rows = R.c; v.k = m; v.trans = 1; v.b = 1; v.rd = drd + j;
       oz::GemmTask g{};
       g.crow = rows; g.rd = drd + j; g.m = m; g.n = R.c; g.chunks = oz::chunks_of(m);
-      g.ea = reinterpret_cast<const int32_t*>(mat);  // the pack task, until the buffers are known
       v.src = 1; g.dst = 1; g.sign = -1.0;
-      vec[q] = v; gemms[q] = g;
+      vec[q] = v; gemms[q] = g; left_of[q] = mat;
       v.src = 2; g.dst = 2; g.sign = 1.0;
-      vec[nst + q] = v; gemms[nst + q] = g;
+      vec[nst + q] = v; gemms[nst + q] = g; left_of[nst + q] = mat;
       fl_sigma += 8.0 * m * (double)m * R.c;
       if (side == 0 && R.gamma_l && !R.whole) {
         g.dst = 3; g.crow = nullptr;  // takes the digits of x_L that the residual wrote
-        g.ea = reinterpret_cast<const int32_t*>(matrix(R.gamma_l, m));
+        left_of[2 * nst + j] = matrix(R.gamma_l, m);
         vec[2 * nst + j] = v; gemms[2 * nst + j] = g;
         fl_gamma += 8.0 * m * (double)m * R.c;
       }
@@ -736,7 +736,7 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
   }
   for (size_t e = 0; e < gemms.size(); ++e) {
     if (!gemms[e].m) continue;
-    const size_t mat = reinterpret_cast<size_t>(gemms[e].ea), q = e < 2 * nst ? e % nst : (e - 2 * nst) * SLICE_SIDES;
+    const size_t mat = left_of[e], q = e < 2 * nst ? e % nst : (e - 2 * nst) * SLICE_SIDES;
     gemms[e].a = packs[mat].dig;
     gemms[e].ea = packs[mat].exp;
     gemms[e].b = vec[e].dig = dvec + vec_off[q];
@@ -1979,7 +1979,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
       // threshold is then 0 x Inf, a NaN. (Reading a root once more: 4 us of 0.8 ms on one 32 x 32 square.)
       scale_of(0.0, first, count, pmax, cls);
       for (int k0 = 0; k0 < pmax; k0 += GJ_KB) {
-        launch(cls, flops / panels, 0.0, [&] { launch_panel_sweep<double>(ctx, dinv + first, count, k0, pmax - k0, tol, 0, djobs, status); });
+        launch(cls, flops / panels, 0.0, [&] { launch_panel_sweep<double>(ctx, dinv + first, count, k0, pmax - k0, tol, djobs, status); });
         const int rows = trail ? nmax - k0 : nmax;  // rows and columns of the update, at most
         launch(cls, 0.0, 0.0, [&] {
           if (trail) {

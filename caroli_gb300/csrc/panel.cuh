@@ -66,7 +66,7 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(tc::smem_addr(p)), "r"(rank));
   return r;
 }
-// 16 (8) bytes into a CTA of the cluster, counted on its barrier when they have arrived.
+// 16 bytes into a CTA of the cluster, counted on its barrier when they have arrived.
 __device__ __forceinline__ void store_remote(uint32_t addr, uint4 v, uint32_t bar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
                "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
@@ -74,11 +74,6 @@ __device__ __forceinline__ void store_remote(uint32_t addr, uint4 v, uint32_t ba
 }
 __device__ __forceinline__ void store_remote(uint32_t addr, double2 v, uint32_t bar) {
   store_remote(addr, *reinterpret_cast<const uint4*>(&v), bar);
-}
-__device__ __forceinline__ void store_remote(uint32_t addr, float2 v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr),
-               "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(bar)
-               : "memory");
 }
 // Waits (bounded) for a phase completed by other CTAs of the cluster.
 __device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t parity, uint32_t limit) {
@@ -130,7 +125,7 @@ __global__ void __launch_bounds__(256) panel_scale_kernel(const InvTask* __restr
 // warp is kept to integers, and entries are taken 8 rows x 4 columns at a time to leave few idle lanes.
 template <typename T>
 __global__ void __launch_bounds__(PS_THREADS) panel_sweep_kernel(const InvTask* __restrict__ tasks, int k0, double tol,
-                                                                 int perturb, int R, const JobDesc* __restrict__ jobs,
+                                                                 int R, const JobDesc* __restrict__ jobs,
                                                                  int32_t* __restrict__ status, uint32_t wait_limit) {
   using V = typename Cx<T>::V;
   namespace cg = cooperative_groups;
@@ -170,10 +165,9 @@ __global__ void __launch_bounds__(PS_THREADS) panel_sweep_kernel(const InvTask* 
       if (j == 0) cb[i] = v;
     }
   __syncthreads();
-  const double scale2 = *t.scale2;
-  const unsigned long long refuse = refuse_key<T>(tol * tol * scale2);
+  const unsigned long long refuse = refuse_key<T>(tol * tol * *t.scale2);
   // The CTA's best candidate of column k among its rows at or past k: key, local row and the
-  // reciprocal of the (possibly perturbed) pivot. One warp, the candidates' entries in `col`.
+  // reciprocal of the pivot. One warp, the candidates' entries in `col`.
   auto search = [&](int k, const V* col) {
     unsigned long long key = 0;
     int loc = 0x7fffffff;
@@ -188,19 +182,9 @@ __global__ void __launch_bounds__(PS_THREADS) panel_sweep_kernel(const InvTask* 
       return;
     }
     if (lane != win) return;
-    V d = col[loc];
-    if (!(key > refuse)) {
-      if (perturb && scale2 > 0.0) {  // static pivoting (see gj_sweep)
-        const double mag = sqrt(key_norm<T>(key)), target = tol * sqrt(scale2);
-        if (mag > 0.0) { d.x = (T)(d.x / mag * target); d.y = (T)(d.y / mag * target); }
-        else { d.x = (T)target; d.y = (T)0; }
-      } else {
-        loc |= 1 << 30;
-      }
-    }
-    s_inv = cinv(d);
+    s_inv = cinv(col[loc]);
     s_key = key;
-    s_loc = loc;
+    s_loc = key > refuse ? loc : loc | 1 << 30;
   };
   // Publishes the candidate found by `search`, scaled (warps 0-3: eight columns each, the CTAs split four
   // ways over the lanes), and row k if it is here (warps 4-7).

@@ -1531,6 +1531,10 @@ void trace_pairs(caroli_ctx* ctx, const std::vector<TracePair>& pairs, double fl
     const size_t pb = packs.size() * sizeof(oz::PackTask), gb = gemms.size() * sizeof(oz::GemmTask),
                  db = dots.size() * sizeof(oz::DotTask);
     unsigned char* dt = static_cast<unsigned char*>(ctx->tr_tasks.get(pb + gb + db));
+    for (size_t k = 0; k < gemms.size(); ++k) {
+      gemms[k].pa = reinterpret_cast<const oz::PackTask*>(dt) + mats[2 * k];
+      gemms[k].pb = reinterpret_cast<const oz::PackTask*>(dt) + mats[2 * k + 1];
+    }
     CK(cudaMemcpyAsync(dt, packs.data(), pb, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(dt + pb, gemms.data(), gb, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(dt + pb + gb, dots.data(), db, cudaMemcpyHostToDevice, s));

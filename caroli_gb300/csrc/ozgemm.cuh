@@ -37,6 +37,7 @@ struct GemmTask {
   int64_t ldc;
   const int32_t* crow;  // row i goes to row crow[i] of C (null: i)
   const RefineDesc* rd; // a refinement vector instead of c: see `dst`
+  const PackTask *pa, *pb;  // outputs far below the largest entries' product again from these (null: as they are)
   int32_t* status;      // set to ST_TIMEOUT by a wait that runs out (null: the solve of rd is marked late)
   int32_t m, n, chunks;
   int32_t dst;          // 0: c; 1: V_{step + 1} (accumulated); 2: r (accumulated); 3: gx
@@ -56,6 +57,14 @@ __device__ __forceinline__ bool pack_idle(const RefineDesc* rd, bool inner) {
   return rd && (rd->done || (inner && rd->inner_done));
 }
 
+// Entry k of row r of an operand in memory (src 0).
+__device__ __forceinline__ double2 pack_entry(const PackTask& t, int r, int k) {
+  const int64_t row = t.r0 + (t.rmap ? t.rmap[r] : r), kk = t.k0 + (t.kmap ? t.kmap[k] : k);
+  double2 v = static_cast<const double2*>(t.p)[t.trans ? kk + row * t.ld : row + kk * t.ld];
+  if (t.conj) v.y = -v.y;
+  return t.kscale ? cmul(v, t.kscale[k]) : v;
+}
+
 // Four lanes per (row, chunk). grid (pieces of 64 (row, chunk) pairs, tasks); with a job list, task
 // jl[y / per] * per + y % per (`per` tasks per job).
 __global__ void __launch_bounds__(256) pack_kernel(const PackTask* __restrict__ tasks, const int32_t* __restrict__ jl, int per,
@@ -68,10 +77,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackTask* __restrict__ 
   const int h = threadIdx.x & 3;
   const bool act = pair < (int64_t)t.rows * nch;
   const int r = act ? (int)(pair % t.rows) : 0, ch = act ? (int)(pair / t.rows) : 0;
-  const double2* p = static_cast<const double2*>(t.p);
-  const float2* pf = nullptr;
-  if (t.src == 1) pf = t.rd->Z + (int64_t)step * t.rd->nblk * t.rd->c;
-  else if (t.src == 2) p = t.rd->x;
+  const float2* pf = t.src == 1 ? t.rd->Z + (int64_t)step * t.rd->nblk * t.rd->c : nullptr;
   const int64_t row = t.r0 + (t.rmap ? t.rmap[r] : r);
   double2 a[GJ_KB / 4];
 #pragma unroll
@@ -79,16 +85,13 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackTask* __restrict__ 
     const int k = ch * GJ_KB + 4 * i + h;
     double2 v = make_double2(0.0, 0.0);
     if (act && k < t.k) {
-      const int64_t kk = t.k0 + (t.kmap ? t.kmap[k] : k);
-      const int64_t at = t.trans ? kk + row * t.ld : row + kk * t.ld;
-      if (pf) {
-        const float2 f = pf[at];
-        v = make_double2((double)f.x, (double)f.y);
-      } else {
-        v = p[at];
+      if (t.src == 0) {
+        v = pack_entry(t, r, k);
+      } else {  // a refinement vector: as it is, or transposed
+        const int64_t kk = t.k0 + (t.kmap ? t.kmap[k] : k), at = t.trans ? kk + row * t.ld : row + kk * t.ld;
+        if (pf) v = make_double2((double)pf[at].x, (double)pf[at].y);
+        else v = t.rd->x[at];
       }
-      if (t.conj) v.y = -v.y;
-      if (t.kscale) v = cmul(v, t.kscale[k]);
     }
     a[i] = v;
   }
@@ -177,8 +180,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
     const int r = i0 + 32 * q + lane, c0 = j0 + part * 4;
     const bool row_in = r < t.m;
     double2 sum[4];
+    int top[4];  // largest exponent of a product of the chunks' largest entries
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sum[j] = make_double2(0.0, 0.0);
+    for (int j = 0; j < 4; ++j) {
+      sum[j] = make_double2(0.0, 0.0);
+      top[j] = 0;
+    }
     bool ok = true;
     for (int ch = 0; ch < nch; ++ch) {
       const int a = ch & 1;
@@ -212,6 +219,25 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
         }
         sum[j].x += combine(x, ec[j]);
         sum[j].y += combine(y, ec[j]);
+        top[j] = max(top[j], ec[j]);
+      }
+    }
+    if (ok && row_in && t.pa) {  // see far_below; sums start at zero
+      uint32_t far = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) far |= (c0 + j < t.n && far_below(top[j], 1u, sum[j], sum[j]) ? 1u : 0u) << j;
+      if (far) {
+        const PackTask pa = *t.pa, pb = *t.pb;
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          if (!(far >> j & 1u)) continue;
+          double2 s = make_double2(0.0, 0.0);
+#pragma unroll 4
+          for (int k = 0; k < pa.k; ++k) s = cfma(s, pack_entry(pa, r, k), pack_entry(pb, c0 + j, k));
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (i == j) sum[i] = s;
+        }
       }
     }
     if (ok && row_in) {

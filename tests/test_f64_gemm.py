@@ -107,3 +107,39 @@ def test_wide_slices_go_block_by_block():
         nested._CONTEXTS.pop(0)
         if kept is not None:
             nested._CONTEXTS[0] = kept
+
+
+@pytest.mark.parametrize("half", [1, 7, 20, 40])
+@pytest.mark.parametrize("coupling", [1e-6, 1e-12, 1e-20])
+def test_transmission_between_weakly_coupled_halves(half, coupling):
+    """Left lead open on one half of the slice only, right lead on the other, the halves coupled by `coupling`: T (of its
+    square's size) comes from entries of G far below those of the same columns that the closed half holds."""
+    clean = square()
+    width = 2 * half
+    s = NestedTwoTerminal.from_model(clean, clean, Region.cuboid(clean.lattice, [2, width, 0]), 0)
+    plan, y = s.plan(), s.system
+    rows, cols = np.repeat(np.arange(y.n), np.diff(y.row_ptr)), y.cols.astype(int)
+    across = np.asarray(y.cells)[np.repeat(np.arange(len(y.site_offsets)), y.site_orbitals), 1] >= half
+    h = y.values[0] * np.where(across[rows] != across[cols], coupling, 1.0)
+    plan.upload_values(h[None])
+    blk = y.blocks[0]
+    sl = np.diag(np.where(across[blk.left], 0.3, -0.5j))
+    sr = np.diag(np.where(across[blk.right], -0.4j, 0.2))
+    plan.upload_sigma(0, 0.31, [(np.asfortranarray(sl), np.asfortranarray(sr))], [np.zeros((width, 1), complex)])
+    a = 0.31 * np.eye(y.n, dtype=complex)
+    a[rows, cols] -= h
+    a[np.ix_(blk.left, blk.left)] -= sl
+    a[np.ix_(blk.right, blk.right)] -= sr
+    # To first order in the coupling, exact to coupling^2: G_ab = G_aa H_ab G_bb of the uncoupled halves.
+    i, j = np.nonzero(~across)[0], np.nonzero(across)[0]
+    ga, gb = np.linalg.inv(a[np.ix_(i, i)]), np.linalg.inv(a[np.ix_(j, j)])
+    g = np.zeros((y.n, y.n), complex)
+    g[np.ix_(i, j)] = -ga @ a[np.ix_(i, j)] @ gb
+    gl, gr = 1j * (sl - sl.conj().T), 1j * (sr - sr.conj().T)
+    g = g[np.ix_(blk.left, blk.right)]
+    ref = np.trace(gl @ g @ gr @ g.conj().T).real
+    t, st, _ = plan.ctx.solve_multi([plan], [0], [0])
+    assert st[0] == 0 and ref > 0.0
+    cond = np.linalg.cond(a)
+    bound = 2.0 * y.n * EPS * cond + 4.0 * (coupling * cond) ** 2  # both halves' inverses; the next order
+    assert abs(t[0] - ref) <= bound * ref

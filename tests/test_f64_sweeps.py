@@ -174,3 +174,14 @@ def test_transmission_of_localised_devices(model, shape, strength):
     t = s.transmission_with(sigma)
     assert 0.0 < ref < 1e-10
     assert abs(t - ref) <= 1e-9 * ref
+
+
+def test_localised_devices_in_a_batch():
+    """Outputs computed again are the same whatever form the batch takes (a CTA per 128 rows and columns, or per 32)."""
+    clean = square()
+    region = Region.cuboid(clean.lattice, [40, 48, 0])
+    device = disordered(clean, region, [{"kind": "anderson", "strength": 20.0}], 7)
+    s = NestedTwoTerminal.from_models([device], clean, region, 0)
+    sigmas = [s.self_energies(e) for e in np.linspace(-0.8, 0.7, 11)]
+    alone = [s.transmission_with(x) for x in sigmas]
+    assert s.transmissions_with(sigmas * 30) == alone * 30

@@ -1972,7 +1972,7 @@ void run_jobs(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& specs, M
         inv_finish_kernel<decltype(tag)><<<dim3((unsigned)count, ch), 256, smf, s>>>(dinv + first, djobs, status);
       });
     };
-    // FP64 sweeps: panels over clusters, updates from exact digit products on the tensor cores
+    // FP64 sweeps: panels over clusters, updates from digit products on the tensor cores
     // (panel.cuh, ozaki.cuh).
     auto sweep_f64 = [&](size_t first, size_t count, int nmax, int pmax, double tol, bool trail, KClass cls, double flops,
                          KClass ucls, double uflops, double ubytes) {

@@ -501,8 +501,8 @@ __device__ __forceinline__ void replay_boundary(typename Cx<T>::V* F, int ld, in
 // the entries past k only. An FP64 instruction costs the same with one active lane as with 32, and these fronts
 // are bound by that pipe: against whole rows per warp (replay_boundary), 64 lanes' worth for 33 columns and
 // every column at every step, the small and tiny fronts of 16 BHZ 200 x 64 solves took 9.13 ms, then 8.71 (with
-// four warps per front; 6.8 with what followed: integer pivot keys, tiny.cuh), those of graphene over 64 energies
-// 0.95, then 0.87 (0.69).
+// four warps per front; 6.8 with what followed: integer pivot keys, tiny.cuh), those of eight energies of a
+// 64 x 64 graphene sample 0.95, then 0.87 (0.69).
 __device__ __forceinline__ void replay_schur(const double2* F, int ld, int n, int ne, const double2* prows, double2* out) {
   constexpr int Q = 8;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, h = lane & 7;

@@ -1,7 +1,7 @@
-// Complex FP64 GEMMs on the tcgen05 tensor cores, from exact digit products as the rank-32 updates of
+// Complex FP64 GEMMs on the tcgen05 tensor cores, from digit products as the rank-32 updates of
 // ozaki.cuh: C = (C +) sign A B. Operands are first written as digits (oz_pack_kernel), 32 entries of the
 // inner dimension at a time, each 32 with its own power-of-two scale per row of A and column of B; the
-// chunks' products, rounded once each, are summed in FP64 registers.
+// chunks' products, rounded each, are summed in FP64 registers.
 //
 // They carry the dense FP64 products of the framework: the slices' Σ and Γ against the refinement's
 // right-hand sides, the Caroli traces Tr[Γ_p G_pq Γ_q G_pq^†], and the lead self-energies Y diag(λ) Y^†.

@@ -4,7 +4,7 @@
 // A 32-column panel is a chain of 32 pivot steps over its candidate rows. FP64 runs at about two
 // multiply-adds per clock and SM here, so one CTA per matrix is bound by its own SM's FP64 pipe as
 // soon as there are fewer matrices than SMs: the chain itself is short. Two kernels replace it:
-//   panel_sweep_kernel  the candidate rows split over the CTAs of a cluster, a cluster barrier per
+//   panel_sweep_kernel  the candidate rows split over the CTAs of a cluster, an exchange per
 //                       pivot step; each CTA publishes its best candidate row, already scaled by the
 //                       reciprocal of its pivot, into every CTA's shared memory, so a step costs one
 //                       exchange and no CTA computes a reciprocal or a pivot search twice;
@@ -22,8 +22,9 @@
 //          of the scaled pivot rows); L11 with the reciprocals of the pivots on its diagonal.
 // Measured with ozaki.cuh against the former FP64 path (one CTA per matrix and panel, rank-32 updates on
 // the FP64 pipe, every row and column updated): panels + updates of two 48 x 24 x 24 cubic wires (fronts
-// up to 1 728, root 1 152) 337 -> 24 ms, of 16 BHZ 200 x 64 solves (fronts up to 384) 88 -> 13 ms, of one
-// 32 x 32 square (fronts up to 94) 1.57 -> 0.39 ms.
+// up to 1 728, root 1 152) 337 -> 27 ms, of 16 BHZ 200 x 64 solves (fronts up to 384) 88 -> 16 ms, of one
+// 32 x 32 square (fronts up to 94) 1.57 -> 0.40 ms (24, 13 and 0.39 before outputs far below the largest were computed
+// again, see oz::far_below).
 //
 // The pivots (largest modulus among the candidate rows, ties to the smaller row) and the test
 // |pivot| > tol max|F11| are those of inv_panel_kernel.

@@ -6,10 +6,10 @@
 // The replay is a triangular recursion of 496 complex multiply-adds per vector, bound by the FP64 pipe (two
 // multiply-adds per clock and SM: 127 000 clocks for 128 vectors). Here only its four diagonal blocks of
 // 8 x 8 stay there (112 multiply-adds); the blocks between them, 8 -> 8 columns twice and 16 -> 16 once, are
-// products of 128 vectors with a small matrix, taken as exact digit products on the tensor cores (ozaki.cuh:
-// same digits, levels and rounding). Blocks of 16 would leave 240 multiply-adds, blocks of 4 would leave 48
-// but need seven products, with 48 outputs per vector to put together in place of 32, and their
-// eight operand columns are half of an MMA's K.
+// products of 128 vectors with a small matrix, taken as digit products on the tensor cores (ozaki.cuh:
+// same digits, levels, rounding and entries computed again). Blocks of 16 would leave 240 multiply-adds,
+// blocks of 4 would leave 48 but need seven products, with 48 outputs per vector to put together in place of
+// 32, and their eight operand columns are half of an MMA's K.
 //
 // Digits are cut relative to the largest entry of a row of L and of a column of U, and the pivot rows are scaled
 // by the pivots' reciprocals: behind a small pivot p, row k of U (of size 1 / p) would take its place in the
@@ -18,9 +18,10 @@
 // entries by more than p^(-1/2). (U11 likewise; L11's columns are at most 1 against their pivots.)
 //
 // Measured against the whole replay on the FP64 pipe: 3 584 fronts of 16 BHZ 200 x 64 solves (first panel)
-// 1.47 -> 0.78 ms, all panels of these solves 9.0 -> 5.3 ms; the panels (with their sweeps) of two
-// 48 x 24 x 24 cubic wires 11.1 -> 9.9 ms. The FP64 pipe is then busy half of the time, one or two warps per
-// scheduler being all that 32 FP64 entries per thread leave room for.
+// 1.47 -> 0.83 ms, all panels of these solves 9.0 -> 5.5 ms; the panels (with their sweeps) of two
+// 48 x 24 x 24 cubic wires 11.1 -> 10.6 ms (0.78, 5.3 and 9.9 before oz::far_below had entries kept and computed
+// again). The FP64 pipe is then busy half of the time, one or two warps per scheduler being all that 32 FP64
+// entries per thread leave room for.
 #pragma once
 #include "ozaki.cuh"
 

@@ -18,8 +18,8 @@
 // A 128 x 16 complex tile takes 15 Mflop on the f16 cores in place of 0.52 Mflop on the FP64 pipe (80 us
 // on one SM). Measured: the updates of two 48 x 24 x 24 cubic wires' fronts 121 -> 9.2 ms
 // (a factor 1.4 of it from the trailing form), of 16 BHZ 200 x 64 solves 58.8 -> 6.2 ms (6.9 and 3.9 without what
-// far_below has computed again); T
-// against 64 bits equal to the FP64 pipe's within its scatter (1e-15 to 5e-12 on these devices).
+// far_below has computed again); T against 64 bits equal to the FP64 pipe's within its scatter (1e-15 to 5e-12 on
+// these devices).
 //
 // The complex product is a real GEMM D = A' B'^T with the row's 32 complex entries as K = 64 and
 // two columns of D per complex column:
@@ -239,8 +239,9 @@ __device__ __forceinline__ void mma_tile(uint32_t acc, const unsigned char* sa, 
 // rate; a 128 x 32 x 16 MMA per digit pair took 53 clocks, 6 000 per tile) into one of two sets of seven
 // 32-column accumulators, warps 2-17 (four per lane quarter, four complex columns each) add the other set's
 // tile to the old values (zero on the pivot rows of the full form) and compute again what is far below (far_below):
-// with their FP64 adds that keeps the pipe 37 % busy on BHZ fronts, the integer pipe as much. Two sets of 32-column tiles would not
-// fit in tensor memory. Waits are bounded as in tc_update_kernel. grid (row tiles, matrices, column groups).
+// with their FP64 adds that keeps the pipe 37 % busy on BHZ fronts, the integer pipe as much. Two sets of 32-column
+// tiles would not fit in tensor memory. Waits are bounded as in tc_update_kernel. grid (row tiles, matrices,
+// column groups).
 __global__ void __launch_bounds__(THREADS, 1) update_kernel(const InvTask* __restrict__ tasks, int k0, int group,
                                                             int32_t* __restrict__ status, uint32_t wait_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -550,6 +550,12 @@ struct LevelRange {
 // 1.4e-13 and 2.6e-11. It costs about a tenth more Arnoldi steps (16 solves of BHZ 100 x 40: 14.1 -> 15.2 ms; more
 // where a solve needs another outer step for it).
 constexpr double GRAD_TIGHTER = 1e-2;
+// Slice products of the refinement are computed again below 2^-20 of the largest entries' product (oz::far_below): the
+// digits leave 2^-37 of such an output, under the refinement's tolerance. Eight energies of a BHZ cross, whose solution
+// falls off from the edges of a slice, take 17.4 ms (19.0 with 12 bits, 15.6 with 28, 15.1 with none computed again);
+// the other refined cases take the same time with any. (Without, T between two halves coupled by 1e-9 was off by 4e-10, by
+// 1e-12 by 1e-7.)
+constexpr int FAR_REFINED = 20;
 
 // FP64 iterative refinement of the jobs [begin, begin + cj) after their f32 factorization. `tighter`: the fraction of
 // the context's tolerances to aim at.
@@ -747,6 +753,12 @@ RefineDesc* refine(caroli_ctx* ctx, System* sys, const std::vector<JobSpec>& spe
   packs.insert(packs.end(), vec.begin(), vec.end());
   oz::PackTask* dpacks = static_cast<oz::PackTask*>(rb.spack.get(packs.size() * sizeof(oz::PackTask)));
   oz::GemmTask* dgemms = static_cast<oz::GemmTask*>(rb.sgemm.get(gemms.size() * sizeof(oz::GemmTask)));
+  for (size_t e = 0; e < gemms.size(); ++e)
+    if (gemms[e].m) {
+      gemms[e].pa = dpacks + left_of[e];
+      gemms[e].pb = dpacks + npacks + e;
+      gemms[e].far = FAR_REFINED;
+    }
   CK(cudaMemcpyAsync(dpacks, packs.data(), packs.size() * sizeof(oz::PackTask), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(dgemms, gemms.data(), gemms.size() * sizeof(oz::GemmTask), cudaMemcpyHostToDevice, s));
   in_pieces(npacks, [&](size_t f0, size_t c) {
@@ -1534,6 +1546,7 @@ void trace_pairs(caroli_ctx* ctx, const std::vector<TracePair>& pairs, double fl
     for (size_t k = 0; k < gemms.size(); ++k) {
       gemms[k].pa = reinterpret_cast<const oz::PackTask*>(dt) + mats[2 * k];
       gemms[k].pb = reinterpret_cast<const oz::PackTask*>(dt) + mats[2 * k + 1];
+      gemms[k].far = oz::FAR;
     }
     CK(cudaMemcpyAsync(dt, packs.data(), pb, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(dt + pb, gemms.data(), gb, cudaMemcpyHostToDevice, s));

@@ -84,8 +84,8 @@ __device__ __forceinline__ bool is_zero(double2 v) {
 }
 __device__ __forceinline__ int top_exponent(double2 v) { return max(biased_exponent(v.x), biased_exponent(v.y)); }
 // ec: sum of the row's and the column's biased exponents; common: their common nonzero entries.
-__device__ __forceinline__ bool far_below(int ec, uint32_t common, double2 old, double2 out) {
-  return common && max(top_exponent(old), top_exponent(out)) < ec - 1023 - FAR;
+__device__ __forceinline__ bool far_below(int ec, uint32_t common, double2 old, double2 out, int far = FAR) {
+  return common && max(top_exponent(old), top_exponent(out)) < ec - 1023 - far;
 }
 
 // x as a 62-bit fixed-point number, x 2^(1084 - e) rounded toward zero (e the biased exponent of the largest

@@ -37,10 +37,11 @@ struct GemmTask {
   int64_t ldc;
   const int32_t* crow;  // row i goes to row crow[i] of C (null: i)
   const RefineDesc* rd; // a refinement vector instead of c: see `dst`
-  const PackTask *pa, *pb;  // outputs far below the largest entries' product again from these (null: as they are)
+  const PackTask *pa, *pb;  // outputs far below the largest entries' product: again from these (null: as they are)
   int32_t* status;      // set to ST_TIMEOUT by a wait that runs out (null: the solve of rd is marked late)
   int32_t m, n, chunks;
   int32_t dst;          // 0: c; 1: V_{step + 1} (accumulated); 2: r (accumulated); 3: gx
+  int32_t far;          // how many bits far below (with pa)
   double sign;
 };
 
@@ -57,10 +58,17 @@ __device__ __forceinline__ bool pack_idle(const RefineDesc* rd, bool inner) {
   return rd && (rd->done || (inner && rd->inner_done));
 }
 
-// Entry k of row r of an operand in memory (src 0).
-__device__ __forceinline__ double2 pack_entry(const PackTask& t, int r, int k) {
+// Entry k of row r of an operand.
+__device__ __forceinline__ double2 pack_entry(const PackTask& t, int r, int k, int step) {
   const int64_t row = t.r0 + (t.rmap ? t.rmap[r] : r), kk = t.k0 + (t.kmap ? t.kmap[k] : k);
-  double2 v = static_cast<const double2*>(t.p)[t.trans ? kk + row * t.ld : row + kk * t.ld];
+  const int64_t at = t.trans ? kk + row * t.ld : row + kk * t.ld;
+  double2 v;
+  if (t.src == 1) {
+    const float2 f = t.rd->Z[(int64_t)step * t.rd->nblk * t.rd->c + at];
+    v = make_double2((double)f.x, (double)f.y);
+  } else {
+    v = t.src == 2 ? t.rd->x[at] : static_cast<const double2*>(t.p)[at];
+  }
   if (t.conj) v.y = -v.y;
   return t.kscale ? cmul(v, t.kscale[k]) : v;
 }
@@ -77,23 +85,11 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackTask* __restrict__ 
   const int h = threadIdx.x & 3;
   const bool act = pair < (int64_t)t.rows * nch;
   const int r = act ? (int)(pair % t.rows) : 0, ch = act ? (int)(pair / t.rows) : 0;
-  const float2* pf = t.src == 1 ? t.rd->Z + (int64_t)step * t.rd->nblk * t.rd->c : nullptr;
-  const int64_t row = t.r0 + (t.rmap ? t.rmap[r] : r);
   double2 a[GJ_KB / 4];
 #pragma unroll
   for (int i = 0; i < GJ_KB / 4; ++i) {
     const int k = ch * GJ_KB + 4 * i + h;
-    double2 v = make_double2(0.0, 0.0);
-    if (act && k < t.k) {
-      if (t.src == 0) {
-        v = pack_entry(t, r, k);
-      } else {  // a refinement vector: as it is, or transposed
-        const int64_t kk = t.k0 + (t.kmap ? t.kmap[k] : k), at = t.trans ? kk + row * t.ld : row + kk * t.ld;
-        if (pf) v = make_double2((double)pf[at].x, (double)pf[at].y);
-        else v = t.rd->x[at];
-      }
-    }
-    a[i] = v;
+    a[i] = act && k < t.k ? pack_entry(t, r, k, step) : make_double2(0.0, 0.0);
   }
   if (t.b) write_b<4>(t.dig + (size_t)ch * B_TILE, t.exp + (size_t)ch * t.rows, r, h, act, a, (size_t)nch * B_TILE);
   else write_a<4>(t.dig + (size_t)ch * A_TILE, t.exp + (size_t)ch * t.rows, r, h, act, a, (size_t)nch * A_TILE);
@@ -222,24 +218,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
         top[j] = max(top[j], ec[j]);
       }
     }
-    if (ok && row_in && t.pa) {  // see far_below; sums start at zero
-      uint32_t far = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) far |= (c0 + j < t.n && far_below(top[j], 1u, sum[j], sum[j]) ? 1u : 0u) << j;
-      if (far) {
-        const PackTask pa = *t.pa, pb = *t.pb;
-#pragma unroll 1
-        for (int j = 0; j < 4; ++j) {
-          if (!(far >> j & 1u)) continue;
-          double2 s = make_double2(0.0, 0.0);
-#pragma unroll 4
-          for (int k = 0; k < pa.k; ++k) s = cfma(s, pack_entry(pa, r, k), pack_entry(pb, c0 + j, k));
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (i == j) sum[i] = s;
-        }
-      }
-    }
     if (ok && row_in) {
       double2* C = t.c;
       int64_t ldc = t.ldc;
@@ -247,11 +225,34 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const GemmTask* __rest
       if (t.dst == 1) { C = t.rd->V + (int64_t)(step + 1) * t.rd->nblk * t.rd->c; ldc = t.rd->nblk; }
       else if (t.dst == 2) { C = t.rd->r; ldc = t.rd->nblk; }
       else if (t.dst == 3) { C = t.rd->gx; ldc = t.rd->nl; }
-      const int64_t row = t.crow ? t.crow[r] : r;
+      C += (t.crow ? t.crow[r] : r) + (int64_t)c0 * ldc;
+      if (t.pa) {  // see far_below
+        uint32_t far = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (c0 + j < t.n && far_below(top[j], 1u, sum[j], add ? C[j * ldc] : sum[j], t.far)) far |= 1u << j;
+        if (far) {
+          const PackTask pa = *t.pa, pb = *t.pb;
+#pragma unroll 1
+          for (int j = 0; j < 4; ++j) {
+            if (!(far >> j & 1u)) continue;
+            double2 s = make_double2(0.0, 0.0);
+            for (int ch = 0; ch < nch; ++ch) {
+              if (t.ea[(size_t)ch * t.m + r] <= 1 || t.eb[(size_t)ch * t.n + c0 + j] <= 1) continue;  // zeros
+#pragma unroll 4
+              for (int k = ch * GJ_KB; k < min(pa.k, (ch + 1) * GJ_KB); ++k)
+                s = cfma(s, pack_entry(pa, r, k, step), pack_entry(pb, c0 + j, k, step));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (i == j) sum[i] = s;
+          }
+        }
+      }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (c0 + j >= t.n) break;
-        double2& o = C[row + (int64_t)(c0 + j) * ldc];
+        double2& o = C[j * ldc];
         const double2 v = make_double2(t.sign * sum[j].x, t.sign * sum[j].y);
         o = add ? make_double2(o.x + v.x, o.y + v.y) : v;
       }

@@ -143,3 +143,28 @@ def test_transmission_between_weakly_coupled_halves(half, coupling):
     cond = np.linalg.cond(a)
     bound = 2.0 * y.n * EPS * cond + 4.0 * (coupling * cond) ** 2  # both halves' inverses; the next order
     assert abs(t[0] - ref) <= bound * ref
+
+
+@pytest.mark.parametrize("length,half", [(2, 7), (2, 40), (20, 20), (30, 12)])
+@pytest.mark.parametrize("coupling", [1e-3, 1e-9, 1e-20])
+def test_refined_transmission_between_weakly_coupled_halves(length, half, coupling):
+    """The same device refined: the products of Σ with the solution hold both halves, and the open one's entries
+    are `coupling` of the closed one's. Against the FP64 path; 1e-9 is ten times the refinement's tolerance."""
+    clean = square()
+    width = 2 * half
+    s = NestedTwoTerminal.from_model(clean, clean, Region.cuboid(clean.lattice, [length, width, 0]), 0)
+    plan, y = s.plan(), s.system
+    rows, cols = np.repeat(np.arange(y.n), np.diff(y.row_ptr)), y.cols.astype(int)
+    across = np.asarray(y.cells)[np.repeat(np.arange(len(y.site_offsets)), y.site_orbitals), 1] >= half
+    plan.upload_values((y.values[0] * np.where(across[rows] != across[cols], coupling, 1.0))[None])
+    blk = y.blocks[0]
+    sl = np.diag(np.where(across[blk.left], 0.3, -0.5j))
+    sr = np.diag(np.where(across[blk.right], -0.4j, 0.2))
+    w = np.zeros((width, half), complex)
+    w[np.nonzero(across[blk.right])[0], np.arange(half)] = np.sqrt(0.8)
+    plan.upload_sigma(0, 0.31, [(np.asfortranarray(sl), np.asfortranarray(sr))], [np.asfortranarray(w)])
+    ref, st, _ = plan.ctx.solve_multi([plan], [0], [0])
+    assert st[0] == 0
+    t, st, _ = plan.ctx.solve_multi([plan], [0], [0], Precision.MIXED)
+    assert st[0] == 0
+    assert abs(t[0] - ref[0]) <= 1e-9 * ref[0]
